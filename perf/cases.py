@@ -1,7 +1,7 @@
 """The work this library is measured on: single-GPU (one-rank) forms of its public entry points over the sizes they are
 used at. `listed()` names the fixed cases, `draw()` gives more of the same ranges, `prepare()` builds what a program
 holds before the call, `run()` is one call, `work()` what it cannot do without, `tolerance()` how far another correct
-implementation of the same precision may be off.
+implementation of the same precision may be off, `exact()` the results in float64.
 
 Kinds of case:
   decode   one decode step of paged GQA attention (plain op, its partial O||LSE form, or the sequence-parallel layer)
@@ -165,6 +165,7 @@ def prepare(case, seed):
         s["x"] = _normal(gen, (M, H))
         s["b1"], s["b2"] = _normal(gen, (E, H, I), torch.bfloat16, H ** -0.5), _normal(gen, (E, I, H), torch.bfloat16, I ** -0.5)
         ids, w = moe_utils.topk_softmax(_normal(gen, (M, E), torch.float32), topk, renormalize=True)
+        s["ids"], s["w"] = ids, w
         s["up"] = moe_tp.create_ag_group_gemm_intra_node_context(None, s["x"], s["b1"], ids, E, max_M=M, rank=0, num_ranks=1,
                                                                  heap=heap)
         s["down"] = moe_tp.create_moe_rs_context(None, 0, 1, 1, M, H, E, topk, torch.bfloat16, torch.bfloat16, s["x"].device,
@@ -246,3 +247,69 @@ def tolerance(case):
     if kind == "a2a":
         return {"rel": 9e-3, "max": 3e-2}
     return {"rel": 1.4e-2, "max": 8.5e-2}
+
+
+def exact(case, seed):
+    """What `run` returns for `prepare(case, seed)`, in float64 torch. fp8 operands are the quantised values themselves;
+    16-bit intermediates (attention probabilities, activations between two GEMMs) are not rounded. None: an output that
+    is the quantisation itself."""
+    s = prepare(case, seed)
+    kind = case["kind"]
+    if kind == "decode":
+        return _exact_decode(case, s)
+    if kind == "linear":
+        return s["a"].double() @ s["b"].double().t()
+    if kind == "mlp":
+        act = {"gelu": lambda h: F.gelu(h, approximate="tanh"), "silu": F.silu, "relu": F.relu}[case["activation"]]
+        return act(s["x"].double() @ s["block"].w1.double().t()) @ s["block"].w2.double().t()
+    if kind == "fp8":
+        a, sa = _quantised(s["x"])
+        sb = s["sb"].double().repeat_interleave(128, 0)[:case["N"]].repeat_interleave(128, 1)
+        return (a.double() * sa.double().repeat_interleave(128, 1)) @ (s["b"].double() * sb).t()
+    if kind == "a2a":
+        p = torch.softmax(s["logits"].double(), -1)
+        w = p.topk(case["topk"], -1).values
+        q, scale = _quantised(s["x"])
+        x = q.double() * scale.double().repeat_interleave(128, 1)
+        return {"rows": None, "scales": None, "splits": None, "out": w.sum(-1, keepdim=True) * x}
+    x, M = s["x"].double(), s["x"].shape[0]
+    if kind == "ep_moe":
+        block, E = s["block"], case["E"]
+        p, ids = torch.softmax(x @ block.gate.double().t(), -1).topk(case["topk"], -1)
+        w = p / p.sum(-1, keepdim=True)
+        up = lambda e: block.w1[e].double().t()    # noqa: E731
+        down = lambda e: block.w2[e].double().t()  # noqa: E731
+    else:
+        E, ids, w = case["E"], s["ids"].long(), s["w"].double()
+        up, down = (lambda e: s["b1"][e].double()), (lambda e: s["b2"][e].double())
+    out = torch.zeros((M, case["hidden"]), dtype=torch.float64, device="cuda")
+    for e in range(E):
+        tok, slot = torch.nonzero(ids == e, as_tuple=True)
+        if tok.numel():
+            out.index_add_(0, tok, (F.silu(x[tok] @ up(e)) @ down(e)) * w[tok, slot].unsqueeze(1))
+    return out
+
+
+def _quantised(x):
+    """Per row and 128 values: the e4m3 values and their fp32 scale (largest magnitude / 448)."""
+    g = x.float().view(x.shape[0], -1, 128)
+    scale = g.abs().amax(-1).clamp_min(1e-12) / 448.0
+    return (g / scale.unsqueeze(-1)).to(torch.float8_e4m3fn).view(x.shape), scale
+
+
+def _exact_decode(case, s):
+    B, hq, hkv, D, cap = case["B"], case["hq"], case["hkv"], case["head_dim"], case["soft_cap"]
+    out = torch.empty((B, hq, D + 1), dtype=torch.float64, device="cuda")
+    lens = s["lens"].view(B).tolist()
+    for b in range(B):
+        pages, n = s["table"][b].long(), lens[b]
+        for h in range(hkv):
+            heads = slice(h * hq // hkv, (h + 1) * hq // hkv)
+            k = s["k"][pages, :, h].reshape(-1, D)[:n].double()
+            v = s["v"][pages, :, h].reshape(-1, D)[:n].double()
+            t = s["q"][b, heads].double() @ k.t() * s["scale"]
+            if cap > 0:
+                t = cap * torch.tanh(t / cap)
+            out[b, heads, :D] = torch.softmax(t, -1) @ v
+            out[b, heads, D] = torch.logsumexp(t, -1)
+    return out if case["entry"] == "partial" else out[..., :D]
