@@ -36,6 +36,22 @@ def test_quantisers_round_trip(cuda_device):
     torch.testing.assert_close(F.dequantize_fp8(a2, sa2, 1), x, rtol=0.07, atol=1e-6)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("M,K", [(1, 128), (3, 384), (63, 128), (65, 128), (1000, 7168)])
+def test_rowwise_quantiser_gives_the_bytes_of_its_torch_statement(cuda_device, M, K, dtype):
+    g = torch.Generator(device="cpu").manual_seed(M + K)
+    x = torch.randn(M, K, generator=g) * torch.exp2(torch.randint(-14, 15, (M, K // 128), generator=g).float()).repeat_interleave(128, 1)
+    x = x.to(dtype).to(cuda_device)
+    x[0, :128] = 0
+    if K > 128 and M > 2:   # an infinity, a NaN, the largest and the smallest values of the type
+        x[1, 5], x[1, 6], x[2, 7] = float("inf"), 1.0, float("nan")
+        x[2, 128:256] = torch.finfo(dtype).max
+        x[2, 256:384] = torch.finfo(dtype).smallest_normal
+    (q, s), (qt, st) = F.quantize_fp8_rowwise(x), F._quantize_rowwise_torch(x)
+    assert torch.equal(q.view(torch.uint8), qt.view(torch.uint8))
+    torch.testing.assert_close(s, st, rtol=0, atol=0, equal_nan=True)
+
+
 @pytest.mark.parametrize("M,N,K", [(128, 256, 128), (256, 512, 512), (300, 264, 384), (1000, 1000, 896), (4096, 768, 2048)])
 def test_plain_fp8_gemm_matches_fp32_reference(cuda_device, M, N, K):
     a, sa, b, sb = _operands(M, N, K, cuda_device, M + N + K)

@@ -227,6 +227,7 @@ def _declare(lib):
     lib.tdist_gemm_schedule_check.argtypes = [C.c_int] * 8 + [C.POINTER(C.c_int), C.POINTER(C.c_int)]
     lib.tdist_gemm_schedule_check.restype = C.c_int
     lib.tdist_gemm_fp8_run.argtypes = [C.POINTER(GemmFp8Args)]
+    lib.tdist_quant_fp8_rowwise.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_longlong, C.c_int, C.c_int, C.c_void_p]
     lib.tdist_allgather.argtypes = [C.POINTER(CollArgs)]
     lib.tdist_nvls.argtypes = [C.POINTER(NvlsArgs)]
     lib.tdist_reduce_scatter.argtypes = [C.POINTER(CollArgs)]

@@ -161,6 +161,9 @@ typedef struct TdistGemmFp8Args {
 } TdistGemmFp8Args;
 
 int tdist_gemm_fp8_run(const TdistGemmFp8Args* args);
+/* Activations of the above: x [rows, k] (bf16 / fp16 / fp32, 16-byte aligned) -> q e4m3 [rows, k], scale fp32
+ * [rows, k / 128]; value = q * scale. */
+int tdist_quant_fp8_rowwise(const void* x, void* q, void* scale, long long rows, int k, int dtype, void* stream);
 
 /* ------------------------------------------------------------------ standalone collectives */
 /* PUSH_ORDERED: like PUSH, but all copy CTAs serve one destination after the other, rank - 1 first (the order in which the

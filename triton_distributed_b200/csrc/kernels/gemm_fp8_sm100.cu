@@ -28,6 +28,9 @@
 // (reference kernels/nvidia/allgather_group_gemm.py:348); the 1x128 / 128x128 scale layout is the
 // DeepSeek-V3 one its tutorial 04 quantises to.
 #include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+#include <cuda_fp8.h>
 #include <cuda_runtime.h>
 
 #include <cstring>
@@ -384,6 +387,69 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_fp8_kernel(const __grid_const
     if (warp == 1) tmem_dealloc<1>(tmem_base, TMEM_COLS);
 }
 
+// ------------------------------------------------------------------------------------------
+// Row-wise quantisation of the activations: every 128 values of a row become e4m3 with one fp32 scale.
+// Bound by memory: it reads x once and writes half (bf16) or a quarter (fp32) of that. 16 lanes own a group, 8 values
+// each, so that a lane loads 16 (bf16 / fp16) or 32 bytes at once and the group's largest magnitude takes four shuffles;
+// QUANT_UNROLL groups per lane are loaded before the first is used. M 8192, K 4096, bf16, with the N 6144 product that
+// follows: 599 us with the seven elementwise passes this replaces, 282 us here.
+// The arithmetic is theirs to the bit: scale = amax x fl(1 / 448) (how a tensor is divided by a host scalar), then an
+// IEEE division per value; a NaN anywhere in a group makes its scale NaN.
+// ------------------------------------------------------------------------------------------
+constexpr int QUANT_THREADS = 256, QUANT_UNROLL = 4;
+constexpr int QUANT_GROUPS = QUANT_THREADS / 16 * QUANT_UNROLL;   // groups of 128 values per CTA
+
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+template <typename T>
+struct QuantLoad {
+    uint4 raw[sizeof(T) / 2];
+    __device__ __forceinline__ void load(const T* src) {
+#pragma unroll
+        for (int i = 0; i < static_cast<int>(sizeof(T) / 2); ++i) raw[i] = __ldg(reinterpret_cast<const uint4*>(src) + i);
+    }
+    __device__ __forceinline__ void unpack(float (&v)[8]) const {
+        const T* e = reinterpret_cast<const T*>(raw);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = static_cast<float>(e[i]);
+    }
+};
+
+template <typename T>
+__global__ void __launch_bounds__(QUANT_THREADS) quant_rowwise_kernel(const T* x, uint2* q, float* scale, long long groups) {
+    const int sub = static_cast<int>(threadIdx.x) & 15;
+    const long long g0 = static_cast<long long>(blockIdx.x) * QUANT_GROUPS + (threadIdx.x >> 4);
+    QuantLoad<T> in[QUANT_UNROLL];
+#pragma unroll
+    for (int u = 0; u < QUANT_UNROLL; ++u) {
+        const long long g = g0 + u * (QUANT_THREADS / 16);
+        if (g < groups) in[u].load(x + g * 128 + sub * 8);
+    }
+#pragma unroll
+    for (int u = 0; u < QUANT_UNROLL; ++u) {
+        const long long g = g0 + u * (QUANT_THREADS / 16);
+        if (g >= groups) continue;   // the 16 lanes of a group leave together
+        float v[8];
+        in[u].unpack(v);
+        float amax = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) amax = max_nan(amax, fabsf(v[i]));
+        const unsigned lanes = 0xffffu << (threadIdx.x & 16);
+#pragma unroll
+        for (int o = 8; o >= 1; o >>= 1) amax = max_nan(amax, __shfl_xor_sync(lanes, amax, o));
+        const float s = max_nan(amax, 1e-12f) * (1.f / 448.f);
+        uint32_t w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            w[i] = __nv_cvt_float2_to_fp8x2(make_float2(__fdiv_rn(v[2 * i], s), __fdiv_rn(v[2 * i + 1], s)), __NV_SATFINITE, __NV_E4M3);
+        q[g * 16 + sub] = make_uint2(w[0] | (w[1] << 16), w[2] | (w[3] << 16));
+        if (sub == 0) scale[g] = s;
+    }
+}
+
 }  // namespace fp8
 }  // namespace tdist
 
@@ -491,5 +557,25 @@ extern "C" int tdist_gemm_fp8_run(const TdistGemmFp8Args* a) {
     const void* fn = reinterpret_cast<const void*>(&gemm_fp8_kernel<16>);  // 8-column staging measured the same
     TDIST_CUDA_OK(cudaLaunchKernel(fn, dim3(gemm_ctas + p.num_comm), dim3(THREADS), kargs,
                                    SMEM_BYTES, static_cast<cudaStream_t>(a->stream)));
+    return 0;
+}
+
+extern "C" int tdist_quant_fp8_rowwise(const void* x, void* q, void* scale, long long rows, int k, int dtype, void* stream) {
+    using namespace tdist::fp8;
+    if (!x || !q || !scale) return fail(TDIST_EINVAL, "fp8 quantisation: null pointer");
+    if (rows < 1 || k < 128 || k % 128) return fail(TDIST_EINVAL, "fp8 quantisation: K must be a positive multiple of 128");
+    if (reinterpret_cast<uintptr_t>(x) % 16 || reinterpret_cast<uintptr_t>(q) % 8) return fail(TDIST_EINVAL, "fp8 quantisation: x must be 16-byte and q 8-byte aligned");
+    const long long groups = rows * (k / 128);
+    const long long ctas = (groups + QUANT_GROUPS - 1) / QUANT_GROUPS;
+    if (ctas > 0x7fffffffLL) return fail(TDIST_ELIMIT, "fp8 quantisation: too many values for one launch");
+    const dim3 grid(static_cast<unsigned>(ctas));
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    uint2* qo = static_cast<uint2*>(q);
+    float* so = static_cast<float*>(scale);
+    if (dtype == TDIST_BF16) quant_rowwise_kernel<<<grid, QUANT_THREADS, 0, s>>>(static_cast<const __nv_bfloat16*>(x), qo, so, groups);
+    else if (dtype == TDIST_F16) quant_rowwise_kernel<<<grid, QUANT_THREADS, 0, s>>>(static_cast<const __half*>(x), qo, so, groups);
+    else if (dtype == TDIST_F32) quant_rowwise_kernel<<<grid, QUANT_THREADS, 0, s>>>(static_cast<const float*>(x), qo, so, groups);
+    else return fail(TDIST_EINVAL, "fp8 quantisation: dtype must be bf16, fp16 or fp32");
+    TDIST_CUDA_OK(cudaGetLastError());
     return 0;
 }
