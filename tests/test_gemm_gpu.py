@@ -215,3 +215,29 @@ def test_gemm_rs_random_m_sweep(cuda_device, tiling, world):
             check_status()
             torch.testing.assert_close(out.float(), total[r * mpr:(r + 1) * mpr], atol=3e-2, rtol=3e-2,
                                        msg=lambda m: f"iteration {it}, mpr={mpr}, rank {r}: {m}")
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("N,K", [(8, 8), (136, 72), (256, 4096), (1288, 8192 + 8), (6144, 1536), (20480, 256)])
+def test_few_row_gemm_matches_fp32_reference(cuda_device, N, K, dtype):
+    """The automatic choice at few rows: every token-tile width (1 row to 4 x 128 with remainders), N and K off the tile
+    edges, one to eight CTAs per cluster. Tolerance: the 16-bit rounding of the result (half an ulp) and fp32 sums of K
+    products of unit-variance terms, whose order changes nothing above 1e-5."""
+    import ctypes as C
+    torch.manual_seed(N + K)
+    b = _rand((N, K), dtype, cuda_device, K ** -0.5)
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    few = 0
+    for M in (1, 2, 15, 16, 17, 31, 48, 64, 65, 100, 127, 128, 129, 255, 257, 385, 500, 512):
+        a = _rand((M, K), dtype, cuda_device)
+        guard = torch.full((M + 1, N), 7.0, dtype=dtype, device=cuda_device)
+        c = G.gemm_persistent(a, b, out=guard[:M])
+        check_status()
+        torch.testing.assert_close(c.float(), a.float() @ b.float().t(), atol=eps / 16, rtol=eps)
+        assert (guard[M] == 7.0).all()   # nothing written past the last row
+        g = G._base_args(a, b, 1, 0, _lib.GEMM_PLAIN)
+        g.c, g.m_per_rank = c.data_ptr(), M
+        out = (C.c_int * 4)()
+        assert _lib.lib().tdist_gemm_plan(C.byref(g), out) == 0
+        few += out[0] == 1 and out[3] % (-(-N // 128)) == 0
+    assert few >= 8 or K < 1024   # the few-row kernel did run (with so short a K the large tiles are as good)

@@ -1,0 +1,16 @@
+// Few-row GEMM (gemm_skinny_sm100.cu): plan and launch, used by the dispatch in gemm_sm100.cu.
+#pragma once
+#include "../include/tdist.h"
+
+namespace tdist_host {
+
+struct SkinnyPlan {
+    int tok, m_tiles, n_tiles, split, stages, grid;
+};
+
+// True when the few-row kernel is expected to finish a plain product before `other_s` seconds (the estimate for the
+// large-tile kernel); fills the plan. Looks at sizes only.
+bool skinny_plan(int m, int n, int k, double other_s, SkinnyPlan* plan);
+int skinny_run(const TdistGemmArgs* a, const SkinnyPlan& plan);
+
+}  // namespace tdist_host

@@ -46,6 +46,7 @@
 #include "../device/signal.cuh"
 #include "../include/tdist.h"
 #include "../runtime/host_common.h"
+#include "gemm_skinny.h"
 
 namespace tdist {
 
@@ -1332,6 +1333,8 @@ static bool use_wide(const TdistGemmArgs* a) {
 
 struct GridPlan {
     int ctas_per_tile, wide, num_comm, num_tiles, grid;
+    bool few_rows;                     // a plain product of few rows goes to the kernel in gemm_skinny_sm100.cu
+    tdist_host::SkinnyPlan skinny;
 };
 
 template <int CTAS, bool WIDE>
@@ -1447,8 +1450,29 @@ static void plan_ag(const TdistGemmArgs* a, int sms, int n_tiles, GridPlan& g) {
     g.num_tiles = seg_m_tiles * (g.wide ? (n_tiles + 1) / 2 : n_tiles) * a->world;
 }
 
+// Plain products of one rank whose caller asked for no particular tiling, CTA count or timeline. C is written with plain
+// stores there, so a C that the TMA store here would refuse is left to that refusal.
+static bool may_be_few_rows(const TdistGemmArgs* a) {
+    return (a->mode == TDIST_GEMM_PLAIN || a->mode == TDIST_GEMM_AG) && a->world == 1 && a->expert_ids == nullptr &&
+           a->num_m_blocks == nullptr && a->a_gather == nullptr && a->c_scatter == nullptr && a->block_rot == nullptr &&
+           a->trace == nullptr && a->cta_pair < 0 && a->num_sms <= 0 && a->c != nullptr && reinterpret_cast<uintptr_t>(a->c) % 16 == 0;
+}
+
+// Expected time of a plain product on this kernel: the longest unit's share of 256-column tiles at the rate a CTA or a
+// pair sustains, or the operands' trip through HBM. A single CTA's tile is bound by its L2 -> shared-memory loads
+// (48 KB per K block at 64 bytes per clock: m16 n6144 k12288 measured 77 us, 10.5 TFLOP/s of the padded tile), a pair's by the MMAs.
+static double plain_time(const TdistGemmArgs* a, const GridPlan& g) {
+    const int units = g.grid / g.ctas_per_tile;
+    const double rate = g.ctas_per_tile == 1 ? 10.4e12 : (g.wide ? 20.5e12 : 20.0e12);
+    const double tile_s = 2.0 * BM * g.ctas_per_tile * BN * a->k / rate + (g.wide ? 1.5e-6 : 0.5e-6);
+    const double sm_s = schedule_cost(g.num_tiles, units, g.wide) * tile_s;
+    const double hbm_s = 2.0 * (static_cast<double>(a->n) * a->k + static_cast<double>(a->m_per_rank) * (a->k + a->n)) / 6.3e12;
+    return (sm_s > hbm_s ? sm_s : hbm_s) + 4e-6;
+}
+
 static GridPlan plan_grid(const TdistGemmArgs* a) {
     GridPlan g;
+    g.few_rows = false;
     g.ctas_per_tile = use_pair(a) ? 2 : 1;
     g.wide = use_wide(a) ? 1 : 0;
     const int seg_m_tiles = (a->m_per_rank + BM * g.ctas_per_tile - 1) / (BM * g.ctas_per_tile);
@@ -1477,6 +1501,12 @@ static GridPlan plan_grid(const TdistGemmArgs* a) {
     if (units > most) units = most;
     if (units < 1) units = 1;
     g.grid = units * g.ctas_per_tile + g.num_comm;
+    if (may_be_few_rows(a) && tdist_host::skinny_plan(a->m_per_rank, a->n, a->k, plain_time(a, g), &g.skinny)) {
+        g.few_rows = true;
+        g.ctas_per_tile = 1;
+        g.wide = 0;
+        g.grid = g.skinny.grid;
+    }
     return g;
 }
 
@@ -1564,6 +1594,7 @@ extern "C" int tdist_gemm_run(const TdistGemmArgs* a) {
     }
 
     const GridPlan plan = plan_grid(a);
+    if (plan.few_rows) return tdist_host::skinny_run(a, plan.skinny);
     const int ctas = plan.ctas_per_tile;
     GemmParams p;
     memset(&p, 0, sizeof(p));
