@@ -6,6 +6,7 @@ import pytest
 import torch
 
 from triton_distributed_b200.ops import all_to_all as A
+from triton_distributed_b200.ops import moe_tp as MT
 from triton_distributed_b200.ops import moe_utils as MU
 from triton_distributed_b200.runtime import LocalWorld, check_status
 
@@ -234,3 +235,49 @@ def test_ep_dispatch_compact_layout_and_pull_combine(cuda_device, world, T, E, K
         for r in range(world):
             live = (ids[r] >= 0).sum(-1, keepdim=True).float()
             torch.testing.assert_close(outs[r].float(), xs[r].float() * live, atol=2e-2, rtol=2e-2)
+
+
+@pytest.mark.parametrize("E", [1, 8, 31, 32, 33, 60, 64, 100, 256, 300, 1024])
+def test_topk_softmax_over_every_register_width(cuda_device, E):
+    torch.manual_seed(E)
+    logits = torch.randn(37, E, device=cuda_device)
+    logits[3] = 0.0                               # ties: the lower expert ids
+    logits[4, 1:] = torch.finfo(torch.float32).min
+    k = min(E, 8)
+    for renorm in (False, True):
+        ids, w = MU.topk_softmax(logits, k, renormalize=renorm)
+        ids_c, w_c = MU.topk_softmax(logits.cpu(), k, renormalize=renorm)
+        rows = [i for i in range(37) if i != 4]   # row 4: equal (zero) probabilities in any order after the first
+        assert torch.equal(ids.cpu()[rows], ids_c[rows]) and ids[4, 0] == 0
+        torch.testing.assert_close(w.cpu(), w_c, rtol=1e-5, atol=1e-7)
+
+
+@pytest.mark.parametrize("T,hidden,E,k", [(1, 32, 8, 1), (3, 512, 8, 2), (16, 544, 16, 4), (17, 2048, 32, 8), (128, 7168, 32, 8),
+                                          (33, 1024, 60, 5), (50, 4096, 64, 8), (40, 512, 130, 6), (9, 64, 1024, 8)])
+def test_gate_topk_is_no_further_from_float64_than_the_fp32_product(cuda_device, T, hidden, E, k):
+    torch.manual_seed(T + hidden + E)
+    x = torch.randn(T, hidden, device=cuda_device).bfloat16()
+    gate = (torch.randn(E, hidden, device=cuda_device) * hidden ** -0.5).bfloat16()
+    logits = torch.empty(T, E, device=cuda_device)
+    ids, w = MU.gate_topk(x, gate, k, renormalize=True, logits=logits)
+    exact = x.double() @ gate.double().t()
+    before = (x.float() @ gate.float().t()).double()
+    assert (logits.double() - exact).norm() <= max((before - exact).norm().item(), 1e-7 * exact.norm().item())
+    ids_t, w_t = MU.topk_softmax(logits, k, renormalize=True)
+    assert torch.equal(ids, ids_t)
+    torch.testing.assert_close(w, w_t, rtol=1e-6, atol=0)
+
+
+@pytest.mark.parametrize("T,k,hidden", [(1, 1, 8), (5, 2, 1024), (64, 3, 1032), (7, 8, 7168), (300, 2, 4096), (2, 1, 1016)])
+def test_topk_reduce_over_ragged_rows_and_rejected_pairs(cuda_device, T, k, hidden):
+    torch.manual_seed(T + hidden)
+    y = torch.randn(T * k + 3, hidden, device=cuda_device).bfloat16()
+    pos = torch.randperm(T * k + 3, device=cuda_device)[:T * k].to(torch.int32)
+    w = torch.rand(T, k, device=cuda_device)
+    if T > 2:
+        pos[k] = -1                               # a pair that routing rejected contributes nothing
+    rows = torch.where((pos >= 0).unsqueeze(1), y[pos.long().clamp(min=0)].float(), torch.zeros((), device=cuda_device)).view(T, k, hidden)
+    for weights in (w, None):
+        ref = (rows * (weights.unsqueeze(-1) if weights is not None else 1.0)).sum(1)
+        out = MT.topk_reduce(y, pos, weights, T, k)
+        torch.testing.assert_close(out.float(), ref, rtol=2.0 ** -8, atol=1e-5)

@@ -252,6 +252,8 @@ def _declare(lib):
     lib.tdist_gather_rows.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p]
     lib.tdist_topk_reduce.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p]
     lib.tdist_moe_topk_softmax.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p]
+    lib.tdist_moe_gate_topk.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p,
+                                        C.c_void_p, C.c_void_p]
     lib.tdist_stream_write_value.argtypes = [C.c_void_p, C.c_uint64, C.c_uint64, C.c_int]
     lib.tdist_stream_wait_value.argtypes = [C.c_void_p, C.c_uint64, C.c_uint64, C.c_int, C.c_int]
 

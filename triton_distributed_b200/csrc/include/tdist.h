@@ -348,6 +348,11 @@ int tdist_topk_reduce(const void* y, const void* pos_of, const void* weights, in
 int tdist_moe_topk_softmax(const void* logits_f32, int ntok, int num_experts, int topk, int renormalize,
                            void* ids, void* weights, void* stream);
 
+/* The same on logits = x . gate^T computed in the launch: x [ntok, hidden], gate [num_experts, hidden] bf16, fp32 sums;
+ * logits (fp32 [ntok, num_experts]) may be NULL. hidden must be a multiple of 32. */
+int tdist_moe_gate_topk(const void* x, const void* gate, int ntok, int hidden, int num_experts, int topk, int renormalize,
+                        void* ids, void* weights, void* logits, void* stream);
+
 /* ------------------------------------------------------------------ GQA flash decode */
 typedef struct TdistDecodeArgs {
     const void* q;            /* [B, Hq, D] bf16/fp16 */

@@ -7,6 +7,7 @@
 // (csrc/lib/moe_utils.cu:60-192) with its Python oracle `full_moe_align_block_size`
 // (kernels/nvidia/moe_reduce_rs.py:87-177). The sorts here are stable (ascending pair index inside
 // an expert), so results are reproducible and comparable element by element with the oracle.
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <math_constants.h>
 
@@ -110,17 +111,16 @@ __global__ void __launch_bounds__(kMoeThreads) moe_align_kernel(const int* ids, 
 }
 
 // ---------------------------------------------------------------------------- softmax + top-k
-// One warp per token; E <= 1024. weights = softmax probabilities of the selected experts,
-// optionally renormalised to sum to one. Ties go to the lower expert index.
-__global__ void moe_topk_softmax_kernel(const float* logits, int ntok, int E, int topk, int renorm, int* ids, float* w) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (warp >= ntok) return;
-    const float* row = logits + static_cast<size_t>(warp) * E;
-    float v[32];
+// One warp per token; E <= 1024, J = ceil(E / 32) logits per lane rounded up to a power of two: the selection walks them
+// topk times, so 32 per lane whatever E is costs more than the loads (128 tokens, 8 of 256: 6.2 us with 32 per lane, 4.1 us with 8).
+// weights = softmax probabilities of the selected experts, optionally renormalised to sum to one. Ties go to the lower
+// expert index.
+template <int J>
+__device__ __forceinline__ void topk_softmax_row(const float* row, int E, int topk, int renorm, int lane, int* ids, float* w) {
+    float v[J];
     float mx = -CUDART_INF_F;
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
+    for (int j = 0; j < J; ++j) {
         const int e = j * 32 + lane;
         v[j] = e < E ? row[e] : -CUDART_INF_F;
         mx = fmaxf(mx, v[j]);
@@ -129,7 +129,7 @@ __global__ void moe_topk_softmax_kernel(const float* logits, int ntok, int E, in
     for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     float sum = 0.f;
 #pragma unroll
-    for (int j = 0; j < 32; ++j) sum += (j * 32 + lane < E) ? __expf(v[j] - mx) : 0.f;
+    for (int j = 0; j < J; ++j) sum += (j * 32 + lane < E) ? __expf(v[j] - mx) : 0.f;
 #pragma unroll
     for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     float picked_sum = 0.f;
@@ -139,7 +139,7 @@ __global__ void moe_topk_softmax_kernel(const float* logits, int ntok, int E, in
         float best = -CUDART_INF_F;
         int best_e = 0x7fffffff;
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
+        for (int j = 0; j < J; ++j) {
             const int e = j * 32 + lane;
             if (v[j] > best) {
                 best = v[j];
@@ -163,14 +163,107 @@ __global__ void moe_topk_softmax_kernel(const float* logits, int ntok, int E, in
         }
         if ((best_e & 31) == lane) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j)
+            for (int j = 0; j < J; ++j)
                 if (j == (best_e >> 5)) v[j] = -CUDART_INF_F;
         }
     }
     if (lane < topk) {
-        ids[static_cast<size_t>(warp) * topk + lane] = my_id;
-        w[static_cast<size_t>(warp) * topk + lane] = renorm ? my_w / picked_sum : my_w;
+        ids[lane] = my_id;
+        w[lane] = renorm ? my_w / picked_sum : my_w;
     }
+}
+__device__ __forceinline__ void topk_softmax_any(const float* row, int E, int topk, int renorm, int lane, int* ids, float* w) {
+    if (E <= 32) topk_softmax_row<1>(row, E, topk, renorm, lane, ids, w);
+    else if (E <= 64) topk_softmax_row<2>(row, E, topk, renorm, lane, ids, w);
+    else if (E <= 128) topk_softmax_row<4>(row, E, topk, renorm, lane, ids, w);
+    else if (E <= 256) topk_softmax_row<8>(row, E, topk, renorm, lane, ids, w);
+    else topk_softmax_row<32>(row, E, topk, renorm, lane, ids, w);
+}
+__global__ void moe_topk_softmax_kernel(const float* logits, int ntok, int E, int topk, int renorm, int* ids, float* w) {
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (warp >= ntok) return;
+    const size_t at = static_cast<size_t>(warp) * topk;
+    topk_softmax_any(logits + static_cast<size_t>(warp) * E, E, topk, renorm, static_cast<int>(threadIdx.x) & 31, ids + at, w + at);
+}
+
+// ---------------------------------------------------------------------------- gate: logits, softmax and top-k in one launch
+// logits[t, e] = x[t, :] . gate[e, :] (bf16 in, fp32 sums), then the selection above. A decode step has few tokens and
+// few experts, so the product is short of parallelism, not of arithmetic: a CTA takes 16 tokens and ALL experts, and its
+// 16 warps split the hidden dimension 32 values at a time (what a cuBLAS SGEMM of the fp32 copies does serially; 128 x
+// 7168 x 32 experts: 53 us as two copies, SGEMM, reduction and selection, 12 us here). mma.sync m16n8k16: the products of bf16 values are exact in
+// fp32, the tensor core sums 32 of them at a time (its accumulator truncates, so longer chains there would lose bits
+// against an fp32 FMA loop), the rest is added in fp32: 1/16 of the hidden dimension per warp, then 16 partial sums. A tcgen05
+// tile (M 128) would leave all but 16 rows of this split idle. Any order of k will do as long as x and gate agree, so a
+// thread takes 8 consecutive values of its row per step: one 16-byte load feeds two MMAs.
+constexpr int kGateTok = 16, kGateThreads = 512, kGateWarps = kGateThreads / 32;
+
+__device__ __forceinline__ void mma_bf16_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// NT: groups of 8 experts per pass over the tokens' rows
+template <int NT>
+__global__ void __launch_bounds__(kGateThreads, 1) moe_gate_topk_kernel(const __nv_bfloat16* x, const __nv_bfloat16* gate, int ntok, int hidden, int E,
+                                                                        int topk, int renorm, int* ids, float* w, float* logits) {
+    extern __shared__ float gate_sm[];
+    constexpr int COLS = NT * 8;
+    float* part = gate_sm;                                   // [warps][16 tokens][COLS]
+    float* row_s = gate_sm + kGateWarps * kGateTok * COLS;   // [16 tokens][E]
+    const int tid = static_cast<int>(threadIdx.x), warp = tid >> 5, lane = tid & 31;
+    const int g = lane >> 2, tig = lane & 3;                 // row / column group of the MMA fragments
+    const int t0 = static_cast<int>(blockIdx.x) * kGateTok;
+    const int steps = hidden / 32;
+    // rows past the end repeat the last one; their results are not used
+    const __nv_bfloat16* xa = x + static_cast<size_t>(min(t0 + g, ntok - 1)) * hidden + tig * 8;
+    const __nv_bfloat16* xb = x + static_cast<size_t>(min(t0 + g + 8, ntok - 1)) * hidden + tig * 8;
+    for (int e0 = 0; e0 < E; e0 += COLS) {
+        const __nv_bfloat16* ge[NT];
+        float acc[NT][4];
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+            ge[n] = gate + static_cast<size_t>(min(e0 + n * 8 + g, E - 1)) * hidden + tig * 8;
+            acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+        }
+#pragma unroll(NT == 8 ? 1 : 2)
+        for (int s = warp; s < steps; s += kGateWarps) {
+            const uint4 a = __ldg(reinterpret_cast<const uint4*>(xa + s * 32));
+            const uint4 c = __ldg(reinterpret_cast<const uint4*>(xb + s * 32));
+            uint4 b[NT];
+#pragma unroll
+            for (int n = 0; n < NT; ++n) b[n] = __ldg(reinterpret_cast<const uint4*>(ge[n] + s * 32));
+#pragma unroll
+            for (int n = 0; n < NT; ++n) {
+                float d[4] = {0.f, 0.f, 0.f, 0.f};
+                mma_bf16_16816(d, a.x, c.x, a.y, c.y, b[n].x, b[n].y);
+                mma_bf16_16816(d, a.z, c.z, a.w, c.w, b[n].z, b[n].w);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) acc[n][i] += d[i];
+            }
+        }
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+            float* p = part + (warp * kGateTok + g) * COLS + n * 8 + tig * 2;
+            *reinterpret_cast<float2*>(p) = make_float2(acc[n][0], acc[n][1]);
+            *reinterpret_cast<float2*>(p + 8 * COLS) = make_float2(acc[n][2], acc[n][3]);
+        }
+        __syncthreads();
+        for (int i = tid; i < kGateTok * COLS; i += kGateThreads) {
+            const int t = i / COLS, e = e0 + i % COLS;
+            float sum = 0.f;
+#pragma unroll
+            for (int k = 0; k < kGateWarps; ++k) sum += part[k * kGateTok * COLS + i];
+            if (e < E) {
+                row_s[t * E + e] = sum;
+                if (logits != nullptr && t0 + t < ntok) logits[static_cast<size_t>(t0 + t) * E + e] = sum;
+            }
+        }
+        __syncthreads();
+    }
+    const int t = t0 + warp;   // a warp per token: kGateWarps == kGateTok
+    static_assert(kGateWarps == kGateTok, "a warp per token");
+    if (t < ntok) topk_softmax_any(row_s + warp * E, E, topk, renorm, lane, ids + static_cast<size_t>(t) * topk, w + static_cast<size_t>(t) * topk);
 }
 
 // ---------------------------------------------------------------------------- row gather / top-k reduce
@@ -191,36 +284,55 @@ __global__ void gather_rows_kernel(const uint4* src, const int* index, int rows_
     }
 }
 
-// out[t] = sum_k w[t*topk+k] * y[pos_of[t*topk+k]] in fp32 (bf16 in/out). One warp per token.
-__global__ void topk_reduce_kernel(const uint4* y, const int* pos_of, const float* w, int ntok, int topk, int vec_per_row,
-                                   uint4* out) {
+// out[t] = sum_k w[t*topk+k] * y[pos_of[t*topk+k]] in fp32 (bf16 in/out), bound by reading y. A warp takes a token's 128
+// vectors of 16 bytes at a time (a row shorter than that still goes to one warp): four loads per lane and row are in
+// flight, twice that with two rows (8192 tokens x 4096, top 2: 53 us with one load per lane and row, 30 us).
+constexpr int kReduceVecs = 4;
+__global__ void __launch_bounds__(256) topk_reduce_kernel(const uint4* y, const int* pos_of, const float* w, int ntok, int topk, int vec_per_row,
+                                                          uint4* out) {
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (int t = warp; t < ntok; t += nwarps) {
-        for (int c = lane; c < vec_per_row; c += 32) {
-            float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            for (int k = 0; k < topk; ++k) {
-                const int pos = pos_of[t * topk + k];
-                if (pos < 0) continue;   // a pair that routing rejected contributes nothing
-                const float wk = w ? w[t * topk + k] : 1.f;
-                const uint4 q = y[static_cast<size_t>(pos) * vec_per_row + c];
-                const uint32_t u[4] = {q.x, q.y, q.z, q.w};
+    const int segs = (vec_per_row + 32 * kReduceVecs - 1) / (32 * kReduceVecs);
+    for (long long item = warp; item < static_cast<long long>(ntok) * segs; item += nwarps) {
+        const int t = static_cast<int>(item / segs);
+        const int c0 = static_cast<int>(item - static_cast<long long>(t) * segs) * 32 * kReduceVecs + lane;
+        float acc[kReduceVecs][8];
+#pragma unroll
+        for (int u = 0; u < kReduceVecs; ++u)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[u][i] = 0.f;
+#pragma unroll 2
+        for (int k = 0; k < topk; ++k) {
+            const int pos = pos_of[static_cast<size_t>(t) * topk + k];
+            // a pair that routing rejected contributes nothing
+            const float wk = pos < 0 ? 0.f : (w ? w[static_cast<size_t>(t) * topk + k] : 1.f);
+            uint4 q[kReduceVecs];
+#pragma unroll
+            for (int u = 0; u < kReduceVecs; ++u)
+                q[u] = pos >= 0 && c0 + u * 32 < vec_per_row ? __ldg(y + static_cast<size_t>(pos) * vec_per_row + c0 + u * 32) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+            for (int u = 0; u < kReduceVecs; ++u) {
+                const uint32_t v[4] = {q[u].x, q[u].y, q[u].z, q[u].w};
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    acc[2 * i] += wk * __uint_as_float(u[i] << 16);
-                    acc[2 * i + 1] += wk * __uint_as_float(u[i] & 0xffff0000u);
+                    acc[u][2 * i] += wk * __uint_as_float(v[i] << 16);
+                    acc[u][2 * i + 1] += wk * __uint_as_float(v[i] & 0xffff0000u);
                 }
             }
+        }
+#pragma unroll
+        for (int u = 0; u < kReduceVecs; ++u) {
+            if (c0 + u * 32 >= vec_per_row) continue;
             uint4 o;
             uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 uint32_t r;
-                asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(acc[2 * i + 1]), "f"(acc[2 * i]));
+                asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(acc[u][2 * i + 1]), "f"(acc[u][2 * i]));
                 ow[i] = r;
             }
-            out[static_cast<size_t>(t) * vec_per_row + c] = o;
+            out[static_cast<size_t>(t) * vec_per_row + c0 + u * 32] = o;
         }
     }
 }
@@ -292,6 +404,32 @@ extern "C" int tdist_moe_topk_softmax(const void* logits, int ntok, int num_expe
     return 0;
 }
 
+extern "C" int tdist_moe_gate_topk(const void* x, const void* gate, int ntok, int hidden, int num_experts, int topk, int renormalize,
+                                   void* ids, void* weights, void* logits, void* stream) {
+    if (num_experts < 1 || num_experts > 1024) return fail(TDIST_ELIMIT, "moe_gate_topk: at most 1024 experts");
+    if (topk < 1 || topk > 32 || topk > num_experts) return fail(TDIST_EINVAL, "moe_gate_topk: topk must be in [1, min(32, experts)]");
+    if (hidden < 32 || hidden % 32) return fail(TDIST_EINVAL, "moe_gate_topk: hidden must be a multiple of 32");
+    if (reinterpret_cast<uintptr_t>(x) % 16 || reinterpret_cast<uintptr_t>(gate) % 16) return fail(TDIST_EINVAL, "moe_gate_topk: x and gate must be 16-byte aligned");
+    if (ntok <= 0) return 0;
+    const int nt = num_experts <= 8 ? 1 : (num_experts <= 16 ? 2 : (num_experts <= 32 ? 4 : 8));
+    const int smem = (kGateWarps * kGateTok * nt * 8 + kGateTok * num_experts) * static_cast<int>(sizeof(float));
+    const dim3 grid((ntok + kGateTok - 1) / kGateTok);
+#define TDIST_GATE_CASE(NT)                                                                                                     \
+    {                                                                                                                           \
+        if (int rc = ensure_smem(moe_gate_topk_kernel<NT>, smem)) return rc;                                                    \
+        moe_gate_topk_kernel<NT><<<grid, kGateThreads, smem, static_cast<cudaStream_t>(stream)>>>(                              \
+            static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gate), ntok, hidden, num_experts, topk,     \
+            renormalize, static_cast<int*>(ids), static_cast<float*>(weights), static_cast<float*>(logits));                    \
+    }
+    if (nt == 1) TDIST_GATE_CASE(1)
+    else if (nt == 2) TDIST_GATE_CASE(2)
+    else if (nt == 4) TDIST_GATE_CASE(4)
+    else TDIST_GATE_CASE(8)
+#undef TDIST_GATE_CASE
+    TDIST_CUDA_OK(cudaGetLastError());
+    return 0;
+}
+
 extern "C" int tdist_gather_rows(const void* src, const void* index, int rows_out, int div, int limit, int row_bytes,
                                  void* dst, void* pos_of, void* stream) {
     if (row_bytes % 16 || div < 1) return fail(TDIST_EINVAL, "gather_rows: rows must be multiples of 16 bytes");
@@ -308,7 +446,8 @@ extern "C" int tdist_topk_reduce(const void* y, const void* pos_of, const void* 
                                  void* out, void* stream) {
     if (row_bytes % 16 || topk < 1) return fail(TDIST_EINVAL, "topk_reduce: rows must be multiples of 16 bytes");
     if (ntok <= 0) return 0;
-    const int blocks = (ntok + 7) / 8 < 1184 ? (ntok + 7) / 8 : 1184;
+    const long long items = static_cast<long long>(ntok) * ((row_bytes / 16 + 32 * kReduceVecs - 1) / (32 * kReduceVecs));
+    const int blocks = static_cast<int>((items + 7) / 8 < 1184 ? (items + 7) / 8 : 1184);
     topk_reduce_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const uint4*>(y), static_cast<const int*>(pos_of), static_cast<const float*>(weights), ntok, topk,
         row_bytes / 16, static_cast<uint4*>(out));

@@ -50,7 +50,7 @@ class EPMoE:
     The dispatch kernel writes the received rows grouped by local expert with every group starting on a 128-row
     boundary, together with the expert of every 128-row block, so the receive buffer is the A operand of the
     grouped GEMM as it stands; the second GEMM writes into the symmetric buffer the combine kernels of the source
-    ranks read. Five launches (top-k, dispatch, GEMM, activation, GEMM) + combine, no host synchronisation."""
+    ranks read. Five launches (gate, dispatch, GEMM, activation, GEMM) + combine, no host synchronisation."""
 
     def __init__(self, gate: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor, topk: int, rank: int, world: int, max_tokens: int,
                  group=None, heap=None):
@@ -67,8 +67,7 @@ class EPMoE:
         return MT.group_gemm(F.silu(h), self.w2, self.ctx.block_expert, self.ctx.num_blocks, out=out)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        logits = x.float() @ self.gate.float().t()
-        ids, w = MU.topk_softmax(logits, self.topk, renormalize=True)
+        ids, w = MU.gate_topk(x, self.gate, self.topk, renormalize=True)
         rows, _, _, _ = EP.ep_dispatch(self.ctx, x, ids, w)
         if x.device.type != "cuda":
             return EP.ep_combine(self.ctx, self._experts_cpu(rows), weighted=True)

@@ -19,6 +19,7 @@ from typing import NamedTuple, Optional, Tuple
 import torch
 
 from .. import _lib
+from ..utils.misc import plain_cuda
 
 launch_count = 0
 
@@ -60,6 +61,28 @@ def topk_softmax(logits: torch.Tensor, topk: int, renormalize: bool = False) -> 
                                                  w.data_ptr(), _stream(x)), "tdist_moe_topk_softmax")
     launch_count += 1
     return ids, w
+
+
+def gate_topk(x: torch.Tensor, gate: torch.Tensor, topk: int, renormalize: bool = False,
+              logits: Optional[torch.Tensor] = None) -> Tuple[torch.Tensor, torch.Tensor]:
+    """:func:`topk_softmax` of ``x[T, hidden] @ gate[E, hidden].T`` with fp32 sums; one launch for bf16 operands.
+    ``logits`` (fp32 ``[T, E]``), if given, receives the product."""
+    global launch_count
+    T, hidden = x.shape
+    E = gate.shape[0]
+    if x.dtype == gate.dtype == torch.bfloat16 and T > 0 and hidden >= 32 and hidden % 32 == 0 and 1 <= topk <= min(32, E) and E <= 1024 \
+            and gate.shape[1] == hidden and plain_cuda(x, gate):
+        ids = torch.empty((T, topk), dtype=torch.int32, device=x.device)
+        w = torch.empty((T, topk), dtype=torch.float32, device=x.device)
+        _lib.check(_lib.lib().tdist_moe_gate_topk(x.data_ptr(), gate.data_ptr(), T, hidden, E, topk, int(renormalize), ids.data_ptr(),
+                                                  w.data_ptr(), logits.data_ptr() if logits is not None else None, _stream(x)),
+                   "tdist_moe_gate_topk")
+        launch_count += 1
+        return ids, w
+    out = x.float() @ gate.float().t()
+    if logits is not None:
+        logits.copy_(out)
+    return topk_softmax(out, topk, renormalize)
 
 
 def route(topk_ids: torch.Tensor, num_experts: int, out: Optional[Routing] = None) -> Routing:
