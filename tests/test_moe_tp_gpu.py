@@ -146,3 +146,47 @@ def test_group_gemm_staged_gather_rotation_and_scatter(cuda_device, T, E, K, N, 
         assert torch.equal(got_sorted[live], want_sorted[live])
         assert torch.equal(got, want)
         assert int(ready[n // 128:].abs().sum()) == 0      # the kernel leaves its counters at zero for the next launch
+
+
+@pytest.mark.parametrize("world,tpr,E,K,N,topk", [(1, 2000, 4, 264, 520, 2), (1, 3000, 3, 4104, 776, 2), (1, 300, 8, 256, 512, 2),
+                                                  (4, 700, 2, 512, 264, 2), (1, 90, 2, 64, 8, 1)])
+def test_grouped_gemm_on_block_pairs(cuda_device, monkeypatch, world, tpr, E, K, N, topk):
+    """Two blocks of an expert per CTA pair, odd blocks alone (forced where they are many), ragged last blocks, narrow and
+    wide tiles; up-projection with staged rows, rotation and scatter, then down-projection with staged rows and top-k reduce.
+    Tolerance as above: 16-bit results and the 16-bit intermediate of the reduce."""
+    monkeypatch.setattr(MT, "PAIR_MAX_OVERHEAD", 2.0)
+    torch.manual_seed(tpr + E)
+    lw = LocalWorld(world, cuda_device)
+    M = world * tpr
+    shards = [torch.randn(tpr, K, device=cuda_device).to(torch.bfloat16) for _ in range(world)]
+    bs = [(torch.randn(E, K, N, device=cuda_device) * K ** -0.5).to(torch.bfloat16) for _ in range(world)]
+    ids = torch.stack([torch.randperm(E, device=cuda_device)[:topk] for _ in range(M)]).to(torch.int32)
+    ctxs = [MT.create_ag_group_gemm_intra_node_context(None, shards[r], bs[r], ids, E, max_M=M, rank=r, num_ranks=world,
+                                                       heap=lw.heap(r)) for r in range(world)]
+    assert all(c.pairs is not None for c in ctxs)
+    for r in range(world if world > 1 else 0):
+        MT.ag_group_gemm_intra_node(shards[r], bs[r], ctxs[r], phase=1)
+    rows = torch.cat(shards)[torch.arange(M * topk, device=cuda_device) // topk]
+    for r in range(world):
+        for _ in range(2 if world == 1 else 1):
+            out = MT.ag_group_gemm_intra_node(shards[r], bs[r], ctxs[r], phase=2 if world > 1 else 3)
+            check_status()
+            torch.testing.assert_close(out.float(), _expert_matmul(rows, ids.reshape(-1), bs[r]), atol=3e-2, rtol=3e-2)
+    if world == 1:
+        w = torch.rand(M, topk, device=cuda_device)
+        down = MT.create_moe_rs_context(None, 0, 1, 1, M, N, E, topk, torch.bfloat16, torch.bfloat16, cuda_device, full_topk_ids=ids,
+                                        full_topk_weight=w, heap=lw.heap(0))
+        assert down.pairs is not None
+        y = MT.moe_reduce_rs(0, 1, 1, rows, bs[0], down)
+        check_status()
+        ref = (_expert_matmul(rows, ids.reshape(-1), bs[0]).view(M, topk, N) * w.unsqueeze(-1)).sum(1)
+        torch.testing.assert_close(y.float(), ref, atol=6e-2, rtol=3e-2)
+
+
+def test_pair_blocks_keeps_experts_and_ranks_apart():
+    experts = torch.tensor([0, 0, 0, 1, 1, 1, 1, 2, 2, 0, 0, 3, 3], dtype=torch.int32)
+    ranks = torch.tensor([0] * 9 + [1] * 4, dtype=torch.int32)
+    pairs = MT.pair_blocks(experts, ranks, 13, 9)
+    assert pairs.block.tolist() == [0, 5, 6, 10, 14, 18, 22] and pairs.rot.tolist() == [5]
+    assert MT.pair_blocks(torch.arange(6, dtype=torch.int32), torch.zeros(6, dtype=torch.int32), 6) is None
+    assert MT.pair_blocks(experts, ranks, 0) is None

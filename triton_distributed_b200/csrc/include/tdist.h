@@ -117,6 +117,11 @@ typedef struct TdistGemmArgs {
      * int32) of the matrix at `c` ([c_rows, N]); rows whose index is outside [0, c_rows) are dropped (padding). */
     const void* c_scatter;
     int c_rows;
+    /* Grouped GEMM on CTA pairs, optional: device int32 per pair, block * 2 + 1 for a block on its own and block * 2 for
+     * one whose successor has the same expert and the same source rank, every live block in exactly one pair, in order;
+     * block_rot then counts pairs. Two blocks share their loads of B, so this pays where an expert has several blocks. */
+    const void* pair_block;
+    int num_pairs;
 } TdistGemmArgs;
 
 int tdist_gemm_run(const TdistGemmArgs* args);

@@ -116,6 +116,9 @@ struct GemmParams {
     unsigned long long* trace;  // optional timeline (see tdist.h), nullptr = off
     const int* expert_ids;      // grouped GEMM: expert (slice of B) of every 128-row block, nullptr = plain
     const int* num_m_blocks;    // grouped GEMM: device count of live 128-row blocks (rest is padding)
+    // Grouped GEMM on CTA pairs: row of tiles i is block pair_block[i] >> 1 and, unless bit 0 is set, the block after it,
+    // which has the same expert (and source rank). nullptr: one CTA per block.
+    const int* pair_block;
     // Row-gathering A operand (PLAIN, one CTA per tile): row r of the logical A is row a_gather[r] of the matrix
     // at a_raw ([a_gather_rows, K], K contiguous); indices >= a_gather_rows read as zeros. With block_src set,
     // the rows of 128-row block b come from rank block_src[b]'s segment of an all-gather in flight: the
@@ -134,7 +137,7 @@ struct GemmParams {
     uint32_t* gather_counter;   // 4 + blocks words, zero between launches: prologue arrivals, claim cursor, exits, per-block arrivals
     int gather_pro_blocks;      // blocks the prologue stages
     const int* block_rot;       // device scalar: block the schedule starts at (cyclic), nullptr = 0
-    // Scattering epilogue (PLAIN, one CTA per tile): row r of the product goes to row c_scatter[r] of c_out.
+    // Scattering epilogue (PLAIN, grouped): row r of the product goes to row c_scatter[r] of c_out.
     const int* c_scatter;
     char* c_out;
     int c_rows;
@@ -145,6 +148,17 @@ struct GemmParams {
 __device__ __forceinline__ int rotate_block(int i, int rot, int live) {
     int b = i + rot;
     return b >= live ? b - live : b;
+}
+
+// 128-row block of this CTA in a work item's row of tiles (inside its segment); -1: a pair's second CTA without a block.
+template <int CTAS>
+__device__ __forceinline__ int block_of(const GemmParams& p, int m_in_seg, int cta_rank, int rot, int live) {
+    if (CTAS == 2 && p.pair_block != nullptr) {
+        const int pb = p.pair_block[rotate_block(m_in_seg, rot, p.seg_m_tiles)];
+        return (cta_rank && (pb & 1)) ? -1 : (pb >> 1) + cta_rank;
+    }
+    const int block = m_in_seg * CTAS + cta_rank;
+    return CTAS == 1 && p.block_rot != nullptr ? rotate_block(block, rot, live) : block;
 }
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int src_bytes) {
@@ -748,11 +762,13 @@ __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : THREADS, 1) gemm_sm1
     }
 
     // ---------------- staged row gather (grouped GEMM): every CTA copies its share of the first wave's rows ----------------
-    constexpr bool STAGED = MODE == TDIST_GEMM_PLAIN && CTAS == 1 && !GATHER;
+    constexpr bool STAGED = MODE == TDIST_GEMM_PLAIN && !GATHER;
     int gather_live = 0, gather_rot = 0, gather_pro = 0;
     if (STAGED && p.gather_dst != nullptr) {
         gather_live = min(p.seg_blocks, p.num_m_blocks ? *p.num_m_blocks : p.seg_blocks);
-        gather_rot = p.block_rot ? min(max(*p.block_rot, 0), max(gather_live - 1, 0)) : 0;
+        gather_rot = p.block_rot ? max(*p.block_rot, 0) : 0;
+        if (CTAS == 2 && p.pair_block != nullptr) gather_rot = p.pair_block[min(gather_rot, p.seg_m_tiles - 1)] >> 1;
+        gather_rot = min(gather_rot, max(gather_live - 1, 0));
         gather_pro = gather_prologue_blocks(p, gather_live, gather_rot);
         if (gather_pro > 0) gather_prologue(p, gather_pro, gather_live, gather_rot);
     }
@@ -817,7 +833,7 @@ __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : THREADS, 1) gemm_sm1
         constexpr int LAG = 2;
         const int r = static_cast<int>(threadIdx.x) - THREADS;
         uint32_t it = 0, signaled = 0;
-        const int live_blocks = p.num_m_blocks ? *p.num_m_blocks : 0x7fffffff;
+        const int live_blocks = p.num_m_blocks && p.pair_block == nullptr ? *p.num_m_blocks : 0x7fffffff;
         auto drain = [&]() {
             cp_async_wait<0>();
             fence_proxy_async();
@@ -875,7 +891,7 @@ __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : THREADS, 1) gemm_sm1
         // ===================== B-only TMA producer of the gather variant ==========
         if (lane == 0) {
             uint32_t it = 0;
-            const int live_blocks = p.num_m_blocks ? *p.num_m_blocks : 0x7fffffff;
+            const int live_blocks = p.num_m_blocks && p.pair_block == nullptr ? *p.num_m_blocks : 0x7fffffff;
             for (int t = unit; t < p.num_tiles; t += num_units) {
                 const TileCoord tc = decode_tile(t, first_seg, p.world, p.seg_m_tiles, p.n_tiles, p.group_m);
                 const int block = tc.m_in_seg;
@@ -898,18 +914,18 @@ __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : THREADS, 1) gemm_sm1
             unsigned long long* tr = (p.trace != nullptr && cta < 64) ? p.trace + 1024 + cta * 4 : nullptr;
             unsigned long long waited = 0, blocked = 0;
             if (tr) tr[0] = globaltimer_ns();
-            const int live_blocks = p.num_m_blocks ? *p.num_m_blocks : 0x7fffffff;
+            const int live_blocks = p.num_m_blocks && p.pair_block == nullptr ? *p.num_m_blocks : 0x7fffffff;
             const int block_rot = p.block_rot ? min(max(*p.block_rot, 0), max(min(live_blocks, p.seg_m_tiles) - 1, 0)) : 0;
             Work tc;
             for (int round = 0; get_work<WIDE>(p, unit, num_units, round, first_seg, tc); ++round) {
                 if (tc.halves == 0 || tc.m_in_seg * CTAS >= live_blocks) continue;  // padding tile of a grouped GEMM: every role skips it
-                int block = tc.m_in_seg * CTAS + cta_rank;  // 128-row block inside the segment
-                if (MODE == TDIST_GEMM_PLAIN && CTAS == 1 && p.block_rot != nullptr)
-                    block = rotate_block(block, block_rot, min(live_blocks, p.seg_m_tiles));
-                const int bz = p.expert_ids ? p.expert_ids[block] : 0;
+                // 128-row block inside the segment; a pair's second CTA without one reads the zeros past the last row
+                const int located = block_of<CTAS>(p, tc.m_in_seg, cta_rank, block_rot, min(live_blocks, p.seg_m_tiles));
+                const int block = located < 0 ? p.seg_blocks : located;
+                const int bz = p.expert_ids ? p.expert_ids[CTAS == 2 ? block_of<CTAS>(p, tc.m_in_seg, 0, block_rot, 0) : block] : 0;
                 const CUtensorMap* am = &p.tm_a;
                 int az = tc.seg;
-                if (MODE == TDIST_GEMM_PLAIN && CTAS == 1 && p.block_ready != nullptr) {
+                if (MODE == TDIST_GEMM_PLAIN && p.block_ready != nullptr && located >= 0) {
                     // this block's rows have been staged (generic-proxy stores, read next by TMA)
                     wait_flag_ge_gpu(p.block_ready + block, p.epoch, p.wctx, -1, block, 7);
                     fence_proxy_async();
@@ -964,7 +980,7 @@ __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : THREADS, 1) gemm_sm1
             const uint32_t idesc = umma_idesc(p.is_f16 ? 0u : 1u, p.is_f16 ? 0u : 1u, BM * CTAS, BN);
             uint32_t it = 0;
             uint32_t uses0 = 0, uses1 = 0, next_narrow = 0;   // per-slot use counts give the barrier phases
-            const int live_blocks = p.num_m_blocks ? *p.num_m_blocks : 0x7fffffff;
+            const int live_blocks = p.num_m_blocks && p.pair_block == nullptr ? *p.num_m_blocks : 0x7fffffff;
             // optional timeline of the issuing thread: cycles in all, cycles waiting for operands, cycles waiting for the
             // epilogue to hand a TMEM slot back, tiles
             unsigned long long* mtr = (p.trace != nullptr && unit < 64) ? p.trace + 1536 + unit * 4 : nullptr;
@@ -1053,18 +1069,17 @@ __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : THREADS, 1) gemm_sm1
         // eight groups, i.e. the two younger tiles' four chunks each, are complete) costs nothing.
         uint32_t* pend0 = nullptr;   // older
         uint32_t* pend1 = nullptr;   // younger
-        const int live_blocks = p.num_m_blocks ? *p.num_m_blocks : 0x7fffffff;
+        const int live_blocks = p.num_m_blocks && p.pair_block == nullptr ? *p.num_m_blocks : 0x7fffffff;
         const int block_rot = p.block_rot ? min(max(*p.block_rot, 0), max(min(live_blocks, p.seg_m_tiles) - 1, 0)) : 0;
-        const bool scatter = MODE == TDIST_GEMM_PLAIN && CTAS == 1 && p.c_scatter != nullptr;
+        const bool scatter = MODE == TDIST_GEMM_PLAIN && p.c_scatter != nullptr;
         GatherCursor gcur{-1, 0};
         Work tc;
         for (int round = 0; get_work<WIDE>(p, unit, num_units, round, first_seg, tc); ++round) {
             if (tc.halves == 0 || tc.m_in_seg * CTAS >= live_blocks) continue;
             const CUtensorMap* cm = (MODE == TDIST_GEMM_RS) ? &p.tm_c[tc.seg] : &p.tm_c[0];
             const int cz = (MODE == TDIST_GEMM_RS) ? p.rank : tc.seg;
-            int block = tc.m_in_seg * CTAS + cta_rank;
-            if (MODE == TDIST_GEMM_PLAIN && CTAS == 1 && p.block_rot != nullptr)
-                block = rotate_block(block, block_rot, min(live_blocks, p.seg_m_tiles));
+            const int located = block_of<CTAS>(p, tc.m_in_seg, cta_rank, block_rot, min(live_blocks, p.seg_m_tiles));
+            const int block = located < 0 ? p.seg_blocks : located;   // none: nothing past the last row is stored
             const int row = block * BM;
             // scattering epilogue: the output row of this thread's row of the tile (-1 = padding, dropped)
             int out_row = -1;
@@ -1313,6 +1328,7 @@ using namespace tdist;
 using tdist_host::fail;
 
 static bool use_pair(const TdistGemmArgs* a) {
+    if (a->pair_block != nullptr) return true;   // the caller has paired the blocks of each expert
     if (a->expert_ids != nullptr || a->a_gather != nullptr || a->c_scatter != nullptr || a->block_rot != nullptr)
         return false;  // one expert / one source / one output row per 128-row block and thread
     if (a->cta_pair == 0) return false;
@@ -1323,7 +1339,8 @@ static bool use_pair(const TdistGemmArgs* a) {
 // The wide tiling pays when the main loop of a 256 x 512 tile is long against its epilogue, which only
 // overlaps the next tile half by half: from K = 4096 on, and only where a row of tiles has a pair to form.
 static bool use_wide(const TdistGemmArgs* a) {
-    if (!use_pair(a)) return false;
+    if (!use_pair(a) || a->pair_block != nullptr) return false;   // grouped: the longer main loop does not make up for
+    // the half-overlapped epilogue (4096 -> 1792 for 8192 tokens, top 2 of 8: 244 us wide, 216 us with single blocks)
     if (a->cta_pair == 2) return true;
     if (a->cta_pair == 1) return false;
     // RS: the epilogue of a wide tile stores 128 KB per CTA over NVLink with the MMAs of the next tile held up, so the
@@ -1475,7 +1492,7 @@ static GridPlan plan_grid(const TdistGemmArgs* a) {
     g.few_rows = false;
     g.ctas_per_tile = use_pair(a) ? 2 : 1;
     g.wide = use_wide(a) ? 1 : 0;
-    const int seg_m_tiles = (a->m_per_rank + BM * g.ctas_per_tile - 1) / (BM * g.ctas_per_tile);
+    const int seg_m_tiles = a->pair_block ? a->num_pairs : (a->m_per_rank + BM * g.ctas_per_tile - 1) / (BM * g.ctas_per_tile);
     const int n_tiles = (a->n + BN - 1) / BN;
     g.num_tiles = seg_m_tiles * (g.wide ? (n_tiles + 1) / 2 : n_tiles) * a->world;
     int capacity = resident_ctas(g.ctas_per_tile, g.wide, a->mode);
@@ -1584,8 +1601,10 @@ extern "C" int tdist_gemm_run(const TdistGemmArgs* a) {
     if ((a->gather_dst != nullptr) != (a->block_ready != nullptr) || (a->gather_dst != nullptr) != (a->gather_counter != nullptr) ||
         (a->gather_dst != nullptr && a->a_gather == nullptr))
         return fail(TDIST_EINVAL, "the staged row gather needs a_gather, gather_dst, block_ready and gather_counter together");
-    if ((a->c_scatter != nullptr || a->block_rot != nullptr) && (a->mode != TDIST_GEMM_PLAIN || a->world != 1 || a->cta_pair > 0))
-        return fail(TDIST_EINVAL, "c_scatter / block_rot are plain-mode, one-CTA-per-tile features");
+    if (a->pair_block != nullptr && (a->expert_ids == nullptr || a->num_pairs < 1 || (a->a_gather != nullptr && a->gather_dst == nullptr)))
+        return fail(TDIST_EINVAL, "paired blocks belong to a grouped GEMM whose rows are in place or staged");
+    if ((a->c_scatter != nullptr || a->block_rot != nullptr) && (a->mode != TDIST_GEMM_PLAIN || a->world != 1 || (a->cta_pair > 0 && a->pair_block == nullptr)))
+        return fail(TDIST_EINVAL, "c_scatter / block_rot are plain-mode features of one CTA per tile or paired blocks");
     if (a->a_gather != nullptr) {
         if (a->mode != TDIST_GEMM_PLAIN || a->world != 1) return fail(TDIST_EINVAL, "row-gathering A is a plain-mode feature (world = 1 in the GEMM's own terms)");
         if (a->a_gather_rows < 1) return fail(TDIST_EINVAL, "row-gathering A needs the number of source rows");
@@ -1661,8 +1680,9 @@ extern "C" int tdist_gemm_run(const TdistGemmArgs* a) {
         // the first wave of tiles: one tile per GEMM CTA, rows of tiles GROUP_M blocks deep
         const int gm = a->group_m > 0 ? a->group_m : DEFAULT_GROUP_M;
         const int n_tiles = (a->n + BN - 1) / BN;
-        const int first_wave = (plan.grid - plan.num_comm + n_tiles - 1) / n_tiles;
-        p.gather_pro_blocks = a->gather_counter != nullptr ? (first_wave + gm - 1) / gm * gm : 0;
+        const int per_row = plan.wide ? (n_tiles + 1) / 2 : n_tiles;
+        const int first_wave = ((plan.grid - plan.num_comm) / ctas + per_row - 1) / per_row;   // rows of tiles
+        p.gather_pro_blocks = a->gather_counter != nullptr ? (first_wave + gm - 1) / gm * gm * ctas : 0;
     }
     p.block_rot = static_cast<const int*>(a->block_rot);
     p.c_scatter = static_cast<const int*>(a->c_scatter);
@@ -1685,7 +1705,8 @@ extern "C" int tdist_gemm_run(const TdistGemmArgs* a) {
     p.world = a->world;
     p.rank = a->rank;
     p.seg_blocks = (a->m_per_rank + BM - 1) / BM;
-    p.seg_m_tiles = (a->m_per_rank + BM * ctas - 1) / (BM * ctas);
+    p.seg_m_tiles = a->pair_block ? a->num_pairs : (a->m_per_rank + BM * ctas - 1) / (BM * ctas);
+    p.pair_block = static_cast<const int*>(a->pair_block);
     p.n_tiles = (a->n + BN - 1) / BN;
     p.n_pairs = (p.n_tiles + 1) / 2;
     p.k_blocks = (a->k + BK - 1) / BK;
