@@ -241,3 +241,33 @@ def test_few_row_gemm_matches_fp32_reference(cuda_device, N, K, dtype):
         assert _lib.lib().tdist_gemm_plan(C.byref(g), out) == 0
         few += out[0] == 1 and out[3] % (-(-N // 128)) == 0
     assert few >= 8 or K < 1024   # the few-row kernel did run (with so short a K the large tiles are as good)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("activation", ["gelu", "silu", "relu"])
+@pytest.mark.parametrize("M,N,K", [(5, 264, 136), (100, 520, 4096), (300, 264, 136), (128, 1288, 8192)])
+def test_epilogue_activation_matches_fp32_reference(cuda_device, M, N, K, activation, dtype):
+    """Few-row and one-CTA kernels, and the pass of its own above 128 rows (two roundings there). Pre-activations reach +-40, far into both tails. Tolerance: the 16-bit
+    rounding of the result, and for gelu / silu fp32 sums whose error (1e-5 of their spread) the activation passes on."""
+    torch.manual_seed(M + N)
+    a, b = _rand((M, K), dtype, cuda_device, 8.0), _rand((N, K), dtype, cuda_device, K ** -0.5)
+    ctx = G.create_ag_gemm_intra_node_context(a, b, 0, 1, max_M=M)
+    h = a.double() @ b.double().t()
+    ref = {"gelu": lambda v: torch.nn.functional.gelu(v, approximate="tanh"), "silu": torch.nn.functional.silu,
+           "relu": torch.nn.functional.relu}[activation](h)
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for pair in (-1, 0, 1):
+        ctx.cta_pair = pair
+        out = G.ag_gemm_intra_node(a, b, ctx, activation=activation)
+        check_status()
+        torch.testing.assert_close(out.double(), ref, atol=2e-4 if M <= 128 and pair <= 0 else 40 * eps, rtol=2 * eps)
+
+
+def test_activation_of_a_nan_is_a_nan(cuda_device):
+    a = torch.ones(4, 64, dtype=torch.bfloat16, device=cuda_device)
+    a[1, 3] = float("nan")
+    b = torch.ones(8, 64, dtype=torch.bfloat16, device=cuda_device)
+    ctx = G.create_ag_gemm_intra_node_context(a, b, 0, 1, max_M=4)
+    for activation in ("gelu", "silu", "relu"):
+        out = G.ag_gemm_intra_node(a, b, ctx, activation=activation)
+        assert out[1].isnan().all() and not out[[0, 2, 3]].isnan().any()

@@ -190,3 +190,17 @@ def test_pair_blocks_keeps_experts_and_ranks_apart():
     assert pairs.block.tolist() == [0, 5, 6, 10, 14, 18, 22] and pairs.rot.tolist() == [5]
     assert MT.pair_blocks(torch.arange(6, dtype=torch.int32), torch.zeros(6, dtype=torch.int32), 6) is None
     assert MT.pair_blocks(experts, ranks, 0) is None
+
+
+@pytest.mark.parametrize("blocks,E,K,N", [(3, 2, 264, 520), (9, 4, 1024, 256)])
+def test_grouped_gemm_applies_silu_to_the_fp32_sums(cuda_device, blocks, E, K, N):
+    torch.manual_seed(blocks)
+    a = torch.randn(blocks * 128, K, device=cuda_device).mul_(4).to(torch.bfloat16)
+    b = (torch.randn(E, N, K, device=cuda_device) * K ** -0.5).to(torch.bfloat16)
+    experts = torch.randint(0, E, (blocks,), dtype=torch.int32, device=cuda_device)
+    out = MT.group_gemm(a, b, experts, activation="silu")
+    check_status()
+    for i in range(blocks):
+        blk = slice(128 * i, 128 * i + 128)
+        ref = torch.nn.functional.silu(a[blk].double() @ b[int(experts[i])].double().t())
+        torch.testing.assert_close(out[blk].double(), ref, atol=1e-4, rtol=2.0 ** -8)

@@ -59,7 +59,7 @@ class GemmArgs(C.Structure):
         ("src_epoch", C.c_uint64), ("src_rank", C.c_int), ("src_world", C.c_int),
         ("gather_dst", C.c_void_p), ("block_ready", C.c_void_p), ("gather_counter", C.c_void_p), ("block_rot", C.c_void_p),
         ("c_scatter", C.c_void_p), ("c_rows", C.c_int),
-        ("pair_block", C.c_void_p), ("num_pairs", C.c_int),
+        ("pair_block", C.c_void_p), ("num_pairs", C.c_int), ("act", C.c_int),
     ]
 
 
@@ -196,6 +196,7 @@ class PrimArgs(C.Structure):
  PRIM_FCOLLECT, PRIM_GRID_BARRIER, PRIM_SCOPED_OPS, PRIM_BARRIER, PRIM_BOUNDS_PROBE) = range(12)
 GEMM_PLAIN, GEMM_AG, GEMM_RS = 0, 1, 2
 A2A_DISPATCH, A2A_COMBINE = 0, 1
+ACTIVATIONS = {None: 0, "gelu": 1, "silu": 2, "relu": 3}   # TDIST_ACT_*
 DT_BF16, DT_F16, DT_F32, DT_I32 = 0, 1, 2, 3
 AG_PULL, AG_PUSH, AG_LL, AG_PUSH_ORDERED = 0, 1, 2, 3
 

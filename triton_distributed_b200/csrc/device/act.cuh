@@ -1,0 +1,24 @@
+// Activations of the GEMM epilogues, on the fp32 accumulator.
+#pragma once
+#include <cuda_runtime.h>
+
+#include "../include/tdist.h"
+
+namespace tdist {
+
+// GELU (tanh form) and SiLU are both v * sigmoid(z): one exponential and one division, and no cancellation where
+// 1 + tanh(z / 2) of the textbook form has one. Their error is a few fp32 ulps. (Two special-function results per value:
+// in the epilogue of a 256 x 512 tile, most of which is exposed, that costs more than a separate pass over the result:
+// m2048, 4096 -> 14336 -> 4096 with GELU 443 us fused, 428 us apart. So only the epilogues of memory-bound tiles apply them.)
+__device__ __forceinline__ float activate(float v, int act) {
+    if (act == TDIST_ACT_RELU) return v < 0.f ? 0.f : v;   // NaN stays NaN
+    const float z = act == TDIST_ACT_GELU ? 1.5957691216057308f * v * (1.f + 0.044715f * v * v) : v;
+    return v / (1.f + __expf(-z));
+}
+template <int N>
+__device__ __forceinline__ void activate(uint32_t (&r)[N], int act) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) r[i] = __float_as_uint(activate(__uint_as_float(r[i]), act));
+}
+
+}  // namespace tdist

@@ -33,6 +33,8 @@ int tdist_status_destroy(void* device_ptr);
 enum { TDIST_GEMM_PLAIN = 0, TDIST_GEMM_AG = 1, TDIST_GEMM_RS = 2 };
 enum { TDIST_BF16 = 0, TDIST_F16 = 1, TDIST_F32 = 2, TDIST_I32 = 3 };
 
+enum { TDIST_ACT_NONE = 0, TDIST_ACT_GELU = 1, TDIST_ACT_SILU = 2, TDIST_ACT_RELU = 3 };
+
 typedef struct TdistGemmArgs {
     /* A operand. PLAIN/RS: the whole local A, [world*m_per_rank, K] row-major (K contiguous).
      * AG: this rank's shard [m_per_rank, K]. */
@@ -122,6 +124,9 @@ typedef struct TdistGemmArgs {
      * block_rot then counts pairs. Two blocks share their loads of B, so this pays where an expert has several blocks. */
     const void* pair_block;
     int num_pairs;
+    /* PLAIN / AG with one rank, optional: applied to the fp32 accumulator before C is rounded (TDIST_ACT_*; GELU is the tanh
+     * form). Few-row products and one CTA per tile only (m_per_rank <= 128, or grouped without pair_block). */
+    int act;
 } TdistGemmArgs;
 
 int tdist_gemm_run(const TdistGemmArgs* args);

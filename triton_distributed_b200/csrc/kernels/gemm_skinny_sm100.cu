@@ -21,6 +21,7 @@
 #include <cstring>
 #include <mutex>
 
+#include "../device/act.cuh"
 #include "../device/ptx.cuh"
 #include "../device/signal.cuh"
 #include "../include/tdist.h"
@@ -47,7 +48,7 @@ struct Params {
     CUtensorMap tm_w;   // {K, N}, box {64, 128}
     CUtensorMap tm_x;   // {K, M}, box {64, tok}
     void* out;          // [M, N] bf16 / fp16
-    int m, n, k_blocks, tok, m_tiles, split, stages, is_f16, tmem_cols;
+    int m, n, k_blocks, tok, m_tiles, split, stages, is_f16, act, tmem_cols;
     WaitCtx wctx;
 };
 
@@ -177,6 +178,10 @@ __global__ void __launch_bounds__(THREADS, 2) gemm_skinny_kernel(const __grid_co
             acc.x += v.x;
             acc.y += v.y;
         }
+        if (p.act != TDIST_ACT_NONE) {
+            acc.x = activate(acc.x, p.act);
+            acc.y = activate(acc.y, p.act);
+        }
         const uint32_t w = p.is_f16 ? pack_f16x2(acc.x, acc.y) : pack_bf16x2(acc.x, acc.y);
         *reinterpret_cast<uint32_t*>(static_cast<char*>(p.out) + (static_cast<size_t>(m0 + t0 + t) * p.n + n0 + c) * 2) = w;
     }
@@ -298,6 +303,7 @@ int skinny_run(const TdistGemmArgs* a, const SkinnyPlan& plan) {
     p.split = plan.split;
     p.stages = plan.stages;
     p.is_f16 = a->dtype == TDIST_F16;
+    p.act = a->act;
     p.tmem_cols = plan.tok <= 32 ? 32 : (plan.tok <= 64 ? 64 : 128);
     p.wctx.status = static_cast<Status*>(a->status);
     p.wctx.timeout_ns = a->timeout_ns;

@@ -42,6 +42,7 @@
 #include <cstdlib>
 #include <string>
 
+#include "../device/act.cuh"
 #include "../device/ptx.cuh"
 #include "../device/signal.cuh"
 #include "../include/tdist.h"
@@ -111,6 +112,7 @@ struct GemmParams {
     uint32_t* push_count;       // [(world - 1) * seg_blocks] slice arrivals per (hop, block), zero between launches
     int group_m;
     int is_f16;
+    int act;                    // ACT kernels: TDIST_ACT_* the epilogue applies
     uint32_t epoch;
     int debug_delay_ns;
     unsigned long long* trace;  // optional timeline (see tdist.h), nullptr = off
@@ -734,7 +736,8 @@ __device__ __forceinline__ void rs_reduce_tile(const GemmParams& p, int block, i
 // GATHER (PLAIN, one CTA per tile): four extra warps (threads 192..319) copy the A rows by index with cp.async,
 // warp 0 then only issues the TMA loads of B.
 constexpr int GATHER_THREADS = THREADS + 128;
-template <int MODE, int CTAS, bool GATHER = false, bool WIDE = false>
+// ACT: the epilogue applies p.act. A kernel of its own: the branch alone slowed the others' epilogues (3 % of a grouped GEMM).
+template <int MODE, int CTAS, bool GATHER = false, bool WIDE = false, bool ACT = false>
 __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : THREADS, 1) gemm_sm100_kernel(const __grid_constant__ GemmParams p) {
     using T = Tiling<CTAS, WIDE>;
     static_assert(!(GATHER && WIDE), "the row-gathering producer feeds narrow tiles");
@@ -1129,6 +1132,10 @@ __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : THREADS, 1) gemm_sm1
                             else mbar_arrive_cluster(bar_tempty(buf), 0);
                         }
                     }
+                    if (ACT) {
+                        activate(r0, p.act);
+                        activate(r1, p.act);
+                    }
                     if (reduce_here) {
                         // every thread owns one row of the tile: add the 64 columns of every other rank's partial (fp32)
                         // and store the finished 128 bytes of the output row
@@ -1361,6 +1368,11 @@ static const void* kernel_for(int mode) {
         case TDIST_GEMM_AG: return reinterpret_cast<const void*>(&gemm_sm100_kernel<TDIST_GEMM_AG, CTAS, false, WIDE>);
         default: return reinterpret_cast<const void*>(&gemm_sm100_kernel<TDIST_GEMM_RS, CTAS, false, WIDE>);
     }
+}
+// with an activation in the epilogue: one CTA per tile, plain or AG
+static const void* act_kernel_of(int mode) {
+    return mode == TDIST_GEMM_AG ? reinterpret_cast<const void*>(&gemm_sm100_kernel<TDIST_GEMM_AG, 1, false, false, true>)
+                                 : reinterpret_cast<const void*>(&gemm_sm100_kernel<TDIST_GEMM_PLAIN, 1, false, false, true>);
 }
 static const void* kernel_of(int ctas, int wide, int mode) {
     if (ctas == 1) return kernel_for<1, false>(mode);
@@ -1596,6 +1608,8 @@ extern "C" int tdist_gemm_run(const TdistGemmArgs* a) {
     if (a->k % 8 != 0 || a->n % 8 != 0)
         return fail(TDIST_EINVAL, "K and N must be multiples of 8 (16-byte rows for TMA)");
     if (a->mode < TDIST_GEMM_PLAIN || a->mode > TDIST_GEMM_RS) return fail(TDIST_EINVAL, "bad mode");
+    if (a->act < TDIST_ACT_NONE || a->act > TDIST_ACT_RELU || (a->act != TDIST_ACT_NONE && (a->mode == TDIST_GEMM_RS || a->world != 1)))
+        return fail(TDIST_EINVAL, "unknown activation, or one on more than one rank");
     if (a->expert_ids != nullptr && (a->mode != TDIST_GEMM_PLAIN || a->world != 1))
         return fail(TDIST_EINVAL, "grouped GEMM (expert_ids) is a single-rank plain-mode feature");
     if ((a->gather_dst != nullptr) != (a->block_ready != nullptr) || (a->gather_dst != nullptr) != (a->gather_counter != nullptr) ||
@@ -1615,6 +1629,8 @@ extern "C" int tdist_gemm_run(const TdistGemmArgs* a) {
     const GridPlan plan = plan_grid(a);
     if (plan.few_rows) return tdist_host::skinny_run(a, plan.skinny);
     const int ctas = plan.ctas_per_tile;
+    if (a->act != TDIST_ACT_NONE && (ctas != 1 || (a->a_gather != nullptr && a->gather_dst == nullptr)))
+        return fail(TDIST_EINVAL, "an activation in the epilogue needs one CTA per tile");
     GemmParams p;
     memset(&p, 0, sizeof(p));
     const CUtensorMapDataType dt = a->dtype == TDIST_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -1711,6 +1727,7 @@ extern "C" int tdist_gemm_run(const TdistGemmArgs* a) {
     p.n_pairs = (p.n_tiles + 1) / 2;
     p.k_blocks = (a->k + BK - 1) / BK;
     p.is_f16 = a->dtype == TDIST_F16;
+    p.act = a->act;
     p.epoch = a->epoch;
     p.debug_delay_ns = a->debug_delay_ns;
     p.trace = static_cast<unsigned long long*>(a->trace);
@@ -1764,6 +1781,16 @@ extern "C" int tdist_gemm_run(const TdistGemmArgs* a) {
     cudaStream_t stream = static_cast<cudaStream_t>(a->stream);
     const void* fn = kernel_of(ctas, plan.wide, a->mode);  // smem opt-in done by resident_ctas()
     int block_threads = THREADS;
+    if (a->act != TDIST_ACT_NONE) {
+        fn = act_kernel_of(a->mode);
+        static bool attr_set[64][2] = {};
+        int dev = 0;
+        TDIST_CUDA_OK(cudaGetDevice(&dev));
+        if (dev >= 0 && dev < 64 && !attr_set[dev][a->mode == TDIST_GEMM_AG]) {
+            TDIST_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+            attr_set[dev][a->mode == TDIST_GEMM_AG] = true;
+        }
+    }
     if (a->a_gather != nullptr && a->gather_dst == nullptr) {
         fn = reinterpret_cast<const void*>(&gemm_sm100_kernel<TDIST_GEMM_PLAIN, 1, true>);
         block_threads = GATHER_THREADS;

@@ -15,7 +15,8 @@ class TPMLP:
     """Megatron-style tensor/sequence-parallel MLP over ``world`` ranks:
     ``y = reduce_scatter(act(allgather(x) @ W1_shard^T) @ W2_shard^T)``. ``x`` is this rank's
     ``[M/ws, hidden]`` token shard, ``w1`` ``[ffn/ws, hidden]``, ``w2`` ``[hidden, ffn/ws]``; the output
-    is this rank's ``[M/ws, hidden]`` rows. Two kernel launches: AG-GEMM and GEMM-RS (+ activation)."""
+    is this rank's ``[M/ws, hidden]`` rows. Two kernel launches: AG-GEMM and GEMM-RS (+ activation, where the
+    AG-GEMM does not apply it)."""
 
     def __init__(self, w1: torch.Tensor, w2: torch.Tensor, rank: int, world: int, max_M: int, activation: str = "gelu",
                  group=None, heap=None):
@@ -36,8 +37,11 @@ class TPMLP:
         return h
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        h = G.ag_gemm_intra_node(x, self.w1, self.ag_ctx)
-        return G.gemm_rs(self._act(h), self.w2, self.rs_ctx)
+        if getattr(self._act, "__func__", None) is TPMLP._act and self.activation in ("gelu", "silu", "relu"):
+            h = G.ag_gemm_intra_node(x, self.w1, self.ag_ctx, activation=self.activation)
+        else:   # an activation of the caller's own, or none
+            h = self._act(G.ag_gemm_intra_node(x, self.w1, self.ag_ctx))
+        return G.gemm_rs(h, self.w2, self.rs_ctx)
 
     __call__ = forward
 
@@ -50,7 +54,7 @@ class EPMoE:
     The dispatch kernel writes the received rows grouped by local expert with every group starting on a 128-row
     boundary, together with the expert of every 128-row block, so the receive buffer is the A operand of the
     grouped GEMM as it stands; the second GEMM writes into the symmetric buffer the combine kernels of the source
-    ranks read. Five launches (gate, dispatch, GEMM, activation, GEMM) + combine, no host synchronisation."""
+    ranks read. Four launches (gate, dispatch, GEMM + SiLU, GEMM) + combine, no host synchronisation."""
 
     def __init__(self, gate: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor, topk: int, rank: int, world: int, max_tokens: int,
                  group=None, heap=None):
@@ -63,8 +67,8 @@ class EPMoE:
 
     def experts(self, rows: torch.Tensor, out: torch.Tensor = None) -> torch.Tensor:
         """This rank's experts over the dispatched rows (``[capacity, hidden]``, block-aligned groups)."""
-        h = MT.group_gemm(rows, self.w1, self.ctx.block_expert, self.ctx.num_blocks)
-        return MT.group_gemm(F.silu(h), self.w2, self.ctx.block_expert, self.ctx.num_blocks, out=out)
+        h = MT.group_gemm(rows, self.w1, self.ctx.block_expert, self.ctx.num_blocks, activation="silu")
+        return MT.group_gemm(h, self.w2, self.ctx.block_expert, self.ctx.num_blocks, out=out)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         ids, w = MU.gate_topk(x, self.gate, self.topk, renormalize=True)

@@ -22,6 +22,7 @@ from typing import Optional
 
 import torch
 import torch.distributed as dist
+import torch.nn.functional as F
 
 from .. import _lib
 from ..utils.profile import nvtx_range
@@ -173,9 +174,10 @@ def create_ag_gemm_intra_node_context(tensor_A: torch.Tensor, tensor_B: torch.Te
 @nvtx_range("tdist.ag_gemm_intra_node")
 def ag_gemm_intra_node(a: torch.Tensor, b: torch.Tensor, ctx: Optional[AllGatherGEMMTensorParallelContext] = None,
                        rank: Optional[int] = None, num_ranks: Optional[int] = None, persistent: bool = True,
-                       out: Optional[torch.Tensor] = None) -> torch.Tensor:
+                       out: Optional[torch.Tensor] = None, activation: Optional[str] = None) -> torch.Tensor:
     """``allgather(a) @ b.T``: ``a`` is this rank's ``[M/ws, K]`` row shard, ``b`` this rank's
-    ``[N/ws, K]`` weight shard; returns ``[M, N/ws]``."""
+    ``[N/ws, K]`` weight shard; returns ``[M, N/ws]``. ``activation`` ("gelu" in its tanh form, "silu", "relu") is applied
+    to it: by the epilogue, on the fp32 sums, for the 128 rows of a decode step of one rank; as a pass of its own otherwise."""
     if ctx is None:
         if rank is None or num_ranks is None:
             raise ValueError("ag_gemm_intra_node needs a context or rank and num_ranks")
@@ -183,7 +185,7 @@ def ag_gemm_intra_node(a: torch.Tensor, b: torch.Tensor, ctx: Optional[AllGather
     mpr, K = a.shape
     N = b.shape[0]
     if a.device.type != "cuda":
-        return _ag_gemm_cpu(a, b, ctx)
+        return apply_activation(_ag_gemm_cpu(a, b, ctx), activation)
     _check_operands(a, b)
     if mpr > ctx.max_m_per_rank or K != ctx.k:
         raise ValueError(f"shard {tuple(a.shape)} exceeds the context (max rows {ctx.max_m_per_rank}, K {ctx.k})")
@@ -191,6 +193,9 @@ def ag_gemm_intra_node(a: torch.Tensor, b: torch.Tensor, ctx: Optional[AllGather
     g = _base_args(a, b, ctx.world, ctx.rank, _lib.GEMM_AG, cta_pair=ctx.cta_pair)
     g.c = c.data_ptr()
     g.m_per_rank = mpr
+    fused = activation is not None and ctx.world == 1 and mpr <= BLOCK_M_TILE and g.cta_pair <= 0
+    if fused:
+        g.act = _lib.ACTIVATIONS[activation]
     ctx.epoch += 1
     g.epoch = ctx.epoch
     g.num_sms = ctx.num_sms
@@ -210,7 +215,18 @@ def ag_gemm_intra_node(a: torch.Tensor, b: torch.Tensor, ctx: Optional[AllGather
         if ctx.workspace.mc is not None and (AG_NVLS == 2 or (AG_NVLS == 1 and ctx.world >= 4)):
             g.a_ws_mc = ctx.workspace.mc[half].data_ptr()   # the pushers multicast through the switch
     _launch(g)
+    if activation is not None and not fused:
+        act = apply_activation(c, activation)
+        return act if out is None else out.copy_(act)
     return c
+
+
+def apply_activation(h: torch.Tensor, activation: Optional[str]) -> torch.Tensor:
+    if activation is None:
+        return h
+    if activation == "gelu":
+        return F.gelu(h, approximate="tanh")
+    return {"silu": F.silu, "relu": F.relu}[activation](h)
 
 
 def _ag_gemm_cpu(a, b, ctx):

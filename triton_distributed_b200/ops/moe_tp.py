@@ -121,10 +121,11 @@ def topk_reduce(y: torch.Tensor, pos_of: torch.Tensor, weights: Optional[torch.T
 
 
 def group_gemm(a_sorted: torch.Tensor, b: torch.Tensor, expert_ids: torch.Tensor, num_blocks: Optional[torch.Tensor] = None,
-               out: Optional[torch.Tensor] = None) -> torch.Tensor:
+               out: Optional[torch.Tensor] = None, activation: Optional[str] = None) -> torch.Tensor:
     """``out[i*128:(i+1)*128] = a_sorted[i*128:(i+1)*128] @ b[expert_ids[i]].T`` for every live
     128-row block. ``a_sorted`` ``[blocks*128, K]``, ``b`` ``[E, N, K]`` (K contiguous), ``num_blocks``
-    an int32 device scalar (blocks past it are padding and are skipped)."""
+    an int32 device scalar (blocks past it are padding and are skipped). ``activation`` ("gelu" in its tanh form, "silu",
+    "relu") is applied to the fp32 sums by the epilogue."""
     rows, K = a_sorted.shape
     E, N, _ = b.shape
     if rows % GROUP_BLOCK_M:
@@ -135,7 +136,7 @@ def group_gemm(a_sorted: torch.Tensor, b: torch.Tensor, expert_ids: torch.Tensor
         for i in range(nb):
             blk = slice(i * GROUP_BLOCK_M, (i + 1) * GROUP_BLOCK_M)
             o[blk] = (a_sorted[blk].float() @ b[int(expert_ids[i])].float().t()).to(o.dtype)
-        return o
+        return G.apply_activation(o, activation)
     G._check_operands(a_sorted, b.view(E * N, K))
     c = out if out is not None else torch.empty((rows, N), dtype=a_sorted.dtype, device=a_sorted.device)
     g = G._base_args(a_sorted, b.view(E * N, K), 1, 0, _lib.GEMM_PLAIN)
@@ -146,6 +147,7 @@ def group_gemm(a_sorted: torch.Tensor, b: torch.Tensor, expert_ids: torch.Tensor
     g.expert_ids = expert_ids.data_ptr()
     g.num_m_blocks = num_blocks.data_ptr() if num_blocks is not None else None
     g.num_experts = E
+    g.act = _lib.ACTIVATIONS[activation]
     G._launch(g)
     return c
 
