@@ -281,3 +281,38 @@ def test_topk_reduce_over_ragged_rows_and_rejected_pairs(cuda_device, T, k, hidd
         ref = (rows * (weights.unsqueeze(-1) if weights is not None else 1.0)).sum(1)
         out = MT.topk_reduce(y, pos, weights, T, k)
         torch.testing.assert_close(out.float(), ref, rtol=2.0 ** -8, atol=1e-5)
+
+
+@pytest.mark.parametrize("T,topk,E", [(1, 1, 1), (31, 1, 8), (64, 8, 32), (513, 1, 16), (171, 3, 60), (1024, 8, 256), (300, 2, 1024)])
+@pytest.mark.parametrize("align", [1, 128])
+def test_dispatch_sorts_the_pairs_stably(cuda_device, T, topk, E, align):
+    """Rows land in stable expert order for pair counts around the 32 and 512 pairs the sort steps by, and up to the most
+    it routes in place; some pairs are rejected (id -1 and E)."""
+    from triton_distributed_b200.ops import moe_ep as EP
+    from triton_distributed_b200.runtime import global_status
+    torch.manual_seed(T + E)
+    x = torch.randn(T, 256, device=cuda_device).to(torch.bfloat16)
+    ids = torch.randint(0, E, (T, topk), dtype=torch.int32, device=cuda_device)
+    ctx = EP.create_ep_context(T, 256, topk, E, 0, 1, quant=False, compact=True, align=align, heap=LocalWorld(1, cuda_device).heap(0))
+    for bad in (False, True):
+        if bad and T > 30:
+            ids[3, 0], ids[T - 1, topk - 1] = -1, E
+        recv, _, splits, num = EP.ep_dispatch(ctx, x, ids, None)
+        torch.cuda.synchronize()
+        if bad and T > 30:
+            with pytest.raises(Exception, match="bad argument"):
+                global_status().check()
+        else:
+            check_status()
+        flat = ids.reshape(-1).long()
+        counts = torch.bincount(flat[(flat >= 0) & (flat < E)], minlength=E)
+        assert torch.equal(splits.view(-1).long(), counts) and int(num) == int(counts.sum())
+        padded = (counts + align - 1) // align * align
+        start = torch.cumsum(padded, 0) - padded
+        for e in range(E):
+            tokens = torch.nonzero(flat == e).flatten() // topk
+            assert torch.equal(recv[start[e]: start[e] + tokens.numel()], x[tokens])
+        blocks = int(padded.sum()) // align
+        assert int(ctx.num_blocks) == blocks
+        want = torch.repeat_interleave(torch.arange(E, device=cuda_device), padded // align)
+        assert torch.equal(ctx.block_expert[:blocks].long(), want)
