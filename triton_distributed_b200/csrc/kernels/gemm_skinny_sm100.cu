@@ -18,6 +18,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <cstring>
 #include <mutex>
 
@@ -168,22 +169,39 @@ __global__ void __launch_bounds__(THREADS, 2) gemm_skinny_kernel(const __grid_co
         tmem_dealloc<1>(tmem_base, static_cast<uint32_t>(p.tmem_cols));
     }
     const int t0 = part * per;
-    const int count = min(per, live - t0);   // tokens of this CTA's share (may be <= 0)
-    for (int i = static_cast<int>(threadIdx.x); i < count * (ROWS / 2); i += THREADS) {
-        const int t = i / (ROWS / 2), c = (i % (ROWS / 2)) * 2;
-        if (n0 + c >= p.n) continue;   // N is even: both columns or none
-        float2 acc = make_float2(0.f, 0.f);
+    const int items = min(per, live - t0) * (ROWS / 4);   // 4 columns of a token each; this CTA's share may be empty
+    constexpr int UNROLL = 4;   // items per thread and step: their loads of one source part are in flight together
+    for (int i0 = static_cast<int>(threadIdx.x); i0 < items; i0 += UNROLL * THREADS) {
+        float4 acc[UNROLL];
+#pragma unroll
+        for (int u = 0; u < UNROLL; ++u) acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
         for (int s = 0; s < p.split; ++s) {
-            const float2 v = *reinterpret_cast<const float2*>(sums + (s * per + t) * ROWS + c);
-            acc.x += v.x;
-            acc.y += v.y;
+            const float4* src = reinterpret_cast<const float4*>(sums + s * per * ROWS);
+#pragma unroll
+            for (int u = 0; u < UNROLL; ++u) {
+                if (i0 + u * THREADS >= items) continue;
+                const float4 v = src[i0 + u * THREADS];
+                acc[u].x += v.x;
+                acc[u].y += v.y;
+                acc[u].z += v.z;
+                acc[u].w += v.w;
+            }
         }
-        if (p.act != TDIST_ACT_NONE) {
-            acc.x = activate(acc.x, p.act);
-            acc.y = activate(acc.y, p.act);
+#pragma unroll
+        for (int u = 0; u < UNROLL; ++u) {
+            const int i = i0 + u * THREADS;
+            const int t = i / (ROWS / 4), c = (i % (ROWS / 4)) * 4;
+            if (i >= items || n0 + c >= p.n) continue;   // N is a multiple of 8: all four columns or none
+            float4 v = acc[u];
+            if (p.act != TDIST_ACT_NONE) {
+                v.x = activate(v.x, p.act);
+                v.y = activate(v.y, p.act);
+                v.z = activate(v.z, p.act);
+                v.w = activate(v.w, p.act);
+            }
+            const uint2 w = p.is_f16 ? make_uint2(pack_f16x2(v.x, v.y), pack_f16x2(v.z, v.w)) : make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
+            *reinterpret_cast<uint2*>(static_cast<char*>(p.out) + (static_cast<size_t>(m0 + t0 + t) * p.n + n0 + c) * 2) = w;
         }
-        const uint32_t w = p.is_f16 ? pack_f16x2(acc.x, acc.y) : pack_bf16x2(acc.x, acc.y);
-        *reinterpret_cast<uint32_t*>(static_cast<char*>(p.out) + (static_cast<size_t>(m0 + t0 + t) * p.n + n0 + c) * 2) = w;
     }
 }
 
@@ -195,8 +213,9 @@ using tdist_host::fail;
 
 namespace {
 
-// CTAs of the kernel that are resident at once when they come in clusters of `split` (a cluster needs its SMs in one
-// GPC, so sizes that do not divide a GPC leave some unused). Cached per device.
+// CTAs of the kernel that are resident at once when they come in clusters of `split` (a cluster needs its SMs in one GPC,
+// so sizes that do not divide a GPC leave some unused). The occupancy query counts one CTA per SM here whatever the
+// carveout; two do run (clusters of four, n6144 k12288: 192 CTAs finish sooner than 144 in clusters of three). Cached per device.
 int skinny_slots(int split) {
     using namespace tdist::skinny;
     static int cache[64][MAX_SPLIT + 1] = {};
@@ -226,7 +245,7 @@ int skinny_slots(int split) {
     cfg.numAttrs = 1;
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) == cudaSuccess &&
         cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) == cudaSuccess && clusters > 0)
-        slot = clusters * split;
+        slot = clusters * split <= tdist_host::sm_count() ? 2 * clusters * split : clusters * split;
     else
         slot = nominal;
     cudaGetLastError();
@@ -245,21 +264,26 @@ bool skinny_plan(int m, int n, int k, double other_s, SkinnyPlan* plan) {
     const int n_tiles = (n + ROWS - 1) / ROWS;
     const int k_blocks = (k + BK - 1) / BK;
     const int tiles = n_tiles * m_tiles;
-    // Model of a run: an SM takes 64 bytes per clock from L2 whichever of its two CTAs asks; HBM delivers 6.3 TB/s; a
-    // launch costs 4 us beside its loads (prologue, first loads, exchange), and a larger cluster starts and meets later.
-    const double block_s = (W_BYTES + tok * BK * 2) / 64.0 / 1.8e9;
-    const double hbm_s = 2.0 * (static_cast<double>(n) * k + static_cast<double>(m) * (k + n)) / 6.3e12;
+    // Model of a run, fitted to sweeps over M 1..512, N 256..49152, K 1024..16384 and every split: a CTA moves 70 GB/s
+    // whatever its tile (twice the stages on a CTA that has its SM to itself changed nothing), HBM delivers 6.4 TB/s and
+    // the two bend into one another; launch, first loads and the exchange of the partial sums cost 5.3 us and 15-50 ns per
+    // token of the tile, the most where two CTAs share an SM; half of that again for every further round. Chosen splits are within 8 % of the best one measured
+    // (m16 n14336 k4096: 2, 24 us; 3, which needs a second wave, 29 us; 1, 27 us).
+    const double stage = W_BYTES + tok * BK * 2;
+    const double hbm_s = 2.0 * (static_cast<double>(n) * k + static_cast<double>(m) * (k + n)) / 6.4e12;
+    const int sms = tdist_host::sm_count();
     double best = 1e30;
     int best_split = 1;
     for (int split = 1; split <= MAX_SPLIT; ++split) {
-        if (split > 1 && k_blocks < 4 * split) break;   // a part shorter than the pipeline only adds partial sums
+        if (split > 1 && k_blocks < 3 * split) break;   // a part shorter than the pipeline only adds partial sums
         const int slots = skinny_slots(split);
         const int ctas = tiles * split;
-        const int full = ctas / slots, rest = ctas - full * slots;
         const int blocks = (k_blocks + split - 1) / split;
-        const double rounds = 2.0 * full + (rest == 0 ? 0.0 : (2 * rest <= slots ? 1.0 : 2.0));
-        const double sm_s = rounds * blocks * block_s;
-        const double t = (sm_s > hbm_s ? sm_s : hbm_s) + 4e-6 + 0.2e-6 * split;
+        const int rounds = (ctas + slots - 1) / slots;
+        const double sm_s = rounds * blocks * stage / 70e9;
+        const double loads = std::pow(std::pow(sm_s * 1e6, 6) + std::pow(hbm_s * 1e6, 6), 1.0 / 6) * 1e-6;
+        const double fixed = 5.3e-6 + tok * (15e-9 + 16e-9 / split + (ctas > sms ? 20e-9 : 0.0)) + 0.05e-6 * split;
+        const double t = loads + fixed * (1 + 0.5 * (rounds - 1));
         if (t < best) {
             best = t;
             best_split = split;
