@@ -143,3 +143,32 @@ def test_sequence_parallel_decode_with_device_call_number(cuda_device, world, B,
     done = 4 + (1 if graph else 0)
     for r in range(world):
         assert int(ctxs[r].epoch_dev[0]) == done and int(ctxs[r].epoch_dev[1]) == 0
+
+
+@pytest.mark.parametrize("splits", [1, 2, 3, 4, 5, 7, 8, 9, 12])
+@pytest.mark.parametrize("Hq,Hkv,D", [(32, 8, 128), (16, 16, 64), (16, 1, 256), (64, 4, 128)])
+def test_splits_meet_in_the_ring_or_in_global_memory(cuda_device, splits, Hq, Hkv, D):
+    """Partials of up to eight splits land in the ring of the cluster's first CTA while that is still merging its warps;
+    with 16 heads per kv head and eight splits they no longer fit and go through global memory. Ragged, empty and
+    one-key sequences."""
+    torch.manual_seed(splits + D)
+    lens = [3000, 0, 1, 17, 1024]
+    B, page, per = len(lens), 16, -(-3000 // 16)
+    k = torch.randn(B * per, page, Hkv, D, device=cuda_device).to(torch.bfloat16)
+    v = torch.randn(B * per, page, Hkv, D, device=cuda_device).to(torch.bfloat16)
+    q = torch.randn(B, Hq, D, device=cuda_device).to(torch.bfloat16)
+    table = torch.randperm(B * per, device=cuda_device).to(torch.int32).view(B, per)
+    kv = torch.tensor(lens, dtype=torch.int32, device=cuda_device)
+    ref = FD.ref_paged_attn(q, k, v, kv, table, D ** -0.5)
+    for _ in range(3):
+        out = FD.gqa_fwd_batch_decode(q, k, v, None, None, kv, table, D ** -0.5, kv_split=splits)
+        check_status()
+        torch.testing.assert_close(out.float(), ref, atol=2e-2, rtol=2e-2)
+
+
+def test_batch_splits_fill_the_last_wave_and_even_out_lengths():
+    assert FD._batch_splits(32 * 8, 8192, 128, 148, 1) == 2        # ragged batches gain, full ones lose next to nothing
+    assert FD._batch_splits(8 * 8, 32768, 128, 148, 4) == 4        # one wave of 256 CTAs is hard to beat
+    assert FD._batch_splits(48 * 8, 4096, 128, 148, 1) == 2        # 384 CTAs are 1.3 waves, 768 are 2.6
+    assert FD._batch_splits(64 * 8, 512, 128, 148, 1) == 1         # short sequences: the fixed cost decides
+    assert FD._batch_splits(16 * 8, 1024, 128, 148, 2) == 2

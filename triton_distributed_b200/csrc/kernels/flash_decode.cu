@@ -148,15 +148,6 @@ __global__ void __launch_bounds__(kDecodeThreads, (D <= 128 ? 2 : 1)) flash_deco
     const T* vc = static_cast<const T*>(p.v_cache) + static_cast<size_t>(kvh) * p.stride_head;
     const int* table = p.block_table + static_cast<size_t>(b) * p.max_blocks;
 
-    // ---- Q tile into shared memory (rows >= G are zero)
-    for (int c = tid; c < 16 * CH; c += kDecodeThreads) {
-        const int row = c / CH, ch = c % CH;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (row < G) v = *reinterpret_cast<const uint4*>(q + static_cast<size_t>(row) * D + ch * 8);
-        *reinterpret_cast<uint4*>(q_s + tile_off<D>(row, ch)) = v;
-    }
-    __syncthreads();
-
     // ---- this CTA's KV range, in 16-token blocks dealt round-robin to the warps
     const int kv_len = p.kv_lens[b];
     const int nblk_total = (kv_len + kTok - 1) / kTok;
@@ -195,12 +186,6 @@ __global__ void __launch_bounds__(kDecodeThreads, (D <= 128 ? 2 : 1)) flash_deco
         }
     };
 
-    float o[NT][4];
-#pragma unroll
-    for (int i = 0; i < NT; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-    float m_run[2] = {-CUDART_INF_F, -CUDART_INF_F}, l_run[2] = {0.f, 0.f};
-    const float sl2 = p.scale * 1.4426950408889634f;
-
     long long base_next = lookup(0);
     for (int i = 0; i < NS - 1; ++i) {
         const long long base = base_next;
@@ -208,6 +193,21 @@ __global__ void __launch_bounds__(kDecodeThreads, (D <= 128 ? 2 : 1)) flash_deco
         if (i < my_blocks) issue(i, base);
         cp_async_commit();
     }
+    // ---- Q tile into shared memory (rows >= G are zero), under the first K / V loads
+    for (int c = tid; c < 16 * CH; c += kDecodeThreads) {
+        const int row = c / CH, ch = c % CH;
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (row < G) v = *reinterpret_cast<const uint4*>(q + static_cast<size_t>(row) * D + ch * 8);
+        *reinterpret_cast<uint4*>(q_s + tile_off<D>(row, ch)) = v;
+    }
+    __syncthreads();
+
+    float o[NT][4];
+#pragma unroll
+    for (int i = 0; i < NT; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+    float m_run[2] = {-CUDART_INF_F, -CUDART_INF_F}, l_run[2] = {0.f, 0.f};
+    const float sl2 = p.scale * 1.4426950408889634f;
+
     for (int i = 0; i < my_blocks; ++i) {
         if (i + NS - 1 < my_blocks) {
             const long long base = base_next;
@@ -310,11 +310,18 @@ __global__ void __launch_bounds__(kDecodeThreads, (D <= 128 ? 2 : 1)) flash_deco
             *reinterpret_cast<float2*>(base + static_cast<size_t>(r0 + 8) * D + col) = make_float2(o[nt][2], o[nt][3]);
         }
     }
-    __syncthreads();
     const int W2 = D + 2;  // floats per head in the workspace and in the gather buffers: O, LSE, pad
-    // cluster merge: the partials of all splits land behind the ring of the cluster's first CTA
-    float* part_s = reinterpret_cast<float*>(ring + static_cast<size_t>(kDecodeWarps) * NS * 2 * TILE);
+    // cluster merge: the partials of all splits land in the ring of the cluster's first CTA, behind the results of that
+    // CTA's warps (shared memory of their own would leave room for one CTA per SM instead of two), so every CTA of the
+    // cluster has to be done with its ring first
+    float* part_s = o_s + kDecodeWarps * 16 * D;
     const uint32_t part_leader = p.cluster_merge ? mapa_u32(smem_u32(part_s), 0) : 0u;
+    if (p.cluster_merge) {
+        cluster_arrive();
+        cluster_wait();
+    } else {
+        __syncthreads();
+    }
     for (int idx = tid; idx < G * D; idx += kDecodeThreads) {
         const int g = idx / D, c = idx % D;
         float mm = -CUDART_INF_F;
@@ -525,20 +532,20 @@ __global__ void lse_combine_kernel(const float* parts, int R, int heads, int D, 
 using namespace tdist;
 using tdist_host::fail;
 
-// Largest cluster (splits of one (batch, kv head)) the merge through shared memory is used for, and the bytes it may add
-// to a CTA's shared memory. Above either limit the splits meet in global memory (workspace + arrival counter).
+// Largest cluster (splits of one (batch, kv head)) the merge through shared memory is used for. Above it, or when the
+// partials do not fit the ring, the splits meet in global memory (workspace + arrival counter).
 // Eight is the portable cluster size; 16-CTA clusters were measured and dropped: with 133 KB of shared memory per CTA
 // only some of them are resident at once (batch 1, 8 kv heads, 16384 keys, 16 splits: 37.1 us against 22.6 us through
 // global memory). Up to eight splits the cluster form is 5-10 % faster (4096 keys: 14.4 / 20.6 us against 15.4 / 22.6 us
 // with 8 / 4 splits).
 constexpr int kClusterMergeMaxSplits = 8;
-constexpr int kClusterMergeMaxBytes = 48 * 1024;
 
 template <typename T, int D>
 static int launch_decode(DecodeParams& p, cudaStream_t stream) {
     constexpr int NS = decode_stages(D);
     constexpr int smem = kTok * D * 2 + kDecodeWarps * NS * 2 * kTok * D * 2;
-    static_assert(smem >= kDecodeWarps * 16 * D * 4, "the warp-merge buffer reuses the ring");
+    constexpr int part_room = kDecodeWarps * NS * 2 * kTok * D * 2 - kDecodeWarps * 16 * D * 4;   // ring behind the warps' results
+    static_assert(part_room > 0, "the warp-merge buffer reuses the ring");
     static bool done[64] = {};
     static std::mutex setup_lock;
     static const bool cluster_enabled = [] {
@@ -551,19 +558,19 @@ static int launch_decode(DecodeParams& p, cudaStream_t stream) {
     {
         std::lock_guard<std::mutex> guard(setup_lock);
         if (!done[dev]) {
-            TDIST_CUDA_OK(cudaFuncSetAttribute(flash_decode_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem + kClusterMergeMaxBytes));
+            TDIST_CUDA_OK(cudaFuncSetAttribute(flash_decode_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
             done[dev] = true;
         }
     }
     const int G = p.Hq / p.Hkv;
     const int part_bytes = G * p.splits * (D + 2) * static_cast<int>(sizeof(float));
-    const bool cluster = cluster_enabled && p.splits >= 2 && p.splits <= kClusterMergeMaxSplits && part_bytes <= kClusterMergeMaxBytes;
+    const bool cluster = cluster_enabled && p.splits >= 2 && p.splits <= kClusterMergeMaxSplits && part_bytes <= part_room;
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(static_cast<unsigned>(p.B * p.Hkv * p.splits));
     cfg.blockDim = dim3(kDecodeThreads);
     cfg.stream = stream;
-    cfg.dynamicSmemBytes = cluster ? smem + part_bytes : smem;
+    cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute attr[1];
     if (cluster) {
         attr[0].id = cudaLaunchAttributeClusterDimension;
