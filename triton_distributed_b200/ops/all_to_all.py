@@ -25,7 +25,7 @@ import torch.distributed as dist
 
 from .. import _lib
 from ..utils.profile import nvtx_range
-from ..runtime import SymmTensor, default_timeout_ns, global_status, symm_heap
+from ..runtime import SymmTensor, default_timeout_ns, global_status, stream_ptr, symm_heap
 from . import moe_utils
 
 launch_count = 0
@@ -84,7 +84,7 @@ def _fill_common(a: "_lib.A2AArgs", ctx: AllToAllContext, half: int, phase: int,
     st = global_status()
     a.status = st.device_ptr if st is not None else None
     a.timeout_ns = default_timeout_ns()
-    a.stream = (stream or torch.cuda.current_stream(device)).cuda_stream
+    a.stream = stream_ptr(device, stream)
 
 
 def _next_call(ctx: AllToAllContext, phase: int) -> int:
@@ -256,7 +256,7 @@ def dequant_fp8(x: torch.Tensor, scale: torch.Tensor, rows: Optional[int] = None
     if out is None:
         out = torch.empty((x.shape[0], hidden), dtype=torch.bfloat16, device=x.device)
     _lib.check(_lib.lib().tdist_dequant_fp8(x.data_ptr(), scale.data_ptr(), out.data_ptr(), R, hidden,
-                                            torch.cuda.current_stream(x.device).cuda_stream), "tdist_dequant_fp8")
+                                            stream_ptr(x.device)), "tdist_dequant_fp8")
     launch_count += 1
     return out
 

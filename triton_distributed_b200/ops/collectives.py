@@ -27,7 +27,7 @@ import torch.distributed as dist
 
 from .. import _lib
 from ..utils.profile import nvtx_range
-from ..runtime import SymmTensor, default_timeout_ns, global_status, symm_heap
+from ..runtime import SymmTensor, default_timeout_ns, global_status, stream_ptr, symm_heap
 
 launch_count = 0
 
@@ -48,7 +48,7 @@ def _status_ptr():
 
 
 def _stream_ptr(device, stream=None):
-    return (stream or torch.cuda.current_stream(device)).cuda_stream
+    return stream_ptr(device, stream)
 
 
 # ---------------------------------------------------------------------------- barrier / flags

@@ -29,7 +29,7 @@ import torch.distributed as dist
 
 from .. import _lib
 from ..utils.profile import nvtx_range
-from ..runtime import SymmTensor, default_timeout_ns, global_status, symm_heap
+from ..runtime import SymmTensor, default_timeout_ns, global_status, stream_ptr, symm_heap
 
 launch_count = 0
 _DTYPES = {torch.bfloat16: _lib.DT_BF16, torch.float16: _lib.DT_F16}
@@ -185,7 +185,7 @@ def _launch(q, k_cache, v_cache, kv_lens, block_table, scale, soft_cap, out, mod
     st = global_status()
     a.status = st.device_ptr if st is not None else None
     a.timeout_ns = default_timeout_ns()
-    a.stream = (stream or torch.cuda.current_stream(q.device)).cuda_stream
+    a.stream = stream_ptr(q.device, stream)
     if stream is not None:
         # copies made on the current stream are read on `stream`: order the two, and keep the allocator from
         # handing the copies' memory out again before `stream` is done with them
@@ -263,7 +263,7 @@ def inter_rank_combine(partials: torch.Tensor, out_dtype=torch.bfloat16, out: Op
     parts = partials.float().contiguous()
     o = out if out is not None else torch.empty((B, Hq, D), dtype=out_dtype, device=partials.device)
     _lib.check(_lib.lib().tdist_lse_combine(parts.data_ptr(), R, B * Hq, D, o.data_ptr(), _DTYPES[o.dtype],
-                                            torch.cuda.current_stream(parts.device).cuda_stream), "tdist_lse_combine")
+                                            stream_ptr(parts.device)), "tdist_lse_combine")
     launch_count += 1
     return o
 

@@ -26,7 +26,7 @@ import torch.nn.functional as F
 
 from .. import _lib
 from ..utils.profile import nvtx_range
-from ..runtime import SymmTensor, counters_clean, default_timeout_ns, global_status, symm_heap
+from ..runtime import SymmTensor, counters_clean, default_timeout_ns, global_status, stream_ptr, symm_heap
 
 BLOCK_M = 128
 BLOCK_N = 256
@@ -84,7 +84,7 @@ def _base_args(a, b, world, rank, mode, stream=None, cta_pair: int = -1) -> "_li
     g.group_m = GROUP_M
     if TRACE is not None:
         g.trace = TRACE.data_ptr()
-    g.stream = (stream or torch.cuda.current_stream(a.device)).cuda_stream
+    g.stream = stream_ptr(a.device, stream)
     return g
 
 

@@ -27,7 +27,7 @@ import torch.distributed as dist
 from .. import _lib
 from ..utils.misc import plain_cuda
 from ..utils.profile import nvtx_range
-from ..runtime import SymmTensor, default_timeout_ns, global_status, symm_heap
+from ..runtime import SymmTensor, default_timeout_ns, global_status, stream_ptr, symm_heap
 
 FP8 = torch.float8_e4m3fn
 FP8_MAX = 448.0
@@ -49,7 +49,7 @@ def quantize_fp8_rowwise(x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
         q = torch.empty((M, K), dtype=FP8, device=x.device)
         scale = torch.empty((M, K // 128), dtype=torch.float32, device=x.device)
         _lib.check(_lib.lib().tdist_quant_fp8_rowwise(x.data_ptr(), q.data_ptr(), scale.data_ptr(), M, K, _QUANT_DTYPES[x.dtype],
-                                                      torch.cuda.current_stream(x.device).cuda_stream), "tdist_quant_fp8_rowwise")
+                                                      stream_ptr(x.device)), "tdist_quant_fp8_rowwise")
         return q, scale
     return _quantize_rowwise_torch(x)
 
@@ -115,7 +115,7 @@ def _base(a, sa, b, sb, world, rank, mode) -> "_lib.GemmFp8Args":
     st = global_status()
     g.status = st.device_ptr if st is not None else None
     g.timeout_ns = default_timeout_ns()
-    g.stream = torch.cuda.current_stream(a.device).cuda_stream
+    g.stream = stream_ptr(a.device)
     return g
 
 

@@ -31,7 +31,7 @@ import torch
 import torch.distributed as dist
 
 from .. import _lib
-from ..runtime import SymmTensor, default_timeout_ns, global_status, symm_heap
+from ..runtime import SymmTensor, default_timeout_ns, global_status, stream_ptr, symm_heap
 from ..utils.profile import nvtx_range
 from . import moe_utils
 
@@ -73,6 +73,8 @@ class EPContext:
     topk_ids: Optional[torch.Tensor] = None
     topk_weights: Optional[torch.Tensor] = None
     num_ctas: int = 0
+    # what the launch arguments of this context have in common, per call parity: [dispatch, combine]
+    templates: Optional[list] = None
 
     @property
     def experts_per_rank(self) -> int:
@@ -115,7 +117,37 @@ def create_ep_context(max_tokens: int, hidden: int, topk: int, num_experts: int,
         ctx.num_recv = torch.zeros(1, dtype=torch.int32, device=dev)
         ctx.block_expert = torch.zeros(max(1, rows // max(1, align)), dtype=torch.int32, device=dev)
         ctx.num_blocks = torch.zeros(1, dtype=torch.int32, device=dev)
+        ctx.templates = [(_dispatch_template(ctx, h), _combine_template(ctx, h)) for h in range(2)]
     return ctx
+
+
+def _dispatch_template(ctx: EPContext, half: int) -> "_lib.MoeDispatchArgs":
+    a = _lib.MoeDispatchArgs()
+    a.recv_peer = ctx.recv_buf.half_ptr_arrays()[half]
+    if ctx.quant:
+        a.scale_peer = ctx.scale_buf.half_ptr_arrays()[half]
+    a.counts_peer = ctx.counts_buf.half_ptr_arrays()[half]
+    a.sig_peer = ctx.sig.cached_ptr_array()
+    a.counters = ctx.counters.data_ptr()
+    a.pair_row, a.send_splits = ctx.pair_row.data_ptr(), ctx.send_splits.data_ptr()
+    a.recv_splits, a.recv_offset = ctx.recv_splits.data_ptr(), ctx.recv_offset.data_ptr()
+    a.num_recv = ctx.num_recv.data_ptr()
+    if ctx.compact:
+        a.block_expert, a.num_blocks = ctx.block_expert.data_ptr(), ctx.num_blocks.data_ptr()
+    a.topk, a.hidden, a.num_experts = ctx.topk, ctx.hidden, ctx.num_experts
+    a.world, a.rank = ctx.world, ctx.rank
+    a.max_m, a.quant, a.compact, a.align = ctx.max_m, int(ctx.quant), int(ctx.compact), ctx.align
+    return a
+
+
+def _combine_template(ctx: EPContext, half: int) -> "_lib.MoeCombineArgs":
+    a = _lib.MoeCombineArgs()
+    a.buf_peer = ctx.out_buf.half_ptr_arrays()[half]
+    a.sig_peer = ctx.comb_sig.cached_ptr_array()
+    a.pair_row = ctx.pair_row.data_ptr()
+    a.topk, a.hidden, a.epr = ctx.topk, ctx.hidden, ctx.experts_per_rank
+    a.world, a.rank = ctx.world, ctx.rank
+    return a
 
 
 @nvtx_range("tdist.ep_dispatch")
@@ -145,34 +177,21 @@ def ep_dispatch(ctx: EPContext, x: torch.Tensor, topk_ids: torch.Tensor, topk_we
         ctx.topk_weights = None if topk_weights is None else topk_weights.to(torch.float32).contiguous()
         ctx.ntok = T
     half = ctx.call_count & 1
-    a = _lib.MoeDispatchArgs()
+    a = _lib.MoeDispatchArgs.from_buffer_copy(ctx.templates[half][0])
     a.x, a.topk_ids = x.data_ptr(), ctx.topk_ids.data_ptr()
     routed = None
     if T * ctx.topk > ROUTE_IN_PLACE_MAX:
         routed = moe_utils.route(ctx.topk_ids, ctx.num_experts)     # large batches: routing as a launch of its own
         a.slot_of, a.cumsum = routed.slot_of.data_ptr(), routed.cumsum.data_ptr()
-    a.recv_peer = ctx.recv_buf.half_ptr_arrays()[half]
-    if ctx.quant:
-        a.scale_peer = ctx.scale_buf.half_ptr_arrays()[half]
-    a.counts_peer = ctx.counts_buf.half_ptr_arrays()[half]
-    a.sig_peer = ctx.sig.cached_ptr_array()
-    a.counters = ctx.counters.data_ptr()
-    a.pair_row, a.send_splits = ctx.pair_row.data_ptr(), ctx.send_splits.data_ptr()
-    a.recv_splits, a.recv_offset = ctx.recv_splits.data_ptr(), ctx.recv_offset.data_ptr()
-    a.num_recv = ctx.num_recv.data_ptr()
-    if ctx.compact:
-        a.block_expert, a.num_blocks = ctx.block_expert.data_ptr(), ctx.num_blocks.data_ptr()
-    a.ntok, a.topk, a.hidden, a.num_experts = T, ctx.topk, ctx.hidden, ctx.num_experts
-    a.world, a.rank = ctx.world, ctx.rank
-    a.max_m, a.quant, a.compact, a.align = ctx.max_m, int(ctx.quant), int(ctx.compact), ctx.align
+    a.ntok = T
     a.phase, a.num_ctas, a.epoch = phase, ctx.num_ctas, ctx.call_count
     st = global_status()
     a.status = st.device_ptr if st is not None else None
     a.timeout_ns = default_timeout_ns()
-    a.stream = (stream or torch.cuda.current_stream(x.device)).cuda_stream
+    a.stream = stream_ptr(x.device, stream)
     _lib.check(_lib.lib().tdist_moe_dispatch(C.byref(a)), "tdist_moe_dispatch")
     launch_count += 1
-    return (ctx.recv_buf.local[half], ctx.scale_buf.local[half] if ctx.quant else None, ctx.recv_splits, ctx.num_recv)
+    return (ctx.recv_buf.half(half), ctx.scale_buf.half(half) if ctx.quant else None, ctx.recv_splits, ctx.num_recv)
 
 
 def expert_out_buffer(ctx: EPContext) -> torch.Tensor:
@@ -180,7 +199,7 @@ def expert_out_buffer(ctx: EPContext) -> torch.Tensor:
     (row ``i`` answers row ``i`` of the receive buffer); ``ep_combine`` of the peers reads it in place."""
     if ctx.out_buf is None:
         raise ValueError("no symmetric buffers on this device")
-    return ctx.out_buf.local[ctx.call_count & 1]
+    return ctx.out_buf.half(ctx.call_count & 1)
 
 
 @nvtx_range("tdist.ep_combine")
@@ -195,7 +214,7 @@ def ep_combine(ctx: EPContext, expert_out: Optional[torch.Tensor] = None, weight
     if ctx.out_buf is None:
         return _ep_combine_cpu(ctx, expert_out, weighted)
     half = ctx.call_count & 1
-    buf = ctx.out_buf.local[half]
+    buf = ctx.out_buf.half(half)
     if expert_out is not None and expert_out.data_ptr() != buf.data_ptr() and (phase & 1):
         if expert_out.dtype != torch.bfloat16 or expert_out.shape[1] != ctx.hidden or expert_out.shape[0] > ctx.rows:
             raise ValueError("expert_out must be bf16 [rows, hidden] in the receive layout")
@@ -203,18 +222,14 @@ def ep_combine(ctx: EPContext, expert_out: Optional[torch.Tensor] = None, weight
     if phase & 1:
         ctx.combine_count += 1
     o = out if out is not None else torch.empty((T, ctx.hidden), dtype=torch.bfloat16, device=buf.device)
-    a = _lib.MoeCombineArgs()
-    a.buf_peer = ctx.out_buf.half_ptr_arrays()[half]
-    a.sig_peer = ctx.comb_sig.cached_ptr_array()
+    a = _lib.MoeCombineArgs.from_buffer_copy(ctx.templates[half][1])
     a.topk_ids = ctx.topk_ids.data_ptr()
     a.topk_w = ctx.topk_weights.data_ptr() if (weighted and ctx.topk_weights is not None) else None
-    a.pair_row, a.out = ctx.pair_row.data_ptr(), o.data_ptr()
-    a.ntok, a.topk, a.hidden, a.epr = T, ctx.topk, ctx.hidden, ctx.experts_per_rank
-    a.world, a.rank, a.phase, a.num_ctas, a.epoch = ctx.world, ctx.rank, phase, 0, ctx.combine_count
+    a.out, a.ntok, a.phase, a.epoch = o.data_ptr(), T, phase, ctx.combine_count
     st = global_status()
     a.status = st.device_ptr if st is not None else None
     a.timeout_ns = default_timeout_ns()
-    a.stream = (stream or torch.cuda.current_stream(buf.device)).cuda_stream
+    a.stream = stream_ptr(buf.device, stream)
     _lib.check(_lib.lib().tdist_moe_combine(C.byref(a)), "tdist_moe_combine")
     launch_count += 1
     return o

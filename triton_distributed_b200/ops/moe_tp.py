@@ -30,7 +30,7 @@ import torch
 import torch.distributed as dist
 
 from .. import _lib
-from ..runtime import counters_clean, symm_heap
+from ..runtime import counters_clean, stream_ptr, symm_heap
 from . import collectives as CO
 from . import gemm as G
 from . import moe_utils as MU
@@ -65,7 +65,7 @@ launch_count = 0
 
 
 def _stream(t):
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return stream_ptr(t.device)
 
 
 def select_experts(pg, num_ranks: int, topk: int, input_dtype, device, router_logits: torch.Tensor

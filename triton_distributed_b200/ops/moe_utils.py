@@ -19,13 +19,14 @@ from typing import NamedTuple, Optional, Tuple
 import torch
 
 from .. import _lib
+from ..runtime import stream_ptr
 from ..utils.misc import plain_cuda
 
 launch_count = 0
 
 
 def _stream(t: torch.Tensor, stream=None):
-    return (stream or torch.cuda.current_stream(t.device)).cuda_stream
+    return stream_ptr(t.device, stream)
 
 
 def _status_ptr():

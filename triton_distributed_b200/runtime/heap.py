@@ -83,6 +83,14 @@ class SymmTensor:
             object.__setattr__(self, "_half_arrays", cached)
         return cached
 
+    def half(self, h: int) -> torch.Tensor:
+        """``local[h]`` of such an object; the two views are built once."""
+        cached = getattr(self, "_halves", None)
+        if cached is None:
+            cached = (self.local[0], self.local[1])
+            object.__setattr__(self, "_halves", cached)
+        return cached[h]
+
     def cached_ptr_array(self):
         cached = getattr(self, "_ptr_array", None)
         if cached is None:

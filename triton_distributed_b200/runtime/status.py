@@ -30,6 +30,14 @@ def default_timeout_ns() -> int:
     return _TIMEOUT_CACHE[1]
 
 
+def stream_ptr(device, stream=None) -> int:
+    """Raw handle of ``stream``, or of the current stream of ``device``: without the ``torch.cuda.Stream`` object, whose
+    construction costs half as much as the native launch (2.3 us of a 14 us call)."""
+    if stream is not None:
+        return stream.cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device.index is None else device.index)
+
+
 class StatusBlock:
     """One per process, in device memory. ``device_ptr`` goes into kernel arguments; :meth:`check`
     is called after the stream has been synchronised, copies the block back and raises

@@ -296,13 +296,13 @@ def plain_cuda(*tensors: torch.Tensor) -> bool:
     """True when a raw-pointer kernel may stand in for torch operations on ``tensors``: dense CUDA tensors of the current
     device, 16-byte aligned, whose operations nothing else has to see (no autograd or forward-mode graph, no vmap / functorch
     wrapper, no tensor subclass, no dispatch mode or compilation in progress)."""
-    if torch.compiler.is_compiling() or torch.utils._python_dispatch._get_current_dispatch_mode() is not None:
-        return False
-    device = torch.cuda.current_device() if torch.cuda.is_available() else -1
+    device = -1
     for t in tensors:
-        if type(t) not in (torch.Tensor, torch.nn.Parameter) or torch._C._functorch.is_functorch_wrapped_tensor(t):
+        if t.device.type != "cuda" or type(t) not in (torch.Tensor, torch.nn.Parameter) or torch._C._functorch.is_functorch_wrapped_tensor(t):
             return False
-        if t.device.type != "cuda" or t.device.index != device or t.layout != torch.strided or not t.is_contiguous():
+        if device < 0:
+            device = torch.cuda.current_device()
+        if t.device.index != device or t.layout != torch.strided or not t.is_contiguous():
             return False
         if t.requires_grad and torch.is_grad_enabled():
             return False
@@ -310,4 +310,4 @@ def plain_cuda(*tensors: torch.Tensor) -> bool:
             return False
         if t.is_conj() or t.is_neg() or t.data_ptr() % 16:
             return False
-    return True
+    return not torch.compiler.is_compiling() and torch.utils._python_dispatch._get_current_dispatch_mode() is None
