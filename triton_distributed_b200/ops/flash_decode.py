@@ -157,7 +157,10 @@ def _launch(q, k_cache, v_cache, kv_lens, block_table, scale, soft_cap, out, mod
             max_kv = page * block_table.shape[1]
         splits = default_splits(B, Hkv, max_kv, q.device, D)
         if B > 1:
-            splits = _batch_splits(B * Hkv, max_kv, D, _sm_count(q.device), splits)
+            more = _batch_splits(B * Hkv, max_kv, D, _sm_count(q.device), splits)
+            # only where the partials meet in shared memory: the shared workspace is not for calls that did without it
+            if (Hq // Hkv) * more * (D + 2) * 4 <= 48 * 1024:
+                splits = more
     partial, counters = workspace if workspace is not None else _Workspace.get(q.device, B, Hq, Hkv, D, splits)
     a = _lib.DecodeArgs()
     a.q, a.k_cache, a.v_cache = q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr()
