@@ -271,3 +271,32 @@ def test_activation_of_a_nan_is_a_nan(cuda_device):
     for activation in ("gelu", "silu", "relu"):
         out = G.ag_gemm_intra_node(a, b, ctx, activation=activation)
         assert out[1].isnan().all() and not out[[0, 2, 3]].isnan().any()
+
+
+def _tile_width(M, N, K):
+    g = _lib.GemmArgs()
+    g.mode, g.world, g.rank, g.m_per_rank, g.n, g.k, g.cta_pair, g.c = _lib.GEMM_PLAIN, 1, 0, M, N, K, -1, 16
+    return _lib.lib().tdist_gemm_tile_width(g)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K", [(1000, 5504, 4096), (999, 5496, 4104), (520, 2048, 512), (600, 2056, 520), (512, 6144, 12288), (777, 1928, 5000)])
+def test_automatic_tile_width_matches_fp32_reference(cuda_device, M, N, K, dtype):
+    """Narrow and wide pair tiles of fewer than 256 columns, with remainders in M, N and K. Tolerance: half an ulp of
+    the 16-bit result, and K / 16 accumulation steps on partial sums below 3, each off by less than 2^-23 of them."""
+    torch.manual_seed(M + N)
+    a, b = _rand((M, K), dtype, cuda_device), _rand((N, K), dtype, cuda_device, K ** -0.5)
+    guard = torch.full((M + 1, N), 7.0, dtype=dtype, device=cuda_device)
+    c = G.gemm_persistent(a, b, out=guard[:M])
+    check_status()
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    torch.testing.assert_close(c.double(), a.double() @ b.double().t(), atol=eps / 16 + 3 * K / 16 * 2.0 ** -23, rtol=eps)
+    assert (guard[M] == 7.0).all()
+
+
+def test_narrower_tiles_only_where_a_round_is_nearly_empty(cuda_device):
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("calibrated for 148 SMs")
+    assert _tile_width(8192, 49152, 12288) == 256       # many rounds
+    assert _tile_width(1000, 5504, 4096) == 192         # 44 wide tiles of 2 x 256 on 74 pairs, or 60 of 2 x 192
+    assert _tile_width(16, 6144, 12288) == 0            # few rows

@@ -204,3 +204,21 @@ def test_grouped_gemm_applies_silu_to_the_fp32_sums(cuda_device, blocks, E, K, N
         blk = slice(128 * i, 128 * i + 128)
         ref = torch.nn.functional.silu(a[blk].double() @ b[int(experts[i])].double().t())
         torch.testing.assert_close(out[blk].double(), ref, atol=1e-4, rtol=2.0 ** -8)
+
+
+@pytest.mark.parametrize("blocks,most,E,K,N", [(4, 2, 4, 264, 520), (8, 3, 4, 1024, 2048), (40, 0, 8, 512, 136), (60, 30, 60, 256, 1024)])
+def test_grouped_gemm_tile_width_follows_the_live_blocks(cuda_device, blocks, most, E, K, N):
+    """64 to 256 columns per tile by the number of blocks the host knows of; the count on the device may be lower, and
+    blocks past it stay untouched."""
+    torch.manual_seed(blocks + N)
+    a = torch.randn(blocks * 128, K, device=cuda_device).to(torch.bfloat16)
+    b = (torch.randn(E, N, K, device=cuda_device) * K ** -0.5).to(torch.bfloat16)
+    experts = torch.randint(0, E, (blocks,), dtype=torch.int32, device=cuda_device)
+    live = max(1, (most or blocks) - 1)
+    out = torch.full((blocks * 128, N), 7.0, dtype=torch.bfloat16, device=cuda_device)
+    MT.group_gemm(a, b, experts, torch.tensor([live], dtype=torch.int32, device=cuda_device), out=out, max_blocks=most)
+    check_status()
+    for i in range(live):
+        blk = slice(128 * i, 128 * i + 128)
+        torch.testing.assert_close(out[blk].float(), a[blk].float() @ b[int(experts[i])].float().t(), atol=2.0 ** -8 / 4, rtol=2.0 ** -8)
+    assert (out[128 * live:] == 7.0).all()

@@ -59,7 +59,7 @@ class GemmArgs(C.Structure):
         ("src_epoch", C.c_uint64), ("src_rank", C.c_int), ("src_world", C.c_int),
         ("gather_dst", C.c_void_p), ("block_ready", C.c_void_p), ("gather_counter", C.c_void_p), ("block_rot", C.c_void_p),
         ("c_scatter", C.c_void_p), ("c_rows", C.c_int),
-        ("pair_block", C.c_void_p), ("num_pairs", C.c_int), ("act", C.c_int),
+        ("pair_block", C.c_void_p), ("num_pairs", C.c_int), ("act", C.c_int), ("max_m_blocks", C.c_int),
     ]
 
 
@@ -224,6 +224,7 @@ def _declare(lib):
     lib.tdist_status_destroy.argtypes = [C.c_void_p]
     lib.tdist_gemm_run.argtypes = [C.POINTER(GemmArgs)]
     lib.tdist_gemm_grid.argtypes = [C.POINTER(GemmArgs)]
+    lib.tdist_gemm_tile_width.argtypes = [C.POINTER(GemmArgs)]
     lib.tdist_gemm_plan.argtypes = [C.POINTER(GemmArgs), C.POINTER(C.c_int)]
     lib.tdist_gemm_plan.restype = C.c_int
     lib.tdist_gemm_schedule_check.argtypes = [C.c_int] * 8 + [C.POINTER(C.c_int), C.POINTER(C.c_int)]

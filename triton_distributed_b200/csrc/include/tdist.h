@@ -127,6 +127,7 @@ typedef struct TdistGemmArgs {
     /* PLAIN / AG with one rank, optional: applied to the fp32 accumulator before C is rounded (TDIST_ACT_*; GELU is the tanh
      * form). Few-row products and one CTA per tile only (m_per_rank <= 128, or grouped without pair_block). */
     int act;
+    int max_m_blocks;   /* grouped: the most live 128-row blocks the host knows of (0 = m_per_rank / 128), for the choice of tile */
 } TdistGemmArgs;
 
 int tdist_gemm_run(const TdistGemmArgs* args);
@@ -135,6 +136,8 @@ int tdist_gemm_grid(const TdistGemmArgs* args);
 /* The launch plan of a call with these arguments: out4 = {CTAs per tile (1 or 2), wide tiling (0 / 1), pusher CTAs,
  * grid size}. Launches nothing. */
 int tdist_gemm_plan(const TdistGemmArgs* args, int* out4);
+/* Columns of a tile (of each half of a wide one) such a call uses; 0 = it goes to the few-row kernel. */
+int tdist_gemm_tile_width(const TdistGemmArgs* args);
 /* Host-side replay of the kernel's static tile schedule (no GPU needed): `num_units` CTAs or CTA pairs over a problem
  * of `world` segments of seg_m_tiles x n_tiles 256-column tiles, wide (items of two neighbouring tiles) or narrow,
  * with `split_first` own items cut in two in round 0. Returns 0 when every tile is given out exactly once;

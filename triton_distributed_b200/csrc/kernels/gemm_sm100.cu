@@ -105,7 +105,8 @@ struct GemmParams {
     int seg_blocks;  // 128-row blocks per segment (flag granularity)
     int num_tiles;   // work items of the schedule: 256-column tiles, or 512-column tiles (wide tiling)
     int split_first; // wide tiling, AG: own items cut into halves in round 0 (see get_work)
-    int n_pairs;     // wide tiling: 512-column tiles per row of tiles = ceil(n_tiles / 2)
+    int n_pairs;     // wide tiling: two-half tiles per row of tiles = ceil(n_tiles / 2)
+    int bn;          // columns of a tile, or of each half of a wide one (a multiple of 64; 256 unless the plan chose less)
     int num_comm;
     int push_ahead;             // chunks the pusher's loads run ahead of its stores (1..PUSH_AHEAD)
     int push_parts;             // row slices a 128-row block is pushed in (AG, unicast pushers)
@@ -949,14 +950,14 @@ __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : THREADS, 1) gemm_sm1
                     }
                 }
                 const int row = block * BM;
-                const int col = tc.n_tile * BN + cta_rank * T::B_ROWS;
-                const uint32_t stage_tx = A_BYTES + tc.halves * T::B_BYTES;
+                const int col = tc.n_tile * p.bn + cta_rank * (p.bn / CTAS);
+                const uint32_t stage_tx = A_BYTES + tc.halves * (p.bn / CTAS) * (BK * 2);
                 for (int kb = 0; kb < p.k_blocks; ++kb, ++it) {
                     const uint32_t s = it % STAGES;
                     mbar_wait(bar_empty(s), ((it / STAGES) & 1u) ^ 1u, p.wctx, 2);
                     const uint32_t sa = smem_u32(smem + s * STAGE_BYTES);
                     if (CTAS == 1) {
-                        mbar_expect_tx(bar_full(s), STAGE_BYTES);
+                        mbar_expect_tx(bar_full(s), stage_tx);
                         tma_load_3d(sa, am, bar_full(s), kb * BK, row, az);
                         tma_load_3d(sa + A_BYTES, &p.tm_b, bar_full(s), kb * BK, col, bz);
                     } else {
@@ -966,7 +967,7 @@ __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : THREADS, 1) gemm_sm1
                         tma_load_3d_pair(sa, am, leader_full, kb * BK, row, az);
                         tma_load_3d_pair(sa + A_BYTES, &p.tm_b, leader_full, kb * BK, col, bz);
                         if (WIDE && tc.halves == 2)
-                            tma_load_3d_pair(sa + A_BYTES + T::B_BYTES, &p.tm_b, leader_full, kb * BK, col + BN, bz);
+                            tma_load_3d_pair(sa + A_BYTES + T::B_BYTES, &p.tm_b, leader_full, kb * BK, col + p.bn, bz);
                     }
                 }
             }
@@ -980,7 +981,7 @@ __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : THREADS, 1) gemm_sm1
     } else if (warp == 1) {
         // ===================== MMA issuer (leader CTA only when CTAS == 2) =====================
         if (lane == 0 && cta_rank == 0) {
-            const uint32_t idesc = umma_idesc(p.is_f16 ? 0u : 1u, p.is_f16 ? 0u : 1u, BM * CTAS, BN);
+            const uint32_t idesc = umma_idesc(p.is_f16 ? 0u : 1u, p.is_f16 ? 0u : 1u, BM * CTAS, static_cast<uint32_t>(p.bn));
             uint32_t it = 0;
             uint32_t uses0 = 0, uses1 = 0, next_narrow = 0;   // per-slot use counts give the barrier phases
             const int live_blocks = p.num_m_blocks && p.pair_block == nullptr ? *p.num_m_blocks : 0x7fffffff;
@@ -1070,6 +1071,7 @@ __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : THREADS, 1) gemm_sm1
         // Waiting for that right after issuing them would stall the epilogue for an NVLink round trip per tile, so
         // the flag of a tile is published two tiles later, when `cp.async.bulk.wait_group 8` (all but the newest
         // eight groups, i.e. the two younger tiles' four chunks each, are complete) costs nothing.
+        uint32_t chunk = 0;          // running count: consecutive chunks alternate between the two staging buffers
         uint32_t* pend0 = nullptr;   // older
         uint32_t* pend1 = nullptr;   // younger
         const int live_blocks = p.num_m_blocks && p.pair_block == nullptr ? *p.num_m_blocks : 0x7fffffff;
@@ -1099,7 +1101,7 @@ __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : THREADS, 1) gemm_sm1
                 tc_fence_after();
                 if (buf) ++uses1;
                 else ++uses0;
-                const int col = (tc.n_tile + h) * BN;
+                const int col = (tc.n_tile + h) * p.bn;
                 // RS, this rank's own rows: the other ranks' partials of this tile are added here, so wait for them first
                 // (they were computed one segment-time ago or earlier; only the MMAs of the next tile run meanwhile)
                 const bool reduce_here = MODE == TDIST_GEMM_RS && p.rs_fused && tc.seg == p.rank;
@@ -1117,13 +1119,13 @@ __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : THREADS, 1) gemm_sm1
                     wait_flag_ge_sys(p.flags + (block * p.n_tiles + tc.n_tile + h) * p.world + lane, p.epoch, p.wctx, lane, block, 6);
                 if (reduce_here) __syncwarp();
 #pragma unroll 1
-                for (int c = 0; c < BN / EPI_COLS; ++c) {
+                for (int c = 0; c < p.bn / EPI_COLS; ++c) {
                     uint32_t r0[32], r1[32];
                     const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * BN + c * EPI_COLS;
                     tmem_ld_32x32(taddr, r0);
                     tmem_ld_32x32(taddr + 32, r1);
                     tmem_ld_wait();
-                    if (c == BN / EPI_COLS - 1) {
+                    if (c == p.bn / EPI_COLS - 1) {
                         // accumulator fully read: hand the TMEM slot back to the MMA issuer
                         tc_fence_before();
                         __syncwarp();
@@ -1220,7 +1222,7 @@ __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : THREADS, 1) gemm_sm1
                         }
                         continue;
                     }
-                    uint8_t* cs = cstage + (c & 1) * EPI_BYTES;
+                    uint8_t* cs = cstage + (chunk++ & 1) * EPI_BYTES;
                     named_barrier(1, 128);  // the store that last read this buffer has drained
                     uint8_t* rowp = cs + row_in_tile * 128;
                     const int sw = row_in_tile & 7;
@@ -1357,6 +1359,7 @@ static bool use_wide(const TdistGemmArgs* a) {
 
 struct GridPlan {
     int ctas_per_tile, wide, num_comm, num_tiles, grid;
+    int bn;                            // columns of a tile (of each half of a wide one)
     bool few_rows;                     // a plain product of few rows goes to the kernel in gemm_skinny_sm100.cu
     tdist_host::SkinnyPlan skinny;
 };
@@ -1479,34 +1482,51 @@ static void plan_ag(const TdistGemmArgs* a, int sms, int n_tiles, GridPlan& g) {
     g.num_tiles = seg_m_tiles * (g.wide ? (n_tiles + 1) / 2 : n_tiles) * a->world;
 }
 
-// Plain products of one rank whose caller asked for no particular tiling, CTA count or timeline. C is written with plain
-// stores there, so a C that the TMA store here would refuse is left to that refusal.
-static bool may_be_few_rows(const TdistGemmArgs* a) {
+// Plain products of one rank whose caller asked for no particular tiling, CTA count or timeline.
+static bool may_replan(const TdistGemmArgs* a) {
     return (a->mode == TDIST_GEMM_PLAIN || a->mode == TDIST_GEMM_AG) && a->world == 1 && a->expert_ids == nullptr &&
            a->num_m_blocks == nullptr && a->a_gather == nullptr && a->c_scatter == nullptr && a->block_rot == nullptr &&
-           a->trace == nullptr && a->cta_pair < 0 && a->num_sms <= 0 && a->c != nullptr && reinterpret_cast<uintptr_t>(a->c) % 16 == 0;
+           a->trace == nullptr && a->cta_pair < 0 && a->num_sms <= 0;
 }
 
-// Expected time of a plain product on this kernel: the longest unit's share of 256-column tiles at the rate a CTA or a
-// pair sustains, or the operands' trip through HBM. A single CTA's tile is bound by its L2 -> shared-memory loads
-// (48 KB per K block at 64 bytes per clock: m16 n6144 k12288 measured 77 us, 10.5 TFLOP/s of the padded tile), a pair's by the MMAs.
+// Expected time of a plain product on this kernel: the longest unit's tiles, or the operands' trip through HBM. Nanoseconds
+// per 64-wide K block, measured with one tile per unit (M 1024, K 4096 and 16384): a CTA pair's narrow tile 336 at 128
+// columns and 382 at 256 (the latency of its loads, hardly its width), a wide one 175 + 2.1 per column of a half; a single
+// CTA's 128 x 256 tile 400 (48 KB at what an SM takes from L2; m16 n6144 k12288 as 24 such tiles: 77 us).
 static double plain_time(const TdistGemmArgs* a, const GridPlan& g) {
     const int units = g.grid / g.ctas_per_tile;
-    const double rate = g.ctas_per_tile == 1 ? 10.4e12 : 22.0e12;
-    const double tile_s = 2.0 * BM * g.ctas_per_tile * BN * a->k / rate + (g.wide ? 1.5e-6 : 0.5e-6);
-    const double sm_s = schedule_cost(g.num_tiles, units, g.wide) * tile_s;
+    const int k_blocks = (a->k + BK - 1) / BK;
+    const double narrow_s = k_blocks * (g.ctas_per_tile == 1 ? 400e-9 : (290 + 0.36 * g.bn) * 1e-9) + 0.3e-6;
+    const double wide_s = k_blocks * (175 + 2.1 * g.bn) * 1e-9 + 3e-6;
+    // the rounds get_work() deals out: a last, partial round of wide tiles may be cut into halves
+    const int full = g.num_tiles / units, rest = g.num_tiles - full * units;
+    const double whole = g.wide ? wide_s : narrow_s;
+    const double sm_s = full * whole + (rest == 0 ? 0.0 : (g.wide && 2 * rest <= units ? narrow_s : whole));
     // single CTAs reach 5.6 TB/s (m16 n49152 k4096: 79 us, 69 us on the few-row kernel)
     const double hbm_s = 2.0 * (static_cast<double>(a->n) * a->k + static_cast<double>(a->m_per_rank) * (a->k + a->n)) / (g.ctas_per_tile == 1 ? 5.6e12 : 6.3e12);
-    return (sm_s > hbm_s ? sm_s : hbm_s) + 4e-6;
+    return (sm_s > hbm_s ? sm_s : hbm_s) + 5e-6;
 }
 
 static GridPlan plan_grid(const TdistGemmArgs* a) {
     GridPlan g;
     g.few_rows = false;
+    g.bn = BN;
     g.ctas_per_tile = use_pair(a) ? 2 : 1;
     g.wide = use_wide(a) ? 1 : 0;
     const int seg_m_tiles = a->pair_block ? a->num_pairs : (a->m_per_rank + BM * g.ctas_per_tile - 1) / (BM * g.ctas_per_tile);
-    const int n_tiles = (a->n + BN - 1) / BN;
+    int n_tiles = (a->n + BN - 1) / BN;
+    if (a->expert_ids != nullptr && g.ctas_per_tile == 1 && a->num_sms <= 0 && (a->a_gather == nullptr || a->gather_dst != nullptr)) {
+        // Grouped GEMM of a decode step: its blocks are a few rows each, so it is bound by the loads of B, and a CTA's rate by
+        // what an SM takes from L2. While 256-column tiles leave SMs idle, narrower ones that still run as one round bring
+        // more of them in (both GEMMs of the experts, 16 tokens, top 2 of 8, 4096 x 2048: 71 -> 67 us; 64 tokens, top 4 of
+        // 16, 4096 x 512: 58 -> 51 us). Beyond one round they lose: the A rows are loaded again for every tile (128 tokens,
+        // top 8 of 32, 7168 x 2048 with 192 columns: 350 us against 330).
+        const int blocks = a->max_m_blocks > 0 && a->max_m_blocks < seg_m_tiles ? a->max_m_blocks : seg_m_tiles;
+        const long long sms = tdist_host::sm_count();
+        for (int bn = BN - 64; bn >= 64; bn -= 64)
+            if (static_cast<long long>(blocks) * ((a->n + bn - 1) / bn) <= sms) g.bn = bn;
+        n_tiles = (a->n + g.bn - 1) / g.bn;
+    }
     g.num_tiles = seg_m_tiles * (g.wide ? (n_tiles + 1) / 2 : n_tiles) * a->world;
     int capacity = resident_ctas(g.ctas_per_tile, g.wide, a->mode);
     if (a->mode == TDIST_GEMM_AG && a->world > 1 && g.ctas_per_tile == 2) {
@@ -1525,19 +1545,56 @@ static GridPlan plan_grid(const TdistGemmArgs* a) {
         if (g.num_comm > sms - g.ctas_per_tile) g.num_comm = sms - g.ctas_per_tile;
         if (g.num_comm < g.ctas_per_tile) g.num_comm = g.ctas_per_tile;
     }
-    int units = (sms - g.num_comm) / g.ctas_per_tile;
-    // a wide schedule may split its last round in two: allow up to twice the items
-    const int most = g.wide ? 2 * g.num_tiles : g.num_tiles;
-    if (units > most) units = most;
-    if (units < 1) units = 1;
-    g.grid = units * g.ctas_per_tile + g.num_comm;
-    if (may_be_few_rows(a) && tdist_host::skinny_plan(a->m_per_rank, a->n, a->k, plain_time(a, g), &g.skinny)) {
+    const auto set_grid = [&](GridPlan& p) {
+        int units = (sms - p.num_comm) / p.ctas_per_tile;
+        // a wide schedule may split its last round in two: allow up to twice the items
+        const int most = p.wide ? 2 * p.num_tiles : p.num_tiles;
+        if (units > most) units = most;
+        if (units < 1) units = 1;
+        p.grid = units * p.ctas_per_tile + p.num_comm;
+    };
+    set_grid(g);
+    if (!may_replan(a)) return g;
+    // A problem of a few rounds: the tile width, narrow or wide, whose last round is the least empty for what its K blocks
+    // cost (m1000 n5504 k4096: 44 wide tiles of 2 x 256 columns on 74 pairs 53.6 us, 60 of 2 x 192 44.3 us; m2048 n14336
+    // k4096: 3.5 rounds of 2 x 256 187.6 us, 7 narrow rounds 172.7 us). The rule above keeps its choice on a near tie: long
+    // runs are bound by power, and the wide tile moves the fewest bytes.
+    double best = plain_time(a, g);
+    if (g.ctas_per_tile == 2) {
+        const GridPlan first = g;
+        for (int wide = 0; wide <= first.wide; ++wide)
+            for (int bn = BN; bn >= 128; bn -= 64) {
+                GridPlan c = first;
+                const int tiles = (a->n + bn - 1) / bn;
+                if (wide && tiles < 2) continue;
+                c.bn = bn;
+                c.wide = wide;
+                c.num_tiles = seg_m_tiles * (wide ? (tiles + 1) / 2 : tiles);
+                set_grid(c);
+                const double t = plain_time(a, c);
+                if (t < 0.96 * plain_time(a, first) && t < best) {
+                    best = t;
+                    g = c;
+                }
+            }
+        if (g.wide != first.wide) resident_ctas(2, g.wide, a->mode);   // opts in to the shared memory of that kernel
+    }
+    // Few rows: the kernel in gemm_skinny_sm100.cu. It writes C with plain stores, so a C that the TMA store here would
+    // refuse is left to that refusal.
+    if (a->c != nullptr && reinterpret_cast<uintptr_t>(a->c) % 16 == 0 &&
+        tdist_host::skinny_plan(a->m_per_rank, a->n, a->k, best, &g.skinny)) {
         g.few_rows = true;
         g.ctas_per_tile = 1;
         g.wide = 0;
         g.grid = g.skinny.grid;
     }
     return g;
+}
+
+// Columns of a tile (of each half of a wide one), 0 = the few-row kernel.
+extern "C" int tdist_gemm_tile_width(const TdistGemmArgs* a) {
+    const GridPlan g = plan_grid(a);
+    return g.few_rows ? 0 : g.bn;
 }
 
 extern "C" int tdist_gemm_grid(const TdistGemmArgs* a) { return plan_grid(a).grid; }
@@ -1658,7 +1715,7 @@ extern "C" int tdist_gemm_run(const TdistGemmArgs* a) {
         const uint64_t E = a->num_experts > 0 ? a->num_experts : 1;
         uint64_t dims[3] = {K, N, E};
         uint64_t strides[2] = {K * 2, N * K * 2};
-        uint32_t box[3] = {BK, static_cast<uint32_t>(BN / ctas), 1};
+        uint32_t box[3] = {BK, static_cast<uint32_t>(plan.bn / ctas), 1};
         if ((rc = tdist_host::encode_tmap(&p.tm_b, dt, 2, 3, a->b, dims, strides, box, tdist_host::Swizzle::B128))) return rc;
     }
     {
@@ -1696,7 +1753,7 @@ extern "C" int tdist_gemm_run(const TdistGemmArgs* a) {
     {
         // the first wave of tiles: one tile per GEMM CTA, rows of tiles GROUP_M blocks deep
         const int gm = a->group_m > 0 ? a->group_m : DEFAULT_GROUP_M;
-        const int n_tiles = (a->n + BN - 1) / BN;
+        const int n_tiles = (a->n + plan.bn - 1) / plan.bn;
         const int per_row = plan.wide ? (n_tiles + 1) / 2 : n_tiles;
         const int first_wave = ((plan.grid - plan.num_comm) / ctas + per_row - 1) / per_row;   // rows of tiles
         p.gather_pro_blocks = a->gather_counter != nullptr ? (first_wave + gm - 1) / gm * gm * ctas : 0;
@@ -1724,7 +1781,8 @@ extern "C" int tdist_gemm_run(const TdistGemmArgs* a) {
     p.seg_blocks = (a->m_per_rank + BM - 1) / BM;
     p.seg_m_tiles = a->pair_block ? a->num_pairs : (a->m_per_rank + BM * ctas - 1) / (BM * ctas);
     p.pair_block = static_cast<const int*>(a->pair_block);
-    p.n_tiles = (a->n + BN - 1) / BN;
+    p.bn = plan.bn;
+    p.n_tiles = (a->n + plan.bn - 1) / plan.bn;
     p.n_pairs = (p.n_tiles + 1) / 2;
     p.k_blocks = (a->k + BK - 1) / BK;
     p.is_f16 = a->dtype == TDIST_F16;

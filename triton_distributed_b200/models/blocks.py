@@ -67,8 +67,10 @@ class EPMoE:
 
     def experts(self, rows: torch.Tensor, out: torch.Tensor = None) -> torch.Tensor:
         """This rank's experts over the dispatched rows (``[capacity, hidden]``, block-aligned groups)."""
-        h = MT.group_gemm(rows, self.w1, self.ctx.block_expert, self.ctx.num_blocks, activation="silu")
-        return MT.group_gemm(h, self.w2, self.ctx.block_expert, self.ctx.num_blocks, out=out)
+        # one rank: no more blocks than pairs; otherwise the other ranks' pairs are not known here
+        most = self.ctx.ntok * self.topk if self.world == 1 else 0
+        h = MT.group_gemm(rows, self.w1, self.ctx.block_expert, self.ctx.num_blocks, activation="silu", max_blocks=most)
+        return MT.group_gemm(h, self.w2, self.ctx.block_expert, self.ctx.num_blocks, out=out, max_blocks=most)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         ids, w = MU.gate_topk(x, self.gate, self.topk, renormalize=True)

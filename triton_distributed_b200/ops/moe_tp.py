@@ -121,11 +121,13 @@ def topk_reduce(y: torch.Tensor, pos_of: torch.Tensor, weights: Optional[torch.T
 
 
 def group_gemm(a_sorted: torch.Tensor, b: torch.Tensor, expert_ids: torch.Tensor, num_blocks: Optional[torch.Tensor] = None,
-               out: Optional[torch.Tensor] = None, activation: Optional[str] = None) -> torch.Tensor:
+               out: Optional[torch.Tensor] = None, activation: Optional[str] = None,
+               max_blocks: int = 0) -> torch.Tensor:
     """``out[i*128:(i+1)*128] = a_sorted[i*128:(i+1)*128] @ b[expert_ids[i]].T`` for every live
     128-row block. ``a_sorted`` ``[blocks*128, K]``, ``b`` ``[E, N, K]`` (K contiguous), ``num_blocks``
     an int32 device scalar (blocks past it are padding and are skipped). ``activation`` ("gelu" in its tanh form, "silu",
-    "relu") is applied to the fp32 sums by the epilogue."""
+    "relu") is applied to the fp32 sums by the epilogue. ``max_blocks``: the most live blocks the caller knows of (0 = all
+    of ``a_sorted``); the tile is chosen for that many."""
     rows, K = a_sorted.shape
     E, N, _ = b.shape
     if rows % GROUP_BLOCK_M:
@@ -148,6 +150,7 @@ def group_gemm(a_sorted: torch.Tensor, b: torch.Tensor, expert_ids: torch.Tensor
     g.num_m_blocks = num_blocks.data_ptr() if num_blocks is not None else None
     g.num_experts = E
     g.act = _lib.ACTIVATIONS[activation]
+    g.max_m_blocks = max_blocks
     G._launch(g)
     return c
 
