@@ -116,6 +116,16 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
     return r;
 }
 
+// ---------------------------------------------------------------- programmatic dependent launch
+// Every kernel launched with tdist_host::pdl_attribute() calls this before it touches memory that an earlier kernel of the
+// stream may still write or read: the launch itself, barrier set-up and TMEM allocation then run under the tail of that
+// kernel. wait returns when all earlier kernels are complete and their writes visible; only then is the next kernel of the
+// stream let in, which bounds how many grids hold resources at once.
+__device__ __forceinline__ void pdl_wait_and_release() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // ---------------------------------------------------------------- TMA (no multicast)
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* m) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory");

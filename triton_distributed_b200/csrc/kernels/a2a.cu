@@ -19,6 +19,7 @@
 #include <cuda_fp8.h>
 #include <cuda_runtime.h>
 
+#include "../device/ptx.cuh"
 #include "../device/shmem.cuh"
 #include "../include/tdist.h"
 #include "../runtime/host_common.h"
@@ -241,6 +242,7 @@ __global__ void __launch_bounds__(kA2AThreads, 2) a2a_kernel(const A2AParams p) 
 // fp8 e4m3 rows + per-128 scales -> bf16 rows (expert-side dequantisation; reference
 // tutorials/04-deepseek-infer-all2all.py `_dequant_kernel`).
 __global__ void dequant_fp8_kernel(const uint8_t* x, const float* scale, __nv_bfloat16* out, int rows, int hidden) {
+    pdl_wait_and_release();
     const int groups = hidden / 128;
     const size_t total = static_cast<size_t>(rows) * hidden / 8;
     for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
@@ -339,8 +341,7 @@ extern "C" int tdist_dequant_fp8(const void* x, const void* scale, void* out, in
     if (rows <= 0) return 0;
     const size_t total = static_cast<size_t>(rows) * hidden / 8;
     const int blocks = static_cast<int>(min(static_cast<size_t>(592), (total + 255) / 256));
-    dequant_fp8_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const uint8_t*>(x), static_cast<const float*>(scale), static_cast<__nv_bfloat16*>(out), rows, hidden);
-    TDIST_CUDA_OK(cudaGetLastError());
+    TDIST_CUDA_OK(tdist_host::launch_pdl(dequant_fp8_kernel, dim3(blocks), 256, 0, static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(x),
+                                         static_cast<const float*>(scale), static_cast<__nv_bfloat16*>(out), rows, hidden));
     return 0;
 }

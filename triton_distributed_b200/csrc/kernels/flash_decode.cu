@@ -139,6 +139,7 @@ __global__ void __launch_bounds__(kDecodeThreads, (D <= 128 ? 2 : 1)) flash_deco
 
     const int tid = static_cast<int>(threadIdx.x);
     const int warp = tid >> 5, lane = tid & 31;
+    pdl_wait_and_release();
     const int split = static_cast<int>(blockIdx.x) % p.splits;
     const int kvh = (static_cast<int>(blockIdx.x) / p.splits) % p.Hkv;
     const int b = static_cast<int>(blockIdx.x) / (p.splits * p.Hkv);
@@ -571,14 +572,16 @@ static int launch_decode(DecodeParams& p, cudaStream_t stream) {
     cfg.blockDim = dim3(kDecodeThreads);
     cfg.stream = stream;
     cfg.dynamicSmemBytes = smem;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    attr[0] = tdist_host::pdl_attribute();
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
     if (cluster) {
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = static_cast<unsigned>(p.splits);
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = static_cast<unsigned>(p.splits);
+        attr[1].val.clusterDim.y = 1;
+        attr[1].val.clusterDim.z = 1;
+        cfg.numAttrs = 2;
     }
     p.cluster_merge = cluster ? 1 : 0;
     TDIST_CUDA_OK(cudaLaunchKernelEx(&cfg, flash_decode_kernel<T, D>, p));

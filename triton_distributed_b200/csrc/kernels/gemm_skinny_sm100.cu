@@ -92,6 +92,7 @@ __global__ void __launch_bounds__(THREADS, 2) gemm_skinny_kernel(const __grid_co
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
+    pdl_wait_and_release();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -341,13 +342,14 @@ int skinny_run(const TdistGemmArgs* a, const SkinnyPlan& plan) {
     cfg.blockDim = dim3(THREADS);
     cfg.dynamicSmemBytes = SMEM_BYTES;
     cfg.stream = static_cast<cudaStream_t>(a->stream);
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = static_cast<unsigned>(plan.split);
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1] = pdl_attribute();
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     TDIST_CUDA_OK(cudaLaunchKernelEx(&cfg, gemm_skinny_kernel, p));
     return 0;
 }

@@ -755,6 +755,7 @@ __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : THREADS, 1) gemm_sm1
 
     // ---------------- pusher CTAs (AG only; whole clusters when CTAS == 2) ----------------
     if (MODE == TDIST_GEMM_AG && static_cast<int>(blockIdx.x) < p.num_comm) {
+        pdl_wait_and_release();
         if (threadIdx.x == 0) {
             for (int s = 0; s < PUSH_STAGES; ++s) mbar_init(smem_u32(&bars[s]), 1);
             fence_mbar_init();
@@ -769,6 +770,7 @@ __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : THREADS, 1) gemm_sm1
     constexpr bool STAGED = MODE == TDIST_GEMM_PLAIN && !GATHER;
     int gather_live = 0, gather_rot = 0, gather_pro = 0;
     if (STAGED && p.gather_dst != nullptr) {
+        pdl_wait_and_release();
         gather_live = min(p.seg_blocks, p.num_m_blocks ? *p.num_m_blocks : p.seg_blocks);
         gather_rot = p.block_rot ? max(*p.block_rot, 0) : 0;
         if (CTAS == 2 && p.pair_block != nullptr) gather_rot = p.pair_block[min(gather_rot, p.seg_m_tiles - 1)] >> 1;
@@ -825,6 +827,7 @@ __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : THREADS, 1) gemm_sm1
     }
     tc_fence_after();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
+    if (!(STAGED && p.gather_dst != nullptr)) pdl_wait_and_release();
 
     if (GATHER && warp >= THREADS / 32) {
         // ===================== gathering producers: A rows by index with cp.async ==========
@@ -1868,13 +1871,14 @@ extern "C" int tdist_gemm_run(const TdistGemmArgs* a) {
     cfg.blockDim = dim3(block_threads);
     cfg.dynamicSmemBytes = SMEM_BYTES;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = ctas;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1] = tdist_host::pdl_attribute();
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = a->gather_dst != nullptr ? 1 : 2;   // (a staged row gather starts on every SM at once: 1 % slower early)
     TDIST_CUDA_OK(cudaLaunchKernelExC(&cfg, fn, kargs));
     return 0;
 }

@@ -12,6 +12,7 @@
 #include <math_constants.h>
 
 #include "../device/moe_sort.cuh"
+#include "../device/ptx.cuh"
 #include "../device/signal.cuh"
 #include "../include/tdist.h"
 #include "../runtime/host_common.h"
@@ -181,6 +182,7 @@ __device__ __forceinline__ void topk_softmax_any(const float* row, int E, int to
 }
 __global__ void moe_topk_softmax_kernel(const float* logits, int ntok, int E, int topk, int renorm, int* ids, float* w) {
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    pdl_wait_and_release();
     if (warp >= ntok) return;
     const size_t at = static_cast<size_t>(warp) * topk;
     topk_softmax_any(logits + static_cast<size_t>(warp) * E, E, topk, renorm, static_cast<int>(threadIdx.x) & 31, ids + at, w + at);
@@ -215,6 +217,7 @@ __global__ void __launch_bounds__(kGateThreads, 1) moe_gate_topk_kernel(const __
     const int g = lane >> 2, tig = lane & 3;                 // row / column group of the MMA fragments
     const int t0 = static_cast<int>(blockIdx.x) * kGateTok;
     const int steps = hidden / 32;
+    pdl_wait_and_release();
     // rows past the end repeat the last one; their results are not used
     const __nv_bfloat16* xa = x + static_cast<size_t>(min(t0 + g, ntok - 1)) * hidden + tig * 8;
     const __nv_bfloat16* xb = x + static_cast<size_t>(min(t0 + g + 8, ntok - 1)) * hidden + tig * 8;
@@ -294,6 +297,7 @@ __global__ void __launch_bounds__(256) topk_reduce_kernel(const uint4* y, const 
     const int lane = threadIdx.x & 31;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     const int segs = (vec_per_row + 32 * kReduceVecs - 1) / (32 * kReduceVecs);
+    pdl_wait_and_release();
     for (long long item = warp; item < static_cast<long long>(ntok) * segs; item += nwarps) {
         const int t = static_cast<int>(item / segs);
         const int c0 = static_cast<int>(item - static_cast<long long>(t) * segs) * 32 * kReduceVecs + lane;
@@ -397,10 +401,9 @@ extern "C" int tdist_moe_topk_softmax(const void* logits, int ntok, int num_expe
     if (ntok <= 0) return 0;
     const int warps_per_block = 8;
     const int blocks = (ntok + warps_per_block - 1) / warps_per_block;
-    moe_topk_softmax_kernel<<<blocks, warps_per_block * 32, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const float*>(logits), ntok, num_experts, topk, renormalize, static_cast<int*>(ids),
-        static_cast<float*>(weights));
-    TDIST_CUDA_OK(cudaGetLastError());
+    TDIST_CUDA_OK(tdist_host::launch_pdl(moe_topk_softmax_kernel, dim3(blocks), warps_per_block * 32, 0, static_cast<cudaStream_t>(stream),
+                                         static_cast<const float*>(logits), ntok, num_experts, topk, renormalize,
+                                         static_cast<int*>(ids), static_cast<float*>(weights)));
     return 0;
 }
 
@@ -417,16 +420,16 @@ extern "C" int tdist_moe_gate_topk(const void* x, const void* gate, int ntok, in
 #define TDIST_GATE_CASE(NT)                                                                                                     \
     {                                                                                                                           \
         if (int rc = ensure_smem(moe_gate_topk_kernel<NT>, smem)) return rc;                                                    \
-        moe_gate_topk_kernel<NT><<<grid, kGateThreads, smem, static_cast<cudaStream_t>(stream)>>>(                              \
-            static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gate), ntok, hidden, num_experts, topk,     \
-            renormalize, static_cast<int*>(ids), static_cast<float*>(weights), static_cast<float*>(logits));                    \
+        TDIST_CUDA_OK(tdist_host::launch_pdl(moe_gate_topk_kernel<NT>, grid, kGateThreads, smem, static_cast<cudaStream_t>(stream), \
+                                             static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gate), ntok,   \
+                                             hidden, num_experts, topk, renormalize, static_cast<int*>(ids),                    \
+                                             static_cast<float*>(weights), static_cast<float*>(logits)));                       \
     }
     if (nt == 1) TDIST_GATE_CASE(1)
     else if (nt == 2) TDIST_GATE_CASE(2)
     else if (nt == 4) TDIST_GATE_CASE(4)
     else TDIST_GATE_CASE(8)
 #undef TDIST_GATE_CASE
-    TDIST_CUDA_OK(cudaGetLastError());
     return 0;
 }
 
@@ -448,9 +451,8 @@ extern "C" int tdist_topk_reduce(const void* y, const void* pos_of, const void* 
     if (ntok <= 0) return 0;
     const long long items = static_cast<long long>(ntok) * ((row_bytes / 16 + 32 * kReduceVecs - 1) / (32 * kReduceVecs));
     const int blocks = static_cast<int>((items + 7) / 8 < 1184 ? (items + 7) / 8 : 1184);
-    topk_reduce_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const uint4*>(y), static_cast<const int*>(pos_of), static_cast<const float*>(weights), ntok, topk,
-        row_bytes / 16, static_cast<uint4*>(out));
-    TDIST_CUDA_OK(cudaGetLastError());
+    TDIST_CUDA_OK(tdist_host::launch_pdl(topk_reduce_kernel, dim3(blocks), 256, 0, static_cast<cudaStream_t>(stream), static_cast<const uint4*>(y),
+                                         static_cast<const int*>(pos_of), static_cast<const float*>(weights), ntok, topk, row_bytes / 16,
+                                         static_cast<uint4*>(out)));
     return 0;
 }

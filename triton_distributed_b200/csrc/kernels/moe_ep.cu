@@ -26,6 +26,7 @@
 #include <cuda_runtime.h>
 
 #include "../device/moe_sort.cuh"
+#include "../device/ptx.cuh"
 #include "../device/shmem.cuh"
 #include "../include/tdist.h"
 #include "../runtime/host_common.h"
@@ -165,6 +166,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_dispatch_kernel(const __gr
     const int gw = static_cast<int>(blockIdx.x) * kMoeWarps + warp;
     const int nw = static_cast<int>(gridDim.x) * kMoeWarps;
     uint4 raw[kEpSegLoads];
+    pdl_wait_and_release();
     if ((p.phase & 2) && gw < p.ntok * segs)
         load_segment(p.x + static_cast<size_t>(gw / segs) * p.hidden * 2, p.hidden, gw % segs, lane, p.quant != 0, raw);
 
@@ -432,6 +434,7 @@ struct CombineParams {
 __global__ void __launch_bounds__(kMoeThreads, 2) moe_combine_kernel(const __grid_constant__ CombineParams p) {
     const int tid = static_cast<int>(threadIdx.x);
     const int warp = tid >> 5, lane = tid & 31;
+    pdl_wait_and_release();
     if ((p.phase & 1) && blockIdx.x == 0 && tid < p.world) {
         // the expert outputs were written by earlier work of this stream: complete and visible to peer reads
         fence_acq_rel_sys();
@@ -566,8 +569,7 @@ extern "C" int tdist_moe_dispatch(const TdistMoeDispatchArgs* a) {
     const int sms = tdist_host::sm_count();
     if (ctas > sms) ctas = sms;
     if (ctas < 1 || !(p.phase & 2)) ctas = 1;   // counts-only and wait-only launches need one CTA
-    moe_dispatch_kernel<<<ctas, kMoeThreads, smem, static_cast<cudaStream_t>(a->stream)>>>(p);
-    TDIST_CUDA_OK(cudaGetLastError());
+    TDIST_CUDA_OK(tdist_host::launch_pdl(moe_dispatch_kernel, dim3(ctas), kMoeThreads, smem, static_cast<cudaStream_t>(a->stream), p));
     return 0;
 }
 
@@ -606,7 +608,6 @@ extern "C" int tdist_moe_combine(const TdistMoeCombineArgs* a) {
     const int cap = 2 * tdist_host::sm_count();
     if (ctas > cap) ctas = cap;
     if (ctas < 1 || !(p.phase & 2)) ctas = 1;
-    moe_combine_kernel<<<ctas, kMoeThreads, 0, static_cast<cudaStream_t>(a->stream)>>>(p);
-    TDIST_CUDA_OK(cudaGetLastError());
+    TDIST_CUDA_OK(tdist_host::launch_pdl(moe_combine_kernel, dim3(ctas), kMoeThreads, 0, static_cast<cudaStream_t>(a->stream), p));
     return 0;
 }
