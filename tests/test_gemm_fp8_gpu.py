@@ -107,3 +107,22 @@ def test_ag_fp8_gemm_single_rank_kernels_against_prepared_peers(cuda_device, wor
             if s != r:
                 assert torch.equal(ws[s], ops[s][0].view(torch.uint8)), f"rank {r} rows of {s}"
                 assert torch.equal(sws[s], ops[s][1]), f"rank {r} scales of {s}"
+
+
+@pytest.mark.parametrize("N,K", [(8, 128), (264, 384), (1000, 896), (4096, 8192), (520, 16384)])
+def test_few_row_fp8_gemm_matches_fp32_reference(cuda_device, N, K):
+    """The automatic choice at few rows: one or two groups of folding warps, token and weight-row remainders, one to eight
+    CTAs per cluster. Tolerance: half an ulp of bf16 and fp32 sums (1e-5 of the terms' spread)."""
+    b = sb = None
+    for M in (1, 5, 16, 17, 31, 63, 64, 65, 100, 127, 128, 129, 200, 256):
+        a, sa, bn, sbn = _operands(M, N, K, cuda_device, M)
+        if b is None:
+            b, sb = bn, sbn
+        guard = torch.full((M + 1, N), 7.0, dtype=torch.bfloat16, device=cuda_device)
+        c = F.gemm_fp8_blockscaled(a, sa, b, sb, out=guard[:M])
+        check_status()
+        ref = F.dequantize_fp8(a, sa, 1).double() @ F.dequantize_fp8(b, sb, 128).double().t()
+        torch.testing.assert_close(c.double(), ref, rtol=2.0 ** -8, atol=1e-5 * ref.abs().max().item())
+        assert (guard[M] == 7.0).all()
+        again = F.gemm_fp8_blockscaled(a, sa, b, sb, num_sms=148)   # the large tiles
+        torch.testing.assert_close(again.double(), ref, rtol=2.0 ** -8, atol=1e-5 * ref.abs().max().item())

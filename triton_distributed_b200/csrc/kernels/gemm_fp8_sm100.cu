@@ -40,6 +40,7 @@
 #include "../device/signal.cuh"
 #include "../include/tdist.h"
 #include "../runtime/host_common.h"
+#include "gemm_skinny.h"
 
 namespace tdist {
 namespace fp8 {
@@ -487,6 +488,17 @@ extern "C" int tdist_gemm_fp8_run(const TdistGemmFp8Args* a) {
     if (a->k % 128 != 0) return fail(TDIST_EINVAL, "fp8 gemm: K must be a multiple of 128 (one scale per 128 values)");
     if (a->n % 8 != 0) return fail(TDIST_EINVAL, "fp8 gemm: N must be a multiple of 8");
     if (!a->a || !a->b || !a->c || !a->sa || !a->sb) return fail(TDIST_EINVAL, "fp8 gemm: null operand");
+    if (a->world == 1 && a->num_sms <= 0 && reinterpret_cast<uintptr_t>(a->c) % 16 == 0) {
+        // Few rows: expected time of the tiles below (a K block of one takes 0.52 us, or its share of 5.6 TB/s) against the
+        // few-row kernel's. (A C that the TMA store here would refuse is left to that refusal.)
+        const long long tiles = static_cast<long long>((a->m_per_rank + BM - 1) / BM) * ((a->n + BN - 1) / BN);
+        const int sms = tdist_host::sm_count();
+        const double sm_s = static_cast<double>((tiles + sms - 1) / sms) * (a->k / BK) * 0.52e-6;
+        const double hbm_s = (static_cast<double>(a->n) * a->k + static_cast<double>(a->m_per_rank) * (a->k + 2.0 * a->n)) / 5.6e12;
+        tdist_host::SkinnyPlan plan;
+        if (tdist_host::fp8_skinny_plan(a->m_per_rank, a->n, a->k, (sm_s > hbm_s ? sm_s : hbm_s) + 4.5e-6, &plan))
+            return tdist_host::fp8_skinny_run(a, plan);
+    }
     Params p;
     memset(&p, 0, sizeof(p));
     const uint64_t K = a->k, N = a->n, MPR = a->m_per_rank, W = a->world;

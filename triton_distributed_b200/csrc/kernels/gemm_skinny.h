@@ -1,4 +1,4 @@
-// Few-row GEMM (gemm_skinny_sm100.cu): plan and launch, used by the dispatch in gemm_sm100.cu.
+// Few-row GEMMs: plan and launch, used by the dispatch in gemm_sm100.cu and gemm_fp8_sm100.cu.
 #pragma once
 #include "../include/tdist.h"
 
@@ -12,5 +12,9 @@ struct SkinnyPlan {
 // large-tile kernel); fills the plan. Looks at sizes only.
 bool skinny_plan(int m, int n, int k, double other_s, SkinnyPlan* plan);
 int skinny_run(const TdistGemmArgs* a, const SkinnyPlan& plan);
+
+// The same for the block-scaled fp8 product (gemm_fp8_skinny_sm100.cu).
+bool fp8_skinny_plan(int m, int n, int k, double other_s, SkinnyPlan* plan);
+int fp8_skinny_run(const TdistGemmFp8Args* a, const SkinnyPlan& plan);
 
 }  // namespace tdist_host
