@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_dispatch_kernel(const __gr
             p.counts_peer[d][p.rank * E + e] = hist[e];
         }
         __syncthreads();
-        if (tid < p.world) {
+        if (tid < p.world && tid != p.rank) {
             fence_acq_rel_sys();
             st_release_sys_u64(p.sig_peer[tid] + p.world + p.rank, p.epoch);
         }
@@ -230,13 +230,14 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_dispatch_kernel(const __gr
     if (p.phase & 2) {
         // ---------------------------------------------------------------- start row of each expert's group at its owner
         if (p.compact) {
-            if (tid < p.world) signal_wait_until(p.sig_peer[p.rank] + p.world + tid, kCmpGe, p.epoch, p.wctx, tid, 1);
+            // (every CTA counted this rank's own pairs itself: nothing to wait for there)
+            if (tid < p.world && tid != p.rank) signal_wait_until(p.sig_peer[p.rank] + p.world + tid, kCmpGe, p.epoch, p.wctx, tid, 1);
             __syncthreads();
-            const int* counts = p.counts_peer[p.rank];   // [world][E], complete after the waits above
+            const int* counts = p.counts_peer[p.rank];   // [world][E], the other ranks' rows complete after the waits above
             for (int e = tid; e < E; e += kMoeThreads) {
                 int tot = 0, before = 0;   // rows of expert e over all sources, and from lower ranks
                 for (int s = 0; s < p.world; ++s) {
-                    const int c = ld_relaxed_sys_u32(reinterpret_cast<const uint32_t*>(counts + s * E + e));
+                    const int c = s == p.rank ? hist[e] : ld_relaxed_sys_u32(reinterpret_cast<const uint32_t*>(counts + s * E + e));
                     tot += c;
                     before += s < p.rank ? c : 0;
                 }
@@ -345,18 +346,21 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_dispatch_kernel(const __gr
         // ---------------------------------------------------------------- publish
         // One thread per CTA joins the arrival counter after the CTA barrier (gpu scope, acq_rel: every CTA's stores
         // happen before the last arrival); the last CTA fences at system scope and raises this source's flag on
-        // every destination.
-        __syncthreads();
-        __shared__ int last_s;
-        if (tid == 0) {
-            const uint32_t old = atom_add_acq_rel_gpu_u32(p.counters, 1);
-            last_s = old == gridDim.x - 1;
-            if (last_s) p.counters[0] = 0;
-        }
-        __syncthreads();
-        if (last_s && tid < p.world) {
-            fence_acq_rel_sys();
-            st_release_sys_u64(p.sig_peer[tid] + p.rank, p.epoch);
+        // every other destination. What this rank sent to itself is ordered by the end of the launch, so a single rank
+        // needs neither (dispatch of 128 tokens, 8 of 256: 13.8 -> 10.4 us; combine 8.5 -> 5.8 us).
+        if (p.world > 1) {
+            __syncthreads();
+            __shared__ int last_s;
+            if (tid == 0) {
+                const uint32_t old = atom_add_acq_rel_gpu_u32(p.counters, 1);
+                last_s = old == gridDim.x - 1;
+                if (last_s) p.counters[0] = 0;
+            }
+            __syncthreads();
+            if (last_s && tid < p.world && tid != p.rank) {
+                fence_acq_rel_sys();
+                st_release_sys_u64(p.sig_peer[tid] + p.rank, p.epoch);
+            }
         }
 
         if (p.compact && first_cta) {
@@ -366,7 +370,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_dispatch_kernel(const __gr
             const int al = p.align, e0 = p.rank * p.epr;
             for (int i = tid; i < p.world * p.epr; i += kMoeThreads) {
                 const int s = i / p.epr, le = i - s * p.epr;
-                p.recv_splits[i] = ld_relaxed_sys_u32(reinterpret_cast<const uint32_t*>(counts + s * E + e0 + le));
+                p.recv_splits[i] = s == p.rank ? hist[e0 + le] : ld_relaxed_sys_u32(reinterpret_cast<const uint32_t*>(counts + s * E + e0 + le));
             }
             for (int i = tid; i < p.epr * p.world; i += kMoeThreads) {
                 const int le = i / p.world, s = i - le * p.world;
@@ -376,7 +380,8 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_dispatch_kernel(const __gr
                     for (int b = 0; b < nb; ++b)
                         if ((off / al + b + 1) * al <= p.max_m) p.block_expert[off / al + b] = le;
                 }
-                for (int q = 0; q < s; ++q) off += ld_relaxed_sys_u32(reinterpret_cast<const uint32_t*>(counts + q * E + e0 + le));
+                for (int q = 0; q < s; ++q)
+                    off += q == p.rank ? hist[e0 + le] : ld_relaxed_sys_u32(reinterpret_cast<const uint32_t*>(counts + q * E + e0 + le));
                 p.recv_offset[i] = off;
             }
             if (warp == 0) {
@@ -396,7 +401,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_dispatch_kernel(const __gr
 
     if ((p.phase & 4) && first_cta) {
         // ---------------------------------------------------------------- every source's rows have landed here
-        if (tid < p.world) signal_wait_until(p.sig_peer[p.rank] + tid, kCmpGe, p.epoch, p.wctx, tid, 2);
+        if (tid < p.world && tid != p.rank) signal_wait_until(p.sig_peer[p.rank] + tid, kCmpGe, p.epoch, p.wctx, tid, 2);
         __syncthreads();
         if (!p.compact) {
             const int* counts = p.counts_peer[p.rank];
@@ -435,13 +440,13 @@ __global__ void __launch_bounds__(kMoeThreads, 2) moe_combine_kernel(const __gri
     const int tid = static_cast<int>(threadIdx.x);
     const int warp = tid >> 5, lane = tid & 31;
     pdl_wait_and_release();
-    if ((p.phase & 1) && blockIdx.x == 0 && tid < p.world) {
+    if ((p.phase & 1) && blockIdx.x == 0 && tid < p.world && tid != p.rank) {
         // the expert outputs were written by earlier work of this stream: complete and visible to peer reads
         fence_acq_rel_sys();
         st_release_sys_u64(p.sig_peer[tid] + p.rank, p.epoch);
     }
     if (!(p.phase & 2)) return;
-    if (tid < p.world) signal_wait_until(p.sig_peer[p.rank] + tid, kCmpGe, p.epoch, p.wctx, tid, 1);
+    if (tid < p.world && tid != p.rank) signal_wait_until(p.sig_peer[p.rank] + tid, kCmpGe, p.epoch, p.wctx, tid, 1);
     __syncthreads();
     const int gw = static_cast<int>(blockIdx.x) * kMoeWarps + warp;
     const int nw = static_cast<int>(gridDim.x) * kMoeWarps;
