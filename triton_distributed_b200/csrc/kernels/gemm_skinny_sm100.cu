@@ -12,6 +12,9 @@
 // then), and CTA r adds them in the order of K and writes bf16 / fp16 once. No workspace, no counters, no atomics, so
 // calls on any number of streams are independent and the result does not depend on timing.
 //
+// Measured, weights from HBM every time, before (128 x 256 tiles over all of K) and here: m16 n6144 k12288 77.9 us (1.9 TB/s)
+// and 27.3 us (5.5 TB/s); m16 n1024 k8192 52 and 9 us; m128 n4096 k4096 30 and 15 us; m16 n49152 k4096 79 and 69 us.
+//
 // Warps (192 threads): 0 = TMA producer, 1 = MMA issuer and TMEM owner, 2..5 = epilogue. One tile per CTA.
 #include <cuda.h>
 #include <cuda_bf16.h>
