@@ -300,3 +300,22 @@ def test_narrower_tiles_only_where_a_round_is_nearly_empty(cuda_device):
     assert _tile_width(8192, 49152, 12288) == 256       # many rounds
     assert _tile_width(1000, 5504, 4096) == 192         # 44 wide tiles of 2 x 256 on 74 pairs, or 60 of 2 x 192
     assert _tile_width(16, 6144, 12288) == 0            # few rows
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N", [(129, 8), (200, 1032), (1000, 4104)])
+@pytest.mark.parametrize("activation", ["gelu", "silu", "relu"])
+def test_activation_in_place_behind_the_large_tiles(cuda_device, M, N, activation, dtype):
+    """Above 128 rows the result is rounded, then activated in place: the values of torch's pass over the same result up
+    to an ulp, into `out` as well, and nothing past it."""
+    torch.manual_seed(M + N)
+    K = 264
+    a, b = _rand((M, K), dtype, cuda_device, 8.0), _rand((N, K), dtype, cuda_device, K ** -0.5)
+    ctx = G.create_ag_gemm_intra_node_context(a, b, 0, 1, max_M=M)
+    ref = G.apply_activation(G.ag_gemm_intra_node(a, b, ctx), activation)
+    guard = torch.full((M + 1, N), 7.0, dtype=dtype, device=cuda_device)
+    out = G.ag_gemm_intra_node(a, b, ctx, out=guard[:M], activation=activation)
+    check_status()
+    assert out.data_ptr() == guard.data_ptr() and (guard[M] == 7.0).all()
+    eps = 2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -10
+    torch.testing.assert_close(out.float(), ref.float(), atol=1e-6, rtol=eps)

@@ -223,6 +223,7 @@ def _declare(lib):
     lib.tdist_status_reset.argtypes = [C.c_void_p]
     lib.tdist_status_destroy.argtypes = [C.c_void_p]
     lib.tdist_gemm_run.argtypes = [C.POINTER(GemmArgs)]
+    lib.tdist_activate.argtypes = [C.c_void_p, C.c_longlong, C.c_int, C.c_int, C.c_void_p]
     lib.tdist_gemm_grid.argtypes = [C.POINTER(GemmArgs)]
     lib.tdist_gemm_tile_width.argtypes = [C.POINTER(GemmArgs)]
     lib.tdist_gemm_plan.argtypes = [C.POINTER(GemmArgs), C.POINTER(C.c_int)]

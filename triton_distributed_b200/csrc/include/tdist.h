@@ -131,6 +131,8 @@ typedef struct TdistGemmArgs {
 } TdistGemmArgs;
 
 int tdist_gemm_run(const TdistGemmArgs* args);
+/* h[0, n) = act(h) in place (fp32 inside; bf16 / fp16, 16-byte aligned, n a multiple of 8). */
+int tdist_activate(void* h, long long n, int dtype, int act, void* stream);
 /* Number of CTAs a call with these arguments launches (for occupancy planning and tests). */
 int tdist_gemm_grid(const TdistGemmArgs* args);
 /* The launch plan of a call with these arguments: out4 = {CTAs per tile (1 or 2), wide tiling (0 / 1), pusher CTAs,

@@ -177,7 +177,8 @@ def ag_gemm_intra_node(a: torch.Tensor, b: torch.Tensor, ctx: Optional[AllGather
                        out: Optional[torch.Tensor] = None, activation: Optional[str] = None) -> torch.Tensor:
     """``allgather(a) @ b.T``: ``a`` is this rank's ``[M/ws, K]`` row shard, ``b`` this rank's
     ``[N/ws, K]`` weight shard; returns ``[M, N/ws]``. ``activation`` ("gelu" in its tanh form, "silu", "relu") is applied
-    to it: by the epilogue, on the fp32 sums, for the 128 rows of a decode step of one rank; as a pass of its own otherwise."""
+    to it: by the epilogue, on the fp32 sums, for the 128 rows of a decode step of one rank; in place by a kernel of its own
+    otherwise."""
     if ctx is None:
         if rank is None or num_ranks is None:
             raise ValueError("ag_gemm_intra_node needs a context or rank and num_ranks")
@@ -216,8 +217,7 @@ def ag_gemm_intra_node(a: torch.Tensor, b: torch.Tensor, ctx: Optional[AllGather
             g.a_ws_mc = ctx.workspace.mc[half].data_ptr()   # the pushers multicast through the switch
     _launch(g)
     if activation is not None and not fused:
-        act = apply_activation(c, activation)
-        return act if out is None else out.copy_(act)
+        _lib.check(_lib.lib().tdist_activate(c.data_ptr(), c.numel(), g.dtype, _lib.ACTIVATIONS[activation], g.stream), "tdist_activate")
     return c
 
 
