@@ -1,4 +1,4 @@
-// Activation of a GEMM's result in place, for the results whose epilogue does not apply it (gemm_sm100.cu says why).
+// Activation of a GEMM's result in place, for the results whose epilogue does not apply it (device/act.cuh says why).
 //
 // Bound by the trip of the values: the GEMM has just written them, so up to the size of L2 they are read and written there,
 // which a pass into a second buffer gives away. Two special-function results per value (device/act.cuh) come second: 13 us
