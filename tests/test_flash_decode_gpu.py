@@ -166,6 +166,27 @@ def test_splits_meet_in_the_ring_or_in_global_memory(cuda_device, splits, Hq, Hk
         torch.testing.assert_close(out.float(), ref, atol=2e-2, rtol=2e-2)
 
 
+@pytest.mark.parametrize("B", [1, 2])
+@pytest.mark.parametrize("splits", [2, 10])          # one cluster per (batch, kv head); through global memory
+@pytest.mark.parametrize("blocks_over", [0, 1])      # 2560 keys per CTA and just above: with and without the early launch
+def test_a_decode_reads_the_result_of_the_one_before(cuda_device, B, splits, blocks_over):
+    """Calls in a row whose queries are the outputs of the call before, not synchronised in between."""
+    torch.manual_seed(B + splits)
+    Hq, Hkv, D, page = 32, 8, 128, 16
+    per = splits * (2560 // page + blocks_over)
+    lens = [per * page, 37][:B]
+    k = torch.randn(B * per, page, Hkv, D, device=cuda_device).to(torch.bfloat16)
+    v = torch.randn(B * per, page, Hkv, D, device=cuda_device).to(torch.bfloat16)
+    table = torch.randperm(B * per, device=cuda_device).to(torch.int32).view(B, per)
+    kv = torch.tensor(lens, dtype=torch.int32, device=cuda_device)
+    qs = [4 * torch.randn(B, Hq, D, device=cuda_device).to(torch.bfloat16)]
+    for _ in range(5):
+        qs.append(FD.gqa_fwd_batch_decode(qs[-1], k, v, None, None, kv, table, D ** -0.5, kv_split=splits))
+    check_status()
+    for q, out in zip(qs, qs[1:]):
+        torch.testing.assert_close(out.float(), FD.ref_paged_attn(q, k, v, kv, table, D ** -0.5), atol=2e-2, rtol=2e-2)
+
+
 def test_batch_splits_fill_the_last_wave_and_even_out_lengths():
     assert FD._batch_splits(32 * 8, 8192, 128, 148, 1) == 2        # ragged batches gain, full ones lose next to nothing
     assert FD._batch_splits(8 * 8, 32768, 128, 148, 4) == 4        # one wave of 256 CTAs is hard to beat

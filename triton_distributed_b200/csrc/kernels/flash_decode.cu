@@ -541,6 +541,22 @@ using tdist_host::fail;
 // with 8 / 4 splits).
 constexpr int kClusterMergeMaxSplits = 8;
 
+// Longest key range per CTA with which a batch of several sequences, all of whose CTAs run at once, overlaps the launch
+// before it. CTAs that take their places as that launch's finish sit where its short sequences were, so that two long
+// ones may share an SM; where the lengths are equal or a second round evens them out this does not matter. Batch 2,
+// lengths ragged up to kv, 18 splits, us per call without / with the overlap: kv 20000 (1111 keys per CTA) 35.4 / 33.8,
+// 40000 (2222) 55.5 / 54.8, 60000 (3333) 75.0 / 75.5, 80000 (4444) 95.7 / 96.5, 110000 (6111) 123.5 / 128.1; 64 query
+// heads, 158353 (8797) 177.5 / 186.6. Batch 1, 200000 keys: 143.5 / 138.0; batch 41, 11127 keys (several rounds): 182.4 /
+// 179.5. The lengths are not known on the host: batch 8 of equal 32768 (8192) would gain too, 173.8 / 171.5.
+constexpr long long kOverlapKeys = 2560;
+
+// Whether the CTAs may take their places while the launch before still runs (programmatic dependent launch).
+static bool overlaps_previous(const DecodeParams& p) {
+    const long long ctas = static_cast<long long>(p.B) * p.Hkv * p.splits;
+    const long long keys = static_cast<long long>(p.max_blocks) * p.page_size / p.splits;
+    return p.B == 1 || keys <= kOverlapKeys || ctas > 2LL * tdist_host::sm_count();
+}
+
 template <typename T, int D>
 static int launch_decode(DecodeParams& p, cudaStream_t stream) {
     constexpr int NS = decode_stages(D);
@@ -573,15 +589,14 @@ static int launch_decode(DecodeParams& p, cudaStream_t stream) {
     cfg.stream = stream;
     cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute attr[2];
-    attr[0] = tdist_host::pdl_attribute();
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    if (overlaps_previous(p)) attr[cfg.numAttrs++] = tdist_host::pdl_attribute();
     if (cluster) {
-        attr[1].id = cudaLaunchAttributeClusterDimension;
-        attr[1].val.clusterDim.x = static_cast<unsigned>(p.splits);
-        attr[1].val.clusterDim.y = 1;
-        attr[1].val.clusterDim.z = 1;
-        cfg.numAttrs = 2;
+        cudaLaunchAttribute& dim = attr[cfg.numAttrs++];
+        dim.id = cudaLaunchAttributeClusterDimension;
+        dim.val.clusterDim.x = static_cast<unsigned>(p.splits);
+        dim.val.clusterDim.y = 1;
+        dim.val.clusterDim.z = 1;
     }
     p.cluster_merge = cluster ? 1 : 0;
     TDIST_CUDA_OK(cudaLaunchKernelEx(&cfg, flash_decode_kernel<T, D>, p));
