@@ -316,3 +316,64 @@ def test_dispatch_sorts_the_pairs_stably(cuda_device, T, topk, E, align):
         assert int(ctx.num_blocks) == blocks
         want = torch.repeat_interleave(torch.arange(E, device=cuda_device), padded // align)
         assert torch.equal(ctx.block_expert[:blocks].long(), want)
+
+
+@pytest.mark.parametrize("compact", [False, True])
+def test_halves_launched_apart_meet_at_the_own_flag(cuda_device, monkeypatch, compact):
+    """One rank. The wait half must not return before the send half has raised this rank's flag: with nothing sent it gives
+    up after its limit and names the rank; after the send half (synchronised: the two never run at once) it finds flag,
+    counts and rows, from another stream."""
+    from triton_distributed_b200.ops import moe_ep as EP
+    from triton_distributed_b200.runtime import global_status
+    monkeypatch.setenv("TDIST_WAIT_TIMEOUT_MS", "50")
+    torch.manual_seed(3)
+    T, hidden, E, k = 33, 256, 8, 2
+    x = torch.randn(T, hidden, device=cuda_device).to(torch.bfloat16)
+    ids = torch.stack([torch.randperm(E, device=cuda_device)[:k] for _ in range(T)]).to(torch.int32)
+    ctx = EP.create_ep_context(T, hidden, k, E, 0, 1, quant=False, compact=compact, heap=LocalWorld(1, cuda_device).heap(0))
+
+    ctx.topk_ids, ctx.ntok = ids, T
+
+    def gives_up(launch):
+        launch()
+        torch.cuda.synchronize()
+        rec = global_status().record
+        assert (rec.abort_flag, rec.code, rec.peer) == (1, 1, 0)
+        with pytest.raises(Exception, match="timed out"):
+            check_status()
+
+    send, wait = torch.cuda.Stream(), torch.cuda.Stream()
+    for call in (1, 2):
+        # as a wait half sees it that reaches the GPU before the send half of its call
+        ctx.call_count += 1
+        gives_up(lambda: EP.ep_dispatch(ctx, x, ids, None, phase=4))
+        if compact:
+            gives_up(lambda: EP.ep_dispatch(ctx, x, ids, None, phase=6))   # the counts' flag
+        ctx.call_count -= 1
+        torch.cuda.synchronize()
+        EP.ep_dispatch(ctx, x, ids, None, phase=3, stream=send)
+        send.synchronize()
+        assert int(ctx.sig.local[0]) == ctx.call_count == call
+        rows, _, splits, num = EP.ep_dispatch(ctx, x, ids, None, phase=4, stream=wait)
+        wait.synchronize()
+        check_status()
+        order = torch.sort(ids.reshape(-1).long(), stable=True).indices
+        assert torch.equal(rows[: T * k], x[order // k]) and int(num) == T * k
+        assert torch.equal(splits.view(-1).long(), torch.bincount(ids.reshape(-1).long(), minlength=E))
+        ctx.combine_count += 1
+        gives_up(lambda: EP.ep_combine(ctx, weighted=False, phase=2))
+        ctx.combine_count -= 1
+        out = torch.zeros(T, hidden, dtype=torch.bfloat16, device=cuda_device)
+        EP.ep_combine(ctx, rows, weighted=False, phase=1)
+        torch.cuda.synchronize()
+        assert int(ctx.comb_sig.local[0]) == ctx.combine_count
+        EP.ep_combine(ctx, weighted=False, out=out, phase=2, stream=wait)
+        wait.synchronize()
+        check_status()
+        torch.testing.assert_close(out.float(), k * x.float(), rtol=2.0 ** -8, atol=0)
+    # whole calls in between leave the flags behind; halves after them still meet at theirs
+    EP.ep_dispatch(ctx, x, ids, None)
+    EP.ep_dispatch(ctx, x, ids, None, phase=3)
+    EP.ep_dispatch(ctx, x, ids, None, phase=4)
+    check_status()
+    assert int(ctx.sig.local[0]) == ctx.call_count

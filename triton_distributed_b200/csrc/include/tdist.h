@@ -319,7 +319,9 @@ typedef struct TdistMoeDispatchArgs {
     int quant;     /* 1 = rows travel as fp8 e4m3 with one fp32 scale per 128 values, 0 = as bf16 */
     int compact;   /* 0 = per-source slots [world][max_m], 1 = rows grouped by (local expert, source) back to back */
     int align;     /* compact: every expert's group starts on a multiple of this many rows (0/1 = dense, 128 = grouped GEMM) */
-    int phase;     /* bit 0 publish counts (compact), bit 1 route + send + flag, bit 2 wait for every source; 0 = all */
+    int phase;     /* bit 0 publish counts (compact), bit 1 route + send + flag, bit 2 wait for every source; 0 = all.
+                      A launch that both raises and awaits this rank's own flag leaves it out; halves launched apart, on
+                      whatever streams, meet at the flag, this rank's own included */
     int num_ctas;  /* 0 = sized from the work */
     uint64_t epoch;           /* call number, > 0, the same on every rank */
     void* status;
@@ -335,7 +337,7 @@ typedef struct TdistMoeCombineArgs {
     const void* pair_row;     /* from the matching dispatch */
     void* out;                /* [ntok, hidden] bf16 */
     int ntok, topk, hidden, epr, world, rank;
-    int phase;                /* bit 0 announce, bit 1 wait + gather; 0 = both */
+    int phase;                /* bit 0 announce, bit 1 wait + gather; 0 = both (own flag as above) */
     int num_ctas;
     uint64_t epoch;
     void* status;

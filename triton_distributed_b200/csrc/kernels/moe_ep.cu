@@ -159,6 +159,11 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_dispatch_kernel(const __gr
     const int warp = tid >> 5, lane = tid & 31;
     const bool first_cta = blockIdx.x == 0;
     const int run = (n + kMoeThreads - 1) / kMoeThreads * 32;   // pairs a warp sorts
+    // A rank raises its own flags and waits for them like everybody else's, except where one launch does both: then the order
+    // inside the launch and its end take their place (dispatch of 128 tokens, 8 of 256, one rank: 13.8 -> 10.4 us; combine
+    // 8.5 -> 5.8 us). Halves launched apart may be on two streams, which only the flag orders.
+    const bool skip_own_counts = (p.phase & 3) == 3;
+    const bool skip_own_rows = (p.phase & 6) == 6;
 
     // The rows do not depend on the routing: this warp's first (token, segment) item is loaded now, so that its
     // memory round trip runs under the sort below.
@@ -221,7 +226,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_dispatch_kernel(const __gr
             p.counts_peer[d][p.rank * E + e] = hist[e];
         }
         __syncthreads();
-        if (tid < p.world && tid != p.rank) {
+        if (tid < p.world && !(tid == p.rank && skip_own_counts)) {
             fence_acq_rel_sys();
             st_release_sys_u64(p.sig_peer[tid] + p.world + p.rank, p.epoch);
         }
@@ -230,8 +235,8 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_dispatch_kernel(const __gr
     if (p.phase & 2) {
         // ---------------------------------------------------------------- start row of each expert's group at its owner
         if (p.compact) {
-            // (every CTA counted this rank's own pairs itself: nothing to wait for there)
-            if (tid < p.world && tid != p.rank) signal_wait_until(p.sig_peer[p.rank] + p.world + tid, kCmpGe, p.epoch, p.wctx, tid, 1);
+            // (every CTA counted this rank's own pairs itself: of its own flag only the order between streams matters)
+            if (tid < p.world && !(tid == p.rank && skip_own_counts)) signal_wait_until(p.sig_peer[p.rank] + p.world + tid, kCmpGe, p.epoch, p.wctx, tid, 1);
             __syncthreads();
             const int* counts = p.counts_peer[p.rank];   // [world][E], the other ranks' rows complete after the waits above
             for (int e = tid; e < E; e += kMoeThreads) {
@@ -346,9 +351,8 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_dispatch_kernel(const __gr
         // ---------------------------------------------------------------- publish
         // One thread per CTA joins the arrival counter after the CTA barrier (gpu scope, acq_rel: every CTA's stores
         // happen before the last arrival); the last CTA fences at system scope and raises this source's flag on
-        // every other destination. What this rank sent to itself is ordered by the end of the launch, so a single rank
-        // needs neither (dispatch of 128 tokens, 8 of 256: 13.8 -> 10.4 us; combine 8.5 -> 5.8 us).
-        if (p.world > 1) {
+        // every destination.
+        if (p.world > 1 || !skip_own_rows) {
             __syncthreads();
             __shared__ int last_s;
             if (tid == 0) {
@@ -357,7 +361,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_dispatch_kernel(const __gr
                 if (last_s) p.counters[0] = 0;
             }
             __syncthreads();
-            if (last_s && tid < p.world && tid != p.rank) {
+            if (last_s && tid < p.world && !(tid == p.rank && skip_own_rows)) {
                 fence_acq_rel_sys();
                 st_release_sys_u64(p.sig_peer[tid] + p.rank, p.epoch);
             }
@@ -401,7 +405,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_dispatch_kernel(const __gr
 
     if ((p.phase & 4) && first_cta) {
         // ---------------------------------------------------------------- every source's rows have landed here
-        if (tid < p.world && tid != p.rank) signal_wait_until(p.sig_peer[p.rank] + tid, kCmpGe, p.epoch, p.wctx, tid, 2);
+        if (tid < p.world && !(tid == p.rank && skip_own_rows)) signal_wait_until(p.sig_peer[p.rank] + tid, kCmpGe, p.epoch, p.wctx, tid, 2);
         __syncthreads();
         if (!p.compact) {
             const int* counts = p.counts_peer[p.rank];
@@ -440,13 +444,14 @@ __global__ void __launch_bounds__(kMoeThreads, 2) moe_combine_kernel(const __gri
     const int tid = static_cast<int>(threadIdx.x);
     const int warp = tid >> 5, lane = tid & 31;
     pdl_wait_and_release();
-    if ((p.phase & 1) && blockIdx.x == 0 && tid < p.world && tid != p.rank) {
+    const bool skip_own = (p.phase & 3) == 3;   // as in the dispatch kernel
+    if ((p.phase & 1) && blockIdx.x == 0 && tid < p.world && !(tid == p.rank && skip_own)) {
         // the expert outputs were written by earlier work of this stream: complete and visible to peer reads
         fence_acq_rel_sys();
         st_release_sys_u64(p.sig_peer[tid] + p.rank, p.epoch);
     }
     if (!(p.phase & 2)) return;
-    if (tid < p.world && tid != p.rank) signal_wait_until(p.sig_peer[p.rank] + tid, kCmpGe, p.epoch, p.wctx, tid, 1);
+    if (tid < p.world && !(tid == p.rank && skip_own)) signal_wait_until(p.sig_peer[p.rank] + tid, kCmpGe, p.epoch, p.wctx, tid, 1);
     __syncthreads();
     const int gw = static_cast<int>(blockIdx.x) * kMoeWarps + warp;
     const int nw = static_cast<int>(gridDim.x) * kMoeWarps;

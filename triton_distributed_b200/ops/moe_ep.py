@@ -161,7 +161,8 @@ def ep_dispatch(ctx: EPContext, x: torch.Tensor, topk_ids: torch.Tensor, topk_we
     valid for work enqueued before the next dispatch on this context.
 
     ``phase`` (for running emulated ranks one after the other): bit 0 publishes this rank's per-expert counts
-    (compact layout only), bit 1 routes, sends and raises the flags, bit 2 waits for every source."""
+    (compact layout only), bit 1 routes, sends and raises the flags, bit 2 waits for every source (this rank included when
+    the halves are launched apart, so that they may be on different streams)."""
     global launch_count
     T = x.shape[0]
     if T > ctx.max_tokens:
