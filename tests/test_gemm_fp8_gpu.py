@@ -52,6 +52,69 @@ def test_rowwise_quantiser_gives_the_bytes_of_its_torch_statement(cuda_device, M
     torch.testing.assert_close(s, st, rtol=0, atol=0, equal_nan=True)
 
 
+def _quantised_values(x):
+    q, s = F.quantize_fp8_rowwise(x)
+    return q.float(), s
+
+
+@pytest.mark.parametrize("how", ["jit.trace", "compile", "vmap", "jvp", "grad", "functionalize", "dispatch mode", "saved tensor hooks"])
+def test_rowwise_quantiser_is_torch_operations_to_whoever_traces_it(cuda_device, how):
+    """The one-pass kernel stands in for torch operations only where nothing has to see them; every tracer and transform gets
+    the values of the statement in torch operations, on inputs other than the ones it was traced with too."""
+    g = torch.Generator(device="cpu").manual_seed(7)
+    x, other = (torch.randn(6, 256, generator=g).to(cuda_device) for _ in range(2))
+    want_q, want_s = F._quantize_rowwise_torch(other)
+    want = (want_q.float(), want_s)
+    if how == "jit.trace":
+        got = torch.jit.trace(_quantised_values, (x,), check_trace=False)(other)
+    elif how == "compile":
+        got = torch.compile(_quantised_values, backend="eager", fullgraph=True)(other)
+    elif how == "vmap":
+        got = tuple(t.flatten(0, 1) for t in torch.vmap(_quantised_values)(other.view(2, 3, 256)))
+    elif how == "jvp":
+        # the scale is the largest magnitude / 448, so along x itself its derivative is the scale
+        primal, tangent = torch.func.jvp(lambda v: F.quantize_fp8_rowwise(v)[1], (other,), (other,))
+        torch.testing.assert_close(tangent, primal, rtol=1e-6, atol=0)
+        got = (want[0], primal)
+    elif how == "grad":
+        leaf = other.clone().requires_grad_()
+        F.quantize_fp8_rowwise(leaf)[1].sum().backward()
+        top = other.view(6, 2, 128).abs() == other.view(6, 2, 128).abs().amax(-1, keepdim=True)
+        torch.testing.assert_close(leaf.grad.view(6, 2, 128), top * other.view(6, 2, 128).sign() / 448.0, rtol=1e-6, atol=0)
+        return
+    elif how == "functionalize":
+        got = torch.func.functionalize(_quantised_values)(other)
+    elif how == "dispatch mode":
+        from torch.utils._python_dispatch import TorchDispatchMode
+        seen = []
+
+        class Log(TorchDispatchMode):
+            def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+                seen.append(str(func))
+                return func(*args, **(kwargs or {}))
+
+        with Log():
+            got = _quantised_values(other)
+        assert any("amax" in f for f in seen)
+    else:
+        packed = []
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t.shape) or t, lambda t: t):
+            q, s = F.quantize_fp8_rowwise(other.clone().requires_grad_())
+        assert packed
+        got = (q.float(), s)
+    for have, need in zip(got, want):
+        torch.testing.assert_close(have, need, rtol=0, atol=0)
+
+
+def test_rowwise_quantiser_takes_the_kernel_for_plain_tensors(cuda_device):
+    from triton_distributed_b200.utils.misc import plain_cuda
+    x = torch.randn(4, 128, device=cuda_device)
+    assert plain_cuda(x) and plain_cuda(torch.nn.Parameter(x, requires_grad=False))
+    with torch.no_grad():
+        assert plain_cuda(torch.nn.Parameter(x))
+    assert not plain_cuda(torch.nn.Parameter(x)) and not plain_cuda(x.t()) and not plain_cuda(x.flatten()[1:]) and not plain_cuda(x.cpu())
+
+
 @pytest.mark.parametrize("M,N,K", [(128, 256, 128), (256, 512, 512), (300, 264, 384), (1000, 1000, 896), (4096, 768, 2048)])
 def test_plain_fp8_gemm_matches_fp32_reference(cuda_device, M, N, K):
     a, sa, b, sb = _operands(M, N, K, cuda_device, M + N + K)

@@ -44,7 +44,7 @@ def quantize_fp8_rowwise(x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
     M, K = x.shape
     if K % 128:
         raise ValueError("K must be a multiple of 128")
-    if x.dtype in _QUANT_DTYPES and x.numel() > 0 and plain_cuda(x):
+    if plain_cuda(x) and x.dtype in _QUANT_DTYPES and x.numel() > 0:
         # one pass; the same bytes as the statement below, which everything else takes (CPU, strided, traced tensors)
         q = torch.empty((M, K), dtype=FP8, device=x.device)
         scale = torch.empty((M, K // 128), dtype=torch.float32, device=x.device)

@@ -71,8 +71,8 @@ def gate_topk(x: torch.Tensor, gate: torch.Tensor, topk: int, renormalize: bool 
     global launch_count
     T, hidden = x.shape
     E = gate.shape[0]
-    if x.dtype == gate.dtype == torch.bfloat16 and T > 0 and hidden >= 32 and hidden % 32 == 0 and 1 <= topk <= min(32, E) and E <= 1024 \
-            and gate.shape[1] == hidden and plain_cuda(x, gate):
+    if plain_cuda(x, gate) and x.dtype == gate.dtype == torch.bfloat16 and T > 0 and hidden >= 32 and hidden % 32 == 0 \
+            and 1 <= topk <= min(32, E) and E <= 1024 and gate.shape[1] == hidden:
         ids = torch.empty((T, topk), dtype=torch.int32, device=x.device)
         w = torch.empty((T, topk), dtype=torch.float32, device=x.device)
         _lib.check(_lib.lib().tdist_moe_gate_topk(x.data_ptr(), gate.data_ptr(), T, hidden, E, topk, int(renormalize), ids.data_ptr(),

@@ -295,7 +295,12 @@ def get_numa_node(gpu_index: int = 0) -> int:
 def plain_cuda(*tensors: torch.Tensor) -> bool:
     """True when a raw-pointer kernel may stand in for torch operations on ``tensors``: dense CUDA tensors of the current
     device, 16-byte aligned, whose operations nothing else has to see (no autograd or forward-mode graph, no vmap / functorch
-    wrapper, no tensor subclass, no dispatch mode or compilation in progress)."""
+    wrapper, no tensor subclass, no dispatch mode, tracing or compilation in progress)."""
+    # first: a compiler can trace none of the questions below, and a tracer would record a result that nothing fills
+    if torch.compiler.is_compiling() or torch._C._get_tracing_state() is not None:
+        return False
+    if torch.utils._python_dispatch._get_current_dispatch_mode() is not None:
+        return False
     device = -1
     for t in tensors:
         if t.device.type != "cuda" or type(t) not in (torch.Tensor, torch.nn.Parameter) or torch._C._functorch.is_functorch_wrapped_tensor(t):
@@ -310,4 +315,4 @@ def plain_cuda(*tensors: torch.Tensor) -> bool:
             return False
         if t.is_conj() or t.is_neg() or t.data_ptr() % 16:
             return False
-    return not torch.compiler.is_compiling() and torch.utils._python_dispatch._get_current_dispatch_mode() is None
+    return True
