@@ -268,6 +268,36 @@ def test_gate_topk_is_no_further_from_float64_than_the_fp32_product(cuda_device,
     torch.testing.assert_close(w, w_t, rtol=1e-6, atol=0)
 
 
+@pytest.mark.parametrize("form", ["bf16", "strided", "misaligned", "short", "cpu"])
+def test_gate_topk_writes_logits_of_any_form_or_refuses_them(cuda_device, form):
+    """Only a dense fp32 [T, E] buffer may be handed to the kernel as a pointer; the others are copied into, converted and
+    strided as they are, or refused, and nothing around them is written."""
+    torch.manual_seed(5)
+    T, hidden, E, k = 9, 64, 16, 2
+    x = torch.randn(T, hidden, device=cuda_device).bfloat16()
+    gate = torch.randn(E, hidden, device=cuda_device).bfloat16()
+    want = x.double() @ gate.double().t()
+    room = torch.full((4 * T * E,), 7.0, dtype=torch.bfloat16 if form == "bf16" else torch.float32, device="cpu" if form == "cpu" else cuda_device)
+    if form == "strided":
+        logits = room.view(2 * T, 2 * E)[:T, ::2]
+    elif form == "misaligned":
+        logits = room[1: 1 + T * E].view(T, E)
+    elif form == "short":
+        logits = room[: (T - 1) * E].view(T - 1, E)
+        with pytest.raises(RuntimeError):
+            MU.gate_topk(x, gate, k, logits=logits)
+        assert (room == 7.0).all()
+        return
+    else:
+        logits = room[: T * E].view(T, E)
+    ids, _ = MU.gate_topk(x, gate, k, logits=logits)
+    # fp32 sums of 64 products, then the buffer's rounding
+    torch.testing.assert_close(logits.double().cpu(), want.cpu(), rtol=2.0 ** -8 if form == "bf16" else 1e-5, atol=1e-5)
+    assert torch.equal(ids.long(), want.topk(k, -1).indices)
+    logits.fill_(7.0)
+    assert (room == 7.0).all()
+
+
 @pytest.mark.parametrize("T,k,hidden", [(1, 1, 8), (5, 2, 1024), (64, 3, 1032), (7, 8, 7168), (300, 2, 4096), (2, 1, 1016)])
 def test_topk_reduce_over_ragged_rows_and_rejected_pairs(cuda_device, T, k, hidden):
     torch.manual_seed(T + hidden)

@@ -67,12 +67,13 @@ def topk_softmax(logits: torch.Tensor, topk: int, renormalize: bool = False) -> 
 def gate_topk(x: torch.Tensor, gate: torch.Tensor, topk: int, renormalize: bool = False,
               logits: Optional[torch.Tensor] = None) -> Tuple[torch.Tensor, torch.Tensor]:
     """:func:`topk_softmax` of ``x[T, hidden] @ gate[E, hidden].T`` with fp32 sums; one launch for bf16 operands.
-    ``logits`` (fp32 ``[T, E]``), if given, receives the product."""
+    ``logits`` (``[T, E]``), if given, receives the product; the launch writes it only as dense fp32."""
     global launch_count
     T, hidden = x.shape
     E = gate.shape[0]
-    if plain_cuda(x, gate) and x.dtype == gate.dtype == torch.bfloat16 and T > 0 and hidden >= 32 and hidden % 32 == 0 \
-            and 1 <= topk <= min(32, E) and E <= 1024 and gate.shape[1] == hidden:
+    fits = logits is None or (logits.dtype == torch.float32 and logits.shape == (T, E) and plain_cuda(x, logits))
+    if fits and plain_cuda(x, gate) and x.dtype == gate.dtype == torch.bfloat16 and T > 0 and hidden >= 32 \
+            and hidden % 32 == 0 and 1 <= topk <= min(32, E) and E <= 1024 and gate.shape[1] == hidden:
         ids = torch.empty((T, topk), dtype=torch.int32, device=x.device)
         w = torch.empty((T, topk), dtype=torch.float32, device=x.device)
         _lib.check(_lib.lib().tdist_moe_gate_topk(x.data_ptr(), gate.data_ptr(), T, hidden, E, topk, int(renormalize), ids.data_ptr(),
