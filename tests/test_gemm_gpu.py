@@ -319,3 +319,14 @@ def test_activation_in_place_behind_the_large_tiles(cuda_device, M, N, activatio
     assert out.data_ptr() == guard.data_ptr() and (guard[M] == 7.0).all()
     eps = 2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -10
     torch.testing.assert_close(out.float(), ref.float(), atol=1e-6, rtol=eps)
+
+
+@pytest.mark.parametrize("M", [64, 256])
+def test_an_unknown_activation_launches_nothing(cuda_device, M):
+    a, b = _rand((M, 64), torch.bfloat16, cuda_device), _rand((8, 64), torch.bfloat16, cuda_device)
+    ctx = G.create_ag_gemm_intra_node_context(a, b, 0, 1, max_M=M)
+    out = torch.full((M, 8), 7.0, dtype=torch.bfloat16, device=cuda_device)
+    with pytest.raises(ValueError, match="unknown activation"):
+        G.ag_gemm_intra_node(a, b, ctx, out=out, activation="typo")
+    torch.cuda.synchronize()
+    assert ctx.epoch == 0 and (out == 7.0).all()

@@ -395,3 +395,13 @@ def test_small_utilities_of_the_reference(tmp_path):
     (dev / "numa_node").write_text("1\n")
     assert U.NvidiaSmiUtil.numa_node_of_bus_id("00000000:17:00.0\n", str(tmp_path)) == 1
     assert U.NvidiaSmiUtil.numa_node_of_bus_id("00000000:99:00.0", str(tmp_path)) == -1
+
+
+def test_an_unknown_activation_is_refused_before_anything_runs():
+    from triton_distributed_b200.ops import gemm as G, moe_tp as MT
+    a, b = torch.ones(4, 8), torch.ones(8, 8)
+    ctx = G.create_ag_gemm_intra_node_context(a, b, 0, 1, max_M=4)
+    with pytest.raises(ValueError, match="unknown activation"):
+        G.ag_gemm_intra_node(a, b, ctx, activation="typo")
+    with pytest.raises(ValueError, match="unknown activation"):
+        MT.group_gemm(torch.ones(128, 8), b.view(1, 8, 8), torch.zeros(1, dtype=torch.int32), activation="typo")

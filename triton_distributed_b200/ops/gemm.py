@@ -185,6 +185,7 @@ def ag_gemm_intra_node(a: torch.Tensor, b: torch.Tensor, ctx: Optional[AllGather
         ctx = create_ag_gemm_intra_node_context(a, b, rank, num_ranks)
     mpr, K = a.shape
     N = b.shape[0]
+    act = activation_code(activation)   # an unknown name is refused before anything runs
     if a.device.type != "cuda":
         return apply_activation(_ag_gemm_cpu(a, b, ctx), activation)
     _check_operands(a, b)
@@ -196,7 +197,7 @@ def ag_gemm_intra_node(a: torch.Tensor, b: torch.Tensor, ctx: Optional[AllGather
     g.m_per_rank = mpr
     fused = activation is not None and ctx.world == 1 and mpr <= BLOCK_M_TILE and g.cta_pair <= 0
     if fused:
-        g.act = _lib.ACTIVATIONS[activation]
+        g.act = act
     ctx.epoch += 1
     g.epoch = ctx.epoch
     g.num_sms = ctx.num_sms
@@ -217,8 +218,14 @@ def ag_gemm_intra_node(a: torch.Tensor, b: torch.Tensor, ctx: Optional[AllGather
             g.a_ws_mc = ctx.workspace.mc[half].data_ptr()   # the pushers multicast through the switch
     _launch(g)
     if activation is not None and not fused:
-        _lib.check(_lib.lib().tdist_activate(c.data_ptr(), c.numel(), g.dtype, _lib.ACTIVATIONS[activation], g.stream), "tdist_activate")
+        _lib.check(_lib.lib().tdist_activate(c.data_ptr(), c.numel(), g.dtype, act, g.stream), "tdist_activate")
     return c
+
+
+def activation_code(activation: Optional[str]) -> int:
+    if activation not in _lib.ACTIVATIONS:
+        raise ValueError(f"unknown activation {activation!r}: one of {[k for k in _lib.ACTIVATIONS if k]} or None")
+    return _lib.ACTIVATIONS[activation]
 
 
 def apply_activation(h: torch.Tensor, activation: Optional[str]) -> torch.Tensor:

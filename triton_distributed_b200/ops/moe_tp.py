@@ -128,6 +128,7 @@ def group_gemm(a_sorted: torch.Tensor, b: torch.Tensor, expert_ids: torch.Tensor
     an int32 device scalar (blocks past it are padding and are skipped). ``activation`` ("gelu" in its tanh form, "silu",
     "relu") is applied to the fp32 sums by the epilogue. ``max_blocks``: the most live blocks the caller knows of (0 = all
     of ``a_sorted``); the tile is chosen for that many."""
+    act = G.activation_code(activation)
     rows, K = a_sorted.shape
     E, N, _ = b.shape
     if rows % GROUP_BLOCK_M:
@@ -149,7 +150,7 @@ def group_gemm(a_sorted: torch.Tensor, b: torch.Tensor, expert_ids: torch.Tensor
     g.expert_ids = expert_ids.data_ptr()
     g.num_m_blocks = num_blocks.data_ptr() if num_blocks is not None else None
     g.num_experts = E
-    g.act = _lib.ACTIVATIONS[activation]
+    g.act = act
     g.max_m_blocks = max_blocks
     G._launch(g)
     return c
