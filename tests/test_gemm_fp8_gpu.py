@@ -189,3 +189,22 @@ def test_few_row_fp8_gemm_matches_fp32_reference(cuda_device, N, K):
         assert (guard[M] == 7.0).all()
         again = F.gemm_fp8_blockscaled(a, sa, b, sb, num_sms=148)   # the large tiles
         torch.testing.assert_close(again.double(), ref, rtol=2.0 ** -8, atol=1e-5 * ref.abs().max().item())
+
+
+@pytest.mark.parametrize("M,N,K", [(128, 512, 256), (300, 1000, 4096)])
+def test_fp8_pipeline_stays_whole_when_a_flag_wait_is_abandoned(cuda_device, monkeypatch, M, N, K):
+    """As for the bf16 product: the kernel runs to its end in step and reports the flag and its peer."""
+    monkeypatch.setenv("TDIST_WAIT_TIMEOUT_MS", "50")
+    from triton_distributed_b200.runtime import global_status
+    a, sa, b, sb = _operands(M, N, K, cuda_device, M)
+    ref = F.dequantize_fp8(a, sa, 1).float() @ F.dequantize_fp8(b, sb, 128).float().t()
+    lw = LocalWorld(2, cuda_device)
+    ctxs = [F.create_ag_gemm_fp8_context(2 * M, K, r, 2, heap=lw.heap(r)) for r in range(2)]
+    for _ in range(3):
+        out = F.ag_gemm_fp8(a, sa, b, sb, ctxs[0])
+        torch.cuda.synchronize()
+        rec = global_status().record
+        assert (rec.abort_flag, rec.code, rec.peer) == (1, 1, 1)
+        torch.testing.assert_close(out[:M].float(), ref, atol=3e-2, rtol=2e-2)
+        with pytest.raises(Exception, match="timed out"):
+            check_status()

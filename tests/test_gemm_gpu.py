@@ -132,6 +132,43 @@ def test_abandoned_wait_reports_timeout_and_leaves_the_context_usable(cuda_devic
     torch.testing.assert_close(c.float(), a.float() @ b.float().t(), atol=2e-2, rtol=2e-2)
 
 
+@pytest.mark.parametrize("kind", ["ag", "rs"])
+@pytest.mark.parametrize("tiling", [0, 1, 2])
+@pytest.mark.parametrize("mpr,N,K", [(128, 512, 128), (300, 1032, 4104)])
+def test_pipeline_stays_whole_when_a_flag_wait_is_abandoned(cuda_device, monkeypatch, kind, tiling, mpr, N, K):
+    """K within and well beyond the stages of the pipeline: after the flag wait gives up the copies, MMAs and epilogue run to
+    the end in step, the report names the flag and its peer and not a barrier behind it, and a product launched before anybody has
+    read the report is right."""
+    monkeypatch.setenv("TDIST_WAIT_TIMEOUT_MS", "50")
+    torch.manual_seed(tiling)
+    dtype, world = torch.bfloat16, 2
+    lw = LocalWorld(world, cuda_device)
+    b = _rand((N, K), dtype, cuda_device, K ** -0.5)
+    for _ in range(3):
+        if kind == "ag":
+            a = _rand((mpr, K), dtype, cuda_device)
+            ctxs = [G.create_ag_gemm_intra_node_context(a, b, r, world, max_M=world * mpr, heap=lw.heap(r)) for r in range(world)]
+            ctxs[0].cta_pair = tiling
+            out = G.ag_gemm_intra_node(a, b, ctxs[0])
+            own = a
+        else:
+            a = _rand((world * mpr, K), dtype, cuda_device)
+            ctxs = [G.create_gemm_rs_context(world * mpr, N, r, world, heap=lw.heap(r)) for r in range(world)]
+            ctxs[0].cta_pair = tiling
+            G.gemm_rs(a, b, ctxs[0])
+            own = a[:mpr]
+        after = G.gemm_persistent(own, b, num_sms=148)
+        torch.cuda.synchronize()
+        rec = global_status().record
+        assert (rec.abort_flag, rec.code, rec.peer) == (1, 1, 1)
+        ref = own.float() @ b.float().t()
+        if kind == "ag":   # this rank's own rows do not depend on the missing ones
+            torch.testing.assert_close(out[:mpr].float(), ref, atol=2e-2, rtol=2e-2)
+        torch.testing.assert_close(after.float(), ref, atol=2e-2, rtol=2e-2)
+        with pytest.raises(_lib.TdistTimeoutError):
+            check_status()
+
+
 def test_consumer_blocks_until_the_host_sets_the_flags(cuda_device):
     """The fused AG-GEMM of one emulated rank is launched while the peer's rows are in the workspace but their flags
     are not set; the host sets them a moment later with stream write-values (no kernel involved). The kernel must

@@ -7,8 +7,8 @@
 //
 // Unlike the reference, no wait here is unbounded: every spin has a wall-clock limit
 // (`%globaltimer`), after which the waiter records what it was waiting for in a status
-// block, raises a sticky abort word that makes every later wait in the kernel return at
-// once, and returns `false`. Callers carry on with whatever data is there (all memory they
+// block, raises a sticky abort word that makes every later flag wait return at once (not the
+// mbarrier waits inside a CTA, see mbar_wait), and returns `false`. Callers carry on with whatever data is there (all memory they
 // touch stays valid), so the kernel drains and the host raises from the status block.
 #pragma once
 #include <stdint.h>
@@ -232,17 +232,20 @@ __device__ __forceinline__ bool signal_wait_until(const uint64_t* sig, int cmp, 
     }
 }
 
-// Bounded mbarrier wait. A phase that never completes is a bug or the echo of an abandoned
-// flag wait upstream; either way the waiter gives up after the same limit.
+// Bounded mbarrier wait. Unlike the flag waits it is not cut short by a reported abort: barriers order copies, MMAs and
+// epilogue of one CTA (pair), all of which carry on after an abandoned flag wait with whatever data is there, so their
+// phases still complete. A role that walked on early would arm a barrier whose phase is still open, or leave the CTA with
+// copies into its shared memory in flight (K beyond the pipeline's stages: launch failure). A phase spans at most one flag
+// wait upstream (those of a tile's blocks run side by side), hence twice the flags' limit: what gets reported is the flag,
+// with its peer and index, and not its echo. Only a bug lets this limit run out.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const WaitCtx& w, int where) {
     if (mbar_try_wait(bar, parity)) return true;
-    const uint64_t limit = w.timeout_ns ? w.timeout_ns : kDefaultTimeoutNs;
+    const uint64_t limit = 2 * (w.timeout_ns ? w.timeout_ns : kDefaultTimeoutNs);
     uint64_t t0 = 0;
     uint32_t spins = 0;
     while (true) {
         if (mbar_try_wait(bar, parity)) return true;
         if ((++spins & 255u) == 0) {
-            if (aborted(w)) return false;
             const uint64_t now = globaltimer_ns();
             if (t0 == 0) t0 = now;
             else if (now - t0 > limit) {
