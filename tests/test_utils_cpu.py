@@ -405,3 +405,13 @@ def test_an_unknown_activation_is_refused_before_anything_runs():
         G.ag_gemm_intra_node(a, b, ctx, activation="typo")
     with pytest.raises(ValueError, match="unknown activation"):
         MT.group_gemm(torch.ones(128, 8), b.view(1, 8, 8), torch.zeros(1, dtype=torch.int32), activation="typo")
+
+
+def test_early_launched_kernels_use_no_read_only_loads():
+    """A kernel that is resident while the one before it still writes may not read that memory through the non-coherent path."""
+    from pathlib import Path
+    kernels = Path(U.__file__).resolve().parents[1] / "csrc" / "kernels"
+    early = [f for f in kernels.glob("*.cu") if "pdl_wait" in f.read_text()]
+    assert len(early) >= 8
+    for f in early:
+        assert "__ldg(" not in f.read_text() and "ld.global.nc" not in f.read_text(), f.name

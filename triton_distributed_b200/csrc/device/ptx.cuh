@@ -126,6 +126,15 @@ __device__ __forceinline__ void pdl_wait_and_release() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// 16 bytes by a plain load that stays where it is written. What an earlier kernel of the stream may write is read like this,
+// or by any other ordinary load, and never by __ldg / ld.global.nc: with an early launch that memory is not read-only for the
+// life of the kernel, and the compiler may move such a load above the wait.
+__device__ __forceinline__ uint4 ld_v4(const void* p) {
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+
 // ---------------------------------------------------------------- TMA (no multicast)
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* m) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory");

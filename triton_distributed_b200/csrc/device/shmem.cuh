@@ -28,11 +28,6 @@ __device__ __forceinline__ void fence() { fence_acq_rel_sys(); }
 // Completes this thread's earlier puts (same mechanism on NVLink: a system-scope fence).
 __device__ __forceinline__ void quiet() { fence_acq_rel_sys(); }
 
-__device__ __forceinline__ uint4 ld_nc_v4(const void* p) {
-    uint4 v;
-    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
-    return v;
-}
 __device__ __forceinline__ void st_v4(void* p, const uint4& v) {
     asm volatile("st.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
@@ -46,16 +41,16 @@ __device__ __forceinline__ void copy_coop(void* dst, const void* src, size_t byt
         const size_t nvec = bytes >> 4;
         size_t i = tid;
         for (; i + 3 * static_cast<size_t>(nthreads) < nvec; i += 4 * static_cast<size_t>(nthreads)) {
-            const uint4 a = ld_nc_v4(s + (i << 4));
-            const uint4 b = ld_nc_v4(s + ((i + nthreads) << 4));
-            const uint4 c = ld_nc_v4(s + ((i + 2 * static_cast<size_t>(nthreads)) << 4));
-            const uint4 e = ld_nc_v4(s + ((i + 3 * static_cast<size_t>(nthreads)) << 4));
+            const uint4 a = ld_v4(s + (i << 4));
+            const uint4 b = ld_v4(s + ((i + nthreads) << 4));
+            const uint4 c = ld_v4(s + ((i + 2 * static_cast<size_t>(nthreads)) << 4));
+            const uint4 e = ld_v4(s + ((i + 3 * static_cast<size_t>(nthreads)) << 4));
             st_v4(d + (i << 4), a);
             st_v4(d + ((i + nthreads) << 4), b);
             st_v4(d + ((i + 2 * static_cast<size_t>(nthreads)) << 4), c);
             st_v4(d + ((i + 3 * static_cast<size_t>(nthreads)) << 4), e);
         }
-        for (; i < nvec; i += nthreads) st_v4(d + (i << 4), ld_nc_v4(s + (i << 4)));
+        for (; i < nvec; i += nthreads) st_v4(d + (i << 4), ld_v4(s + (i << 4)));
         for (size_t b = (nvec << 4) + tid; b < bytes; b += nthreads) d[b] = s[b];
     } else {
         for (size_t b = tid; b < bytes; b += nthreads) d[b] = s[b];

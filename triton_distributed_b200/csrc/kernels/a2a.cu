@@ -66,7 +66,7 @@ __device__ __forceinline__ void copy_seg_warp(char* dst, const char* src, int by
 #pragma unroll
     for (int u = 0; u < kSegLoads; ++u) {
         const int i = b0 + u * 512 + lane * 16;
-        if (i < b1) q[u] = ld_nc_v4(src + i);
+        if (i < b1) q[u] = ld_v4(src + i);
     }
 #pragma unroll
     for (int u = 0; u < kSegLoads; ++u) {
@@ -86,7 +86,7 @@ __device__ __forceinline__ void quant_seg_warp(char* dst, float* dst_scale, cons
 #pragma unroll
     for (int u = 0; u < kSegLoads; ++u) {
         const int g = g0 + 2 * u + half;
-        q[u] = g < groups ? ld_nc_v4(src + (static_cast<size_t>(g) * 128 + sub * 8) * 2) : make_uint4(0, 0, 0, 0);
+        q[u] = g < groups ? ld_v4(src + (static_cast<size_t>(g) * 128 + sub * 8) * 2) : make_uint4(0, 0, 0, 0);
     }
 #pragma unroll
     for (int u = 0; u < kSegLoads; ++u) {
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(kA2AThreads, 2) a2a_kernel(const A2AParams p) 
                     const int er = p.topk_ids[pair] / p.epr;
                     const int row = er * p.max_m + (p.slot_of[pair] - p.cumsum[er * p.epr]);
                     w[j] = p.topk_w[pair];
-                    q[j] = ld_nc_v4(rlocal + static_cast<size_t>(row) * p.row_bytes_out + static_cast<size_t>(c0) * 2);
+                    q[j] = ld_v4(rlocal + static_cast<size_t>(row) * p.row_bytes_out + static_cast<size_t>(c0) * 2);
                 }
             }
 #pragma unroll

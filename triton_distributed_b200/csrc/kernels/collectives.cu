@@ -160,7 +160,7 @@ __device__ __forceinline__ void topk_vec(const CollParams& p, size_t t, size_t c
             if (k0 + j < p.topk) {
                 const size_t pair = t * p.topk + k0 + j;
                 w[j] = p.topk_w ? p.topk_w[pair] : 1.f;
-                q[j] = ld_nc_v4(p.input + (static_cast<size_t>(p.pos_of[pair]) * vpr + c) * 16);
+                q[j] = ld_v4(p.input + (static_cast<size_t>(p.pos_of[pair]) * vpr + c) * 16);
             }
         }
 #pragma unroll
@@ -197,14 +197,14 @@ __device__ __forceinline__ void reduce_sources(const CollParams& p, size_t first
             }
         }
         if (!own_done) {
-            const uint4 q = ld_nc_v4(own + i * 16);
+            const uint4 q = ld_v4(own + i * 16);
             const T* e = reinterpret_cast<const T*>(&q);
 #pragma unroll
             for (int j = 0; j < V; ++j) acc[j] = static_cast<Acc>(e[j]);
         }
         for (int s = 0; s < p.world; ++s) {
             if (s == p.rank) continue;
-            const uint4 q = ld_nc_v4(stage + static_cast<size_t>(s) * p.seg_bytes + i * 16);
+            const uint4 q = ld_v4(stage + static_cast<size_t>(s) * p.seg_bytes + i * 16);
             const T* e = reinterpret_cast<const T*>(&q);
 #pragma unroll
             for (int j = 0; j < V; ++j) acc[j] += static_cast<Acc>(e[j]);
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(kCollThreads) ring_reduce_kernel(const char* i
             for (int u = 0; u < 4; ++u) {
                 int s = begin + s0 + u;
                 if (s >= splits) s -= splits;
-                if (s0 + u < splits) q[u] = ld_nc_v4(in + static_cast<size_t>(s) * block_bytes + i * 16);
+                if (s0 + u < splits) q[u] = ld_v4(in + static_cast<size_t>(s) * block_bytes + i * 16);
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {

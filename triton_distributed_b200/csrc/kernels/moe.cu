@@ -231,11 +231,11 @@ __global__ void __launch_bounds__(kGateThreads, 1) moe_gate_topk_kernel(const __
         }
 #pragma unroll(NT == 8 ? 1 : 2)
         for (int s = warp; s < steps; s += kGateWarps) {
-            const uint4 a = __ldg(reinterpret_cast<const uint4*>(xa + s * 32));
-            const uint4 c = __ldg(reinterpret_cast<const uint4*>(xb + s * 32));
+            const uint4 a = ld_v4(xa + s * 32);
+            const uint4 c = ld_v4(xb + s * 32);
             uint4 b[NT];
 #pragma unroll
-            for (int n = 0; n < NT; ++n) b[n] = __ldg(reinterpret_cast<const uint4*>(ge[n] + s * 32));
+            for (int n = 0; n < NT; ++n) b[n] = ld_v4(ge[n] + s * 32);
 #pragma unroll
             for (int n = 0; n < NT; ++n) {
                 float d[4] = {0.f, 0.f, 0.f, 0.f};
@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(256) topk_reduce_kernel(const uint4* y, const 
             uint4 q[kReduceVecs];
 #pragma unroll
             for (int u = 0; u < kReduceVecs; ++u)
-                q[u] = pos >= 0 && c0 + u * 32 < vec_per_row ? __ldg(y + static_cast<size_t>(pos) * vec_per_row + c0 + u * 32) : make_uint4(0, 0, 0, 0);
+                q[u] = pos >= 0 && c0 + u * 32 < vec_per_row ? ld_v4(y + static_cast<size_t>(pos) * vec_per_row + c0 + u * 32) : make_uint4(0, 0, 0, 0);
 #pragma unroll
             for (int u = 0; u < kReduceVecs; ++u) {
                 const uint32_t v[4] = {q[u].x, q[u].y, q[u].z, q[u].w};

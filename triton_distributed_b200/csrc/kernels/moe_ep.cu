@@ -100,7 +100,7 @@ __device__ __forceinline__ void load_segment(const char* src, int hidden, int se
 #pragma unroll
         for (int u = 0; u < kEpSegLoads; ++u) {
             const int g = g0 + 2 * u + half;
-            raw[u] = g < groups ? ld_nc_v4(src + (static_cast<size_t>(g) * 128 + sub * 8) * 2) : make_uint4(0, 0, 0, 0);
+            raw[u] = g < groups ? ld_v4(src + (static_cast<size_t>(g) * 128 + sub * 8) * 2) : make_uint4(0, 0, 0, 0);
         }
     } else {
         const int b0 = seg * kEpSegValues * 2;
@@ -108,7 +108,7 @@ __device__ __forceinline__ void load_segment(const char* src, int hidden, int se
 #pragma unroll
         for (int u = 0; u < kEpSegLoads; ++u) {
             const int off = b0 + u * 512 + lane * 16;
-            raw[u] = off < b1 ? ld_nc_v4(src + off) : make_uint4(0, 0, 0, 0);
+            raw[u] = off < b1 ? ld_v4(src + off) : make_uint4(0, 0, 0, 0);
         }
     }
 }
@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(kMoeThreads, 2) moe_combine_kernel(const __gri
                     const int r = p.pair_row[pair];
                     if (r >= 0) {
                         w[j] = p.topk_w ? p.topk_w[pair] : 1.f;
-                        q[j] = ld_nc_v4(p.buf_peer[p.topk_ids[pair] / p.epr] + static_cast<size_t>(r) * row_bytes + static_cast<size_t>(c0) * 2);
+                        q[j] = ld_v4(p.buf_peer[p.topk_ids[pair] / p.epr] + static_cast<size_t>(r) * row_bytes + static_cast<size_t>(c0) * 2);
                     }
                 }
             }

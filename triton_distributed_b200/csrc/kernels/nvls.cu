@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(kNvlsThreads) nvls_kernel(const NvlsParams p) 
             uint4 v[kNvlsUnroll];
 #pragma unroll
             for (int u = 0; u < kNvlsUnroll; ++u)
-                if (i + u * nthr < nvec) v[u] = ld_nc_v4(p.local + base + (i + u * nthr) * 16);
+                if (i + u * nthr < nvec) v[u] = ld_v4(p.local + base + (i + u * nthr) * 16);
 #pragma unroll
             for (int u = 0; u < kNvlsUnroll; ++u)
                 if (i + u * nthr < nvec) multimem_st_v4(p.mc + base + (i + u * nthr) * 16, v[u]);
