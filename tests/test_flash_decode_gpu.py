@@ -193,3 +193,75 @@ def test_batch_splits_fill_the_last_wave_and_even_out_lengths():
     assert FD._batch_splits(48 * 8, 4096, 128, 148, 1) == 2        # 384 CTAs are 1.3 waves, 768 are 2.6
     assert FD._batch_splits(64 * 8, 512, 128, 148, 1) == 1         # short sequences: the fixed cost decides
     assert FD._batch_splits(16 * 8, 1024, 128, 148, 2) == 2
+
+
+@pytest.mark.parametrize("kind", ["dispatch", "own rows", "combine", "ag_gemm", "gemm_rs", "decode"])
+def test_a_launch_behind_a_waiting_one_leaves_the_machine_free(cuda_device, monkeypatch, kind):
+    """A kernel that waits for a flag of another launch (here one that nothing sets, until its limit) does not let the next
+    launch of its stream in early: that one, here a decode that takes every SM's shared memory, would keep out the work of
+    other streams that the flag may depend on. The product on the other stream waits for nothing and must finish meanwhile."""
+    import time
+    from triton_distributed_b200.ops import gemm as G, moe_ep as EP
+    from triton_distributed_b200.runtime import global_status
+    monkeypatch.setenv("TDIST_WAIT_TIMEOUT_MS", "600")
+    torch.manual_seed(1)
+    lw, keep = LocalWorld(2, cuda_device), []
+    bf = lambda *shape: torch.randn(*shape, device=cuda_device).to(torch.bfloat16)  # noqa: E731
+    x, w = bf(256, 256), bf(512, 256)
+    if kind in ("dispatch", "combine", "own rows"):
+        ids = torch.zeros(4, 1, dtype=torch.int32, device=cuda_device)
+        ranks = 1 if kind == "own rows" else 2
+        heap = LocalWorld(1, cuda_device).heap(0) if ranks == 1 else lw.heap(0)
+        ctx = EP.create_ep_context(4, 256, 1, 2, 0, ranks, compact=False, heap=heap)
+        if ranks == 2:
+            keep.append(EP.create_ep_context(4, 256, 1, 2, 1, 2, compact=False, heap=lw.heap(1)))
+        ctx.topk_ids, ctx.ntok = ids, 4
+        if kind == "combine":
+            EP.ep_dispatch(ctx, x[:4], ids, None, phase=3)
+            wait = lambda: EP.ep_combine(ctx, weighted=False)  # noqa: E731
+        elif kind == "dispatch":
+            wait = lambda: EP.ep_dispatch(ctx, x[:4], ids, None)  # noqa: E731
+        else:
+            ctx.call_count += 1
+            wait = lambda: EP.ep_dispatch(ctx, x[:4], ids, None, phase=4)  # noqa: E731
+    elif kind == "decode":
+        ctxs = [FD.create_sp_decode_context(r, 2, 1, 32, 128, heap=lw.heap(r), device=cuda_device) for r in range(2)]
+        shard = _make_cache(1, [64], 8, 128, 16, torch.bfloat16, cuda_device)
+        q1, glens = bf(1, 32, 128), torch.full((2, 1), 64, dtype=torch.int32, device=cuda_device)
+        wait = lambda: FD.sp_gqa_fwd_batch_decode(ctxs[0], q1, shard[0], shard[1], glens, shard[2])  # noqa: E731
+    else:
+        if kind == "ag_gemm":
+            ctxs = [G.create_ag_gemm_intra_node_context(x, w, r, 2, max_M=512, heap=lw.heap(r)) for r in range(2)]
+            wait = lambda: G.ag_gemm_intra_node(x, w, ctxs[0])  # noqa: E731
+        else:
+            ctxs = [G.create_gemm_rs_context(256, 512, r, 2, heap=lw.heap(r)) for r in range(2)]
+            wait = lambda: G.gemm_rs(x, w, ctxs[0])  # noqa: E731
+        ctxs[0].num_sms = 16
+    # a decode whose 37 x 8 CTAs take two places on each of 148 SMs
+    kv = torch.full((37,), 32, dtype=torch.int32, device=cuda_device)
+    cache = _make_cache(37, [32] * 37, 8, 128, 16, torch.bfloat16, cuda_device)
+    q = bf(37, 32, 128)
+    fill = lambda: FD.gqa_fwd_batch_decode(q, cache[0], cache[1], None, None, kv, cache[2], 128 ** -0.5, kv_split=1)  # noqa: E731
+    other, done, waited = torch.cuda.Stream(), torch.cuda.Event(), torch.cuda.Event()
+    want = fill()
+    G.gemm_persistent(x, w, num_sms=148)
+    torch.cuda.synchronize()
+    wait()
+    got = fill()
+    waited.record()
+    time.sleep(0.05)
+    with torch.cuda.stream(other):
+        c = G.gemm_persistent(x, w, num_sms=148)
+        done.record()
+    until = time.monotonic() + 0.25
+    while not done.query() and time.monotonic() < until:
+        time.sleep(0.005)
+    free, waiting = done.query(), not waited.query()
+    torch.cuda.synchronize()
+    rec = global_status().record
+    assert (rec.abort_flag, rec.code) == (1, 1) and waiting
+    with pytest.raises(Exception, match="timed out"):
+        check_status()
+    assert free
+    torch.testing.assert_close(c.float(), x.float() @ w.float().t(), atol=1e-1, rtol=2e-2)
+    assert torch.equal(got, want)

@@ -120,10 +120,12 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
 // Every kernel launched with tdist_host::pdl_attribute() calls this before it touches memory that an earlier kernel of the
 // stream may still write or read: the launch itself, barrier set-up and TMEM allocation then run under the tail of that
 // kernel. wait returns when all earlier kernels are complete and their writes visible; only then is the next kernel of the
-// stream let in, which bounds how many grids hold resources at once.
-__device__ __forceinline__ void pdl_wait_and_release() {
+// stream let in, which bounds how many grids hold resources at once. A kernel that waits for a flag of another launch (a
+// peer's, or a half of its own operation on another stream) passes false and lets the next one in by its end: early, that one
+// could hold the SMs which the launch that raises the flag still needs.
+__device__ __forceinline__ void pdl_wait_and_release(bool release = true) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (release) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // 16 bytes by a plain load that stays where it is written. What an earlier kernel of the stream may write is read like this,

@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(kDecodeThreads, (D <= 128 ? 2 : 1)) flash_deco
 
     const int tid = static_cast<int>(threadIdx.x);
     const int warp = tid >> 5, lane = tid & 31;
-    pdl_wait_and_release();
+    pdl_wait_and_release(p.mode != 2 || p.world == 1);
     const int split = static_cast<int>(blockIdx.x) % p.splits;
     const int kvh = (static_cast<int>(blockIdx.x) / p.splits) % p.Hkv;
     const int b = static_cast<int>(blockIdx.x) / (p.splits * p.Hkv);

@@ -755,7 +755,7 @@ __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : THREADS, 1) gemm_sm1
 
     // ---------------- pusher CTAs (AG only; whole clusters when CTAS == 2) ----------------
     if (MODE == TDIST_GEMM_AG && static_cast<int>(blockIdx.x) < p.num_comm) {
-        pdl_wait_and_release();
+        pdl_wait_and_release(false);   // only with several ranks
         if (threadIdx.x == 0) {
             for (int s = 0; s < PUSH_STAGES; ++s) mbar_init(smem_u32(&bars[s]), 1);
             fence_mbar_init();
@@ -770,7 +770,7 @@ __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : THREADS, 1) gemm_sm1
     constexpr bool STAGED = MODE == TDIST_GEMM_PLAIN && !GATHER;
     int gather_live = 0, gather_rot = 0, gather_pro = 0;
     if (STAGED && p.gather_dst != nullptr) {
-        pdl_wait_and_release();
+        pdl_wait_and_release(p.block_src == nullptr);
         gather_live = min(p.seg_blocks, p.num_m_blocks ? *p.num_m_blocks : p.seg_blocks);
         gather_rot = p.block_rot ? max(*p.block_rot, 0) : 0;
         if (CTAS == 2 && p.pair_block != nullptr) gather_rot = p.pair_block[min(gather_rot, p.seg_m_tiles - 1)] >> 1;
@@ -827,7 +827,7 @@ __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : THREADS, 1) gemm_sm1
     }
     tc_fence_after();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
-    if (!(STAGED && p.gather_dst != nullptr)) pdl_wait_and_release();
+    if (!(STAGED && p.gather_dst != nullptr)) pdl_wait_and_release(p.world == 1 && p.block_src == nullptr);
 
     if (GATHER && warp >= THREADS / 32) {
         // ===================== gathering producers: A rows by index with cp.async ==========

@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_dispatch_kernel(const __gr
     const int gw = static_cast<int>(blockIdx.x) * kMoeWarps + warp;
     const int nw = static_cast<int>(gridDim.x) * kMoeWarps;
     uint4 raw[kEpSegLoads];
-    pdl_wait_and_release();
+    pdl_wait_and_release(p.world == 1 && (skip_own_counts || !p.compact || !(p.phase & 2)) && (skip_own_rows || !(p.phase & 4)));
     if ((p.phase & 2) && gw < p.ntok * segs)
         load_segment(p.x + static_cast<size_t>(gw / segs) * p.hidden * 2, p.hidden, gw % segs, lane, p.quant != 0, raw);
 
@@ -443,8 +443,8 @@ struct CombineParams {
 __global__ void __launch_bounds__(kMoeThreads, 2) moe_combine_kernel(const __grid_constant__ CombineParams p) {
     const int tid = static_cast<int>(threadIdx.x);
     const int warp = tid >> 5, lane = tid & 31;
-    pdl_wait_and_release();
     const bool skip_own = (p.phase & 3) == 3;   // as in the dispatch kernel
+    pdl_wait_and_release(p.world == 1 && (skip_own || !(p.phase & 2)));
     if ((p.phase & 1) && blockIdx.x == 0 && tid < p.world && !(tid == p.rank && skip_own)) {
         // the expert outputs were written by earlier work of this stream: complete and visible to peer reads
         fence_acq_rel_sys();
