@@ -415,3 +415,14 @@ def test_early_launched_kernels_use_no_read_only_loads():
     assert len(early) >= 8
     for f in early:
         assert "__ldg(" not in f.read_text() and "ld.global.nc" not in f.read_text(), f.name
+
+
+@pytest.mark.parametrize("m,n,k", [(0, 256, 256), (16, 0, 256), (16, 256, 0), (0, 0, 0), (-5, 8, 8), (1000, 0, 4096)])
+def test_plan_queries_answer_for_empty_problems(m, n, k):
+    """The queries launch nothing and take any sizes (in a process of its own: a division by zero there ends the process)."""
+    import subprocess
+    import sys
+    code = ("import ctypes as C; from triton_distributed_b200 import _lib; g = _lib.GemmArgs(); "
+            f"g.world, g.m_per_rank, g.n, g.k, g.cta_pair, g.c = 1, {m}, {n}, {k}, -1, 16; out = (C.c_int * 4)(); lib = _lib.lib(); "
+            "assert lib.tdist_gemm_plan(g, out) == 0 and out[3] >= 1 and lib.tdist_gemm_grid(g) == out[3] and lib.tdist_gemm_tile_width(g) == 256")
+    subprocess.run([sys.executable, "-c", code], check=True)

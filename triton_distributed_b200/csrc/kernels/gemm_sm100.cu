@@ -1488,6 +1488,7 @@ static void plan_ag(const TdistGemmArgs* a, int sms, int n_tiles, GridPlan& g) {
 // Plain products of one rank whose caller asked for no particular tiling, CTA count or timeline.
 static bool may_replan(const TdistGemmArgs* a) {
     return (a->mode == TDIST_GEMM_PLAIN || a->mode == TDIST_GEMM_AG) && a->world == 1 && a->expert_ids == nullptr &&
+           a->m_per_rank > 0 && a->n > 0 && a->k > 0 &&   // the plan queries come here with any sizes
            a->num_m_blocks == nullptr && a->a_gather == nullptr && a->c_scatter == nullptr && a->block_rot == nullptr &&
            a->trace == nullptr && a->cta_pair < 0 && a->num_sms <= 0;
 }
