@@ -222,3 +222,72 @@ def test_grouped_gemm_tile_width_follows_the_live_blocks(cuda_device, blocks, mo
         blk = slice(128 * i, 128 * i + 128)
         torch.testing.assert_close(out[blk].float(), a[blk].float() @ b[int(experts[i])].float().t(), atol=2.0 ** -8 / 4, rtol=2.0 ** -8)
     assert (out[128 * live:] == 7.0).all()
+
+
+@pytest.mark.parametrize("blocks,E,K,N", [(1, 1, 8, 8), (3, 2, 72, 136), (5, 3, 264, 520), (20, 4, 1000, 264), (9, 4, 4104, 1032)])
+def test_grouped_gemm_on_n_major_weights_gives_the_same_bits(cuda_device, blocks, E, K, N):
+    """[E, K, N] read in place against its transposed copy: the same products summed in the same order, for tiles of 64 to 256
+    columns, remainders in K and N, rows in place, gathered by the producers, staged, and staged on block pairs."""
+    torch.manual_seed(blocks + N)
+    rows = blocks * 128
+    a = torch.randn(rows, K, device=cuda_device).to(torch.bfloat16)
+    b = (torch.randn(E, K, N, device=cuda_device) * K ** -0.5).to(torch.bfloat16)
+    t = b.transpose(1, 2).contiguous()
+    experts = torch.sort(torch.randint(0, E, (blocks,), dtype=torch.int32, device=cuda_device)).values.to(torch.int32)
+    for most in (0, 1):
+        want = MT.group_gemm(a, t, experts, max_blocks=most)
+        assert torch.equal(MT.group_gemm(a, b, experts, max_blocks=most, n_major=True), want)
+    for i in range(blocks):
+        blk = slice(128 * i, 128 * i + 128)
+        torch.testing.assert_close(want[blk].double(), a[blk].double() @ b[int(experts[i])].double(), atol=2e-5, rtol=2.0 ** -8)
+    index = torch.randperm(rows, device=cuda_device).to(torch.int32)
+    gathered = MT.group_gemm_gather(a, index, t, experts)
+    assert torch.equal(MT.group_gemm_gather(a, index, b, experts, n_major=True), gathered)
+    count = torch.tensor([blocks], dtype=torch.int32, device=cuda_device)
+    pairs = MT.pair_blocks(experts, torch.zeros_like(experts), blocks)
+    for p in (None, pairs):
+        staging, ready = torch.empty_like(a), MT.staging_flags(rows, cuda_device)
+        for epoch in (1, 2):
+            got = MT.group_gemm_gather(a, index, b, experts, count, staging=staging, block_ready=ready, epoch=epoch, pairs=p, n_major=True)
+            check_status()
+            torch.testing.assert_close(got.float(), gathered.float(), atol=1e-5, rtol=2.0 ** -8)
+    with pytest.raises(ValueError):
+        MT.group_gemm(a, b, experts, activation="silu", n_major=True)
+
+
+@pytest.mark.parametrize("mode", ["fused", "cp_async", "staged"])
+def test_contexts_use_the_weights_of_the_call(cuda_device, monkeypatch, mode):
+    """Other weights on the same context, weights changed in place (through .data as well, which no version counter sees), and
+    weights of every layout: each call multiplies by what it is given."""
+    monkeypatch.setattr(MT, "AG_GROUP_GEMM_MODE", mode)
+    torch.manual_seed(2)
+    M, E, K, N, topk = 300, 4, 264, 136, 2
+    x = torch.randn(M, K, device=cuda_device).to(torch.bfloat16)
+    ids = torch.stack([torch.randperm(E, device=cuda_device)[:topk] for _ in range(M)]).to(torch.int32)
+    w = torch.rand(M, topk, device=cuda_device)
+    make = lambda: (torch.randn(E, K, N, device=cuda_device) * K ** -0.5).to(torch.bfloat16)  # noqa: E731
+    b = make()
+    heap = LocalWorld(1, cuda_device).heap(0)
+    up = MT.create_ag_group_gemm_intra_node_context(None, x, b, ids, E, max_M=M, rank=0, num_ranks=1, heap=heap)
+    down = MT.create_moe_rs_context(None, 0, 1, 1, M, N, E, topk, torch.bfloat16, torch.bfloat16, cuda_device, full_topk_ids=ids,
+                                    full_topk_weight=w, heap=heap)
+    rows = x[torch.arange(M * topk, device=cuda_device) // topk]
+
+    def check(weights):
+        ref = _expert_matmul(rows, ids.reshape(-1), weights)
+        torch.testing.assert_close(MT.ag_group_gemm_intra_node(x, weights, up).float(), ref, atol=3e-2, rtol=3e-2)
+        out = MT.moe_reduce_rs(0, 1, 1, rows, weights, down)
+        check_status()
+        torch.testing.assert_close(out.float(), (ref.view(M, topk, N) * w.unsqueeze(-1)).sum(1), atol=6e-2, rtol=3e-2)
+
+    check(b)
+    check(make())
+    b.neg_()
+    check(b)
+    b.data.copy_(make())
+    check(b)
+    check(make().transpose(1, 2).contiguous().transpose(1, 2))             # K contiguous
+    check(torch.cat([make(), make()], dim=2)[:, :, :N])                    # rows with a gap
+    room = torch.empty(E * K * N + 1, dtype=torch.bfloat16, device=cuda_device)
+    room[1:].copy_(b.flatten())
+    check(room[1:].view(E, K, N))                                          # not 16-byte aligned

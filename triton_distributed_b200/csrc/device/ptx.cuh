@@ -251,6 +251,18 @@ __device__ __forceinline__ uint64_t umma_desc_k_sw128(uint32_t smem_addr) {
     d |= static_cast<uint64_t>(2) << 61;  // SWIZZLE_128B
     return d;
 }
+// The same for an operand whose M / N dimension is contiguous: 64 of its values make a 128-byte row, rows follow K, eight rows
+// are a swizzle atom (1024 bytes to the next eight), and `chunk_bytes` lie between one 64-value chunk and the next.
+__device__ __forceinline__ uint64_t umma_desc_mn_sw128(uint32_t smem_addr, uint32_t chunk_bytes) {
+    uint64_t d = 0;
+    d |= static_cast<uint64_t>((smem_addr & 0x3FFFFu) >> 4);
+    d |= static_cast<uint64_t>(chunk_bytes >> 4) << 16;
+    d |= static_cast<uint64_t>(1024 >> 4) << 32;
+    d |= static_cast<uint64_t>(1) << 46;
+    d |= static_cast<uint64_t>(2) << 61;
+    return d;
+}
+constexpr uint32_t kIdescBNMajor = 1u << 16;   // the instruction descriptor's bit for a B whose N dimension is contiguous
 // Instruction descriptor for kind::f16 / kind::f8f6f4 with fp32 accumulation, both operands
 // K-major. fmt: f16 kinds 0=f16 1=bf16; f8f6f4 kinds 0=e4m3 1=e5m2.
 __host__ __device__ constexpr uint32_t umma_idesc(uint32_t fmt_a, uint32_t fmt_b, uint32_t m,

@@ -127,6 +127,7 @@ typedef struct TdistGemmArgs {
     /* PLAIN / AG with one rank, optional: applied to the fp32 accumulator before C is rounded (TDIST_ACT_*; GELU is the tanh
      * form). Few-row products and one CTA per tile only (m_per_rank <= 128, or grouped without pair_block). */
     int act;
+    int b_n_major;      /* grouped: B is [num_experts, K, N] with N contiguous instead of [num_experts, N, K]; no act */
     int max_m_blocks;   /* grouped: the most live 128-row blocks the host knows of (0 = m_per_rank / 128), for the choice of tile */
 } TdistGemmArgs;
 

@@ -65,6 +65,7 @@ constexpr int THREADS = 192;
 constexpr int TMEM_COLS = 512;
 constexpr int DEFAULT_GROUP_M = 8;
 constexpr int MAX_STAGES = 6;
+constexpr int BNM_CHUNK = 64 * BK * 2;          // N-major B: 64 columns of a stage, BK rows of 128 bytes
 
 template <int CTAS, bool WIDE = false>
 struct Tiling {
@@ -89,7 +90,7 @@ constexpr int kKernelGemm = 1;
 struct GemmParams {
     CUtensorMap tm_a;       // PLAIN/RS: A as {K, m_per_rank, world}; AG: the gather workspace
     CUtensorMap tm_a_own;   // AG: this rank's shard as {K, m_per_rank, 1}
-    CUtensorMap tm_b;       // {K, N, 1}
+    CUtensorMap tm_b;       // {K, N, experts}; BNM kernels: {N, K, experts}, boxes of 64 x 64
     CUtensorMap tm_c[kMaxRanks];  // PLAIN/AG: [0] = C as {N, m_per_rank, world}; RS: per owner
     const char* a_own;            // AG pusher source
     char* a_ws_peer[kMaxRanks];
@@ -738,10 +739,15 @@ __device__ __forceinline__ void rs_reduce_tile(const GemmParams& p, int block, i
 // warp 0 then only issues the TMA loads of B.
 constexpr int GATHER_THREADS = THREADS + 128;
 // ACT: the epilogue applies p.act. A kernel of its own: the branch alone slowed the others' epilogues (3 % of a grouped GEMM).
-template <int MODE, int CTAS, bool GATHER = false, bool WIDE = false, bool ACT = false>
+// BNM (grouped): B is [experts, K, N] as the caller has it, N contiguous. A stage then holds 64 K rows of 128 bytes per 64 columns
+// (a load each) and the MMA takes B with its N dimension contiguous: same bytes, same order of sums, and no transposed copy of
+// the weights, which would have to follow every change of theirs (8192 tokens, top 2 of 8, 4096 -> 1792 -> 4096: 207 us per GEMM
+// on such copies, 207 us here; first call on new weights 941 us and 668 us).
+template <int MODE, int CTAS, bool GATHER = false, bool WIDE = false, bool ACT = false, bool BNM = false>
 __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : THREADS, 1) gemm_sm100_kernel(const __grid_constant__ GemmParams p) {
     using T = Tiling<CTAS, WIDE>;
     static_assert(!(GATHER && WIDE), "the row-gathering producer feeds narrow tiles");
+    static_assert(!BNM || (MODE == TDIST_GEMM_PLAIN && !WIDE && !ACT), "N-major B belongs to the grouped GEMM");
     constexpr int STAGES = T::STAGES;
     constexpr int STAGE_BYTES = T::STAGE_BYTES;
     extern __shared__ uint8_t smem_raw[];
@@ -909,7 +915,12 @@ __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : THREADS, 1) gemm_sm1
                     const uint32_t s = it % STAGES;
                     mbar_wait(bar_empty(s), ((it / STAGES) & 1u) ^ 1u, p.wctx, 2);
                     mbar_expect_tx(bar_full(s), T::B_BYTES);
-                    tma_load_3d(smem_u32(smem + s * STAGE_BYTES) + A_BYTES, &p.tm_b, bar_full(s), kb * BK, col, bz);
+                    const uint32_t sb = smem_u32(smem + s * STAGE_BYTES) + A_BYTES;
+                    if (BNM) {
+                        for (int c = 0; c < BN / 64; ++c) tma_load_3d(sb + c * BNM_CHUNK, &p.tm_b, bar_full(s), col + c * 64, kb * BK, bz);
+                    } else {
+                        tma_load_3d(sb, &p.tm_b, bar_full(s), kb * BK, col, bz);
+                    }
                 }
             }
         }
@@ -962,13 +973,23 @@ __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : THREADS, 1) gemm_sm1
                     if (CTAS == 1) {
                         mbar_expect_tx(bar_full(s), stage_tx);
                         tma_load_3d(sa, am, bar_full(s), kb * BK, row, az);
-                        tma_load_3d(sa + A_BYTES, &p.tm_b, bar_full(s), kb * BK, col, bz);
+                        if (BNM) {
+                            for (int c = 0; c < p.bn / 64; ++c) tma_load_3d(sa + A_BYTES + c * BNM_CHUNK, &p.tm_b, bar_full(s), col + c * 64, kb * BK, bz);
+                        } else {
+                            tma_load_3d(sa + A_BYTES, &p.tm_b, bar_full(s), kb * BK, col, bz);
+                        }
                     } else {
                         // both CTAs' bytes are counted on the leader's barrier
                         if (cta_rank == 0) mbar_expect_tx(bar_full(s), 2 * stage_tx);
                         const uint32_t leader_full = mapa_u32(bar_full(s), 0);
                         tma_load_3d_pair(sa, am, leader_full, kb * BK, row, az);
-                        tma_load_3d_pair(sa + A_BYTES, &p.tm_b, leader_full, kb * BK, col, bz);
+                        if (BNM) {
+#pragma unroll
+                            for (int c = 0; c < T::B_ROWS / 64; ++c)   // block pairs: 256 columns
+                                tma_load_3d_pair(sa + A_BYTES + c * BNM_CHUNK, &p.tm_b, leader_full, col + c * 64, kb * BK, bz);
+                        } else {
+                            tma_load_3d_pair(sa + A_BYTES, &p.tm_b, leader_full, kb * BK, col, bz);
+                        }
                         if (WIDE && tc.halves == 2)
                             tma_load_3d_pair(sa + A_BYTES + T::B_BYTES, &p.tm_b, leader_full, kb * BK, col + p.bn, bz);
                     }
@@ -984,7 +1005,7 @@ __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : THREADS, 1) gemm_sm1
     } else if (warp == 1) {
         // ===================== MMA issuer (leader CTA only when CTAS == 2) =====================
         if (lane == 0 && cta_rank == 0) {
-            const uint32_t idesc = umma_idesc(p.is_f16 ? 0u : 1u, p.is_f16 ? 0u : 1u, BM * CTAS, static_cast<uint32_t>(p.bn));
+            const uint32_t idesc = umma_idesc(p.is_f16 ? 0u : 1u, p.is_f16 ? 0u : 1u, BM * CTAS, static_cast<uint32_t>(p.bn)) | (BNM ? kIdescBNMajor : 0u);
             uint32_t it = 0;
             uint32_t uses0 = 0, uses1 = 0, next_narrow = 0;   // per-slot use counts give the barrier phases
             const int live_blocks = p.num_m_blocks && p.pair_block == nullptr ? *p.num_m_blocks : 0x7fffffff;
@@ -1009,11 +1030,11 @@ __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : THREADS, 1) gemm_sm1
                     const uint32_t sa = smem_u32(smem + s * STAGE_BYTES);
                     const uint32_t d_tmem = tmem_base + slot * BN;
                     const uint64_t adesc = umma_desc_k_sw128(sa);
-                    const uint64_t bdesc = umma_desc_k_sw128(sa + A_BYTES + h * T::B_BYTES);
+                    const uint64_t bdesc = BNM ? umma_desc_mn_sw128(sa + A_BYTES, BNM_CHUNK) : umma_desc_k_sw128(sa + A_BYTES + h * T::B_BYTES);
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; ++k) {
-                        // 16 elements of K = 32 bytes = 2 descriptor address units
-                        umma_bf16<CTAS>(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+                        // 16 elements of K = 32 bytes = 2 descriptor address units (N-major B: 16 rows of 128 bytes = 128 units)
+                        umma_bf16<CTAS>(d_tmem, adesc + 2 * k, bdesc + (BNM ? 128 : 2) * k, idesc, (kb | k) != 0 ? 1u : 0u);
                     }
                 };
                 auto release_stage = [&](uint32_t s) {
@@ -1380,6 +1401,12 @@ static const void* act_kernel_of(int mode) {
     return mode == TDIST_GEMM_AG ? reinterpret_cast<const void*>(&gemm_sm100_kernel<TDIST_GEMM_AG, 1, false, false, true>)
                                  : reinterpret_cast<const void*>(&gemm_sm100_kernel<TDIST_GEMM_PLAIN, 1, false, false, true>);
 }
+// with an N-major B: grouped, rows in place, staged or gathered by the producers
+static const void* bnm_kernel_of(int ctas, bool gather) {
+    if (gather) return reinterpret_cast<const void*>(&gemm_sm100_kernel<TDIST_GEMM_PLAIN, 1, true, false, false, true>);
+    return ctas == 2 ? reinterpret_cast<const void*>(&gemm_sm100_kernel<TDIST_GEMM_PLAIN, 2, false, false, false, true>)
+                     : reinterpret_cast<const void*>(&gemm_sm100_kernel<TDIST_GEMM_PLAIN, 1, false, false, false, true>);
+}
 static const void* kernel_of(int ctas, int wide, int mode) {
     if (ctas == 1) return kernel_for<1, false>(mode);
     return wide ? kernel_for<2, true>(mode) : kernel_for<2, false>(mode);
@@ -1674,6 +1701,8 @@ extern "C" int tdist_gemm_run(const TdistGemmArgs* a) {
         return fail(TDIST_EINVAL, "unknown activation, or one on more than one rank");
     if (a->expert_ids != nullptr && (a->mode != TDIST_GEMM_PLAIN || a->world != 1))
         return fail(TDIST_EINVAL, "grouped GEMM (expert_ids) is a single-rank plain-mode feature");
+    if (a->b_n_major && (a->expert_ids == nullptr || a->act != TDIST_ACT_NONE || a->cta_pair > 0))
+        return fail(TDIST_EINVAL, "an N-major B belongs to a grouped GEMM of the automatic tiling without activation");
     if ((a->gather_dst != nullptr) != (a->block_ready != nullptr) || (a->gather_dst != nullptr) != (a->gather_counter != nullptr) ||
         (a->gather_dst != nullptr && a->a_gather == nullptr))
         return fail(TDIST_EINVAL, "the staged row gather needs a_gather, gather_dst, block_ready and gather_counter together");
@@ -1717,9 +1746,10 @@ extern "C" int tdist_gemm_run(const TdistGemmArgs* a) {
     }
     {
         const uint64_t E = a->num_experts > 0 ? a->num_experts : 1;
-        uint64_t dims[3] = {K, N, E};
-        uint64_t strides[2] = {K * 2, N * K * 2};
-        uint32_t box[3] = {BK, static_cast<uint32_t>(plan.bn / ctas), 1};
+        const bool n_major = a->b_n_major != 0;
+        uint64_t dims[3] = {n_major ? N : K, n_major ? K : N, E};
+        uint64_t strides[2] = {dims[0] * 2, N * K * 2};
+        uint32_t box[3] = {n_major ? 64u : static_cast<uint32_t>(BK), n_major ? static_cast<uint32_t>(BK) : static_cast<uint32_t>(plan.bn / ctas), 1};
         if ((rc = tdist_host::encode_tmap(&p.tm_b, dt, 2, 3, a->b, dims, strides, box, tdist_host::Swizzle::B128))) return rc;
     }
     {
@@ -1854,9 +1884,19 @@ extern "C" int tdist_gemm_run(const TdistGemmArgs* a) {
             attr_set[dev][a->mode == TDIST_GEMM_AG] = true;
         }
     }
-    if (a->a_gather != nullptr && a->gather_dst == nullptr) {
+    const bool gather = a->a_gather != nullptr && a->gather_dst == nullptr;
+    if (gather) block_threads = GATHER_THREADS;
+    if (a->b_n_major) {
+        fn = bnm_kernel_of(ctas, gather);
+        static bool attr_set[64][3] = {};
+        int dev = 0;
+        TDIST_CUDA_OK(cudaGetDevice(&dev));
+        if (dev >= 0 && dev < 64 && !attr_set[dev][gather ? 0 : ctas]) {
+            TDIST_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+            attr_set[dev][gather ? 0 : ctas] = true;
+        }
+    } else if (gather) {
         fn = reinterpret_cast<const void*>(&gemm_sm100_kernel<TDIST_GEMM_PLAIN, 1, true>);
-        block_threads = GATHER_THREADS;
         static bool attr_set[64] = {};
         int dev = 0;
         TDIST_CUDA_OK(cudaGetDevice(&dev));

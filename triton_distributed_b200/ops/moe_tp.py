@@ -122,15 +122,18 @@ def topk_reduce(y: torch.Tensor, pos_of: torch.Tensor, weights: Optional[torch.T
 
 def group_gemm(a_sorted: torch.Tensor, b: torch.Tensor, expert_ids: torch.Tensor, num_blocks: Optional[torch.Tensor] = None,
                out: Optional[torch.Tensor] = None, activation: Optional[str] = None,
-               max_blocks: int = 0) -> torch.Tensor:
+               max_blocks: int = 0, n_major: bool = False) -> torch.Tensor:
     """``out[i*128:(i+1)*128] = a_sorted[i*128:(i+1)*128] @ b[expert_ids[i]].T`` for every live
     128-row block. ``a_sorted`` ``[blocks*128, K]``, ``b`` ``[E, N, K]`` (K contiguous), ``num_blocks``
     an int32 device scalar (blocks past it are padding and are skipped). ``activation`` ("gelu" in its tanh form, "silu",
     "relu") is applied to the fp32 sums by the epilogue. ``max_blocks``: the most live blocks the caller knows of (0 = all
-    of ``a_sorted``); the tile is chosen for that many."""
+    of ``a_sorted``); the tile is chosen for that many. ``n_major``: ``b`` is ``[E, K, N]`` (N contiguous) and the product
+    ``@ b[expert_ids[i]]``; no activation."""
     act = G.activation_code(activation)
+    if n_major and act:
+        raise ValueError("an activation needs weights with K contiguous")
     rows, K = a_sorted.shape
-    E, N, _ = b.shape
+    E, N = b.shape[0], b.shape[2 if n_major else 1]
     if rows % GROUP_BLOCK_M:
         raise ValueError("grouped GEMM rows must be a multiple of 128")
     if a_sorted.device.type != "cuda":
@@ -138,22 +141,46 @@ def group_gemm(a_sorted: torch.Tensor, b: torch.Tensor, expert_ids: torch.Tensor
         nb = rows // GROUP_BLOCK_M if num_blocks is None else int(num_blocks)
         for i in range(nb):
             blk = slice(i * GROUP_BLOCK_M, (i + 1) * GROUP_BLOCK_M)
-            o[blk] = (a_sorted[blk].float() @ b[int(expert_ids[i])].float().t()).to(o.dtype)
+            w = b[int(expert_ids[i])].float()
+            o[blk] = (a_sorted[blk].float() @ (w if n_major else w.t())).to(o.dtype)
         return G.apply_activation(o, activation)
-    G._check_operands(a_sorted, b.view(E * N, K))
+    g = _grouped_args(a_sorted, b, n_major)
     c = out if out is not None else torch.empty((rows, N), dtype=a_sorted.dtype, device=a_sorted.device)
-    g = G._base_args(a_sorted, b.view(E * N, K), 1, 0, _lib.GEMM_PLAIN)
-    g.n = N
     g.c = c.data_ptr()
     g.m_per_rank = rows
     g.epoch = 1
     g.expert_ids = expert_ids.data_ptr()
     g.num_m_blocks = num_blocks.data_ptr() if num_blocks is not None else None
-    g.num_experts = E
     g.act = act
     g.max_m_blocks = max_blocks
     G._launch(g)
     return c
+
+
+def _grouped_args(a: torch.Tensor, b: torch.Tensor, n_major: bool) -> "_lib.GemmArgs":
+    """Launch arguments of a grouped GEMM over ``b`` ``[E, N, K]``, or ``[E, K, N]`` when ``n_major``."""
+    E, N, K = b.shape[0], b.shape[2 if n_major else 1], a.shape[1]
+    if n_major and b.shape[1] != K:
+        raise ValueError(f"expected b[E, {K}, N], got {tuple(b.shape)}")
+    flat = b.view(E * N, K)   # the same number of values; raises unless b is dense
+    G._check_operands(a, flat)
+    g = G._base_args(a, flat, 1, 0, _lib.GEMM_PLAIN)
+    g.n = N
+    g.num_experts = E
+    g.b_n_major = int(n_major)
+    return g
+
+
+def _expert_weights(b: torch.Tensor) -> Tuple[torch.Tensor, bool]:
+    """The caller's ``[E, K, N]`` weights as the grouped GEMM reads them, and whether N is contiguous: in place on every call,
+    so that a change of theirs is seen; other layouts, and what a TMA load cannot start on, are copied for the call."""
+    kn = b.transpose(1, 2)
+    if b.data_ptr() % 16 == 0:
+        if b.is_contiguous():
+            return b, True
+        if kn.is_contiguous():
+            return kn, False
+    return b.clone(memory_format=torch.contiguous_format), True
 
 
 def staging_flags(rows: int, device) -> torch.Tensor:
@@ -198,7 +225,7 @@ def group_gemm_gather(a: torch.Tensor, row_index: torch.Tensor, b: torch.Tensor,
                       src_rank: int = 0, src_world: int = 1, staging: Optional[torch.Tensor] = None,
                       block_ready: Optional[torch.Tensor] = None, epoch: int = 1, block_rot: Optional[torch.Tensor] = None,
                       c_scatter: Optional[torch.Tensor] = None, c_rows: int = 0,
-                      pairs: Optional["BlockPairs"] = None) -> torch.Tensor:
+                      pairs: Optional["BlockPairs"] = None, n_major: bool = False) -> torch.Tensor:
     """Grouped GEMM whose A rows are gathered inside the kernel: ``out[r] = a[row_index[r]] @ b[expert_ids[r // 128]].T``
     (rows with ``row_index >= a.shape[0]`` are padding). With ``block_src`` the rows of 128-row
     block ``i`` come from rank ``block_src[i]``'s segment of an all-gather that may still be in flight: the kernel
@@ -211,33 +238,31 @@ def group_gemm_gather(a: torch.Tensor, row_index: torch.Tensor, b: torch.Tensor,
     the rows with cp.async.
     ``block_rot`` (device int32 scalar): block the schedule starts at. ``c_scatter`` (int32 per sorted row): the
     epilogue stores row ``r`` of the product at row ``c_scatter[r]`` of ``out`` (``[c_rows, N]``), dropping rows whose
-    index is not below ``c_rows``. ``pairs`` (:func:`pair_blocks`, with ``staging``): two blocks of an expert per CTA pair."""
+    index is not below ``c_rows``. ``pairs`` (:func:`pair_blocks`, with ``staging``): two blocks of an expert per CTA pair.
+    ``n_major`` as in :func:`group_gemm`."""
     rows = row_index.shape[0]
-    E, N, K = b.shape
+    N, K = b.shape[2 if n_major else 1], b.shape[1 if n_major else 2]
     if rows % GROUP_BLOCK_M:
         raise ValueError("grouped GEMM rows must be a multiple of 128")
     if a.device.type != "cuda":
         padded = torch.cat([a, a.new_zeros((1, K))])
-        prod = group_gemm(padded[row_index.long().clamp(max=a.shape[0])], b, expert_ids, num_blocks)
+        prod = group_gemm(padded[row_index.long().clamp(max=a.shape[0])], b, expert_ids, num_blocks, n_major=n_major)
         if c_scatter is None:
             return prod
         o = out if out is not None else torch.zeros((c_rows, N), dtype=a.dtype)
         live = c_scatter.long() < c_rows
         o[c_scatter.long()[live]] = prod[live]
         return o
-    G._check_operands(a, b.view(E * N, K))
+    g = _grouped_args(a, b, n_major)
     if c_scatter is not None:
         c = out if out is not None else torch.empty((c_rows, N), dtype=a.dtype, device=a.device)
     else:
         c = out if out is not None else torch.empty((rows, N), dtype=a.dtype, device=a.device)
-    g = G._base_args(a, b.view(E * N, K), 1, 0, _lib.GEMM_PLAIN)
-    g.n = N
     g.c = c.data_ptr()
     g.m_per_rank = rows
     g.epoch = epoch
     g.expert_ids = expert_ids.data_ptr()
     g.num_m_blocks = num_blocks.data_ptr() if num_blocks is not None else None
-    g.num_experts = E
     g.cta_pair = 0
     g.a_gather = row_index.data_ptr()
     g.a_gather_rows = a.shape[0]
@@ -286,7 +311,6 @@ class MoEAllGatherGroupGEMMTensorParallelContext:
     rank_block_num: Optional[torch.Tensor] = None
     pairs: Optional[BlockPairs] = None           # blocks of an expert two by two, where most have a partner
     num_blocks: Optional[torch.Tensor] = None    # int32 [1]: live 128-row blocks
-    b_nk: Optional[torch.Tensor] = None          # [E, N, K] copy of the weights (K contiguous)
     row_index: Optional[torch.Tensor] = None     # int32 [sorted rows]: token of every sorted row (padding = M)
     pos_of: Optional[torch.Tensor] = None        # int32 [M * topk]: sorted row of every (token, k) pair
     staging: Optional[torch.Tensor] = None       # [sorted rows, K]: the rows in sorted order, filled inside the GEMM launch
@@ -320,7 +344,6 @@ def create_ag_group_gemm_intra_node_context(tp_pg, A: torch.Tensor, B: torch.Ten
     # set-up time: read the padded length once so that the per-call gather and GEMM cover only live blocks
     ctx.sorted_ids = sorted_ids[: int(post_pad)].contiguous()
     ctx.num_blocks = (post_pad // GROUP_BLOCK_M).to(torch.int32)
-    ctx.b_nk = B.transpose(1, 2).contiguous()
     # static routing: the gather index of the fused kernel and the inverse permutation of its output
     numel = M * topk
     ctx.row_index = torch.div(ctx.sorted_ids, topk, rounding_mode="floor").to(torch.int32).contiguous()   # padding numel -> M
@@ -360,7 +383,7 @@ def ag_group_gemm_intra_node(a: torch.Tensor, b: torch.Tensor, ctx: MoEAllGather
             m = ids == e
             out[m] = (rows[m] @ b[e].float()).to(a.dtype)
         return out
-    b_nk = ctx.b_nk if ctx.b_nk is not None else b.transpose(1, 2).contiguous()
+    b, n_major = _expert_weights(b)
     if ctx.world > 1:
         if phase != 2:
             ctx.calls += 1
@@ -380,8 +403,8 @@ def ag_group_gemm_intra_node(a: torch.Tensor, b: torch.Tensor, ctx: MoEAllGather
             src = dict(block_src=ctx.block_barrier_ids, src_flags=ctx.ag_ctx.signal.local, src_epoch=ctx.ag_ctx.epoch,
                        src_rank=ctx.rank, src_world=ctx.world)
             if mode == "fused":
-                return _fused_group_gemm(ctx, buf.local, b_nk, numel, **src)
-            c_sorted = group_gemm_gather(buf.local, ctx.row_index, b_nk, ctx.expert_ids, ctx.num_blocks, **src)
+                return _fused_group_gemm(ctx, buf.local, b, numel, n_major, **src)
+            c_sorted = group_gemm_gather(buf.local, ctx.row_index, b, ctx.expert_ids, ctx.num_blocks, n_major=n_major, **src)
             out, _ = gather_rows(c_sorted, ctx.pos_of, 1, c_sorted.shape[0])
             return out
         CO.fast_allgather(buf, ctx.ag_ctx, mode="push", phase=phase)
@@ -392,25 +415,26 @@ def ag_group_gemm_intra_node(a: torch.Tensor, b: torch.Tensor, ctx: MoEAllGather
         full = a
     mode = "cp_async" if FUSED_AG_GROUP_GEMM else AG_GROUP_GEMM_MODE
     if mode == "fused":
-        return _fused_group_gemm(ctx, full, b_nk, numel)
+        return _fused_group_gemm(ctx, full, b, numel, n_major)
     if mode == "cp_async":
-        c_sorted = group_gemm_gather(full, ctx.row_index, b_nk, ctx.expert_ids, ctx.num_blocks)
+        c_sorted = group_gemm_gather(full, ctx.row_index, b, ctx.expert_ids, ctx.num_blocks, n_major=n_major)
         out, _ = gather_rows(c_sorted, ctx.pos_of, 1, c_sorted.shape[0])
         return out
     a_sorted, pos_of = gather_rows(full, ctx.sorted_ids, ctx.topk, numel, want_inverse=True)
-    c_sorted = group_gemm(a_sorted, b_nk, ctx.expert_ids, ctx.num_blocks)
+    c_sorted = group_gemm(a_sorted, b, ctx.expert_ids, ctx.num_blocks, n_major=n_major)
     out, _ = gather_rows(c_sorted, pos_of, 1, c_sorted.shape[0])
     return out
 
 
-def _fused_group_gemm(ctx: MoEAllGatherGroupGEMMTensorParallelContext, full: torch.Tensor, b_nk: torch.Tensor, numel: int, **src):
+def _fused_group_gemm(ctx: MoEAllGatherGroupGEMMTensorParallelContext, full: torch.Tensor, b: torch.Tensor, numel: int, n_major: bool,
+                      **src):
     """One launch: the kernel stages the rows block by block itself (all threads for the first wave, then the epilogue
     warps between accumulators), TMA-fed MMAs start at this rank's own blocks, the epilogue stores every row at its
     (token, k) position."""
     ctx.gemm_calls += 1
-    return group_gemm_gather(full, ctx.row_index, b_nk, ctx.expert_ids, ctx.num_blocks, staging=ctx.staging,
+    return group_gemm_gather(full, ctx.row_index, b, ctx.expert_ids, ctx.num_blocks, staging=ctx.staging,
                              block_ready=ctx.block_ready, epoch=ctx.gemm_calls, block_rot=ctx.block_rot,
-                             c_scatter=ctx.sorted_ids, c_rows=numel, pairs=ctx.pairs, **src)
+                             c_scatter=ctx.sorted_ids, c_rows=numel, pairs=ctx.pairs, n_major=n_major, **src)
 
 
 # ---------------------------------------------------------------------------- GroupGEMM + reduce + RS
@@ -429,7 +453,6 @@ class MoEReduceRSContext:
     expert_ids: Optional[torch.Tensor] = None
     num_blocks: Optional[torch.Tensor] = None
     rs_ctx: Optional[CO.ReduceScatter2DContext] = None
-    b_nk: Optional[torch.Tensor] = None   # [E, N, K/ws] copy of the weights, made on first use
     pos_of: Optional[torch.Tensor] = None        # int32 [M * topk]: sorted row of every (token, k) pair
     staging: Optional[torch.Tensor] = None       # [sorted rows, K/ws], allocated on first use
     block_ready: Optional[torch.Tensor] = None
@@ -483,8 +506,7 @@ def moe_reduce_rs(rank: int, world_size: int, local_world_size: int, a: torch.Te
         part = (y.view(M, ctx.topk, N) * ctx.full_topk_weight.view(M, ctx.topk, 1)).sum(1).to(a.dtype)
         return CO.reduce_scatter_2d_op(part, ctx.rs_ctx)
     if phase != 2:
-        if ctx.b_nk is None:
-            ctx.b_nk = b.transpose(1, 2).contiguous()
+        b, n_major = _expert_weights(b)
         if AG_GROUP_GEMM_MODE == "fused":
             # the sort of the rows by expert happens inside the grouped-GEMM launch (in-launch row staging + TMA-fed MMAs)
             if ctx.staging is None or ctx.staging.shape[1] != a.shape[1] or ctx.staging.dtype != a.dtype:
@@ -492,12 +514,12 @@ def moe_reduce_rs(rank: int, world_size: int, local_world_size: int, a: torch.Te
                 ctx.block_ready = staging_flags(ctx.sorted_ids.numel(), a.device)
                 ctx.gemm_calls = 0
             ctx.gemm_calls += 1
-            y = group_gemm_gather(a, ctx.sorted_ids, ctx.b_nk, ctx.expert_ids, ctx.num_blocks, staging=ctx.staging,
-                                  block_ready=ctx.block_ready, epoch=ctx.gemm_calls, pairs=ctx.pairs)
+            y = group_gemm_gather(a, ctx.sorted_ids, b, ctx.expert_ids, ctx.num_blocks, staging=ctx.staging,
+                                  block_ready=ctx.block_ready, epoch=ctx.gemm_calls, pairs=ctx.pairs, n_major=n_major)
             ctx._partial = (y, ctx.pos_of)
         else:
             a_sorted, pos_of = gather_rows(a, ctx.sorted_ids, 1, numel, want_inverse=True)
-            ctx._partial = (group_gemm(a_sorted, ctx.b_nk, ctx.expert_ids, ctx.num_blocks), pos_of)
+            ctx._partial = (group_gemm(a_sorted, b, ctx.expert_ids, ctx.num_blocks, n_major=n_major), pos_of)
     y_sorted, pos_of = ctx._partial
     if FUSED_TOPK_RS and y_sorted.dtype == torch.bfloat16 and M % world_size == 0:
         # top-k weighted reduce and reduce-scatter in one kernel: the [M, N] partial is never written
