@@ -367,3 +367,30 @@ def test_an_unknown_activation_launches_nothing(cuda_device, M):
         G.ag_gemm_intra_node(a, b, ctx, out=out, activation="typo")
     torch.cuda.synchronize()
     assert ctx.epoch == 0 and (out == 7.0).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("activation", ["gelu", "silu", "relu"])
+def test_activation_of_every_16_bit_value(cuda_device, activation, dtype):
+    """The in-place kernel over all 65536 values against float64, tails included. Allowed: the rounding of the result (half a
+    quantum where it is subnormal), (5 + 3.2 |z|) 2^-23 of it for z, __expf and the fast division, and 1.1e-36 where the divisor
+    leaves that division's range."""
+    bits = torch.arange(65536, dtype=torch.int32, device=cuda_device).to(torch.int16)
+    v = bits.view(dtype)
+    h = v.clone()
+    lib = _lib.lib()
+    _lib.check(lib.tdist_activate(h.data_ptr(), h.numel(), G._DTYPES[dtype], _lib.ACTIVATIONS[activation], torch.cuda.current_stream().cuda_stream), "tdist_activate")
+    torch.cuda.synchronize()
+    x = v.double()
+    z = {"gelu": 1.5957691216057308 * x * (1 + 0.044715 * x * x), "silu": x, "relu": torch.zeros_like(x)}[activation]
+    ref = x.clamp_min(0) if activation == "relu" else x / (1 + torch.exp(-z))
+    ok = torch.isfinite(x)
+    rounding, half_quantum = (2.0 ** -8, 2.0 ** -134) if dtype == torch.bfloat16 else (2.0 ** -11, 2.0 ** -25)
+    allowed = ref.abs() * (rounding + (5 + 3.2 * z.abs().clamp_max(200)) * 2.0 ** -23) * (1 + rounding) + half_quantum
+    allowed = allowed + (1.1e-36 if activation != "relu" else 0.0)
+    err = (h.double() - ref).abs()
+    worst = (err / allowed)[ok].max().item()
+    assert worst <= 1.0, (worst, v[ok][(err / allowed)[ok].argmax()].item())
+    edge = lambda t: h[(v == t).nonzero().flatten()]  # noqa: E731
+    assert h[torch.isnan(v)].isnan().all() and (edge(float("inf")) == float("inf")).all()
+    assert (edge(-float("inf")) == 0).all() if activation == "relu" else edge(-float("inf")).isnan().all()   # as torch

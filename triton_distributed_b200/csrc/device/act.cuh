@@ -11,7 +11,11 @@ namespace tdist {
 // in the epilogue of a 256 x 512 tile, most of which is exposed, that costs more than a separate pass over the result:
 // m2048, 4096 -> 14336 -> 4096 with GELU 443 us fused, 428 us apart. So only the epilogues of memory-bound tiles apply them.)
 __device__ __forceinline__ float activate(float v, int act) {
-    if (act == TDIST_ACT_RELU) return v < 0.f ? 0.f : v;   // NaN stays NaN
+    if (act == TDIST_ACT_RELU) {
+        // on the bits: a float comparison would flush subnormals (--use_fast_math), and bf16 has those of fp32. NaN stays NaN.
+        const uint32_t bits = __float_as_uint(v);
+        return bits > 0x80000000u && bits <= 0xff800000u ? 0.f : v;
+    }
     const float z = act == TDIST_ACT_GELU ? 1.5957691216057308f * v * (1.f + 0.044715f * v * v) : v;
     return v / (1.f + __expf(-z));
 }
