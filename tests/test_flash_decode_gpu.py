@@ -193,6 +193,30 @@ def test_batch_splits_fill_the_last_wave_and_even_out_lengths():
     assert FD._batch_splits(48 * 8, 4096, 128, 148, 1) == 2        # 384 CTAs are 1.3 waves, 768 are 2.6
     assert FD._batch_splits(64 * 8, 512, 128, 148, 1) == 1         # short sequences: the fixed cost decides
     assert FD._batch_splits(16 * 8, 1024, 128, 148, 2) == 2
+    assert FD._batch_splits(32 * 8, 131072, 128, 148, 1) == 6
+    assert FD._batch_splits(32 * 8, 131072, 128, 148, 1, True) == 2   # more table than cache: one round of CTAs more at most
+    assert FD._batch_splits(64 * 16, 131072, 128, 148, 1, True) == 1
+
+
+def test_a_table_wider_than_the_cache_does_not_ask_for_more_splits(cuda_device, monkeypatch):
+    """The same sequences and cache behind tables of any width: never more splits than the cache could fill."""
+    asked = []
+    rule = FD._batch_splits
+    monkeypatch.setattr(FD, "_batch_splits", lambda *a: asked.append(a) or rule(*a))
+    torch.manual_seed(0)
+    B, Hq, Hkv, D, page = 32, 32, 8, 128, 16
+    lens = torch.randint(1, 200, (B,), dtype=torch.int32, device=cuda_device)
+    q = torch.randn(B, Hq, D, device=cuda_device).to(torch.bfloat16)
+    k, v, table = _make_cache(B, [256] * B, Hkv, D, page, torch.bfloat16, cuda_device)
+    ref = FD.ref_paged_attn(q, k, v, lens, table, D ** -0.5)
+    for width in (16, 512, 8192):
+        padded = torch.zeros(B, width, dtype=torch.int32, device=cuda_device)
+        padded[:, :16] = table
+        out = FD.gqa_fwd_batch_decode(q, k, v, None, None, lens, padded, D ** -0.5)
+        check_status()
+        torch.testing.assert_close(out.float(), ref, atol=1e-2, rtol=1e-2)
+    held = k.shape[0] * page
+    assert [a[1] for a in asked] == [256, 2 * held // B, 2 * held // B] and [a[5] for a in asked] == [False, True, True]
 
 
 @pytest.mark.parametrize("kind", ["dispatch", "own rows", "combine", "ag_gemm", "gemm_rs", "decode"])

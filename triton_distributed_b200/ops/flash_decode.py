@@ -98,28 +98,33 @@ _CLUSTER_FIT = (1.0, 1.0, 1.0, 0.91, 0.89, 0.88, 0.89, 0.85, 0.81)
 
 
 @functools.lru_cache(maxsize=1024)
-def _batch_splits(pairs: int, max_kv: int, head_dim: int, sms: int, one_wave: int) -> int:
+def _batch_splits(pairs: int, max_kv: int, head_dim: int, sms: int, one_wave: int, wide: bool = False) -> int:
     """Splits for ``pairs`` (sequence, kv head) pairs of at most ``max_kv`` keys. One wave of evenly split CTAs leaves
     the machine idle where the pairs do not divide it, and lets the longest sequence decide where lengths differ (the host
     does not see them); more, shorter CTAs even both out until their fixed cost takes over. Two estimates: all sequences
     full (whole waves), and lengths spread evenly over (0, max_kv] (their sum over the machine, plus the last one to
     start). The least sum decides among the splits that cost full sequences no more than 5 % against one wave; at most
     eight, which merge within their cluster. Measured at one wave / as chosen: 32 ragged sequences x 8 kv heads to 8192
-    keys 136 / 116 us (full ones 169 / 171), 48 full ones of 4096 171 / 146 us, 20 full ones of 6000 109 / 93 us."""
+    keys 136 / 116 us (full ones 169 / 178), 48 full ones of 4096 171 / 146 us, 20 full ones of 6000 109 / 93 us.
+
+    ``wide``: the page table is wider than the cache has keys for, so the sequences are known not to fill it, and the short ones
+    pay the fixed cost of every round of CTAs: then at most one round more than one wave takes (32 sequences in a table of
+    131072 keys, cache of 262144, without / with the limit: 64 keys 37.5 / 12.9 us, 2048 keys 81 / 58, all of 8192 209 / 178,
+    ragged to 8192 125 / 122)."""
     slots = {64: 3, 128: 2}.get(head_dim, 1) * sms
     whole = max_kv * head_dim * 4 / (_HBM_BYTES_PER_US / slots)   # us of a CTA that reads a full sequence of one kv head
 
     def estimate(s: int):
         fit = slots * (_CLUSTER_FIT[s] if s < len(_CLUSTER_FIT) else 1.0)
         part = whole / s
-        full = math.ceil(pairs * s / fit) * (part + _CTA_FIXED_US)
-        return full, max(part + _CTA_FIXED_US, pairs * s / fit * (part / 2 + _CTA_FIXED_US) + part / 2)
+        rounds = math.ceil(pairs * s / fit)
+        return rounds, rounds * (part + _CTA_FIXED_US), max(part + _CTA_FIXED_US, pairs * s / fit * (part / 2 + _CTA_FIXED_US) + part / 2)
 
-    best, (most, ragged) = one_wave, estimate(one_wave)
+    best, (rounds, most, ragged) = one_wave, estimate(one_wave)
     best_t = most + ragged
     for s in range(1, min(8, max(1, max_kv // 1024)) + 1):
-        full, ragged = estimate(s)
-        if full <= 1.05 * most and full + ragged < best_t:
+        r, full, ragged = estimate(s)
+        if (r <= rounds + 1 or not wide) and full <= 1.05 * most and full + ragged < best_t:
             best, best_t = s, full + ragged
     return best
 
@@ -157,7 +162,9 @@ def _launch(q, k_cache, v_cache, kv_lens, block_table, scale, soft_cap, out, mod
             max_kv = page * block_table.shape[1]
         splits = default_splits(B, Hkv, max_kv, q.device, D)
         if B > 1:
-            more = _batch_splits(B * Hkv, max_kv, D, _sm_count(q.device), splits)
+            # a table is often as wide as the longest sequence a server admits; lengths spread evenly over (0, n] take half of it
+            held = blocks * page
+            more = _batch_splits(B * Hkv, min(max_kv, max(1, 2 * held // B)), D, _sm_count(q.device), splits, held < B * max_kv)
             # only where the partials meet in shared memory: the shared workspace is not for calls that did without it
             if (Hq // Hkv) * more * (D + 2) * 4 <= 48 * 1024:
                 splits = more
