@@ -298,7 +298,7 @@ def test_gate_topk_writes_logits_of_any_form_or_refuses_them(cuda_device, form):
     assert (room == 7.0).all()
 
 
-@pytest.mark.parametrize("T,k,hidden", [(1, 1, 8), (5, 2, 1024), (64, 3, 1032), (7, 8, 7168), (300, 2, 4096), (2, 1, 1016)])
+@pytest.mark.parametrize("T,k,hidden", [(1, 1, 8), (3, 2, 0), (5, 2, 1024), (64, 3, 1032), (7, 8, 7168), (300, 2, 4096), (2, 1, 1016)])
 def test_topk_reduce_over_ragged_rows_and_rejected_pairs(cuda_device, T, k, hidden):
     torch.manual_seed(T + hidden)
     y = torch.randn(T * k + 3, hidden, device=cuda_device).bfloat16()

@@ -448,7 +448,7 @@ extern "C" int tdist_gather_rows(const void* src, const void* index, int rows_ou
 extern "C" int tdist_topk_reduce(const void* y, const void* pos_of, const void* weights, int ntok, int topk, int row_bytes,
                                  void* out, void* stream) {
     if (row_bytes % 16 || topk < 1) return fail(TDIST_EINVAL, "topk_reduce: rows must be multiples of 16 bytes");
-    if (ntok <= 0) return 0;
+    if (ntok <= 0 || row_bytes <= 0) return 0;
     const long long items = static_cast<long long>(ntok) * ((row_bytes / 16 + 32 * kReduceVecs - 1) / (32 * kReduceVecs));
     const int blocks = static_cast<int>((items + 7) / 8 < 1184 ? (items + 7) / 8 : 1184);
     TDIST_CUDA_OK(tdist_host::launch_pdl(topk_reduce_kernel, dim3(blocks), 256, 0, static_cast<cudaStream_t>(stream), static_cast<const uint4*>(y),
