@@ -151,8 +151,8 @@ def test_group_gemm_staged_gather_rotation_and_scatter(cuda_device, T, E, K, N, 
 @pytest.mark.parametrize("world,tpr,E,K,N,topk", [(1, 2000, 4, 264, 520, 2), (1, 3000, 3, 4104, 776, 2), (1, 300, 8, 256, 512, 2),
                                                   (4, 700, 2, 512, 264, 2), (1, 90, 2, 64, 8, 1)])
 def test_grouped_gemm_on_block_pairs(cuda_device, monkeypatch, world, tpr, E, K, N, topk):
-    """Two blocks of an expert per CTA pair, odd blocks alone (forced where they are many), ragged last blocks, narrow and
-    wide tiles; up-projection with staged rows, rotation and scatter, then down-projection with staged rows and top-k reduce.
+    """Two blocks of an expert per CTA pair, odd blocks alone (forced where they are many), ragged last blocks, K and N
+    off the tile edges; up-projection with staged rows, rotation and scatter, then down-projection with staged rows and top-k reduce.
     Tolerance as above: 16-bit results and the 16-bit intermediate of the reduce."""
     monkeypatch.setattr(MT, "PAIR_MAX_OVERHEAD", 2.0)
     torch.manual_seed(tpr + E)

@@ -535,10 +535,10 @@ using tdist_host::fail;
 
 // Largest cluster (splits of one (batch, kv head)) the merge through shared memory is used for. Above it, or when the
 // partials do not fit the ring, the splits meet in global memory (workspace + arrival counter).
-// Eight is the portable cluster size; 16-CTA clusters were measured and dropped: with 133 KB of shared memory per CTA
-// only some of them are resident at once (batch 1, 8 kv heads, 16384 keys, 16 splits: 37.1 us against 22.6 us through
-// global memory). Up to eight splits the cluster form is 5-10 % faster (4096 keys: 14.4 / 20.6 us against 15.4 / 22.6 us
-// with 8 / 4 splits).
+// Eight is the portable cluster size. Larger ones were measured only while the partials lay behind the ring (133 KB of shared
+// memory per CTA, so that only some 16-CTA clusters were resident at once: batch 1, 8 kv heads, 16384 keys, 16 splits 37.1 us
+// against 22.6 us through global memory); in the ring (100 KB at head_dim 128, two CTAs per SM) they have not been. Up to
+// eight splits the cluster form was 5-10 % faster then (4096 keys: 14.4 / 20.6 us against 15.4 / 22.6 us with 8 / 4 splits).
 constexpr int kClusterMergeMaxSplits = 8;
 
 // Longest key range per CTA with which a batch of several sequences, all of whose CTAs run at once, overlaps the launch

@@ -41,6 +41,9 @@ ROUTE_IN_PLACE_MAX = 8192   # TDIST_MOE_ROUTE_IN_PLACE_MAX of csrc/include/tdist
 
 @dataclass
 class EPContext:
+    """State of dispatch and combine. The launch arguments that belong to the context (sizes, buffers, peers' addresses) are
+    built once, in ``templates``: its tensors and sizes must not be replaced after :func:`create_ep_context`."""
+
     max_tokens: int
     hidden: int
     topk: int
