@@ -236,23 +236,28 @@ def test_grouped_gemm_on_n_major_weights_gives_the_same_bits(cuda_device, blocks
     experts = torch.sort(torch.randint(0, E, (blocks,), dtype=torch.int32, device=cuda_device)).values.to(torch.int32)
     for most in (0, 1):
         want = MT.group_gemm(a, t, experts, max_blocks=most)
-        assert torch.equal(MT.group_gemm(a, b, experts, max_blocks=most, n_major=True), want)
+        assert torch.equal(MT.group_gemm(a, b, experts, max_blocks=most, kn=True), want)
     for i in range(blocks):
         blk = slice(128 * i, 128 * i + 128)
         torch.testing.assert_close(want[blk].double(), a[blk].double() @ b[int(experts[i])].double(), atol=2e-5, rtol=2.0 ** -8)
     index = torch.randperm(rows, device=cuda_device).to(torch.int32)
     gathered = MT.group_gemm_gather(a, index, t, experts)
-    assert torch.equal(MT.group_gemm_gather(a, index, b, experts, n_major=True), gathered)
+    assert torch.equal(MT.group_gemm_gather(a, index, b, experts, kn=True), gathered)
     count = torch.tensor([blocks], dtype=torch.int32, device=cuda_device)
     pairs = MT.pair_blocks(experts, torch.zeros_like(experts), blocks)
     for p in (None, pairs):
         staging, ready = torch.empty_like(a), MT.staging_flags(rows, cuda_device)
         for epoch in (1, 2):
-            got = MT.group_gemm_gather(a, index, b, experts, count, staging=staging, block_ready=ready, epoch=epoch, pairs=p, n_major=True)
+            got = MT.group_gemm_gather(a, index, b, experts, count, staging=staging, block_ready=ready, epoch=epoch, pairs=p, kn=True)
             check_status()
             torch.testing.assert_close(got.float(), gathered.float(), atol=1e-5, rtol=2.0 ** -8)
     with pytest.raises(ValueError):
-        MT.group_gemm(a, b, experts, activation="silu", n_major=True)
+        MT.group_gemm(a, b, experts, activation="silu", kn=True)
+    wider = torch.cat([b, b], dim=2)
+    assert torch.equal(MT.group_gemm(a, wider[:, :, :N], experts, kn=True), MT.group_gemm(a, t, experts))
+    assert torch.equal(MT.group_gemm(a, t.transpose(1, 2), experts, kn=True), MT.group_gemm(a, t, experts))
+    with pytest.raises(ValueError):
+        MT.group_gemm(a, torch.stack([b, b], dim=3)[..., 0], experts, kn=True)
 
 
 @pytest.mark.parametrize("mode", ["fused", "cp_async", "staged"])
@@ -287,7 +292,11 @@ def test_contexts_use_the_weights_of_the_call(cuda_device, monkeypatch, mode):
     b.data.copy_(make())
     check(b)
     check(make().transpose(1, 2).contiguous().transpose(1, 2))             # K contiguous
-    check(torch.cat([make(), make()], dim=2)[:, :, :N])                    # rows with a gap
+    check(torch.cat([make(), make()], dim=2)[:, :, N:])                    # a shard of wider weights
+    check(torch.cat([make(), make()], dim=1)[:, :K])
+    check(torch.cat([make(), make()], dim=2).transpose(1, 2).contiguous()[:, :N].transpose(1, 2))
+    check(make()[:1].expand(E, K, N))                                      # one expert's weights for all: copied
+    check(torch.stack([make(), make()], dim=3)[..., 0])                    # neither N nor K contiguous: copied
     room = torch.empty(E * K * N + 1, dtype=torch.bfloat16, device=cuda_device)
     room[1:].copy_(b.flatten())
     check(room[1:].view(E, K, N))                                          # not 16-byte aligned

@@ -60,7 +60,7 @@ class GemmArgs(C.Structure):
         ("gather_dst", C.c_void_p), ("block_ready", C.c_void_p), ("gather_counter", C.c_void_p), ("block_rot", C.c_void_p),
         ("c_scatter", C.c_void_p), ("c_rows", C.c_int),
         ("pair_block", C.c_void_p), ("num_pairs", C.c_int), ("act", C.c_int), ("b_n_major", C.c_int),
-        ("max_m_blocks", C.c_int),
+        ("b_row_stride", C.c_longlong), ("b_expert_stride", C.c_longlong), ("max_m_blocks", C.c_int),
     ]
 
 

@@ -128,6 +128,7 @@ typedef struct TdistGemmArgs {
      * form). Few-row products and one CTA per tile only (m_per_rank <= 128, or grouped without pair_block). */
     int act;
     int b_n_major;      /* grouped: B is [num_experts, K, N] with N contiguous instead of [num_experts, N, K]; no act */
+    long long b_row_stride, b_expert_stride;   /* grouped: elements from row to row and expert to expert of B, multiples of 8; 0 = dense */
     int max_m_blocks;   /* grouped: the most live 128-row blocks the host knows of (0 = m_per_rank / 128), for the choice of tile */
 } TdistGemmArgs;
 

@@ -1703,6 +1703,9 @@ extern "C" int tdist_gemm_run(const TdistGemmArgs* a) {
         return fail(TDIST_EINVAL, "grouped GEMM (expert_ids) is a single-rank plain-mode feature");
     if (a->b_n_major && (a->expert_ids == nullptr || a->act != TDIST_ACT_NONE || a->cta_pair > 0))
         return fail(TDIST_EINVAL, "an N-major B belongs to a grouped GEMM of the automatic tiling without activation");
+    if (a->b_row_stride < 0 || a->b_row_stride % 8 || a->b_expert_stride < 0 || a->b_expert_stride % 8 ||
+        (a->b_row_stride != 0) != (a->b_expert_stride != 0) || (a->b_row_stride != 0 && a->expert_ids == nullptr))
+        return fail(TDIST_EINVAL, "strides of B belong to a grouped GEMM, both together, in multiples of 8 elements");
     if ((a->gather_dst != nullptr) != (a->block_ready != nullptr) || (a->gather_dst != nullptr) != (a->gather_counter != nullptr) ||
         (a->gather_dst != nullptr && a->a_gather == nullptr))
         return fail(TDIST_EINVAL, "the staged row gather needs a_gather, gather_dst, block_ready and gather_counter together");
@@ -1748,7 +1751,8 @@ extern "C" int tdist_gemm_run(const TdistGemmArgs* a) {
         const uint64_t E = a->num_experts > 0 ? a->num_experts : 1;
         const bool n_major = a->b_n_major != 0;
         uint64_t dims[3] = {n_major ? N : K, n_major ? K : N, E};
-        uint64_t strides[2] = {dims[0] * 2, N * K * 2};
+        uint64_t strides[2] = {a->b_row_stride ? static_cast<uint64_t>(a->b_row_stride) * 2 : dims[0] * 2,
+                               a->b_expert_stride ? static_cast<uint64_t>(a->b_expert_stride) * 2 : N * K * 2};
         uint32_t box[3] = {n_major ? 64u : static_cast<uint32_t>(BK), n_major ? static_cast<uint32_t>(BK) : static_cast<uint32_t>(plan.bn / ctas), 1};
         if ((rc = tdist_host::encode_tmap(&p.tm_b, dt, 2, 3, a->b, dims, strides, box, tdist_host::Swizzle::B128))) return rc;
     }

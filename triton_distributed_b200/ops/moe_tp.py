@@ -122,18 +122,18 @@ def topk_reduce(y: torch.Tensor, pos_of: torch.Tensor, weights: Optional[torch.T
 
 def group_gemm(a_sorted: torch.Tensor, b: torch.Tensor, expert_ids: torch.Tensor, num_blocks: Optional[torch.Tensor] = None,
                out: Optional[torch.Tensor] = None, activation: Optional[str] = None,
-               max_blocks: int = 0, n_major: bool = False) -> torch.Tensor:
+               max_blocks: int = 0, kn: bool = False) -> torch.Tensor:
     """``out[i*128:(i+1)*128] = a_sorted[i*128:(i+1)*128] @ b[expert_ids[i]].T`` for every live
     128-row block. ``a_sorted`` ``[blocks*128, K]``, ``b`` ``[E, N, K]`` (K contiguous), ``num_blocks``
     an int32 device scalar (blocks past it are padding and are skipped). ``activation`` ("gelu" in its tanh form, "silu",
     "relu") is applied to the fp32 sums by the epilogue. ``max_blocks``: the most live blocks the caller knows of (0 = all
-    of ``a_sorted``); the tile is chosen for that many. ``n_major``: ``b`` is ``[E, K, N]`` (N contiguous) and the product
+    of ``a_sorted``); the tile is chosen for that many. ``kn``: ``b`` is ``[E, K, N]`` (N or K contiguous) and the product
     ``@ b[expert_ids[i]]``; no activation."""
     act = G.activation_code(activation)
-    if n_major and act:
+    if kn and act:
         raise ValueError("an activation needs weights with K contiguous")
     rows, K = a_sorted.shape
-    E, N = b.shape[0], b.shape[2 if n_major else 1]
+    E, N = b.shape[0], b.shape[2 if kn else 1]
     if rows % GROUP_BLOCK_M:
         raise ValueError("grouped GEMM rows must be a multiple of 128")
     if a_sorted.device.type != "cuda":
@@ -142,9 +142,9 @@ def group_gemm(a_sorted: torch.Tensor, b: torch.Tensor, expert_ids: torch.Tensor
         for i in range(nb):
             blk = slice(i * GROUP_BLOCK_M, (i + 1) * GROUP_BLOCK_M)
             w = b[int(expert_ids[i])].float()
-            o[blk] = (a_sorted[blk].float() @ (w if n_major else w.t())).to(o.dtype)
+            o[blk] = (a_sorted[blk].float() @ (w if kn else w.t())).to(o.dtype)
         return G.apply_activation(o, activation)
-    g = _grouped_args(a_sorted, b, n_major)
+    g = _grouped_args(a_sorted, b, kn)
     c = out if out is not None else torch.empty((rows, N), dtype=a_sorted.dtype, device=a_sorted.device)
     g.c = c.data_ptr()
     g.m_per_rank = rows
@@ -157,30 +157,48 @@ def group_gemm(a_sorted: torch.Tensor, b: torch.Tensor, expert_ids: torch.Tensor
     return c
 
 
-def _grouped_args(a: torch.Tensor, b: torch.Tensor, n_major: bool) -> "_lib.GemmArgs":
-    """Launch arguments of a grouped GEMM over ``b`` ``[E, N, K]``, or ``[E, K, N]`` when ``n_major``."""
-    E, N, K = b.shape[0], b.shape[2 if n_major else 1], a.shape[1]
-    if n_major and b.shape[1] != K:
-        raise ValueError(f"expected b[E, {K}, N], got {tuple(b.shape)}")
-    flat = b.view(E * N, K)   # the same number of values; raises unless b is dense
-    G._check_operands(a, flat)
-    g = G._base_args(a, flat, 1, 0, _lib.GEMM_PLAIN)
+def _kn_layout(b: torch.Tensor) -> Optional[Tuple[bool, int, int]]:
+    """How the grouped GEMM reads ``[E, K, N]`` weights in place: (N contiguous, else K; row stride; expert stride), or ``None``
+    where a TMA load cannot (neither contiguous, or something off the 16-byte grid)."""
+    (E, K, N), (se, sk, sn) = b.shape, b.stride()
+    if E == 1:
+        se = K * N
+    if b.data_ptr() % 16 or se <= 0 or se % 8:
+        return None
+    if sn == 1 and sk >= N and sk % 8 == 0:
+        return True, sk, se
+    if sk == 1 and sn >= K and sn % 8 == 0:
+        return False, sn, se
+    return None
+
+
+def _grouped_args(a: torch.Tensor, b: torch.Tensor, kn: bool) -> "_lib.GemmArgs":
+    """Launch arguments of a grouped GEMM over ``b`` ``[E, N, K]``, or ``[E, K, N]`` when ``kn``."""
+    if not kn:
+        E, N, K = b.shape
+        flat = b.view(E * N, K)
+        G._check_operands(a, flat)
+        g = G._base_args(a, flat, 1, 0, _lib.GEMM_PLAIN)
+    else:
+        if a.dtype != b.dtype or a.dtype not in G._DTYPES:
+            raise TypeError(f"GEMM operands must both be bf16 or fp16, got {a.dtype} and {b.dtype}")
+        if a.dim() != 2 or b.dim() != 3 or a.shape[1] != b.shape[1] or not a.is_contiguous():
+            raise ValueError(f"expected a contiguous a[M, K] and b[E, K, N], got {tuple(a.shape)} and {tuple(b.shape)}")
+        E, K, N = b.shape
+        layout = _kn_layout(b)
+        if K % 8 or N % 8 or layout is None:
+            raise ValueError("K and N must be multiples of 8, and b[E, K, N] must have one of them contiguous on a 16-byte grid")
+        g = G._base_args(a, b, 1, 0, _lib.GEMM_PLAIN)
+        g.b_n_major, g.b_row_stride, g.b_expert_stride = layout
     g.n = N
     g.num_experts = E
-    g.b_n_major = int(n_major)
     return g
 
 
-def _expert_weights(b: torch.Tensor) -> Tuple[torch.Tensor, bool]:
-    """The caller's ``[E, K, N]`` weights as the grouped GEMM reads them, and whether N is contiguous: in place on every call,
-    so that a change of theirs is seen; other layouts, and what a TMA load cannot start on, are copied for the call."""
-    kn = b.transpose(1, 2)
-    if b.data_ptr() % 16 == 0:
-        if b.is_contiguous():
-            return b, True
-        if kn.is_contiguous():
-            return kn, False
-    return b.clone(memory_format=torch.contiguous_format), True
+def _expert_weights(b: torch.Tensor) -> torch.Tensor:
+    """The caller's ``[E, K, N]`` weights: read in place on every call, so that a change of theirs is seen, and copied for the
+    call only where a TMA load cannot read them."""
+    return b if _kn_layout(b) is not None else b.clone(memory_format=torch.contiguous_format)
 
 
 def staging_flags(rows: int, device) -> torch.Tensor:
@@ -225,7 +243,7 @@ def group_gemm_gather(a: torch.Tensor, row_index: torch.Tensor, b: torch.Tensor,
                       src_rank: int = 0, src_world: int = 1, staging: Optional[torch.Tensor] = None,
                       block_ready: Optional[torch.Tensor] = None, epoch: int = 1, block_rot: Optional[torch.Tensor] = None,
                       c_scatter: Optional[torch.Tensor] = None, c_rows: int = 0,
-                      pairs: Optional["BlockPairs"] = None, n_major: bool = False) -> torch.Tensor:
+                      pairs: Optional["BlockPairs"] = None, kn: bool = False) -> torch.Tensor:
     """Grouped GEMM whose A rows are gathered inside the kernel: ``out[r] = a[row_index[r]] @ b[expert_ids[r // 128]].T``
     (rows with ``row_index >= a.shape[0]`` are padding). With ``block_src`` the rows of 128-row
     block ``i`` come from rank ``block_src[i]``'s segment of an all-gather that may still be in flight: the kernel
@@ -239,21 +257,21 @@ def group_gemm_gather(a: torch.Tensor, row_index: torch.Tensor, b: torch.Tensor,
     ``block_rot`` (device int32 scalar): block the schedule starts at. ``c_scatter`` (int32 per sorted row): the
     epilogue stores row ``r`` of the product at row ``c_scatter[r]`` of ``out`` (``[c_rows, N]``), dropping rows whose
     index is not below ``c_rows``. ``pairs`` (:func:`pair_blocks`, with ``staging``): two blocks of an expert per CTA pair.
-    ``n_major`` as in :func:`group_gemm`."""
+    ``kn`` as in :func:`group_gemm`."""
     rows = row_index.shape[0]
-    N, K = b.shape[2 if n_major else 1], b.shape[1 if n_major else 2]
+    N, K = b.shape[2 if kn else 1], b.shape[1 if kn else 2]
     if rows % GROUP_BLOCK_M:
         raise ValueError("grouped GEMM rows must be a multiple of 128")
     if a.device.type != "cuda":
         padded = torch.cat([a, a.new_zeros((1, K))])
-        prod = group_gemm(padded[row_index.long().clamp(max=a.shape[0])], b, expert_ids, num_blocks, n_major=n_major)
+        prod = group_gemm(padded[row_index.long().clamp(max=a.shape[0])], b, expert_ids, num_blocks, kn=kn)
         if c_scatter is None:
             return prod
         o = out if out is not None else torch.zeros((c_rows, N), dtype=a.dtype)
         live = c_scatter.long() < c_rows
         o[c_scatter.long()[live]] = prod[live]
         return o
-    g = _grouped_args(a, b, n_major)
+    g = _grouped_args(a, b, kn)
     if c_scatter is not None:
         c = out if out is not None else torch.empty((c_rows, N), dtype=a.dtype, device=a.device)
     else:
@@ -383,7 +401,7 @@ def ag_group_gemm_intra_node(a: torch.Tensor, b: torch.Tensor, ctx: MoEAllGather
             m = ids == e
             out[m] = (rows[m] @ b[e].float()).to(a.dtype)
         return out
-    b, n_major = _expert_weights(b)
+    b = _expert_weights(b)
     if ctx.world > 1:
         if phase != 2:
             ctx.calls += 1
@@ -403,8 +421,8 @@ def ag_group_gemm_intra_node(a: torch.Tensor, b: torch.Tensor, ctx: MoEAllGather
             src = dict(block_src=ctx.block_barrier_ids, src_flags=ctx.ag_ctx.signal.local, src_epoch=ctx.ag_ctx.epoch,
                        src_rank=ctx.rank, src_world=ctx.world)
             if mode == "fused":
-                return _fused_group_gemm(ctx, buf.local, b, numel, n_major, **src)
-            c_sorted = group_gemm_gather(buf.local, ctx.row_index, b, ctx.expert_ids, ctx.num_blocks, n_major=n_major, **src)
+                return _fused_group_gemm(ctx, buf.local, b, numel, **src)
+            c_sorted = group_gemm_gather(buf.local, ctx.row_index, b, ctx.expert_ids, ctx.num_blocks, kn=True, **src)
             out, _ = gather_rows(c_sorted, ctx.pos_of, 1, c_sorted.shape[0])
             return out
         CO.fast_allgather(buf, ctx.ag_ctx, mode="push", phase=phase)
@@ -415,26 +433,25 @@ def ag_group_gemm_intra_node(a: torch.Tensor, b: torch.Tensor, ctx: MoEAllGather
         full = a
     mode = "cp_async" if FUSED_AG_GROUP_GEMM else AG_GROUP_GEMM_MODE
     if mode == "fused":
-        return _fused_group_gemm(ctx, full, b, numel, n_major)
+        return _fused_group_gemm(ctx, full, b, numel)
     if mode == "cp_async":
-        c_sorted = group_gemm_gather(full, ctx.row_index, b, ctx.expert_ids, ctx.num_blocks, n_major=n_major)
+        c_sorted = group_gemm_gather(full, ctx.row_index, b, ctx.expert_ids, ctx.num_blocks, kn=True)
         out, _ = gather_rows(c_sorted, ctx.pos_of, 1, c_sorted.shape[0])
         return out
     a_sorted, pos_of = gather_rows(full, ctx.sorted_ids, ctx.topk, numel, want_inverse=True)
-    c_sorted = group_gemm(a_sorted, b, ctx.expert_ids, ctx.num_blocks, n_major=n_major)
+    c_sorted = group_gemm(a_sorted, b, ctx.expert_ids, ctx.num_blocks, kn=True)
     out, _ = gather_rows(c_sorted, pos_of, 1, c_sorted.shape[0])
     return out
 
 
-def _fused_group_gemm(ctx: MoEAllGatherGroupGEMMTensorParallelContext, full: torch.Tensor, b: torch.Tensor, numel: int, n_major: bool,
-                      **src):
+def _fused_group_gemm(ctx: MoEAllGatherGroupGEMMTensorParallelContext, full: torch.Tensor, b: torch.Tensor, numel: int, **src):
     """One launch: the kernel stages the rows block by block itself (all threads for the first wave, then the epilogue
     warps between accumulators), TMA-fed MMAs start at this rank's own blocks, the epilogue stores every row at its
     (token, k) position."""
     ctx.gemm_calls += 1
     return group_gemm_gather(full, ctx.row_index, b, ctx.expert_ids, ctx.num_blocks, staging=ctx.staging,
                              block_ready=ctx.block_ready, epoch=ctx.gemm_calls, block_rot=ctx.block_rot,
-                             c_scatter=ctx.sorted_ids, c_rows=numel, pairs=ctx.pairs, n_major=n_major, **src)
+                             c_scatter=ctx.sorted_ids, c_rows=numel, pairs=ctx.pairs, kn=True, **src)
 
 
 # ---------------------------------------------------------------------------- GroupGEMM + reduce + RS
@@ -506,7 +523,7 @@ def moe_reduce_rs(rank: int, world_size: int, local_world_size: int, a: torch.Te
         part = (y.view(M, ctx.topk, N) * ctx.full_topk_weight.view(M, ctx.topk, 1)).sum(1).to(a.dtype)
         return CO.reduce_scatter_2d_op(part, ctx.rs_ctx)
     if phase != 2:
-        b, n_major = _expert_weights(b)
+        b = _expert_weights(b)
         if AG_GROUP_GEMM_MODE == "fused":
             # the sort of the rows by expert happens inside the grouped-GEMM launch (in-launch row staging + TMA-fed MMAs)
             if ctx.staging is None or ctx.staging.shape[1] != a.shape[1] or ctx.staging.dtype != a.dtype:
@@ -515,11 +532,11 @@ def moe_reduce_rs(rank: int, world_size: int, local_world_size: int, a: torch.Te
                 ctx.gemm_calls = 0
             ctx.gemm_calls += 1
             y = group_gemm_gather(a, ctx.sorted_ids, b, ctx.expert_ids, ctx.num_blocks, staging=ctx.staging,
-                                  block_ready=ctx.block_ready, epoch=ctx.gemm_calls, pairs=ctx.pairs, n_major=n_major)
+                                  block_ready=ctx.block_ready, epoch=ctx.gemm_calls, pairs=ctx.pairs, kn=True)
             ctx._partial = (y, ctx.pos_of)
         else:
             a_sorted, pos_of = gather_rows(a, ctx.sorted_ids, 1, numel, want_inverse=True)
-            ctx._partial = (group_gemm(a_sorted, b, ctx.expert_ids, ctx.num_blocks, n_major=n_major), pos_of)
+            ctx._partial = (group_gemm(a_sorted, b, ctx.expert_ids, ctx.num_blocks, kn=True), pos_of)
     y_sorted, pos_of = ctx._partial
     if FUSED_TOPK_RS and y_sorted.dtype == torch.bfloat16 and M % world_size == 0:
         # top-k weighted reduce and reduce-scatter in one kernel: the [M, N] partial is never written
