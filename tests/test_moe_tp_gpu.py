@@ -300,3 +300,36 @@ def test_contexts_use_the_weights_of_the_call(cuda_device, monkeypatch, mode):
     room = torch.empty(E * K * N + 1, dtype=torch.bfloat16, device=cuda_device)
     room[1:].copy_(b.flatten())
     check(room[1:].view(E, K, N))                                          # not 16-byte aligned
+
+
+@pytest.mark.parametrize("mode", ["fused", "cp_async"])
+@pytest.mark.parametrize("tpr,E,K,N", [(90, 4, 264, 136), (700, 2, 2048, 520)])   # single blocks, block pairs; K within and beyond the stages
+def test_abandoned_all_gather_leaves_the_grouped_gemm_usable(cuda_device, monkeypatch, mode, tpr, E, K, N):
+    """A peer whose rows never come: the launch gives up, drains in step and reports a flag; the next call on the same context,
+    with the rows there, is right."""
+    from triton_distributed_b200.runtime import global_status
+    monkeypatch.setattr(MT, "AG_GROUP_GEMM_MODE", mode)
+    monkeypatch.setenv("TDIST_WAIT_TIMEOUT_MS", "50")
+    torch.manual_seed(tpr)
+    world, topk = 2, 2
+    lw = LocalWorld(world, cuda_device)
+    M = world * tpr
+    shards = [torch.randn(tpr, K, device=cuda_device).to(torch.bfloat16) for _ in range(world)]
+    b = (torch.randn(E, K, N, device=cuda_device) * K ** -0.5).to(torch.bfloat16)
+    ids = torch.stack([torch.randperm(E, device=cuda_device)[:topk] for _ in range(M)]).to(torch.int32)
+    ctxs = [MT.create_ag_group_gemm_intra_node_context(None, shards[r], b, ids, E, max_M=M, rank=r, num_ranks=world, heap=lw.heap(r))
+            for r in range(world)]
+    rows = torch.cat(shards)[torch.arange(M * topk, device=cuda_device) // topk]
+    for call in range(2):
+        MT.ag_group_gemm_intra_node(shards[0], b, ctxs[0])
+        torch.cuda.synchronize()
+        rec = global_status().record
+        assert (rec.abort_flag, rec.code) == (1, 1)
+        with pytest.raises(Exception, match="timed out"):
+            check_status()
+        MT.ag_group_gemm_intra_node(shards[1], b, ctxs[1], phase=1)    # the peer's send of the call that was given up
+        for r in range(world):
+            MT.ag_group_gemm_intra_node(shards[r], b, ctxs[r], phase=1)
+        out = MT.ag_group_gemm_intra_node(shards[0], b, ctxs[0], phase=2)
+        check_status()
+        torch.testing.assert_close(out.float(), _expert_matmul(rows, ids.reshape(-1), b), atol=3e-2, rtol=3e-2)
