@@ -187,6 +187,39 @@ def test_a_decode_reads_the_result_of_the_one_before(cuda_device, B, splits, blo
         torch.testing.assert_close(out.float(), FD.ref_paged_attn(q, k, v, kv, table, D ** -0.5), atol=2e-2, rtol=2e-2)
 
 
+@pytest.mark.parametrize("explicit", [False, True])   # torch's current stream; a stream handed over
+def test_two_streams_do_not_share_their_scratch(cuda_device, explicit):
+    """16 splits meet in global memory: launches of the same shape on two streams at once, with different queries and caches,
+    each give what they give alone."""
+    torch.manual_seed(9)
+    Hq, Hkv, D, page, per = 32, 8, 128, 16, 256
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    jobs = []
+    for _ in streams:
+        q = torch.randn(1, Hq, D, device=cuda_device).to(torch.bfloat16)
+        k, v, table = _make_cache(1, [per * page], Hkv, D, page, torch.bfloat16, cuda_device)
+        kv = torch.tensor([per * page - 5], dtype=torch.int32, device=cuda_device)
+        ref = FD.gqa_fwd_batch_decode(q, k, v, None, None, kv, table, D ** -0.5, kv_split=16)
+        torch.testing.assert_close(ref.float(), FD.ref_paged_attn(q, k, v, kv, table, D ** -0.5), atol=1e-2, rtol=1e-2)
+        jobs.append((q, k, v, kv, table, ref))
+    torch.cuda.synchronize()
+    outs = [[torch.empty_like(jobs[0][0]) for _ in range(100)] for _ in streams]
+    torch.cuda.synchronize()
+    for n in range(100):
+        for i, s in enumerate(streams):
+            q, k, v, kv, table, _ = jobs[i]
+            if explicit:
+                FD._launch(q, k, v, kv, table, D ** -0.5, 0.0, outs[i][n], 0, 16, stream=s)
+            else:
+                with torch.cuda.stream(s):
+                    FD.gqa_fwd_batch_decode(q, k, v, None, None, kv, table, D ** -0.5, kv_split=16, output_combine=outs[i][n])
+    torch.cuda.synchronize()
+    check_status()
+    for i in range(2):
+        assert all(torch.equal(o, jobs[i][5]) for o in outs[i])
+    assert len({k[1] for k in FD._Workspace.cache if k[1] in (streams[0].cuda_stream, streams[1].cuda_stream)}) == 2
+
+
 def test_batch_splits_fill_the_last_wave_and_even_out_lengths():
     assert FD._batch_splits(32 * 8, 8192, 128, 148, 1) == 2        # ragged batches gain, full ones lose next to nothing
     assert FD._batch_splits(8 * 8, 32768, 128, 148, 4) == 4        # one wave of 256 CTAs is hard to beat

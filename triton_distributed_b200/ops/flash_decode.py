@@ -130,17 +130,20 @@ def _batch_splits(pairs: int, max_kv: int, head_dim: int, sms: int, one_wave: in
 
 
 class _Workspace:
-    """Split-merge scratch, cached per (device, shape)."""
+    """Split-merge scratch, cached per (device, stream, shape): the launches of one stream follow one another, those of two
+    need not. Never given back: a captured launch keeps its addresses. (Launches captured on one stream share theirs, so
+    graphs of them must not be replayed side by side.)"""
 
     cache = {}
 
     @classmethod
-    def get(cls, device, B, Hq, Hkv, D, splits):
-        key = (device, B, Hq, Hkv, D, splits)
+    def get(cls, device, stream, handle, B, Hq, Hkv, D, splits):
+        key = (device, handle, B, Hq, Hkv, D, splits)
         ws = cls.cache.get(key)
         if ws is None:
-            ws = (torch.empty((B, Hq, splits, D + 2), dtype=torch.float32, device=device),
-                  torch.zeros(B * Hkv, dtype=torch.int32, device=device))
+            with torch.cuda.stream(stream):   # the counters are zeroed where they are used (None: the current stream)
+                ws = (torch.empty((B, Hq, splits, D + 2), dtype=torch.float32, device=device),
+                      torch.zeros(B * Hkv, dtype=torch.int32, device=device))
             cls.cache[key] = ws
         return ws
 
@@ -168,7 +171,8 @@ def _launch(q, k_cache, v_cache, kv_lens, block_table, scale, soft_cap, out, mod
             # only where the partials meet in shared memory: the shared workspace is not for calls that did without it
             if (Hq // Hkv) * more * (D + 2) * 4 <= 48 * 1024:
                 splits = more
-    partial, counters = workspace if workspace is not None else _Workspace.get(q.device, B, Hq, Hkv, D, splits)
+    handle = stream_ptr(q.device, stream)
+    partial, counters = workspace if workspace is not None else _Workspace.get(q.device, stream, handle, B, Hq, Hkv, D, splits)
     a = _lib.DecodeArgs()
     a.q, a.k_cache, a.v_cache = q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr()
     bt = block_table if block_table.dtype == torch.int32 else block_table.to(torch.int32)
@@ -195,7 +199,7 @@ def _launch(q, k_cache, v_cache, kv_lens, block_table, scale, soft_cap, out, mod
     st = global_status()
     a.status = st.device_ptr if st is not None else None
     a.timeout_ns = default_timeout_ns()
-    a.stream = stream_ptr(q.device, stream)
+    a.stream = handle
     if stream is not None:
         # copies made on the current stream are read on `stream`: order the two, and keep the allocator from
         # handing the copies' memory out again before `stream` is done with them
