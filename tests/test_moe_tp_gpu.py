@@ -116,6 +116,30 @@ def test_group_gemm_gathers_rows_in_kernel(cuda_device, T, E, K, N, topk):
     assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("K", [8, 40, 256, 264, 504, 1024, 1032, 2048, 2056])
+def test_staged_gather_copies_rows_of_every_length(cuda_device, K):
+    """Rows of one 16-byte vector up to several steps of the copy; T and E leave blocks to the prologue and to the epilogue
+    warps (more blocks than the first wave has), with padding rows in every expert's last block."""
+    torch.manual_seed(K)
+    T, E, N, topk = 2900, 7, 2048, 2
+    x = torch.randn(T, K, device=cuda_device).to(torch.bfloat16)
+    b = (torch.randn(E, N, K, device=cuda_device) * K ** -0.5).to(torch.bfloat16)
+    ids = torch.randint(0, E, (T, topk), dtype=torch.int32, device=cuda_device)
+    sorted_ids, expert_ids, _, _, post_pad = MU.sort_topk_ids_align_block_size(ids, E, 1, T, 128)
+    sid = sorted_ids[:int(post_pad)].contiguous()
+    nb = (post_pad // 128).to(torch.int32)
+    a_sorted, _ = MT.gather_rows(x, sid, topk, T * topk)
+    want = MT.group_gemm(a_sorted, b, expert_ids, nb)
+    row_index = torch.div(sid, topk, rounding_mode="floor").to(torch.int32)
+    staging = torch.full((sid.numel(), K), float("nan"), dtype=x.dtype, device=cuda_device)
+    flags = MT.staging_flags(sid.numel(), cuda_device)
+    live = sid < T * topk
+    for epoch in (1, 2):
+        got = MT.group_gemm_gather(x, row_index, b, expert_ids, nb, staging=staging, block_ready=flags, epoch=epoch)
+        check_status()
+        assert torch.equal(got[live], want[live])
+
+
 @pytest.mark.parametrize("T,E,K,N,topk,rot", [(300, 8, 264, 520, 2, 0), (1500, 16, 512, 776, 3, 7), (128, 4, 64, 256, 1, 1)])
 def test_group_gemm_staged_gather_rotation_and_scatter(cuda_device, T, E, K, N, topk, rot):
     """In-launch row staging (all-thread prologue + epilogue warps) + TMA-fed MMAs + scattering epilogue in one launch against the four-launch path, over several

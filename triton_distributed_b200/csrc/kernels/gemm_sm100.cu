@@ -541,29 +541,77 @@ __device__ __forceinline__ int gather_prologue_blocks(const GemmParams& p, int l
     return pro;
 }
 
-// All CTAs, all threads: copy the rows of the first `pro` blocks (a warp per row, rows dealt round-robin over the grid);
-// the last CTA to finish publishes their flags.
+// Copies the `n` staging rows row0.. of one warp; lane i < n holds row i's source row in `idx`, or -1 for a padding row, whose
+// product is never used. The copy is a chain of two latencies (loads, then stores) and a lane keeps eight 16-byte loads of it in
+// flight, so short rows share a step: four of 800 bytes, all 16 of a group at 256. One row per step, its index loaded by
+// itself, and as many here (both directions of a tensor-parallel MoE layer, one GPU): 3632 tokens, top 6 of 64, 400 -> 464 158 and
+// 112 us; 3596 tokens, top 2 of 32, 928 -> 160 119 and 69 us; 794 tokens, top 6 of 16, 2160 -> 680 118 and 102 us.
+constexpr int GATHER_LOADS = 8;
+__device__ __forceinline__ void gather_copy_rows(const GemmParams& p, int row0, int n, int idx, int lane) {
+    const int vecs = p.k / 8;   // 16-byte vectors of a row (K is a multiple of 8)
+    const size_t row_bytes = static_cast<size_t>(p.k) * 2;
+    if (n == 1) {
+        // a long row: the addresses of its loads are constants apart
+        idx = __shfl_sync(0xffffffffu, idx, 0);
+        if (idx < 0) return;
+        const char* src = p.a_raw + static_cast<size_t>(idx) * row_bytes;
+        char* dst = p.gather_dst + static_cast<size_t>(row0) * row_bytes;
+        for (size_t off = static_cast<size_t>(lane) * 16; off < row_bytes; off += GATHER_LOADS * 512) {
+            uint4 q[GATHER_LOADS];
+#pragma unroll
+            for (int u = 0; u < GATHER_LOADS; ++u)
+                if (off + u * 512 < row_bytes) q[u] = *reinterpret_cast<const uint4*>(src + off + u * 512);
+#pragma unroll
+            for (int u = 0; u < GATHER_LOADS; ++u)
+                if (off + u * 512 < row_bytes) *reinterpret_cast<uint4*>(dst + off + u * 512) = q[u];
+        }
+        return;
+    }
+    const int total = n * vecs;
+    int r = 0, c = lane;        // row and vector of this lane's next load
+    while (c >= vecs) {
+        c -= vecs;
+        ++r;
+    }
+    for (int v0 = 0; v0 < total; v0 += GATHER_LOADS * 32) {
+        uint4 q[GATHER_LOADS];
+        char* dst[GATHER_LOADS];
+#pragma unroll
+        for (int u = 0; u < GATHER_LOADS; ++u) {
+            const int src = __shfl_sync(0xffffffffu, idx, r < n ? r : 0);
+            const bool ok = r < n && src >= 0;
+            dst[u] = ok ? p.gather_dst + static_cast<size_t>(row0 + r) * row_bytes + c * 16 : nullptr;
+            if (ok) q[u] = *reinterpret_cast<const uint4*>(p.a_raw + static_cast<size_t>(src) * row_bytes + c * 16);
+            c += 32;
+            while (c >= vecs) {
+                c -= vecs;
+                ++r;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < GATHER_LOADS; ++u)
+            if (dst[u] != nullptr) *reinterpret_cast<uint4*>(dst[u]) = q[u];
+    }
+}
+// Source row of staging row `row`, -1 for padding.
+__device__ __forceinline__ int gather_source(const GemmParams& p, int row) {
+    const int idx = row < p.m_per_rank ? p.a_gather[row] : -1;
+    return idx < p.a_gather_rows ? idx : -1;
+}
+
+// All CTAs, all threads: copy the rows of the first `pro` blocks (a few neighbouring rows per warp, dealt round-robin over the
+// grid); the last CTA to finish publishes their flags.
 __device__ void gather_prologue(const GemmParams& p, int pro, int live, int rot) {
     const int tid = static_cast<int>(threadIdx.x);
     const int warp = tid >> 5, lane = tid & 31;
     const int nwarps = static_cast<int>(blockDim.x) >> 5;
-    const size_t row_bytes = static_cast<size_t>(p.k) * 2;
-    for (int g = static_cast<int>(blockIdx.x) * nwarps + warp; g < pro * BM; g += static_cast<int>(gridDim.x) * nwarps) {
+    // rows a warp takes at a time: as many as one step of the copy covers, while every warp of the grid still gets some
+    const int warps = static_cast<int>(gridDim.x) * nwarps;
+    int per = 1;
+    while (per < GATHER_LOADS && 2 * per * (p.k / 8) <= GATHER_LOADS * 32 && 2 * per * warps <= pro * BM) per *= 2;
+    for (int g = (static_cast<int>(blockIdx.x) * nwarps + warp) * per; g < pro * BM; g += warps * per) {
         const int row = rotate_block(g / BM, rot, live) * BM + (g % BM);
-        if (row >= p.m_per_rank) continue;
-        const int idx = p.a_gather[row];
-        if (idx < 0 || idx >= p.a_gather_rows) continue;   // padding row: its product is never used
-        const char* src = p.a_raw + static_cast<size_t>(idx) * row_bytes;
-        char* dst = p.gather_dst + static_cast<size_t>(row) * row_bytes;
-        for (size_t off = static_cast<size_t>(lane) * 16; off < row_bytes; off += 8 * 512) {
-            uint4 q[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-                if (off + u * 512 < row_bytes) q[u] = *reinterpret_cast<const uint4*>(src + off + u * 512);
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-                if (off + u * 512 < row_bytes) *reinterpret_cast<uint4*>(dst + off + u * 512) = q[u];
-        }
+        gather_copy_rows(p, row, per, lane < per ? gather_source(p, row + lane) : -1, lane);
     }
     // the CTA barrier orders every thread's stores before thread 0's arrival (gpu scope, acq_rel): the last CTA to
     // arrive has every CTA's rows behind it when it raises the flags
@@ -572,15 +620,17 @@ __device__ void gather_prologue(const GemmParams& p, int pro, int live, int rot)
         const uint32_t old = atom_add_acq_rel_gpu_u32(p.gather_counter + kGatherPrologue, 1);
         if (old == gridDim.x - 1) {
             p.gather_counter[kGatherPrologue] = 0;
+            // one fence, then strong stores: a release store per flag waits for the ones before it (543 tokens, top 5 of 64,
+            // 4184 -> 168: 144 us with them, 121 us without)
             fence_acq_rel_gpu();
-            for (int i = 0; i < pro; ++i) st_release_gpu_u32(p.block_ready + rotate_block(i, rot, live), p.epoch);
+            for (int i = 0; i < pro; ++i) st_relaxed_gpu_u32(p.block_ready + rotate_block(i, rot, live), p.epoch);
         }
     }
 }
 
 // The remaining blocks are staged by the epilogue warps of the GEMM CTAs in the time they would otherwise spend waiting
 // for an accumulator: a warp claims the next 16-row group (in the order the GEMM visits the blocks) from a grid-wide
-// cursor, copies it one row per step, looking at its accumulator barrier between rows, and the warp that completes a
+// cursor, copies it a few rows per step, looking at its accumulator barrier between steps, and the warp that completes a
 // block's last group raises the block's flag. No CTA is taken away from the MMAs and the copy bandwidth grows with the
 // grid (4 warps x 148 CTAs).
 constexpr int GATHER_SUB = 16;              // rows per claimed item
@@ -588,9 +638,10 @@ constexpr int GATHER_SUBS = BM / GATHER_SUB;
 struct GatherCursor {
     int item;   // claimed group in schedule order (-1: none claimed yet)
     int row;    // next row of the group
+    int idx;    // lane i: source row of the group's row i
 };
 
-// One step of a warp's share: claim a group if it holds none, then copy at most one row. False once the cursor has run
+// One step of a warp's share: claim a group if it holds none, then copy the rows of one step. False once the cursor has run
 // past the last block (nothing left for this warp). A group whose rows belong to an all-gather segment that has not
 // arrived yet is kept and retried on the next step.
 __device__ __forceinline__ bool gather_step(const GemmParams& p, GatherCursor& g, int pro, int live, int rot, int lane) {
@@ -610,25 +661,14 @@ __device__ __forceinline__ bool gather_step(const GemmParams& p, GatherCursor& g
             if (!__all_sync(0xffffffffu, here)) return true;
         }
     }
-    const int row = b * BM + (g.item % GATHER_SUBS) * GATHER_SUB + g.row;
-    if (row < p.m_per_rank) {
-        const int idx = p.a_gather[row];
-        if (idx >= 0 && idx < p.a_gather_rows) {   // else a padding row: its product is never used
-            const size_t row_bytes = static_cast<size_t>(p.k) * 2;
-            const char* src = p.a_raw + static_cast<size_t>(idx) * row_bytes;
-            char* dst = p.gather_dst + static_cast<size_t>(row) * row_bytes;
-            for (size_t off = static_cast<size_t>(lane) * 16; off < row_bytes; off += 8 * 512) {
-                uint4 q[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    if (off + u * 512 < row_bytes) q[u] = *reinterpret_cast<const uint4*>(src + off + u * 512);
-#pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    if (off + u * 512 < row_bytes) *reinterpret_cast<uint4*>(dst + off + u * 512) = q[u];
-            }
-        }
-    }
-    if (++g.row == GATHER_SUB) {
+    const int row0 = b * BM + (g.item % GATHER_SUBS) * GATHER_SUB;
+    if (g.row == 0) g.idx = lane < GATHER_SUB ? gather_source(p, row0 + lane) : -1;
+    // rows of one step: one copy's worth of loads, a power of two
+    int n = 1;
+    while (n < GATHER_SUB && 2 * n * (p.k / 8) <= GATHER_LOADS * 32) n *= 2;
+    gather_copy_rows(p, row0 + g.row, n, __shfl_sync(0xffffffffu, g.idx, (g.row + lane) & 31), lane);
+    g.row += n;
+    if (g.row == GATHER_SUB) {
         // the warp barrier orders every lane's stores before lane 0's arrival (gpu scope, acq_rel); the warp that brings
         // the block's count to GATHER_SUBS therefore has all of the block's rows behind it when it raises the flag
         __syncwarp();
@@ -1101,7 +1141,7 @@ __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : THREADS, 1) gemm_sm1
         const int live_blocks = p.num_m_blocks && p.pair_block == nullptr ? *p.num_m_blocks : 0x7fffffff;
         const int block_rot = p.block_rot ? min(max(*p.block_rot, 0), max(min(live_blocks, p.seg_m_tiles) - 1, 0)) : 0;
         const bool scatter = MODE == TDIST_GEMM_PLAIN && p.c_scatter != nullptr;
-        GatherCursor gcur{-1, 0};
+        GatherCursor gcur{-1, 0, -1};
         Work tc;
         for (int round = 0; get_work<WIDE>(p, unit, num_units, round, first_seg, tc); ++round) {
             if (tc.halves == 0 || tc.m_in_seg * CTAS >= live_blocks) continue;
