@@ -39,6 +39,31 @@ def test_decode_matches_reference(cuda_device, Hq, Hkv, D, kv_lens, dtype):
     torch.testing.assert_close(out.float(), ref, atol=1e-2, rtol=1e-2)
 
 
+@pytest.mark.parametrize("G", [1, 7, 8, 9, 16])                       # columns of one MMA tile and of two
+@pytest.mark.parametrize("D,page", [(64, 1), (64, 64), (128, 3), (128, 48), (256, 16)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_decode_tiles_and_pages(cuda_device, G, D, page, dtype):
+    """Lengths at the edges of a 16-token block, of a page and of the copies' ring; 40 sequences (some empty, some equal) are
+    more than one wave of CTAs. The bound is the rounding of the probabilities and of the result, 2^-9 (bf16) or 2^-12 each, of
+    sum p |v| and of the result."""
+    torch.manual_seed(G * D + page)
+    Hkv, splits = 6, 3
+    kv_lens = [0, 1, 15, 16, 17, 47, 48, 49, 63, 64, 65, 255, 256, 257, 1000] + [(37 * i) % 700 for i in range(23)] + [512, 512]
+    B = len(kv_lens)
+    q = torch.randn(B, G * Hkv, D, device=cuda_device).to(dtype)
+    k, v, table = _make_cache(B, kv_lens, Hkv, D, page, dtype, cuda_device)
+    lens = torch.tensor(kv_lens, dtype=torch.int32, device=cuda_device)
+    scale = 1.5 / math.sqrt(D)
+    for cap in (0.0, 20.0):
+        out = FD.gqa_fwd_batch_decode(q, k, v, None, None, lens, table, scale, cap, kv_split=splits).float()
+        check_status()
+        ref = FD.ref_paged_attn(q, k, v, lens, table, scale, cap)
+        spread = FD.ref_paged_attn(q, k, v.abs(), lens, table, scale, cap)
+        u = 2.0 ** (-9 if dtype == torch.bfloat16 else -12)
+        assert ((out - ref).abs() <= u * (spread + ref.abs()) + 1e-3 * spread + 1e-6).all()
+        assert (out[0] == 0).all()
+
+
 @pytest.mark.parametrize("splits", [1, 3, 8, 16, 32])   # up to 8: one cluster per (batch, kv head), merged through shared memory
 @pytest.mark.parametrize("soft_cap", [0.0, 30.0])
 def test_intra_rank_partials_and_merge(cuda_device, splits, soft_cap):

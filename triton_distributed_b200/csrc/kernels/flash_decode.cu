@@ -1,12 +1,17 @@
 // GQA flash-decode over a paged KV cache, split along the KV sequence, with the split merge — and
 // in sequence-parallel mode the cross-rank exchange and merge — fused into the same launch.
 //
-// Grid = batch x kv_heads x splits CTAs of 4 warps. A CTA owns one (batch, kv head, KV range): the
-// G = Hq/Hkv query heads sharing that kv head form the rows of a 16-row Q tile (rows >= G are
-// zero), each warp streams 16-token K/V blocks of the range through its own cp.async ring
-// (no CTA barrier in the main loop) and runs QK^T and PV on tensor cores (mma.sync m16n8k16: at 4..16
-// live rows a tcgen05 tile would be mostly padding and the kernel is HBM-bound anyway), with an
-// online softmax in the exp2 domain. Warps are merged through shared memory, the split result
+// Grid = batch x kv_heads x splits CTAs of 4 warps. A CTA owns one (batch, kv head, KV range): each warp
+// streams 16-token K/V blocks of the range through its own cp.async ring (no CTA barrier in the main loop) and
+// runs S^T = K Q^T and O^T = V^T P^T on tensor cores (mma.sync m16n8k16: at 1..16 live heads a tcgen05 tile would
+// be mostly padding and the kernel is HBM-bound anyway), with an online softmax in the exp2 domain. Tokens (and
+// then head dimensions) are the 16 rows of the MMA, the G = Hq/Hkv query heads sharing the kv head its 8 columns
+// (two tiles of them above 8 heads; columns >= G are zero): with heads as the rows half of every MMA, exponential and
+// accumulator of up to 8 heads was padding, and the kernel was bound by its instructions where a block is small or a
+// score costs much (16 heads of 64, 955863 keys, soft cap: 868 us with heads as rows, 681 us here;
+// 51 ragged sequences to 157988 keys, 6 heads of 64, pages of one: 425 and 404 us;
+// 44 x 23296 keys, 8 heads of 128 per kv head: 713 and 666 us). Q stays in registers.
+// Warps are merged through shared memory, the split result
 // (normalised O, natural-log LSE) goes to a workspace, and the LAST CTA to finish a (batch, kv head)
 // merges all splits. With up to eight splits the CTAs of a (batch, kv head) are launched as one thread-block
 // cluster instead: every CTA stores its result straight into the first CTA's shared memory (st.shared::cluster), a
@@ -53,6 +58,7 @@ struct DecodeParams {
     void* out;              // mode 0/2: T [B, Hq, D]; mode 1: float [B, Hq, D + 1]
     char* ll_peer[kMaxRanks];  // SP: this call's parity of every rank: [world][B*Hq*(D+2)/2] packets
     int B, Hq, Hkv, page_size, max_blocks, splits;
+    int page_shift;         // log2(page_size), or -1
     int cluster_merge;      // 1: the splits of a (batch, kv head) are one thread-block cluster and merge through shared memory
     long long stride_block, stride_token, stride_head;  // cache strides in elements
     float scale, soft_cap;
@@ -120,20 +126,31 @@ __device__ __forceinline__ uint32_t tile_off(int row, int chunk) {
     return static_cast<uint32_t>(row * (D * 2) + ((chunk ^ (row & 7)) << 4));
 }
 
-// Ring depth: D <= 64 -> 4 stages (68 KB, 3 CTAs/SM); D = 128 -> 3 stages (100 KB, 2 CTAs/SM);
-// D = 256 -> 2 stages (136 KB, 1 CTA/SM).
-__host__ __device__ constexpr int decode_stages(int d) { return d <= 64 ? 4 : (d <= 128 ? 3 : 2); }
+// Ring depth: D <= 64 -> 4 stages (64 KB, 3 CTAs/SM); D = 128 -> 3 stages (96 KB, 2 CTAs/SM);
+// D = 256 -> 3 stages (192 KB, 1 CTA/SM; two would
+// leave one block of a warp in flight).
+__host__ __device__ constexpr int decode_stages(int d) { return d <= 64 ? 4 : 3; }
+// floats between the heads of a warp's O in shared memory (the four heads a store writes at once lie in different banks)
+__host__ __device__ constexpr int decode_o_pitch(int d) { return d + 4; }
 
-template <typename T, int D>
-__global__ void __launch_bounds__(kDecodeThreads, (D <= 128 ? 2 : 1)) flash_decode_kernel(const DecodeParams p) {
+__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
+    uint32_t r;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(a));
+    return r;
+}
+
+template <typename T, int D, int NH>
+__global__ void __launch_bounds__(kDecodeThreads, (D <= 64 ? 3 : (D <= 128 ? 2 : 1))) flash_decode_kernel(const DecodeParams p) {
     constexpr int CH = D / 8;                      // 16-byte chunks per row
     constexpr int TILE = kTok * D * 2;             // bytes of one K or V block
     constexpr int NS = decode_stages(D);           // cp.async ring depth per warp
-    constexpr int KS = D / 16;                     // k-steps of QK^T
-    constexpr int NT = D / 8;                      // n-tiles of PV
-    extern __shared__ __align__(128) uint8_t smem[];
-    uint8_t* q_s = smem;                                            // 16 x D
-    uint8_t* ring = smem + kTok * D * 2;                            // [warps][NS][K|V]
+    constexpr int KS = D / 16;                     // k-steps of K Q^T
+    constexpr int MT = D / 16;                     // tiles of 16 head dimensions of V^T P^T
+    constexpr int HEADS = NH * 8;
+    constexpr int OP = decode_o_pitch(D);
+    extern __shared__ uint8_t smem_raw[];
+    // aligned to a row, so that a chunk's address is the row's with some bits flipped
+    uint8_t* ring = smem_raw + ((D * 2 - (smem_u32(smem_raw) & (D * 2 - 1))) & (D * 2 - 1));   // [warps][NS][K|V]
     __shared__ float m_s[kDecodeWarps][16], l_s[kDecodeWarps][16];
     __shared__ int last_s;
 
@@ -158,32 +175,42 @@ __global__ void __launch_bounds__(kDecodeThreads, (D <= 128 ? 2 : 1)) flash_deco
     const int my_blocks = (blk1 - blk0 - warp + kDecodeWarps - 1) / kDecodeWarps;  // may be <= 0
 
     uint8_t* my_ring = ring + static_cast<size_t>(warp) * NS * 2 * TILE;
-    // Page-table lookup for block i of this warp: lane r < 16 resolves token r. It is issued one
-    // block ahead of the copies that need it, so its latency hides behind a block's worth of math
-    // instead of stalling the (in-order) warp right before every batch of cp.async.
+    // Page-table lookup of block i of this warp, issued one block ahead of the copies that need it, so that its latency
+    // hides behind a block's worth of math instead of stalling the (in-order) warp right before every batch of cp.async.
+    // Pages of a multiple of 16 tokens: a block lies in one page, every lane gets the block's offset. Others: lane r < 16
+    // gets token r's offset, or -1 past the end.
+    const bool whole = (p.page_size & (kTok - 1)) == 0;
     auto lookup = [&](int i) -> long long {
         long long base = -1;
-        if (i < my_blocks && lane < kTok) {
-            const int t = (blk0 + warp + i * kDecodeWarps) * kTok + lane;
+        if (i < my_blocks && (whole || lane < kTok)) {
+            const int t = (blk0 + warp + i * kDecodeWarps) * kTok + (whole ? 0 : lane);
             if (t < kv_len) {
-                const int page = table[t / p.page_size];
-                base = static_cast<long long>(page) * p.stride_block + static_cast<long long>(t % p.page_size) * p.stride_token;
+                const int in_table = p.page_shift >= 0 ? t >> p.page_shift : t / p.page_size;
+                const int page = table[in_table];
+                base = static_cast<long long>(page) * p.stride_block + static_cast<long long>(t - in_table * p.page_size) * p.stride_token;
             }
         }
         return base;
     };
+    // this lane's first chunk of a block; its further ones lie 32 / CH rows apart
+    constexpr int ROWS = 32 / CH;                  // rows a warp instruction copies
+    const int lrow = lane / CH, lch = lane % CH;
+    const T* kl = kc + lch * 8;
+    const T* vl = vc + lch * 8;
+    const long long row_off = static_cast<long long>(lrow) * p.stride_token;
     auto issue = [&](int i, long long base) {  // i-th block of this warp -> ring slot i % NS
-        uint8_t* ks = my_ring + static_cast<size_t>(i % NS) * 2 * TILE;
-        uint8_t* vs = ks + TILE;
+        const uint32_t ks = smem_u32(my_ring) + static_cast<uint32_t>(i % NS) * (2 * TILE);
+        const int left = kv_len - (blk0 + warp + i * kDecodeWarps) * kTok;   // tokens from the block's first on
 #pragma unroll
-        for (int j = 0; j < (kTok * CH) / 32; ++j) {
-            const int c = j * 32 + lane;
-            const int row = c / CH, ch = c % CH;
-            const long long rb = __shfl_sync(0xffffffffu, base, row);
-            const int nbytes = rb >= 0 ? 16 : 0;  // rows past the end are zero-filled
-            const long long off = (rb >= 0 ? rb : 0) + ch * 8;
-            cp_async16(smem_u32(ks + tile_off<D>(row, ch)), kc + off, nbytes);
-            cp_async16(smem_u32(vs + tile_off<D>(row, ch)), vc + off, nbytes);
+        for (int j = 0; j < kTok / ROWS; ++j) {
+            const int row = j * ROWS + lrow;
+            long long off = base + row_off + static_cast<long long>(j * ROWS) * p.stride_token;
+            if (!whole) off = __shfl_sync(0xffffffffu, base, row);
+            // rows past the end are zero-filled
+            const int nbytes = row < left ? 16 : 0;
+            if (nbytes == 0) off = 0;
+            cp_async16(ks + tile_off<D>(row, lch), kl + off, nbytes);
+            cp_async16(ks + TILE + tile_off<D>(row, lch), vl + off, nbytes);
         }
     };
 
@@ -194,20 +221,40 @@ __global__ void __launch_bounds__(kDecodeThreads, (D <= 128 ? 2 : 1)) flash_deco
         if (i < my_blocks) issue(i, base);
         cp_async_commit();
     }
-    // ---- Q tile into shared memory (rows >= G are zero), under the first K / V loads
-    for (int c = tid; c < 16 * CH; c += kDecodeThreads) {
-        const int row = c / CH, ch = c % CH;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (row < G) v = *reinterpret_cast<const uint4*>(q + static_cast<size_t>(row) * D + ch * 8);
-        *reinterpret_cast<uint4*>(q_s + tile_off<D>(row, ch)) = v;
-    }
-    __syncthreads();
-
-    float o[NT][4];
+    // ---- Q as the MMA's second operand, in registers, loaded under the first K / V blocks: head 8 h + lane / 4 is a column,
+    // its values 16 k + 2 (lane % 4) + {0, 1} and 8 further on are this lane's
+    uint32_t qf[NH][KS][2];
 #pragma unroll
-    for (int i = 0; i < NT; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-    float m_run[2] = {-CUDART_INF_F, -CUDART_INF_F}, l_run[2] = {0.f, 0.f};
+    for (int h = 0; h < NH; ++h) {
+        const int g = h * 8 + (lane >> 2);
+#pragma unroll
+        for (int k = 0; k < KS; ++k) {
+            const uint32_t* src = reinterpret_cast<const uint32_t*>(q + static_cast<size_t>(g < G ? g : 0) * D + k * 16 + (lane & 3) * 2);
+            qf[h][k][0] = g < G ? src[0] : 0u;
+            qf[h][k][1] = g < G ? src[4] : 0u;
+        }
+    }
+
+    // O^T: rows are dimensions 16 j + lane / 4 (+ 8), columns this lane's heads 8 h + 2 (lane % 4) + {0, 1}
+    float o[NH][MT][4];
+#pragma unroll
+    for (int h = 0; h < NH; ++h)
+#pragma unroll
+        for (int j = 0; j < MT; ++j) o[h][j][0] = o[h][j][1] = o[h][j][2] = o[h][j][3] = 0.f;
+    float m_run[NH][2], m_use[NH][2], l_run[NH][2];
+#pragma unroll
+    for (int h = 0; h < NH; ++h)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            m_run[h][r] = -CUDART_INF_F;
+            m_use[h][r] = l_run[h][r] = 0.f;
+        }
     const float sl2 = p.scale * 1.4426950408889634f;
+    // ldmatrix addresses inside a block: row, and the swizzled chunk with the lane's part of its number
+    const int krow = (lane & 7) + ((lane >> 3) & 1) * 8;
+    const uint32_t k_at = static_cast<uint32_t>(krow * (D * 2)) + static_cast<uint32_t>(((lane >> 4) ^ (krow & 7)) << 4);
+    const int vrow = (lane & 7) + (lane >> 4) * 8;
+    const uint32_t v_at = static_cast<uint32_t>(vrow * (D * 2)) + static_cast<uint32_t>((((lane >> 3) & 1) ^ (vrow & 7)) << 4);
 
     for (int i = 0; i < my_blocks; ++i) {
         if (i + NS - 1 < my_blocks) {
@@ -218,104 +265,117 @@ __global__ void __launch_bounds__(kDecodeThreads, (D <= 128 ? 2 : 1)) flash_deco
         cp_async_commit();
         cp_async_wait<NS - 1>();
         __syncwarp();
-        const uint8_t* ks = my_ring + static_cast<size_t>(i % NS) * 2 * TILE;
-        const uint8_t* vs = ks + TILE;
+        const uint32_t ks = smem_u32(my_ring) + static_cast<uint32_t>(i % NS) * (2 * TILE);
+        const uint32_t ka = ks + k_at, va = ks + TILE + v_at;
         const int tok0 = (blk0 + warp + i * kDecodeWarps) * kTok;
 
-        // S = Q K^T for 16 tokens: two n-tiles of 8
-        float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+        // S^T = K Q^T: rows are tokens lane / 4 (+ 8), columns the lane's two heads of each tile
+        float s[NH][4];
+#pragma unroll
+        for (int h = 0; h < NH; ++h) s[h][0] = s[h][1] = s[h][2] = s[h][3] = 0.f;
 #pragma unroll
         for (int k = 0; k < KS; ++k) {
-            uint32_t a[4], bf[4];
-            ldmatrix_x4(smem_u32(q_s + tile_off<D>((lane & 7) + ((lane >> 3) & 1) * 8, 2 * k + (lane >> 4))), a);
-            ldmatrix_x4(smem_u32(ks + tile_off<D>((lane & 7) + (lane >> 4) * 8, 2 * k + ((lane >> 3) & 1))), bf);
-            mma16816<T>(s[0], a, bf[0], bf[1]);
-            mma16816<T>(s[1], a, bf[2], bf[3]);
-        }
-        // scale, soft cap, mask, online softmax (rows lane/4 and lane/4 + 8)
-        float mx[2] = {-CUDART_INF_F, -CUDART_INF_F};
+            uint32_t a[4];
+            ldmatrix_x4(ka ^ static_cast<uint32_t>(k * 32), a);
 #pragma unroll
-        for (int nt = 0; nt < 2; ++nt)
+            for (int h = 0; h < NH; ++h) mma16816<T>(s[h], a, qf[h][k][0], qf[h][k][1]);
+        }
+        // scale, soft cap, mask, online softmax
+        bool higher = false;
+#pragma unroll
+        for (int h = 0; h < NH; ++h)
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const int tok = tok0 + nt * 8 + (lane & 3) * 2 + (e & 1);
-                float v = s[nt][e];
+                float v = s[h][e];
                 if (p.soft_cap > 0.f) v = p.soft_cap * tanhf(v * p.scale / p.soft_cap) * 1.4426950408889634f;
                 else v *= sl2;
-                v = tok < kv_len ? v : -CUDART_INF_F;
-                s[nt][e] = v;
-                mx[e >> 1] = fmaxf(mx[e >> 1], v);
+                if (tok0 + kTok > kv_len) v = tok0 + (lane >> 2) + (e >> 1) * 8 < kv_len ? v : -CUDART_INF_F;
+                s[h][e] = v;
+                higher |= v > m_run[h][e & 1];
             }
-        float alpha[2], m_use[2];
+        // The maxima rise often in the first blocks and seldom later: a block that raises none needs this vote instead of the
+        // reductions over the lanes and the scaling of O. (Letting scores exceed the old maximum by up to 2^4 before it is
+        // raised saves a little more and costs precision: the largest probability is then rounded too, where it is 1 here.
+        // Error against 64 bits of 4096 bf16 keys 2.2e-3, 2.0e-3 here.)
+        if (__any_sync(0xffffffffu, higher)) {
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
-            mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
-            const float m_new = fmaxf(m_run[r], mx[r]);
-            m_use[r] = m_new == -CUDART_INF_F ? 0.f : m_new;
-            alpha[r] = exp2f(m_run[r] - m_use[r]);
-            m_run[r] = m_new;
+            for (int h = 0; h < NH; ++h)
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    float mx = fmaxf(s[h][r], s[h][2 + r]);
+                    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+                    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+                    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+                    const float m_new = fmaxf(m_run[h][r], mx);
+                    m_use[h][r] = m_new == -CUDART_INF_F ? 0.f : m_new;
+                    const float alpha = exp2f(m_run[h][r] - m_use[h][r]);
+                    m_run[h][r] = m_new;
+                    l_run[h][r] *= alpha;
+#pragma unroll
+                    for (int j = 0; j < MT; ++j) {
+                        o[h][j][r] *= alpha;
+                        o[h][j][2 + r] *= alpha;
+                    }
+                }
         }
-        float rs[2] = {0.f, 0.f};
-        uint32_t pa[4];
+        // P^T as the second operand: tokens in pairs per lane, heads over lane / 4
+        uint32_t pb[NH][2];
 #pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-            const float p0 = exp2f(s[nt][0] - m_use[0]), p1 = exp2f(s[nt][1] - m_use[0]);
-            const float p2 = exp2f(s[nt][2] - m_use[1]), p3 = exp2f(s[nt][3] - m_use[1]);
-            rs[0] += p0 + p1;
-            rs[1] += p2 + p3;
-            pa[nt * 2 + 0] = pack2<T>(p0, p1);
-            pa[nt * 2 + 1] = pack2<T>(p2, p3);
+        for (int h = 0; h < NH; ++h) {
+            const float p0 = exp2f(s[h][0] - m_use[h][0]), p1 = exp2f(s[h][1] - m_use[h][1]);
+            const float p2 = exp2f(s[h][2] - m_use[h][0]), p3 = exp2f(s[h][3] - m_use[h][1]);
+            l_run[h][0] += p0 + p2;   // this lane's tokens; the lanes' sums meet after the loop
+            l_run[h][1] += p1 + p3;
+            pb[h][0] = movmatrix_trans(pack2<T>(p0, p1));
+            pb[h][1] = movmatrix_trans(pack2<T>(p2, p3));
         }
+        // O^T += V^T P^T
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            rs[r] += __shfl_xor_sync(0xffffffffu, rs[r], 1);
-            rs[r] += __shfl_xor_sync(0xffffffffu, rs[r], 2);
-            l_run[r] = l_run[r] * alpha[r] + rs[r];
-        }
-        // O = O * alpha + P V
+        for (int j = 0; j < MT; ++j) {
+            uint32_t a[4];
+            ldmatrix_x4_trans(va ^ static_cast<uint32_t>(j * 32), a);
 #pragma unroll
-        for (int j = 0; j < NT / 2; ++j) {
-            uint32_t bf[4];
-            ldmatrix_x4_trans(smem_u32(vs + tile_off<D>((lane & 7) + ((lane >> 3) & 1) * 8, 2 * j + (lane >> 4))), bf);
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                float (&acc)[4] = o[2 * j + h];
-                acc[0] *= alpha[0];
-                acc[1] *= alpha[0];
-                acc[2] *= alpha[1];
-                acc[3] *= alpha[1];
-                mma16816<T>(acc, pa, bf[2 * h], bf[2 * h + 1]);
-            }
+            for (int h = 0; h < NH; ++h) mma16816<T>(o[h][j], a, pb[h][0], pb[h][1]);
         }
         __syncwarp();
     }
+#pragma unroll
+    for (int h = 0; h < NH; ++h)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            l_run[h][r] += __shfl_xor_sync(0xffffffffu, l_run[h][r], 4);
+            l_run[h][r] += __shfl_xor_sync(0xffffffffu, l_run[h][r], 8);
+            l_run[h][r] += __shfl_xor_sync(0xffffffffu, l_run[h][r], 16);
+        }
     cp_async_wait<0>();
     __syncthreads();
 
     // ---- merge the warps through shared memory (the ring is free now)
-    float* o_s = reinterpret_cast<float*>(ring);  // [warps][16][D]
-    {
-        const int r0 = lane >> 2;
-        if ((lane & 3) == 0) {
-            m_s[warp][r0] = m_run[0];
-            m_s[warp][r0 + 8] = m_run[1];
-            l_s[warp][r0] = l_run[0];
-            l_s[warp][r0 + 8] = l_run[1];
-        }
+    float* o_s = reinterpret_cast<float*>(ring);  // [warps][HEADS][OP]
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-            const int col = nt * 8 + (lane & 3) * 2;
-            float* base = o_s + (static_cast<size_t>(warp) * 16) * D;
-            *reinterpret_cast<float2*>(base + static_cast<size_t>(r0) * D + col) = make_float2(o[nt][0], o[nt][1]);
-            *reinterpret_cast<float2*>(base + static_cast<size_t>(r0 + 8) * D + col) = make_float2(o[nt][2], o[nt][3]);
+    for (int h = 0; h < NH; ++h) {
+        const int g0 = h * 8 + (lane & 3) * 2;
+        if (lane < 4) {
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                m_s[warp][g0 + r] = m_run[h][r];
+                l_s[warp][g0 + r] = l_run[h][r];
+            }
+        }
+        float* base = o_s + (static_cast<size_t>(warp) * HEADS + g0) * OP + (lane >> 2);
+#pragma unroll
+        for (int j = 0; j < MT; ++j) {
+            base[j * 16] = o[h][j][0];
+            base[OP + j * 16] = o[h][j][1];
+            base[j * 16 + 8] = o[h][j][2];
+            base[OP + j * 16 + 8] = o[h][j][3];
         }
     }
     const int W2 = D + 2;  // floats per head in the workspace and in the gather buffers: O, LSE, pad
     // cluster merge: the partials of all splits land in the ring of the cluster's first CTA, behind the results of that
     // CTA's warps (shared memory of their own would leave room for one CTA per SM instead of two), so every CTA of the
     // cluster has to be done with its ring first
-    float* part_s = o_s + kDecodeWarps * 16 * D;
+    float* part_s = o_s + kDecodeWarps * HEADS * OP;
     const uint32_t part_leader = p.cluster_merge ? mapa_u32(smem_u32(part_s), 0) : 0u;
     if (p.cluster_merge) {
         cluster_arrive();
@@ -334,7 +394,7 @@ __global__ void __launch_bounds__(kDecodeThreads, (D <= 128 ? 2 : 1)) flash_deco
         for (int w = 0; w < kDecodeWarps; ++w) {
             const float f = exp2f(m_s[w][g] - mu);
             l += l_s[w][g] * f;
-            acc += o_s[(static_cast<size_t>(w) * 16 + g) * D + c] * f;
+            acc += o_s[(static_cast<size_t>(w) * HEADS + g) * OP + c] * f;
         }
         const float val = l > 0.f ? acc / l : 0.f;
         const float lse = l > 0.f ? mm * 0.6931471805599453f + logf(l) : -CUDART_INF_F;
@@ -466,7 +526,7 @@ __global__ void __launch_bounds__(kDecodeThreads, (D <= 128 ? 2 : 1)) flash_deco
     }
     if (p.push_only) return;
     // gather: lse of every (source, head) first, then the weighted sum
-    float* lse_s = reinterpret_cast<float*>(q_s);  // [world][G]  (Q tile is dead)
+    float* lse_s = w_s;   // [world][G]  (the split weights are dead: every warp is past the merge)
     const char* mine = ll[p.rank];
     for (int idx = tid; idx < p.world * G; idx += kDecodeThreads) {
         const int r = idx / G, g = idx % G;
@@ -557,12 +617,13 @@ static bool overlaps_previous(const DecodeParams& p) {
     return p.B == 1 || keys <= kOverlapKeys || ctas > 2LL * tdist_host::sm_count();
 }
 
-template <typename T, int D>
+template <typename T, int D, int NH>
 static int launch_decode(DecodeParams& p, cudaStream_t stream) {
-    constexpr int NS = decode_stages(D);
-    constexpr int smem = kTok * D * 2 + kDecodeWarps * NS * 2 * kTok * D * 2;
-    constexpr int part_room = kDecodeWarps * NS * 2 * kTok * D * 2 - kDecodeWarps * 16 * D * 4;   // ring behind the warps' results
-    static_assert(part_room > 0, "the warp-merge buffer reuses the ring");
+    constexpr int ring = kDecodeWarps * decode_stages(D) * 2 * kTok * D * 2;
+    constexpr int smem = ring + D * 2;   // and its alignment
+    constexpr int part_room = ring - kDecodeWarps * NH * 8 * decode_o_pitch(D) * 4;   // ring behind the warps' results
+    static_assert(part_room > 0 && 16 * (D + 2) + kDecodeWarps * 256 <= kDecodeWarps * NH * 8 * decode_o_pitch(D),
+                  "the merge's buffers reuse the warps' results, the partials of a cluster lie behind them");
     static bool done[64] = {};
     static std::mutex setup_lock;
     static const bool cluster_enabled = [] {
@@ -575,7 +636,7 @@ static int launch_decode(DecodeParams& p, cudaStream_t stream) {
     {
         std::lock_guard<std::mutex> guard(setup_lock);
         if (!done[dev]) {
-            TDIST_CUDA_OK(cudaFuncSetAttribute(flash_decode_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+            TDIST_CUDA_OK(cudaFuncSetAttribute(flash_decode_kernel<T, D, NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
             done[dev] = true;
         }
     }
@@ -599,7 +660,7 @@ static int launch_decode(DecodeParams& p, cudaStream_t stream) {
         dim.val.clusterDim.z = 1;
     }
     p.cluster_merge = cluster ? 1 : 0;
-    TDIST_CUDA_OK(cudaLaunchKernelEx(&cfg, flash_decode_kernel<T, D>, p));
+    TDIST_CUDA_OK(cudaLaunchKernelEx(&cfg, flash_decode_kernel<T, D, NH>, p));
     return 0;
 }
 
@@ -626,6 +687,7 @@ static int flash_decode_impl(const TdistDecodeArgs* a) {
     p.Hq = a->Hq;
     p.Hkv = a->Hkv;
     p.page_size = a->page_size;
+    p.page_shift = (a->page_size & (a->page_size - 1)) == 0 ? __builtin_ctz(static_cast<unsigned>(a->page_size)) : -1;
     p.max_blocks = a->max_blocks;
     p.splits = a->splits;
     p.stride_block = a->stride_block;
@@ -664,7 +726,8 @@ static int flash_decode_impl(const TdistDecodeArgs* a) {
         }
     }
     cudaStream_t stream = static_cast<cudaStream_t>(a->stream);
-#define TDIST_DECODE_CASE(TT, DD) return launch_decode<TT, DD>(p, stream)
+#define TDIST_DECODE_CASE(TT, DD) return G <= 8 ? launch_decode<TT, DD, 1>(p, stream) : launch_decode<TT, DD, 2>(p, stream)
+    const int G = p.Hq / p.Hkv;
     if (a->dtype == TDIST_BF16) {
         if (a->head_dim == 64) TDIST_DECODE_CASE(__nv_bfloat16, 64);
         if (a->head_dim == 128) TDIST_DECODE_CASE(__nv_bfloat16, 128);
