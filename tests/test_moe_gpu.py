@@ -35,6 +35,29 @@ def test_route_is_a_stable_expert_sort(cuda_device, T, E, K):
         assert torch.equal(got.cpu(), want)
 
 
+@pytest.mark.parametrize("E", [1, 7, 1024, 1025, 2048])   # 1024 | 1025: 32 and 16 warps
+@pytest.mark.parametrize("T,K", [(1, 1), (33, 1), (1024, 1), (1025, 1), (513, 8), (4099, 5)])
+def test_route_runs_of_every_length(cuda_device, T, E, K):
+    """Pairs that end inside a warp's run, runs that are empty, and dropped pairs (id -1 or E) anywhere among them."""
+    from triton_distributed_b200._lib import TdistError
+    torch.manual_seed(T + E)
+    ids = torch.randint(0, E, (T, K), dtype=torch.int32, device=cuda_device)
+    for dropped in (False, True):
+        if dropped:
+            ids.view(-1)[torch.randperm(T * K, device=cuda_device)[: 1 + T * K // 9]] = -1
+            ids[0, 0] = E
+        r, ref = MU.route(ids, E), MU.route(ids.cpu(), E)
+        if dropped:
+            with pytest.raises(TdistError, match="bad argument"):
+                check_status()
+        else:
+            check_status()
+        live = int(ref.splits.sum())
+        for got, want in zip(r, ref):
+            n = live if want is ref.sorted_token else want.numel()
+            assert torch.equal(got.cpu()[:n], want[:n])
+
+
 @pytest.mark.parametrize("ranks,tpr,E,K,bs", [(8, 128, 32, 2, 128), (4, 1000, 8, 4, 64), (2, 17, 256, 8, 16), (1, 300, 60, 5, 128)])
 def test_align_block_size_matches_oracle(cuda_device, ranks, tpr, E, K, bs):
     torch.manual_seed(ranks * tpr)

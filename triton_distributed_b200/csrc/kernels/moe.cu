@@ -21,18 +21,57 @@ namespace tdist {
 
 // ---------------------------------------------------------------------------- routing for EP
 // ids[n] (n = tokens * topk, token-major) -> splits[E], cumsum[E+1], sorted_token[n] (token of the
-// pair at each sorted position), slot_of[n] (sorted position of each pair). One CTA.
-__global__ void __launch_bounds__(kMoeThreads) moe_route_kernel(const int* ids, int n, int topk, int E, int* splits,
-                                                                int* cumsum, int* sorted_token, int* slot_of,
-                                                                WaitCtx w) {
+// pair at each sorted position), slot_of[n] (sorted position of each pair). One CTA; a chain of latencies, so few steps: every
+// warp counts a contiguous run of the pairs by itself (position inside the run's group = count so far + equal ids in lower
+// lanes, kept in slot_of meanwhile), prefix sums over the warps and over the experts follow, then every pair's position is
+// known. (Histogram, then 512 pairs at a time with the CTA meeting four times for each: the
+// whole expert-parallel block of 1194 tokens, top 8 of 16, 280 us, 267 here; 1831 tokens, top 7 of 16, 323 and 314.)
+constexpr int kRouteAhead = 4;   // loads of a lane in flight
+__global__ void __launch_bounds__(1024) moe_route_kernel(const int* ids, int n, int topk, int E, int* splits,
+                                                         int* cumsum, int* sorted_token, int* slot_of, WaitCtx w) {
     extern __shared__ int sm[];
-    int* hist = sm;
-    int* running = sm + E;
-    int* cnt = sm + 2 * E;
-    histogram(ids, n, E, hist, w);
-    if (threadIdx.x < 32) {
+    const int tid = static_cast<int>(threadIdx.x), warp = tid >> 5, lane = tid & 31;
+    const int threads = static_cast<int>(blockDim.x), warps = threads >> 5;
+    int* first = sm;        // sorted position of an expert's first pair
+    int* hist = sm + E;
+    int* cnt = sm + 2 * E;  // [warps][E]
+    for (int j = tid; j < warps * E; j += threads) cnt[j] = 0;
+    pdl_wait_and_release();
+    __syncthreads();
+    const int run = (n + threads - 1) / threads * 32;   // pairs of a warp
+    const int begin = warp * run, end = min(n, begin + run);
+    int* mine = cnt + warp * E;
+    for (int i0 = begin; i0 < end; i0 += 32 * kRouteAhead) {
+        int es[kRouteAhead];
+#pragma unroll
+        for (int u = 0; u < kRouteAhead; ++u) es[u] = i0 + u * 32 + lane < end ? ids[i0 + u * 32 + lane] : -1;
+#pragma unroll
+        for (int u = 0; u < kRouteAhead; ++u) {
+            const int i = i0 + u * 32 + lane, e = es[u];
+            const bool valid = i < end && expert_in_range(e, E);
+            if (i < end && !valid) report_bad_expert(w, i, e, E, 1);
+            const unsigned same = __match_any_sync(0xffffffffu, valid ? e : E + lane);   // idle lanes and rejected ids match nobody
+            const int before = valid ? mine[e] : 0;
+            __syncwarp();
+            if (valid && (same & lanemask_lt()) == 0) mine[e] = before + __popc(same);
+            __syncwarp();
+            if (i < end) slot_of[i] = valid ? before + __popc(same & lanemask_lt()) : -1;   // -1: a pair whose expert id was rejected
+        }
+    }
+    __syncthreads();
+    for (int e = tid; e < E; e += threads) {
+        int total = 0;
+        for (int k = 0; k < warps; ++k) {
+            const int c = cnt[k * E + e];
+            cnt[k * E + e] = total;
+            total += c;
+        }
+        hist[e] = total;
+        splits[e] = total;
+    }
+    __syncthreads();
+    if (warp == 0) {
         // exclusive scan of the histogram by one warp: a contiguous chunk of experts per lane
-        const int lane = threadIdx.x;
         const int per = (E + 31) / 32;
         const int e0 = min(E, lane * per), e1 = min(E, e0 + per);
         int local = 0;
@@ -45,18 +84,31 @@ __global__ void __launch_bounds__(kMoeThreads) moe_route_kernel(const int* ids, 
         }
         int acc = incl - local;
         for (int e = e0; e < e1; ++e) {
-            running[e] = acc;
+            first[e] = acc;
             cumsum[e] = acc;
-            splits[e] = hist[e];
             acc += hist[e];
         }
         if (lane == 31) cumsum[E] = incl;
     }
     __syncthreads();
-    stable_positions(ids, n, E, running, cnt, w, [&](int i, int pos) {
-        slot_of[i] = pos;   // -1 for a pair whose expert id was rejected
-        if (pos >= 0) sorted_token[pos] = i / topk;
-    });
+    // the same lanes as above: they read back their own stores
+    for (int i0 = begin; i0 < end; i0 += 32 * kRouteAhead) {
+        int es[kRouteAhead], in_run[kRouteAhead];
+#pragma unroll
+        for (int u = 0; u < kRouteAhead; ++u) {
+            const int i = i0 + u * 32 + lane;
+            es[u] = i < end ? ids[i] : 0;
+            in_run[u] = i < end ? slot_of[i] : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < kRouteAhead; ++u) {
+            if (in_run[u] < 0) continue;
+            const int i = i0 + u * 32 + lane;
+            const int pos = first[es[u]] + mine[es[u]] + in_run[u];
+            slot_of[i] = pos;
+            sorted_token[pos] = i / topk;
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------- block-aligned sort
@@ -367,13 +419,13 @@ extern "C" int tdist_moe_route(const void* ids, int n, int topk, int num_experts
                                void* sorted_token, void* slot_of, void* status, void* stream) {
     if (num_experts < 1 || num_experts > 2048) return fail(TDIST_ELIMIT, "moe_route: at most 2048 experts");
     if (topk < 1 || n < 0) return fail(TDIST_EINVAL, "moe_route: bad sizes");
-    const int smem = moe_smem_bytes(num_experts);
+    const int threads = num_experts <= 1024 ? 1024 : 512;   // a row of counts per warp has to fit
+    const int smem = (2 + threads / 32) * num_experts * static_cast<int>(sizeof(int));
     int rc = ensure_smem(moe_route_kernel, smem);
     if (rc) return rc;
-    moe_route_kernel<<<1, kMoeThreads, smem, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const int*>(ids), n, topk, num_experts, static_cast<int*>(splits), static_cast<int*>(cumsum),
-        static_cast<int*>(sorted_token), static_cast<int*>(slot_of), moe_wctx(status));
-    TDIST_CUDA_OK(cudaGetLastError());
+    TDIST_CUDA_OK(tdist_host::launch_pdl(moe_route_kernel, dim3(1), threads, smem, static_cast<cudaStream_t>(stream),
+                                         static_cast<const int*>(ids), n, topk, num_experts, static_cast<int*>(splits), static_cast<int*>(cumsum),
+                                         static_cast<int*>(sorted_token), static_cast<int*>(slot_of), moe_wctx(status)));
     return 0;
 }
 
