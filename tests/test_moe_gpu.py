@@ -291,6 +291,24 @@ def test_gate_topk_is_no_further_from_float64_than_the_fp32_product(cuda_device,
     torch.testing.assert_close(w, w_t, rtol=1e-6, atol=0)
 
 
+@pytest.mark.parametrize("T,hidden,E,k", [(1, 1024, 3, 2), (1, 8192, 1024, 8), (15, 2080, 16, 4), (300, 1536, 8, 2), (600, 4096, 64, 6), (1184, 1024, 60, 4)])
+def test_gate_topk_parts_of_the_hidden_dimension(cuda_device, T, hidden, E, k):
+    """One to eight parts, and the token counts from which on there are fewer. The products of bf16 are exact; a sum passes at most
+    hidden / 512 additions in a warp, 16 over the warps, 8 over the parts and two inside an MMA, each off by at most 2^-23 of the
+    sum of the magnitudes."""
+    torch.manual_seed(T + hidden + E)
+    x = torch.randn(T, hidden, device=cuda_device).bfloat16()
+    gate = (torch.randn(E, hidden, device=cuda_device) * hidden ** -0.5).bfloat16()
+    logits = torch.empty(T, E, device=cuda_device)
+    ids, w = MU.gate_topk(x, gate, k, logits=logits)
+    exact = x.double() @ gate.double().t()
+    spread = x.double().abs() @ gate.double().abs().t()
+    assert ((logits.double() - exact).abs() <= (hidden / 512 + 26) * 2.0 ** -23 * spread).all()
+    ids_t, w_t = MU.topk_softmax(logits, k)
+    assert torch.equal(ids, ids_t)
+    torch.testing.assert_close(w, w_t, rtol=1e-6, atol=0)
+
+
 @pytest.mark.parametrize("form", ["bf16", "strided", "misaligned", "short", "cpu"])
 def test_gate_topk_writes_logits_of_any_form_or_refuses_them(cuda_device, form):
     """Only a dense fp32 [T, E] buffer may be handed to the kernel as a pointer; the others are copied into, converted and

@@ -242,14 +242,18 @@ __global__ void moe_topk_softmax_kernel(const float* logits, int ntok, int E, in
 
 // ---------------------------------------------------------------------------- gate: logits, softmax and top-k in one launch
 // logits[t, e] = x[t, :] . gate[e, :] (bf16 in, fp32 sums), then the selection above. A decode step has few tokens and
-// few experts, so the product is short of parallelism, not of arithmetic: a CTA takes 16 tokens and ALL experts, and its
-// 16 warps split the hidden dimension 32 values at a time (what a cuBLAS SGEMM of the fp32 copies does serially; 128 x
+// few experts, so the product is short of parallelism, not of arithmetic: a CTA takes 16 tokens and ALL experts, its
+// 16 warps split the hidden dimension 32 values at a time, and up to eight CTAs of a cluster share it where the tokens leave
+// SMs idle (each adds its part of every token up, sends it to the CTA that selects for the token, which adds the parts:
+// 4 tokens x 4288, 64 experts: 12 us on one CTA, 7 on eight; the whole expert-parallel block 87 and 82) (what a cuBLAS SGEMM of the fp32 copies does serially; 128 x
 // 7168 x 32 experts: 53 us as two copies, SGEMM, reduction and selection, 12 us here). mma.sync m16n8k16: the products of bf16 values are exact in
 // fp32, the tensor core sums 32 of them at a time (its accumulator truncates, so longer chains there would lose bits
 // against an fp32 FMA loop), the rest is added in fp32: 1/16 of the hidden dimension per warp, then 16 partial sums. A tcgen05
 // tile (M 128) would leave all but 16 rows of this split idle. Any order of k will do as long as x and gate agree, so a
 // thread takes 8 consecutive values of its row per step: one 16-byte load feeds two MMAs.
 constexpr int kGateTok = 16, kGateThreads = 512, kGateWarps = kGateThreads / 32;
+
+constexpr int kGateMaxParts = 8;
 
 __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
@@ -260,15 +264,18 @@ __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], uint32_t a0, uint3
 // NT: groups of 8 experts per pass over the tokens' rows
 template <int NT>
 __global__ void __launch_bounds__(kGateThreads, 1) moe_gate_topk_kernel(const __nv_bfloat16* x, const __nv_bfloat16* gate, int ntok, int hidden, int E,
-                                                                        int topk, int renorm, int* ids, float* w, float* logits) {
+                                                                        int topk, int renorm, int parts, int* ids, float* w, float* logits) {
     extern __shared__ float gate_sm[];
     constexpr int COLS = NT * 8;
     float* part = gate_sm;                                   // [warps][16 tokens][COLS]
-    float* row_s = gate_sm + kGateWarps * kGateTok * COLS;   // [16 tokens][E]
+    float* row_s = gate_sm + kGateWarps * kGateTok * COLS;   // [parts][16 / parts tokens][E]: this CTA's tokens, a row per part
     const int tid = static_cast<int>(threadIdx.x), warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, tig = lane & 3;                 // row / column group of the MMA fragments
-    const int t0 = static_cast<int>(blockIdx.x) * kGateTok;
+    const int part_id = parts > 1 ? static_cast<int>(cluster_ctarank()) : 0;
+    const int t0 = static_cast<int>(blockIdx.x) / parts * kGateTok;
+    const int own = kGateTok / parts;   // tokens a CTA selects for
     const int steps = hidden / 32;
+    if (parts > 1) cluster_arrive();    // its counterpart stands before the first store into another CTA
     pdl_wait_and_release();
     // rows past the end repeat the last one; their results are not used
     const __nv_bfloat16* xa = x + static_cast<size_t>(min(t0 + g, ntok - 1)) * hidden + tig * 8;
@@ -282,7 +289,7 @@ __global__ void __launch_bounds__(kGateThreads, 1) moe_gate_topk_kernel(const __
             acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
         }
 #pragma unroll(NT == 8 ? 1 : 2)
-        for (int s = warp; s < steps; s += kGateWarps) {
+        for (int s = part_id * kGateWarps + warp; s < steps; s += parts * kGateWarps) {
             const uint4 a = ld_v4(xa + s * 32);
             const uint4 c = ld_v4(xb + s * 32);
             uint4 b[NT];
@@ -304,21 +311,37 @@ __global__ void __launch_bounds__(kGateThreads, 1) moe_gate_topk_kernel(const __
             *reinterpret_cast<float2*>(p + 8 * COLS) = make_float2(acc[n][2], acc[n][3]);
         }
         __syncthreads();
+        if (parts > 1 && e0 == 0) cluster_wait();   // every CTA of the cluster runs
         for (int i = tid; i < kGateTok * COLS; i += kGateThreads) {
             const int t = i / COLS, e = e0 + i % COLS;
             float sum = 0.f;
 #pragma unroll
             for (int k = 0; k < kGateWarps; ++k) sum += part[k * kGateTok * COLS + i];
-            if (e < E) {
+            if (e >= E) continue;
+            if (parts > 1) {
+                st_shared_cluster_f32(mapa_u32(smem_u32(row_s + (part_id * own + t % own) * E + e), static_cast<uint32_t>(t / own)), sum);
+            } else {
                 row_s[t * E + e] = sum;
                 if (logits != nullptr && t0 + t < ntok) logits[static_cast<size_t>(t0 + t) * E + e] = sum;
             }
         }
         __syncthreads();
     }
-    const int t = t0 + warp;   // a warp per token: kGateWarps == kGateTok
+    if (parts > 1) {
+        cluster_arrive();
+        cluster_wait();
+        for (int i = tid; i < own * E; i += kGateThreads) {
+            float sum = 0.f;
+            for (int k = 0; k < parts; ++k) sum += row_s[k * own * E + i];
+            row_s[i] = sum;   // part 0's own slot: this thread's alone
+            const int t = t0 + part_id * own + i / E;
+            if (logits != nullptr && t < ntok) logits[static_cast<size_t>(t) * E + i % E] = sum;
+        }
+        __syncthreads();
+    }
+    const int t = t0 + part_id * own + warp;   // a warp per token: kGateWarps == kGateTok
     static_assert(kGateWarps == kGateTok, "a warp per token");
-    if (t < ntok) topk_softmax_any(row_s + warp * E, E, topk, renorm, lane, ids + static_cast<size_t>(t) * topk, w + static_cast<size_t>(t) * topk);
+    if (warp < own && t < ntok) topk_softmax_any(row_s + warp * E, E, topk, renorm, lane, ids + static_cast<size_t>(t) * topk, w + static_cast<size_t>(t) * topk);
 }
 
 // ---------------------------------------------------------------------------- row gather / top-k reduce
@@ -468,14 +491,29 @@ extern "C" int tdist_moe_gate_topk(const void* x, const void* gate, int ntok, in
     if (ntok <= 0) return 0;
     const int nt = num_experts <= 8 ? 1 : (num_experts <= 16 ? 2 : (num_experts <= 32 ? 4 : 8));
     const int smem = (kGateWarps * kGateTok * nt * 8 + kGateTok * num_experts) * static_cast<int>(sizeof(float));
-    const dim3 grid((ntok + kGateTok - 1) / kGateTok);
+    // parts of the hidden dimension: while every warp has a step of its own and the CTAs have an SM of their own
+    const int tiles = (ntok + kGateTok - 1) / kGateTok;
+    int parts = 1;
+    while (parts < kGateMaxParts && 2 * parts * kGateWarps * 32 <= hidden && 2 * parts * tiles <= tdist_host::sm_count()) parts *= 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(tiles * parts));
+    cfg.blockDim = dim3(kGateThreads);
+    cfg.dynamicSmemBytes = static_cast<size_t>(smem);
+    cfg.stream = static_cast<cudaStream_t>(stream);
+    cudaLaunchAttribute attr[2];
+    attr[0] = tdist_host::pdl_attribute();
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = static_cast<unsigned>(parts);
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
 #define TDIST_GATE_CASE(NT)                                                                                                     \
     {                                                                                                                           \
         if (int rc = ensure_smem(moe_gate_topk_kernel<NT>, smem)) return rc;                                                    \
-        TDIST_CUDA_OK(tdist_host::launch_pdl(moe_gate_topk_kernel<NT>, grid, kGateThreads, smem, static_cast<cudaStream_t>(stream), \
-                                             static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gate), ntok,   \
-                                             hidden, num_experts, topk, renormalize, static_cast<int*>(ids),                    \
-                                             static_cast<float*>(weights), static_cast<float*>(logits)));                       \
+        TDIST_CUDA_OK(cudaLaunchKernelEx(&cfg, moe_gate_topk_kernel<NT>, static_cast<const __nv_bfloat16*>(x),                  \
+                                         static_cast<const __nv_bfloat16*>(gate), ntok, hidden, num_experts, topk, renormalize, parts, \
+                                         static_cast<int*>(ids), static_cast<float*>(weights), static_cast<float*>(logits)));   \
     }
     if (nt == 1) TDIST_GATE_CASE(1)
     else if (nt == 2) TDIST_GATE_CASE(2)
