@@ -25,6 +25,7 @@ import torch.distributed as dist
 import torch.nn.functional as F
 
 from .. import _lib
+from ..utils.misc import empty_of
 from ..utils.profile import nvtx_range
 from ..runtime import SymmTensor, counters_clean, default_timeout_ns, global_status, stream_ptr, symm_heap
 
@@ -103,7 +104,7 @@ def gemm_persistent(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor
         return (a.float() @ b.float().t()).to(a.dtype)
     _check_operands(a, b)
     M, N = a.shape[0], b.shape[0]
-    c = out if out is not None else torch.empty((M, N), dtype=a.dtype, device=a.device)
+    c = out if out is not None else empty_of(a, M, N)
     g = _base_args(a, b, 1, 0, _lib.GEMM_PLAIN)
     g.c = c.data_ptr()
     g.m_per_rank = M
@@ -191,7 +192,7 @@ def ag_gemm_intra_node(a: torch.Tensor, b: torch.Tensor, ctx: Optional[AllGather
     _check_operands(a, b)
     if mpr > ctx.max_m_per_rank or K != ctx.k:
         raise ValueError(f"shard {tuple(a.shape)} exceeds the context (max rows {ctx.max_m_per_rank}, K {ctx.k})")
-    c = out if out is not None else torch.empty((ctx.world * mpr, N), dtype=a.dtype, device=a.device)
+    c = out if out is not None else empty_of(a, ctx.world * mpr, N)
     g = _base_args(a, b, ctx.world, ctx.rank, _lib.GEMM_AG, cta_pair=ctx.cta_pair)
     g.c = c.data_ptr()
     g.m_per_rank = mpr
@@ -301,7 +302,7 @@ def gemm_rs(a: torch.Tensor, b: torch.Tensor, ctx: GEMMReduceScatterTensorParall
     _check_operands(a, b)
     if mpr > ctx.max_m_per_rank or N != ctx.n:
         raise ValueError(f"problem [{M},{N}] exceeds the context (max rows/rank {ctx.max_m_per_rank}, N {ctx.n})")
-    o = out if out is not None else torch.empty((mpr, N), dtype=a.dtype, device=a.device)
+    o = out if out is not None else empty_of(a, mpr, N)
     if ctx.world == 1:
         return gemm_persistent(a, b, out=o, num_sms=ctx.num_sms)  # nothing to scatter or reduce: skip the staging pass
     g = _base_args(a, b, ctx.world, ctx.rank, _lib.GEMM_RS, cta_pair=ctx.cta_pair)

@@ -32,6 +32,7 @@ import torch.distributed as dist
 
 from .. import _lib
 from ..runtime import SymmTensor, default_timeout_ns, global_status, stream_ptr, symm_heap
+from ..utils.misc import empty_of
 from ..utils.profile import nvtx_range
 from . import moe_utils
 
@@ -225,7 +226,7 @@ def ep_combine(ctx: EPContext, expert_out: Optional[torch.Tensor] = None, weight
         buf[: expert_out.shape[0]].copy_(expert_out)
     if phase & 1:
         ctx.combine_count += 1
-    o = out if out is not None else torch.empty((T, ctx.hidden), dtype=torch.bfloat16, device=buf.device)
+    o = out if out is not None else empty_of(buf, T, ctx.hidden)
     a = _lib.MoeCombineArgs.from_buffer_copy(ctx.templates[half][1])
     a.topk_ids = ctx.topk_ids.data_ptr()
     a.topk_w = ctx.topk_weights.data_ptr() if (weighted and ctx.topk_weights is not None) else None

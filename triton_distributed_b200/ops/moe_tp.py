@@ -31,6 +31,7 @@ import torch.distributed as dist
 
 from .. import _lib
 from ..runtime import counters_clean, stream_ptr, symm_heap
+from ..utils.misc import empty_of
 from . import collectives as CO
 from . import gemm as G
 from . import moe_utils as MU
@@ -108,7 +109,7 @@ def gather_rows(src: torch.Tensor, index: torch.Tensor, div: int, limit: int, wa
 def topk_reduce(y: torch.Tensor, pos_of: torch.Tensor, weights: Optional[torch.Tensor], ntok: int, topk: int) -> torch.Tensor:
     """``out[t] = sum_k weights[t,k] * y[pos_of[t*topk+k]]`` (fp32 accumulation)."""
     global launch_count
-    out = torch.empty((ntok, y.shape[1]), dtype=y.dtype, device=y.device)
+    out = empty_of(y, ntok, y.shape[1])
     if y.device.type != "cuda" or y.dtype != torch.bfloat16:
         rows = y[pos_of.long()].float().view(ntok, topk, -1)
         w = weights.float().view(ntok, topk, 1) if weights is not None else 1.0
@@ -145,7 +146,7 @@ def group_gemm(a_sorted: torch.Tensor, b: torch.Tensor, expert_ids: torch.Tensor
             o[blk] = (a_sorted[blk].float() @ (w if kn else w.t())).to(o.dtype)
         return G.apply_activation(o, activation)
     g = _grouped_args(a_sorted, b, kn)
-    c = out if out is not None else torch.empty((rows, N), dtype=a_sorted.dtype, device=a_sorted.device)
+    c = out if out is not None else empty_of(a_sorted, rows, N)
     g.c = c.data_ptr()
     g.m_per_rank = rows
     g.epoch = 1
@@ -172,8 +173,9 @@ def _kn_layout(b: torch.Tensor) -> Optional[Tuple[bool, int, int]]:
     return None
 
 
-def _grouped_args(a: torch.Tensor, b: torch.Tensor, kn: bool) -> "_lib.GemmArgs":
-    """Launch arguments of a grouped GEMM over ``b`` ``[E, N, K]``, or ``[E, K, N]`` when ``kn``."""
+def _grouped_args(a: torch.Tensor, b: torch.Tensor, kn: bool, layout: Optional[Tuple[bool, int, int]] = None) -> "_lib.GemmArgs":
+    """Launch arguments of a grouped GEMM over ``b`` ``[E, N, K]``, or ``[E, K, N]`` when ``kn`` (``layout``: its
+    :func:`_kn_layout`, where the caller has it)."""
     if not kn:
         E, N, K = b.shape
         flat = b.view(E * N, K)
@@ -185,7 +187,7 @@ def _grouped_args(a: torch.Tensor, b: torch.Tensor, kn: bool) -> "_lib.GemmArgs"
         if a.dim() != 2 or b.dim() != 3 or a.shape[1] != b.shape[1] or not a.is_contiguous():
             raise ValueError(f"expected a contiguous a[M, K] and b[E, K, N], got {tuple(a.shape)} and {tuple(b.shape)}")
         E, K, N = b.shape
-        layout = _kn_layout(b)
+        layout = layout or _kn_layout(b)
         if K % 8 or N % 8 or layout is None:
             raise ValueError("K and N must be multiples of 8, and b[E, K, N] must have one of them contiguous on a 16-byte grid")
         g = G._base_args(a, b, 1, 0, _lib.GEMM_PLAIN)
@@ -195,10 +197,14 @@ def _grouped_args(a: torch.Tensor, b: torch.Tensor, kn: bool) -> "_lib.GemmArgs"
     return g
 
 
-def _expert_weights(b: torch.Tensor) -> torch.Tensor:
-    """The caller's ``[E, K, N]`` weights: read in place on every call, so that a change of theirs is seen, and copied for the
-    call only where a TMA load cannot read them."""
-    return b if _kn_layout(b) is not None else b.clone(memory_format=torch.contiguous_format)
+def _expert_weights(b: torch.Tensor) -> Tuple[torch.Tensor, Optional[Tuple[bool, int, int]]]:
+    """The caller's ``[E, K, N]`` weights with their :func:`_kn_layout`: read in place on every call, so that a change of theirs is
+    seen, and copied for the call only where a TMA load cannot read them."""
+    layout = _kn_layout(b)
+    if layout is not None:
+        return b, layout
+    b = b.clone(memory_format=torch.contiguous_format)
+    return b, _kn_layout(b)
 
 
 def staging_flags(rows: int, device) -> torch.Tensor:
@@ -243,7 +249,8 @@ def group_gemm_gather(a: torch.Tensor, row_index: torch.Tensor, b: torch.Tensor,
                       src_rank: int = 0, src_world: int = 1, staging: Optional[torch.Tensor] = None,
                       block_ready: Optional[torch.Tensor] = None, epoch: int = 1, block_rot: Optional[torch.Tensor] = None,
                       c_scatter: Optional[torch.Tensor] = None, c_rows: int = 0,
-                      pairs: Optional["BlockPairs"] = None, kn: bool = False) -> torch.Tensor:
+                      pairs: Optional["BlockPairs"] = None, kn: bool = False,
+                      layout: Optional[Tuple[bool, int, int]] = None) -> torch.Tensor:
     """Grouped GEMM whose A rows are gathered inside the kernel: ``out[r] = a[row_index[r]] @ b[expert_ids[r // 128]].T``
     (rows with ``row_index >= a.shape[0]`` are padding). With ``block_src`` the rows of 128-row
     block ``i`` come from rank ``block_src[i]``'s segment of an all-gather that may still be in flight: the kernel
@@ -257,7 +264,7 @@ def group_gemm_gather(a: torch.Tensor, row_index: torch.Tensor, b: torch.Tensor,
     ``block_rot`` (device int32 scalar): block the schedule starts at. ``c_scatter`` (int32 per sorted row): the
     epilogue stores row ``r`` of the product at row ``c_scatter[r]`` of ``out`` (``[c_rows, N]``), dropping rows whose
     index is not below ``c_rows``. ``pairs`` (:func:`pair_blocks`, with ``staging``): two blocks of an expert per CTA pair.
-    ``kn`` as in :func:`group_gemm`."""
+    ``kn`` as in :func:`group_gemm`, ``layout`` as in :func:`_grouped_args`."""
     rows = row_index.shape[0]
     N, K = b.shape[2 if kn else 1], b.shape[1 if kn else 2]
     if rows % GROUP_BLOCK_M:
@@ -271,11 +278,8 @@ def group_gemm_gather(a: torch.Tensor, row_index: torch.Tensor, b: torch.Tensor,
         live = c_scatter.long() < c_rows
         o[c_scatter.long()[live]] = prod[live]
         return o
-    g = _grouped_args(a, b, kn)
-    if c_scatter is not None:
-        c = out if out is not None else torch.empty((c_rows, N), dtype=a.dtype, device=a.device)
-    else:
-        c = out if out is not None else torch.empty((rows, N), dtype=a.dtype, device=a.device)
+    g = _grouped_args(a, b, kn, layout)
+    c = out if out is not None else empty_of(a, c_rows if c_scatter is not None else rows, N)
     g.c = c.data_ptr()
     g.m_per_rank = rows
     g.epoch = epoch
@@ -401,7 +405,7 @@ def ag_group_gemm_intra_node(a: torch.Tensor, b: torch.Tensor, ctx: MoEAllGather
             m = ids == e
             out[m] = (rows[m] @ b[e].float()).to(a.dtype)
         return out
-    b = _expert_weights(b)
+    b, layout = _expert_weights(b)
     if ctx.world > 1:
         if phase != 2:
             ctx.calls += 1
@@ -421,7 +425,7 @@ def ag_group_gemm_intra_node(a: torch.Tensor, b: torch.Tensor, ctx: MoEAllGather
             src = dict(block_src=ctx.block_barrier_ids, src_flags=ctx.ag_ctx.signal.local, src_epoch=ctx.ag_ctx.epoch,
                        src_rank=ctx.rank, src_world=ctx.world)
             if mode == "fused":
-                return _fused_group_gemm(ctx, buf.local, b, numel, **src)
+                return _fused_group_gemm(ctx, buf.local, b, numel, layout, **src)
             c_sorted = group_gemm_gather(buf.local, ctx.row_index, b, ctx.expert_ids, ctx.num_blocks, kn=True, **src)
             out, _ = gather_rows(c_sorted, ctx.pos_of, 1, c_sorted.shape[0])
             return out
@@ -433,7 +437,7 @@ def ag_group_gemm_intra_node(a: torch.Tensor, b: torch.Tensor, ctx: MoEAllGather
         full = a
     mode = "cp_async" if FUSED_AG_GROUP_GEMM else AG_GROUP_GEMM_MODE
     if mode == "fused":
-        return _fused_group_gemm(ctx, full, b, numel)
+        return _fused_group_gemm(ctx, full, b, numel, layout)
     if mode == "cp_async":
         c_sorted = group_gemm_gather(full, ctx.row_index, b, ctx.expert_ids, ctx.num_blocks, kn=True)
         out, _ = gather_rows(c_sorted, ctx.pos_of, 1, c_sorted.shape[0])
@@ -444,14 +448,14 @@ def ag_group_gemm_intra_node(a: torch.Tensor, b: torch.Tensor, ctx: MoEAllGather
     return out
 
 
-def _fused_group_gemm(ctx: MoEAllGatherGroupGEMMTensorParallelContext, full: torch.Tensor, b: torch.Tensor, numel: int, **src):
+def _fused_group_gemm(ctx: MoEAllGatherGroupGEMMTensorParallelContext, full: torch.Tensor, b: torch.Tensor, numel: int, layout, **src):
     """One launch: the kernel stages the rows block by block itself (all threads for the first wave, then the epilogue
     warps between accumulators), TMA-fed MMAs start at this rank's own blocks, the epilogue stores every row at its
     (token, k) position."""
     ctx.gemm_calls += 1
     return group_gemm_gather(full, ctx.row_index, b, ctx.expert_ids, ctx.num_blocks, staging=ctx.staging,
                              block_ready=ctx.block_ready, epoch=ctx.gemm_calls, block_rot=ctx.block_rot,
-                             c_scatter=ctx.sorted_ids, c_rows=numel, pairs=ctx.pairs, kn=True, **src)
+                             c_scatter=ctx.sorted_ids, c_rows=numel, pairs=ctx.pairs, kn=True, layout=layout, **src)
 
 
 # ---------------------------------------------------------------------------- GroupGEMM + reduce + RS
@@ -523,7 +527,7 @@ def moe_reduce_rs(rank: int, world_size: int, local_world_size: int, a: torch.Te
         part = (y.view(M, ctx.topk, N) * ctx.full_topk_weight.view(M, ctx.topk, 1)).sum(1).to(a.dtype)
         return CO.reduce_scatter_2d_op(part, ctx.rs_ctx)
     if phase != 2:
-        b = _expert_weights(b)
+        b, layout = _expert_weights(b)
         if AG_GROUP_GEMM_MODE == "fused":
             # the sort of the rows by expert happens inside the grouped-GEMM launch (in-launch row staging + TMA-fed MMAs)
             if ctx.staging is None or ctx.staging.shape[1] != a.shape[1] or ctx.staging.dtype != a.dtype:
@@ -532,7 +536,7 @@ def moe_reduce_rs(rank: int, world_size: int, local_world_size: int, a: torch.Te
                 ctx.gemm_calls = 0
             ctx.gemm_calls += 1
             y = group_gemm_gather(a, ctx.sorted_ids, b, ctx.expert_ids, ctx.num_blocks, staging=ctx.staging,
-                                  block_ready=ctx.block_ready, epoch=ctx.gemm_calls, pairs=ctx.pairs, kn=True)
+                                  block_ready=ctx.block_ready, epoch=ctx.gemm_calls, pairs=ctx.pairs, kn=True, layout=layout)
             ctx._partial = (y, ctx.pos_of)
         else:
             a_sorted, pos_of = gather_rows(a, ctx.sorted_ids, 1, numel, want_inverse=True)

@@ -17,16 +17,18 @@ _CODES = {0: "ok", 1: "flag wait timed out", 2: "mbarrier wait timed out", 3: "b
 _KERNELS = {1: "gemm_sm100", 2: "collectives", 3: "a2a", 4: "flash_decode", 5: "primitives", 6: "moe", 7: "moe_ep", 8: "bounds check"}
 
 
-_TIMEOUT_CACHE = [None, 0]
+_TIMEOUT_KEY = os.environ.encodekey("TDIST_WAIT_TIMEOUT_MS")
+_TIMEOUT_CACHE = [_CODES, 0]   # setting as the environment keeps it (any other object: not looked up yet), nanoseconds
 
 
 def default_timeout_ns() -> int:
     """Limit of every bounded device wait, from TDIST_WAIT_TIMEOUT_MS (default 4 s); the parsed value is
-    cached per distinct setting because this sits on every launch path."""
-    raw = os.environ.get("TDIST_WAIT_TIMEOUT_MS", "4000")
-    if _TIMEOUT_CACHE[0] != raw:
+    cached per distinct setting because this sits on every launch path. The setting is looked up as ``os.environ`` keeps it:
+    its ``get`` encodes the name and decodes the value on every call (0.5 us of a 10 us call, 0.1 here)."""
+    raw = os.environ._data.get(_TIMEOUT_KEY)
+    if raw != _TIMEOUT_CACHE[0]:
+        _TIMEOUT_CACHE[1] = int(float(os.environ.get("TDIST_WAIT_TIMEOUT_MS", "4000")) * 1e6)
         _TIMEOUT_CACHE[0] = raw
-        _TIMEOUT_CACHE[1] = int(float(raw) * 1e6)
     return _TIMEOUT_CACHE[1]
 
 

@@ -292,6 +292,14 @@ def get_numa_node(gpu_index: int = 0) -> int:
         return NvidiaSmiUtil.get_gpu_numa_node(gpu_index)
 
 
+def empty_of(t: torch.Tensor, *shape: int) -> torch.Tensor:
+    """Uninitialised ``shape`` of ``t``'s type and device: ``torch.empty`` without its keyword arguments (2.4 us of a 10 us call,
+    1.8 from the tensor itself)."""
+    if type(t) is torch.Tensor:
+        return t.new_empty(shape)
+    return torch.empty(shape, dtype=t.dtype, device=t.device)
+
+
 def plain_cuda(*tensors: torch.Tensor) -> bool:
     """True when a raw-pointer kernel may stand in for torch operations on ``tensors``: dense CUDA tensors of the current
     device, 16-byte aligned, whose operations nothing else has to see (no autograd or forward-mode graph, no vmap / functorch
