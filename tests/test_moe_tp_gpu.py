@@ -248,6 +248,25 @@ def test_grouped_gemm_tile_width_follows_the_live_blocks(cuda_device, blocks, mo
     assert (out[128 * live:] == 7.0).all()
 
 
+@pytest.mark.parametrize("blocks,E,K,N,width", [(91, 16, 512, 384, 128), (75, 8, 1032, 392, 192), (170, 8, 1032, 392, 256), (300, 4, 64, 72, 128)])
+def test_grouped_gemm_tile_width_beyond_one_round(cuda_device, blocks, E, K, N, width):
+    """Narrower tiles where whole ones leave the last round or the last tile of a row mostly empty, for both layouts of B."""
+    from triton_distributed_b200 import _lib
+    torch.manual_seed(blocks + N)
+    a = torch.randn(blocks * 128, K, device=cuda_device).to(torch.bfloat16)
+    b = (torch.randn(E, K, N, device=cuda_device) * K ** -0.5).to(torch.bfloat16)
+    t = b.transpose(1, 2).contiguous()
+    experts = torch.sort(torch.randint(0, E, (blocks,), dtype=torch.int32, device=cuda_device)).values.to(torch.int32)
+    g = MT._grouped_args(a, t, False)
+    g.m_per_rank, g.expert_ids = blocks * 128, experts.data_ptr()
+    assert _lib.lib().tdist_gemm_tile_width(g) == width
+    out, nm, act = MT.group_gemm(a, t, experts), MT.group_gemm(a, b, experts, kn=True), MT.group_gemm(a, t, experts, activation="relu")
+    check_status()
+    ref = torch.bmm(a.view(blocks, 128, K).double(), b[experts.long()].double()).view(-1, N)
+    torch.testing.assert_close(out.double(), ref, atol=2e-5, rtol=2.0 ** -8)
+    assert torch.equal(nm, out) and torch.equal(act, out.relu())
+
+
 @pytest.mark.parametrize("blocks,E,K,N", [(1, 1, 8, 8), (3, 2, 72, 136), (5, 3, 264, 520), (20, 4, 1000, 264), (9, 4, 4104, 1032)])
 def test_grouped_gemm_on_n_major_weights_gives_the_same_bits(cuda_device, blocks, E, K, N):
     """[E, K, N] read in place against its transposed copy: the same products summed in the same order, for tiles of 64 to 256

@@ -1578,6 +1578,19 @@ static double plain_time(const TdistGemmArgs* a, const GridPlan& g) {
     return (sm_s > hbm_s ? sm_s : hbm_s) + 5e-6;
 }
 
+// Expected time of a grouped product of `blocks` blocks on single CTAs with tiles of `bn` columns: rounds of tiles whose K
+// blocks take what their loads need at the 120 GB/s an SM gets from L2 (the 400 ns above at 256 columns) and whose epilogue
+// (0.4 us per 64 columns) may outlast them, or the weights' and the rows' trip through HBM.
+static double grouped_time(const TdistGemmArgs* a, int blocks, int bn, int sms) {
+    const int k_blocks = (a->k + BK - 1) / BK;
+    const long long tiles = static_cast<long long>(blocks) * ((a->n + bn - 1) / bn);
+    const double main_s = k_blocks * (A_BYTES + bn * BK * 2) / 120e9, epilogue_s = bn / 64 * 0.4e-6;
+    const double sm_s = static_cast<double>((tiles + sms - 1) / sms) * ((main_s > epilogue_s ? main_s : epilogue_s) + 0.3e-6);
+    const double experts = a->num_experts < blocks ? a->num_experts : blocks;
+    const double hbm_s = 2.0 * (experts * a->n * a->k + static_cast<double>(blocks) * BM * (a->k + a->n)) / 6.3e12;
+    return sm_s > hbm_s ? sm_s : hbm_s;
+}
+
 static GridPlan plan_grid(const TdistGemmArgs* a) {
     GridPlan g;
     g.few_rows = false;
@@ -1590,12 +1603,26 @@ static GridPlan plan_grid(const TdistGemmArgs* a) {
         // Grouped GEMM of a decode step: its blocks are a few rows each, so it is bound by the loads of B, and a CTA's rate by
         // what an SM takes from L2. While 256-column tiles leave SMs idle, narrower ones that still run as one round bring
         // more of them in (both GEMMs of the experts, 16 tokens, top 2 of 8, 4096 x 2048: 71 -> 67 us; 64 tokens, top 4 of
-        // 16, 4096 x 512: 58 -> 51 us). Beyond one round they lose: the A rows are loaded again for every tile (128 tokens,
-        // top 8 of 32, 7168 x 2048 with 192 columns: 350 us against 330).
+        // 16, 4096 x 512: 58 -> 51 us).
         const int blocks = a->max_m_blocks > 0 && a->max_m_blocks < seg_m_tiles ? a->max_m_blocks : seg_m_tiles;
         const long long sms = tdist_host::sm_count();
         for (int bn = BN - 64; bn >= 64; bn -= 64)
             if (static_cast<long long>(blocks) * ((a->n + bn - 1) / bn) <= sms) g.bn = bn;
+        // Beyond one round the A rows are loaded again for every tile, which costs a product that is bound by its weights (128
+        // tokens, top 8 of 32, 7168 x 2048 with 192 columns: 350 us against 330) and pays where 256 columns leave the last round
+        // or the last tile of a row mostly empty (1194 tokens, top 8 of 16, 6720 -> 384: 93 us with 256
+        // columns, 78 with 128; the whole expert-parallel block 267 and 257).
+        if (g.bn == BN) {
+            const double whole = grouped_time(a, blocks, BN, static_cast<int>(sms));
+            double best = 0.92 * whole;
+            for (int bn = BN - 64; bn >= 64; bn -= 64) {
+                const double t = grouped_time(a, blocks, bn, static_cast<int>(sms));
+                if (t < best) {
+                    best = t;
+                    g.bn = bn;
+                }
+            }
+        }
         n_tiles = (a->n + g.bn - 1) / g.bn;
     }
     g.num_tiles = seg_m_tiles * (g.wide ? (n_tiles + 1) / 2 : n_tiles) * a->world;
