@@ -307,47 +307,26 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_dispatch_kernel(const __gr
         // ---------------------------------------------------------------- rows: load once, store to every owner
         const int row_bytes_out = p.quant ? p.hidden : p.hidden * 2;
         const int scale_cols = p.hidden / 128;
-        // Row and owner of the item's pairs: lane k looks up pair k (those after the 32nd in further steps), all at once, and the
-        // next item's values are on their way while this one's are stored. (Every pair looked up before its stores, the next
-        // item loaded after them: 1194 tokens x 6720, top 8 of 16, 47 us, 43 here.)
-        const auto look_up = [&](int t, int k0, int& row, int& owner) {
-            row = -1;
-            owner = 0;
-            if (k0 + lane >= p.topk) return;
-            const int i = t * p.topk + k0 + lane;
-            const int e = p.topk_ids[i];
-            if (!expert_in_range(e, E)) return;
-            if (in_place) {
-                row = row_s[i];
-            } else {
-                const int slot = p.slot_in[i];
-                row = slot >= 0 ? base[e] + slot - cum[e] : -1;
-                if (row >= row_limit) row = -1;
-            }
-            owner = e / p.epr;
-        };
-        int row_next = -1, owner_next = 0;
-        if (gw < p.ntok * segs) look_up(gw / segs, 0, row_next, owner_next);
         for (int item = gw; item < p.ntok * segs; item += nw) {
             const int t = item / segs, seg = item - t * segs;
-            uint4 now[kEpSegLoads];
-#pragma unroll
-            for (int u = 0; u < kEpSegLoads; ++u) now[u] = raw[u];
-            int row_k = row_next, owner_k = owner_next;
-            if (item + nw < p.ntok * segs) {
-                const int tn = (item + nw) / segs;
-                load_segment(p.x + static_cast<size_t>(tn) * p.hidden * 2, p.hidden, item + nw - tn * segs, lane, p.quant != 0, raw);
-                look_up(tn, 0, row_next, owner_next);
-            }
+            if (item != gw) load_segment(p.x + static_cast<size_t>(t) * p.hidden * 2, p.hidden, seg, lane, p.quant != 0, raw);
             QuantSeg qs;
-            if (p.quant) quantise_segment(now, qs);
+            if (p.quant) quantise_segment(raw, qs);
             const int half = lane >> 4, sub = lane & 15;
             const int b0 = seg * kEpSegValues * 2;
             const int b1 = min(p.hidden * 2, b0 + kEpSegValues * 2);
             for (int k = 0; k < p.topk; ++k) {
-                if (k > 0 && (k & 31) == 0) look_up(t, k, row_k, owner_k);
-                const int r = __shfl_sync(0xffffffffu, row_k, k & 31), d = __shfl_sync(0xffffffffu, owner_k, k & 31);
+                const int i = t * p.topk + k;
+                int r;
+                if (in_place) {
+                    r = row_s[i];
+                } else {
+                    const int e = p.topk_ids[i];
+                    r = expert_in_range(e, E) && p.slot_in[i] >= 0 ? base[e] + p.slot_in[i] - cum[e] : -1;
+                    if (r >= row_limit) r = -1;
+                }
                 if (r < 0) continue;
+                const int d = p.topk_ids[i] / p.epr;
                 char* dst = p.recv_peer[d] + static_cast<size_t>(r) * row_bytes_out;
                 if (p.quant) {
                     float* dsc = p.scale_peer[d] + static_cast<size_t>(r) * scale_cols;
@@ -363,7 +342,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_dispatch_kernel(const __gr
 #pragma unroll
                     for (int u = 0; u < kEpSegLoads; ++u) {
                         const int off = b0 + u * 512 + lane * 16;
-                        if (off < b1) st_v4(dst + off, now[u]);
+                        if (off < b1) st_v4(dst + off, raw[u]);
                     }
                 }
             }
