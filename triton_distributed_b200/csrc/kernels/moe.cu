@@ -261,21 +261,22 @@ __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], uint32_t a0, uint3
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// NT: groups of 8 experts per pass over the tokens' rows
-template <int NT>
+// NT: groups of 8 experts per pass over the tokens' rows; SPLIT: a cluster of `split` CTAs per 16 tokens
+template <int NT, bool SPLIT>
 __global__ void __launch_bounds__(kGateThreads, 1) moe_gate_topk_kernel(const __nv_bfloat16* x, const __nv_bfloat16* gate, int ntok, int hidden, int E,
-                                                                        int topk, int renorm, int parts, int* ids, float* w, float* logits) {
+                                                                        int topk, int renorm, int split, int* ids, float* w, float* logits) {
+    const int parts = SPLIT ? split : 1;
     extern __shared__ float gate_sm[];
     constexpr int COLS = NT * 8;
     float* part = gate_sm;                                   // [warps][16 tokens][COLS]
     float* row_s = gate_sm + kGateWarps * kGateTok * COLS;   // [parts][16 / parts tokens][E]: this CTA's tokens, a row per part
     const int tid = static_cast<int>(threadIdx.x), warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, tig = lane & 3;                 // row / column group of the MMA fragments
-    const int part_id = parts > 1 ? static_cast<int>(cluster_ctarank()) : 0;
+    const int part_id = SPLIT ? static_cast<int>(cluster_ctarank()) : 0;
     const int t0 = static_cast<int>(blockIdx.x) / parts * kGateTok;
     const int own = kGateTok / parts;   // tokens a CTA selects for
     const int steps = hidden / 32;
-    if (parts > 1) cluster_arrive();    // its counterpart stands before the first store into another CTA
+    if (SPLIT) cluster_arrive();    // its counterpart stands before the first store into another CTA
     pdl_wait_and_release();
     // rows past the end repeat the last one; their results are not used
     const __nv_bfloat16* xa = x + static_cast<size_t>(min(t0 + g, ntok - 1)) * hidden + tig * 8;
@@ -311,14 +312,14 @@ __global__ void __launch_bounds__(kGateThreads, 1) moe_gate_topk_kernel(const __
             *reinterpret_cast<float2*>(p + 8 * COLS) = make_float2(acc[n][2], acc[n][3]);
         }
         __syncthreads();
-        if (parts > 1 && e0 == 0) cluster_wait();   // every CTA of the cluster runs
+        if (SPLIT && e0 == 0) cluster_wait();   // every CTA of the cluster runs
         for (int i = tid; i < kGateTok * COLS; i += kGateThreads) {
             const int t = i / COLS, e = e0 + i % COLS;
             float sum = 0.f;
 #pragma unroll
             for (int k = 0; k < kGateWarps; ++k) sum += part[k * kGateTok * COLS + i];
             if (e >= E) continue;
-            if (parts > 1) {
+            if (SPLIT) {
                 st_shared_cluster_f32(mapa_u32(smem_u32(row_s + (part_id * own + t % own) * E + e), static_cast<uint32_t>(t / own)), sum);
             } else {
                 row_s[t * E + e] = sum;
@@ -327,7 +328,7 @@ __global__ void __launch_bounds__(kGateThreads, 1) moe_gate_topk_kernel(const __
         }
         __syncthreads();
     }
-    if (parts > 1) {
+    if (SPLIT) {
         cluster_arrive();
         cluster_wait();
         for (int i = tid; i < own * E; i += kGateThreads) {
@@ -507,11 +508,12 @@ extern "C" int tdist_moe_gate_topk(const void* x, const void* gate, int ntok, in
     attr[1].val.clusterDim.y = 1;
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 2;
+    cfg.numAttrs = parts > 1 ? 2 : 1;
 #define TDIST_GATE_CASE(NT)                                                                                                     \
     {                                                                                                                           \
-        if (int rc = ensure_smem(moe_gate_topk_kernel<NT>, smem)) return rc;                                                    \
-        TDIST_CUDA_OK(cudaLaunchKernelEx(&cfg, moe_gate_topk_kernel<NT>, static_cast<const __nv_bfloat16*>(x),                  \
+        const auto kernel = parts > 1 ? moe_gate_topk_kernel<NT, true> : moe_gate_topk_kernel<NT, false>;                       \
+        if (int rc = ensure_smem(kernel, smem)) return rc;                                                                      \
+        TDIST_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, static_cast<const __nv_bfloat16*>(x),                                    \
                                          static_cast<const __nv_bfloat16*>(gate), ntok, hidden, num_experts, topk, renormalize, parts, \
                                          static_cast<int*>(ids), static_cast<float*>(weights), static_cast<float*>(logits)));   \
     }
