@@ -104,8 +104,9 @@ def _batch_splits(pairs: int, max_kv: int, head_dim: int, sms: int, one_wave: in
     does not see them); more, shorter CTAs even both out until their fixed cost takes over. Two estimates: all sequences
     full (whole waves), and lengths spread evenly over (0, max_kv] (their sum over the machine, plus the last one to
     start). The least sum decides among the splits that cost full sequences no more than 5 % against one wave; at most
-    eight, which merge within their cluster. Measured at one wave / as chosen: 32 ragged sequences x 8 kv heads to 8192
-    keys 136 / 116 us (full ones 169 / 178), 48 full ones of 4096 171 / 146 us, 20 full ones of 6000 109 / 93 us.
+    eight, which merge within their cluster. Measured at one wave / as chosen (single calls after a flush of L2): 32 ragged
+    sequences x 8 kv heads to 8192 keys 137 / 111 us (full ones 191 / 187), 20 of 6000 91 / 62 us (full ones 107 / 105), 48 full
+    ones of 2048 102 / 96 us.
 
     ``wide``: the page table is wider than the cache has keys for, so the sequences are known not to fill it, and the short ones
     pay the fixed cost of every round of CTAs: then at most one round more than one wave takes (32 sequences in a table of
