@@ -309,6 +309,33 @@ def test_gate_topk_parts_of_the_hidden_dimension(cuda_device, T, hidden, E, k):
     torch.testing.assert_close(w, w_t, rtol=1e-6, atol=0)
 
 
+@pytest.mark.parametrize("T,hidden,E,k", [(1, 256, 64, 1), (37, 1032, 64, 33), (5, 256, 64, 64), (513, 128, 64, 1), (1024, 256, 8, 8), (700, 4096, 16, 5), (1100, 4096, 16, 8)])
+@pytest.mark.parametrize("compact", [False, True])
+def test_dispatch_rows_of_every_pair(cuda_device, T, hidden, E, k, compact):
+    """Runs of pairs shorter and longer than the ids a lane loads at a time, a ragged last segment, more items than warps, and routing
+    both in place and by a launch of its own (1100 x 8 pairs, recorded by all CTAs): every pair's row is its token's, bit by
+    bit; dropped pairs (id -1) have none."""
+    from triton_distributed_b200._lib import TdistError
+    from triton_distributed_b200.ops import moe_ep as EP
+    torch.manual_seed(T + k)
+    x = torch.randn(T, hidden, device=cuda_device).bfloat16()
+    ids = torch.randint(0, E, (T, k), dtype=torch.int32, device=cuda_device)
+    ctx = EP.create_ep_context(T, hidden, k, E, 0, 1, quant=False, compact=compact, heap=LocalWorld(1, cuda_device).heap(0), device=cuda_device)
+    for dropped in (False, True):
+        if dropped:
+            ids[T // 2, k - 1] = -1
+        rows, _, _, num = EP.ep_dispatch(ctx, x, ids)
+        if dropped:
+            with pytest.raises(TdistError, match="bad argument"):
+                check_status()
+        else:
+            check_status()
+        at = ctx.pair_row[: T * k].long()
+        live = ids.reshape(-1) >= 0
+        assert (at[~live] == -1).all() and int(num) == int(live.sum()) == at[live].unique().numel()
+        assert torch.equal(rows[at[live]], x.repeat_interleave(k, 0)[live])
+
+
 @pytest.mark.parametrize("form", ["bf16", "strided", "misaligned", "short", "cpu"])
 def test_gate_topk_writes_logits_of_any_form_or_refuses_them(cuda_device, form):
     """Only a dense fp32 [T, E] buffer may be handed to the kernel as a pointer; the others are copied into, converted and
