@@ -426,3 +426,28 @@ def test_plan_queries_answer_for_empty_problems(m, n, k):
             f"g.world, g.m_per_rank, g.n, g.k, g.cta_pair, g.c = 1, {m}, {n}, {k}, -1, 16; out = (C.c_int * 4)(); lib = _lib.lib(); "
             "assert lib.tdist_gemm_plan(g, out) == 0 and out[3] >= 1 and lib.tdist_gemm_grid(g) == out[3] and lib.tdist_gemm_tile_width(g) == 256")
     subprocess.run([sys.executable, "-c", code], check=True)
+
+
+def test_wait_timeout_follows_any_mapping_in_the_place_of_os_environ(monkeypatch):
+    import os
+
+    from triton_distributed_b200.runtime import default_timeout_ns
+    monkeypatch.delenv("TDIST_WAIT_TIMEOUT_MS", raising=False)
+    assert default_timeout_ns() == 4_000_000_000
+    monkeypatch.setenv("TDIST_WAIT_TIMEOUT_MS", "250")
+    assert default_timeout_ns() == 250_000_000
+    for environ in (os.environ.copy(), {"TDIST_WAIT_TIMEOUT_MS": "250"}):
+        with monkeypatch.context() as m:
+            m.setattr(os, "environ", environ)
+            assert default_timeout_ns() == 250_000_000
+            environ["TDIST_WAIT_TIMEOUT_MS"] = "1.5"
+            assert default_timeout_ns() == 1_500_000
+            del environ["TDIST_WAIT_TIMEOUT_MS"]
+            assert default_timeout_ns() == 4_000_000_000
+        assert default_timeout_ns() == 250_000_000
+    monkeypatch.setenv("TDIST_WAIT_TIMEOUT_MS", "soon")
+    for _ in range(2):                     # refused on every call, not on the first one alone
+        with pytest.raises(ValueError):
+            default_timeout_ns()
+    monkeypatch.setenv("TDIST_WAIT_TIMEOUT_MS", "4000")
+    assert default_timeout_ns() == 4_000_000_000

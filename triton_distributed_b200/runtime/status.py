@@ -17,17 +17,21 @@ _CODES = {0: "ok", 1: "flag wait timed out", 2: "mbarrier wait timed out", 3: "b
 _KERNELS = {1: "gemm_sm100", 2: "collectives", 3: "a2a", 4: "flash_decode", 5: "primitives", 6: "moe", 7: "moe_ep", 8: "bounds check"}
 
 
-_TIMEOUT_KEY = os.environ.encodekey("TDIST_WAIT_TIMEOUT_MS")
+_TIMEOUT_NAME = "TDIST_WAIT_TIMEOUT_MS"
+# CPython's os.environ keeps its settings, encoded, in a dict of its own; another mapping may stand in its place, now or later
+_ENVIRON = type(os.environ) if hasattr(os.environ, "_data") and hasattr(os.environ, "encodekey") else None
+_TIMEOUT_KEY = os.environ.encodekey(_TIMEOUT_NAME) if _ENVIRON is not None else None
 _TIMEOUT_CACHE = [_CODES, 0]   # setting as the environment keeps it (any other object: not looked up yet), nanoseconds
 
 
 def default_timeout_ns() -> int:
     """Limit of every bounded device wait, from TDIST_WAIT_TIMEOUT_MS (default 4 s); the parsed value is
-    cached per distinct setting because this sits on every launch path. The setting is looked up as ``os.environ`` keeps it:
-    its ``get`` encodes the name and decodes the value on every call (0.5 us of a 10 us call, 0.1 here)."""
-    raw = os.environ._data.get(_TIMEOUT_KEY)
+    cached per distinct setting because this sits on every launch path. The setting is looked up as ``os.environ`` keeps it
+    (its ``get`` encodes the name and decodes the value on every call: 0.5 us of a 10 us call, 0.1 here), and by ``get``
+    where ``os.environ`` is some other mapping."""
+    raw = os.environ._data.get(_TIMEOUT_KEY) if type(os.environ) is _ENVIRON else os.environ.get(_TIMEOUT_NAME)
     if raw != _TIMEOUT_CACHE[0]:
-        _TIMEOUT_CACHE[1] = int(float(os.environ.get("TDIST_WAIT_TIMEOUT_MS", "4000")) * 1e6)
+        _TIMEOUT_CACHE[1] = int(float(os.environ.get(_TIMEOUT_NAME, "4000")) * 1e6)
         _TIMEOUT_CACHE[0] = raw
     return _TIMEOUT_CACHE[1]
 
