@@ -309,6 +309,26 @@ def test_gate_topk_parts_of_the_hidden_dimension(cuda_device, T, hidden, E, k):
     torch.testing.assert_close(w, w_t, rtol=1e-6, atol=0)
 
 
+@pytest.mark.parametrize("hidden,E,k", [(64, 3, 1), (544, 8, 2), (992, 40, 4), (1024, 16, 4), (2080, 60, 6), (4096, 8, 2), (7168, 64, 8),
+                                        (8192, 64, 8), (7168, 130, 8), (12288, 64, 8), (2048, 520, 6), (512, 1024, 32)])
+def test_gate_topk_of_a_token_is_the_same_in_any_batch(cuda_device, hidden, E, k):
+    """Every form of the launch, at both sides of the token counts and sizes from which on there is another: bit by bit the
+    logits, experts and weights of the largest batch."""
+    torch.manual_seed(hidden + E)
+    x = torch.randn(1200, hidden, device=cuda_device).bfloat16()
+    gate = (torch.randn(E, hidden, device=cuda_device) * hidden ** -0.5).bfloat16()
+    want = torch.empty(1200, E, device=cuda_device)
+    ids, w = MU.gate_topk(x, gate, k, renormalize=True, logits=want)
+    exact, spread = x.double() @ gate.double().t(), x.double().abs() @ gate.double().abs().t()
+    # additions of a chain, of the chains, and inside an MMA, each off by at most 2^-23 of the sum of the magnitudes
+    assert ((want.double() - exact).abs() <= (hidden / 512 + 18) * 2.0 ** -23 * spread).all()
+    for T in (1, 17, 240, 241, 528, 529, 1184, 1185):
+        logits = torch.empty(T, E, device=cuda_device)
+        ids_t, w_t = MU.gate_topk(x[:T], gate, k, renormalize=True, logits=logits)
+        assert torch.equal(logits, want[:T]), T
+        assert torch.equal(ids_t, ids[:T]) and torch.equal(w_t, w[:T]), T
+
+
 @pytest.mark.parametrize("T,hidden,E,k", [(1, 256, 64, 1), (37, 1032, 64, 33), (5, 256, 64, 64), (513, 128, 64, 1), (1024, 256, 8, 8), (700, 4096, 16, 5), (1100, 4096, 16, 8)])
 @pytest.mark.parametrize("compact", [False, True])
 def test_dispatch_rows_of_every_pair(cuda_device, T, hidden, E, k, compact):

@@ -242,15 +242,22 @@ __global__ void moe_topk_softmax_kernel(const float* logits, int ntok, int E, in
 
 // ---------------------------------------------------------------------------- gate: logits, softmax and top-k in one launch
 // logits[t, e] = x[t, :] . gate[e, :] (bf16 in, fp32 sums), then the selection above. A decode step has few tokens and
-// few experts, so the product is short of parallelism, not of arithmetic: a CTA takes 16 tokens and ALL experts, its
-// 16 warps split the hidden dimension 32 values at a time, and up to eight CTAs of a cluster share it where the tokens leave
-// SMs idle (each adds its part of every token up, sends it to the CTA that selects for the token, which adds the parts:
-// 4 tokens x 4288, 64 experts: 12 us on one CTA, 7 on eight; the whole expert-parallel block 87 and 82) (what a cuBLAS SGEMM of the fp32 copies does serially; 128 x
-// 7168 x 32 experts: 53 us as two copies, SGEMM, reduction and selection, 12 us here). mma.sync m16n8k16: the products of bf16 values are exact in
-// fp32, the tensor core sums 32 of them at a time (its accumulator truncates, so longer chains there would lose bits
-// against an fp32 FMA loop), the rest is added in fp32: 1/16 of the hidden dimension per warp, then 16 partial sums. A tcgen05
-// tile (M 128) would leave all but 16 rows of this split idle. Any order of k will do as long as x and gate agree, so a
-// thread takes 8 consecutive values of its row per step: one 16-byte load feeds two MMAs.
+// few experts, so the product is short of parallelism, not of arithmetic: 16 tokens are a tile, and its hidden dimension, 32 values
+// at a time, is dealt over 16 chains of sums (what a cuBLAS SGEMM of the fp32 copies does serially; 128 x
+// 7168 x 32 experts: 53 us as two copies, SGEMM, reduction and selection, 12 us on one CTA per tile). mma.sync m16n8k16: the
+// products of bf16 values are exact in fp32, the tensor core sums 32 of them at a time (its accumulator truncates, so longer
+// chains there would lose bits against an fp32 FMA loop), the rest is added in fp32: a chain's steps in order, then the 16 chains
+// in order. A tcgen05 tile (M 128) would leave all but 16 rows of this split idle. Any order of k will do as long as x and gate
+// agree, so a thread takes 8 consecutive values of its row per step: one 16-byte load feeds two MMAs.
+//
+// That order of the sums is the same in all forms below, which the number of tokens chooses between: a token's logits, and with
+// them the choice between near ties, do not depend on how many others are in the call. The forms, us per call at 16 tokens x 4096,
+// 8 experts / 128 x 7168, 32 / 300 x 7168, 64 / 1200 x 6720, 64:
+//   a CTA per tile, a chain per warp                                        4.4 / 10.2 / 15.5 / 15.3
+//   a cluster of up to eight CTAs per tile, which share the experts           - /  7.6 /  9.0 / 21.6
+//   a cluster of eight CTAs per tile, two chains each                       2.9 /  5.4 / 14.3 / 36
+// (Up to eight parts of the hidden dimension, each a sum of its own, took 2.9 / 5.7 / 9.5 / 15.3: there the order of the sums followed the
+// number of parts, and that the number of tokens. Eight such sums whatever the number of CTAs: 29 us for the last of these.)
 constexpr int kGateTok = 16, kGateThreads = 512, kGateWarps = kGateThreads / 32;
 
 constexpr int kGateMaxParts = 8;
@@ -261,15 +268,21 @@ __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], uint32_t a0, uint3
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// NT: groups of 8 experts per pass over the tokens' rows; SPLIT: a cluster of `split` CTAs per 16 tokens
+// Rows past the end repeat the last one; their results are not used.
+__device__ __forceinline__ const __nv_bfloat16* gate_row(const __nv_bfloat16* m, int row, int rows, int hidden, int tig) {
+    return m + static_cast<size_t>(min(row, rows - 1)) * hidden + tig * 8;
+}
+
+// NT: groups of 8 experts per pass over the tokens' rows; SPLIT: a cluster of `split` CTAs per tile, which share the experts
 template <int NT, bool SPLIT>
 __global__ void __launch_bounds__(kGateThreads, 1) moe_gate_topk_kernel(const __nv_bfloat16* x, const __nv_bfloat16* gate, int ntok, int hidden, int E,
                                                                         int topk, int renorm, int split, int* ids, float* w, float* logits) {
     const int parts = SPLIT ? split : 1;
     extern __shared__ float gate_sm[];
     constexpr int COLS = NT * 8;
+    constexpr int AHEAD = NT == 1 ? 8 : (NT == 2 ? 4 : (NT == 4 ? 2 : 1));   // steps whose loads are in flight
     float* part = gate_sm;                                   // [warps][16 tokens][COLS]
-    float* row_s = gate_sm + kGateWarps * kGateTok * COLS;   // [parts][16 / parts tokens][E]: this CTA's tokens, a row per part
+    float* row_s = gate_sm + kGateWarps * kGateTok * COLS;   // [16 / parts tokens][E]: the tokens this CTA selects for
     const int tid = static_cast<int>(threadIdx.x), warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, tig = lane & 3;                 // row / column group of the MMA fragments
     const int part_id = SPLIT ? static_cast<int>(cluster_ctarank()) : 0;
@@ -278,31 +291,40 @@ __global__ void __launch_bounds__(kGateThreads, 1) moe_gate_topk_kernel(const __
     const int steps = hidden / 32;
     if (SPLIT) cluster_arrive();    // its counterpart stands before the first store into another CTA
     pdl_wait_and_release();
-    // rows past the end repeat the last one; their results are not used
-    const __nv_bfloat16* xa = x + static_cast<size_t>(min(t0 + g, ntok - 1)) * hidden + tig * 8;
-    const __nv_bfloat16* xb = x + static_cast<size_t>(min(t0 + g + 8, ntok - 1)) * hidden + tig * 8;
-    for (int e0 = 0; e0 < E; e0 += COLS) {
+    const __nv_bfloat16* xa = gate_row(x, t0 + g, ntok, hidden, tig);
+    const __nv_bfloat16* xb = gate_row(x, t0 + g + 8, ntok, hidden, tig);
+    bool apart = SPLIT;   // the other CTAs of the cluster may not run yet
+    for (int e0 = part_id * COLS; e0 < E; e0 += parts * COLS) {
         const __nv_bfloat16* ge[NT];
         float acc[NT][4];
 #pragma unroll
         for (int n = 0; n < NT; ++n) {
-            ge[n] = gate + static_cast<size_t>(min(e0 + n * 8 + g, E - 1)) * hidden + tig * 8;
+            ge[n] = gate_row(gate, e0 + n * 8 + g, E, hidden, tig);
             acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
         }
-#pragma unroll(NT == 8 ? 1 : 2)
-        for (int s = part_id * kGateWarps + warp; s < steps; s += parts * kGateWarps) {
-            const uint4 a = ld_v4(xa + s * 32);
-            const uint4 c = ld_v4(xb + s * 32);
-            uint4 b[NT];
+#pragma unroll 1
+        for (int s0 = warp; s0 < steps; s0 += AHEAD * kGateWarps) {
+            uint4 a[AHEAD], c[AHEAD], b[AHEAD][NT];
 #pragma unroll
-            for (int n = 0; n < NT; ++n) b[n] = ld_v4(ge[n] + s * 32);
+            for (int u = 0; u < AHEAD; ++u) {
+                const int s = s0 + u * kGateWarps;
+                if (s >= steps) break;
+                a[u] = ld_v4(xa + s * 32);
+                c[u] = ld_v4(xb + s * 32);
 #pragma unroll
-            for (int n = 0; n < NT; ++n) {
-                float d[4] = {0.f, 0.f, 0.f, 0.f};
-                mma_bf16_16816(d, a.x, c.x, a.y, c.y, b[n].x, b[n].y);
-                mma_bf16_16816(d, a.z, c.z, a.w, c.w, b[n].z, b[n].w);
+                for (int n = 0; n < NT; ++n) b[u][n] = ld_v4(ge[n] + s * 32);
+            }
 #pragma unroll
-                for (int i = 0; i < 4; ++i) acc[n][i] += d[i];
+            for (int u = 0; u < AHEAD; ++u) {
+                if (s0 + u * kGateWarps >= steps) break;
+#pragma unroll
+                for (int n = 0; n < NT; ++n) {
+                    float d[4] = {0.f, 0.f, 0.f, 0.f};
+                    mma_bf16_16816(d, a[u].x, c[u].x, a[u].y, c[u].y, b[u][n].x, b[u][n].y);
+                    mma_bf16_16816(d, a[u].z, c[u].z, a[u].w, c[u].w, b[u][n].z, b[u][n].w);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) acc[n][i] += d[i];
+                }
             }
         }
 #pragma unroll
@@ -312,7 +334,8 @@ __global__ void __launch_bounds__(kGateThreads, 1) moe_gate_topk_kernel(const __
             *reinterpret_cast<float2*>(p + 8 * COLS) = make_float2(acc[n][2], acc[n][3]);
         }
         __syncthreads();
-        if (SPLIT && e0 == 0) cluster_wait();   // every CTA of the cluster runs
+        if (apart) cluster_wait();
+        apart = false;
         for (int i = tid; i < kGateTok * COLS; i += kGateThreads) {
             const int t = i / COLS, e = e0 + i % COLS;
             float sum = 0.f;
@@ -320,29 +343,109 @@ __global__ void __launch_bounds__(kGateThreads, 1) moe_gate_topk_kernel(const __
             for (int k = 0; k < kGateWarps; ++k) sum += part[k * kGateTok * COLS + i];
             if (e >= E) continue;
             if (SPLIT) {
-                st_shared_cluster_f32(mapa_u32(smem_u32(row_s + (part_id * own + t % own) * E + e), static_cast<uint32_t>(t / own)), sum);
+                st_shared_cluster_f32(mapa_u32(smem_u32(row_s + (t % own) * E + e), static_cast<uint32_t>(t / own)), sum);
             } else {
                 row_s[t * E + e] = sum;
-                if (logits != nullptr && t0 + t < ntok) logits[static_cast<size_t>(t0 + t) * E + e] = sum;
             }
+            if (logits != nullptr && t0 + t < ntok) logits[static_cast<size_t>(t0 + t) * E + e] = sum;
         }
         __syncthreads();
     }
     if (SPLIT) {
+        if (apart) cluster_wait();   // no experts were left for this CTA
         cluster_arrive();
         cluster_wait();
-        for (int i = tid; i < own * E; i += kGateThreads) {
-            float sum = 0.f;
-            for (int k = 0; k < parts; ++k) sum += row_s[k * own * E + i];
-            row_s[i] = sum;   // part 0's own slot: this thread's alone
-            const int t = t0 + part_id * own + i / E;
-            if (logits != nullptr && t < ntok) logits[static_cast<size_t>(t) * E + i % E] = sum;
-        }
-        __syncthreads();
     }
     const int t = t0 + part_id * own + warp;   // a warp per token: kGateWarps == kGateTok
     static_assert(kGateWarps == kGateTok, "a warp per token");
     if (warp < own && t < ntok) topk_softmax_any(row_s + warp * E, E, topk, renorm, lane, ids + static_cast<size_t>(t) * topk, w + static_cast<size_t>(t) * topk);
+}
+
+// A cluster of eight CTAs per tile, two chains each, for at most 8 NT experts. The products of a chain's steps, which eight warps take
+// in turn, meet in shared memory and are added there in order; the chain's sum goes to the CTA that selects for the token, which
+// adds the 16 chains. Every row is read once per tile.
+constexpr int kGateChains = kGateWarps, kGateOwnChains = kGateChains / kGateMaxParts, kGateStepWarps = kGateWarps / kGateOwnChains;
+constexpr int kGateOwnTok = kGateTok / kGateMaxParts;
+// floats between the rows of a step's products: those that a warp stores at once spread over the banks
+__host__ __device__ constexpr int gate_pitch(int nt) { return nt * 8 + 8; }
+static int gate_chains_smem(int hidden, int nt, int E) {
+    const int most = (hidden / 32 + kGateChains - 1) / kGateChains;   // steps of a chain
+    return (kGateOwnChains * most * kGateTok * gate_pitch(nt) + kGateChains * kGateOwnTok * E) * static_cast<int>(sizeof(float));
+}
+
+template <int NT>
+__global__ void __launch_bounds__(kGateThreads, 1) moe_gate_topk_chains_kernel(const __nv_bfloat16* x, const __nv_bfloat16* gate, int ntok, int hidden, int E,
+                                                                               int topk, int renorm, int* ids, float* w, float* logits) {
+    extern __shared__ float gate_sm[];
+    constexpr int COLS = NT * 8, PITCH = gate_pitch(NT), STEP = kGateTok * PITCH;
+    constexpr int AHEAD = NT == 8 ? 1 : 2;
+    const int tid = static_cast<int>(threadIdx.x), warp = tid >> 5, lane = tid & 31;
+    const int g = lane >> 2, tig = lane & 3;
+    const int part_id = static_cast<int>(cluster_ctarank());
+    const int t0 = static_cast<int>(blockIdx.x) / kGateMaxParts * kGateTok;
+    const int steps = hidden / 32, most = (steps + kGateChains - 1) / kGateChains;
+    float* prod = gate_sm;                                     // [own chains][most][16 tokens][PITCH]
+    float* chain_s = gate_sm + kGateOwnChains * most * STEP;   // [16 chains][own tokens][E]
+    cluster_arrive();    // its counterpart stands before the first store into another CTA
+    pdl_wait_and_release();
+    const __nv_bfloat16* xa = gate_row(x, t0 + g, ntok, hidden, tig);
+    const __nv_bfloat16* xb = gate_row(x, t0 + g + 8, ntok, hidden, tig);
+    const __nv_bfloat16* ge[NT];
+#pragma unroll
+    for (int n = 0; n < NT; ++n) ge[n] = gate_row(gate, n * 8 + g, E, hidden, tig);
+    const int mine = warp % kGateOwnChains;                    // this warp's chain, among the CTA's and among all
+    const int chain = part_id * kGateOwnChains + mine;
+#pragma unroll 1
+    for (int j0 = warp / kGateOwnChains; chain + j0 * kGateChains < steps; j0 += AHEAD * kGateStepWarps) {
+        uint4 a[AHEAD], c[AHEAD], b[AHEAD][NT];
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u) {
+            const int s = chain + (j0 + u * kGateStepWarps) * kGateChains;
+            if (s >= steps) break;
+            a[u] = ld_v4(xa + s * 32);
+            c[u] = ld_v4(xb + s * 32);
+#pragma unroll
+            for (int n = 0; n < NT; ++n) b[u][n] = ld_v4(ge[n] + s * 32);
+        }
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u) {
+            const int j = j0 + u * kGateStepWarps;
+            if (chain + j * kGateChains >= steps) break;
+            float* p = prod + (mine * most + j) * STEP + g * PITCH + tig * 2;
+#pragma unroll
+            for (int n = 0; n < NT; ++n) {
+                float d[4] = {0.f, 0.f, 0.f, 0.f};
+                mma_bf16_16816(d, a[u].x, c[u].x, a[u].y, c[u].y, b[u][n].x, b[u][n].y);
+                mma_bf16_16816(d, a[u].z, c[u].z, a[u].w, c[u].w, b[u][n].z, b[u][n].w);
+                *reinterpret_cast<float2*>(p + n * 8) = make_float2(d[0], d[1]);
+                *reinterpret_cast<float2*>(p + 8 * PITCH + n * 8) = make_float2(d[2], d[3]);
+            }
+        }
+    }
+    __syncthreads();
+    cluster_wait();   // every CTA of the cluster runs
+    for (int i = tid; i < kGateOwnChains * kGateTok * COLS; i += kGateThreads) {
+        const int k = i / (kGateTok * COLS), t = i / COLS % kGateTok, e = i % COLS, at = part_id * kGateOwnChains + k;
+        if (e >= E) continue;
+        float sum = 0.f;
+        const float* p = prod + k * most * STEP + t * PITCH + e;
+#pragma unroll 4
+        for (int s = at; s < steps; s += kGateChains, p += STEP) sum += *p;
+        st_shared_cluster_f32(mapa_u32(smem_u32(chain_s + (at * kGateOwnTok + t % kGateOwnTok) * E + e), static_cast<uint32_t>(t / kGateOwnTok)), sum);
+    }
+    cluster_arrive();
+    cluster_wait();
+    for (int i = tid; i < kGateOwnTok * E; i += kGateThreads) {
+        float sum = 0.f;
+#pragma unroll
+        for (int k = 0; k < kGateChains; ++k) sum += chain_s[k * kGateOwnTok * E + i];
+        chain_s[i] = sum;   // chain 0's own slot: this thread's alone
+        const int t = t0 + part_id * kGateOwnTok + i / E;
+        if (logits != nullptr && t < ntok) logits[static_cast<size_t>(t) * E + i % E] = sum;
+    }
+    __syncthreads();
+    const int t = t0 + part_id * kGateOwnTok + warp;
+    if (warp < kGateOwnTok && t < ntok) topk_softmax_any(chain_s + warp * E, E, topk, renorm, lane, ids + static_cast<size_t>(t) * topk, w + static_cast<size_t>(t) * topk);
 }
 
 // ---------------------------------------------------------------------------- row gather / top-k reduce
@@ -490,12 +593,22 @@ extern "C" int tdist_moe_gate_topk(const void* x, const void* gate, int ntok, in
     if (hidden < 32 || hidden % 32) return fail(TDIST_EINVAL, "moe_gate_topk: hidden must be a multiple of 32");
     if (reinterpret_cast<uintptr_t>(x) % 16 || reinterpret_cast<uintptr_t>(gate) % 16) return fail(TDIST_EINVAL, "moe_gate_topk: x and gate must be 16-byte aligned");
     if (ntok <= 0) return 0;
-    const int nt = num_experts <= 8 ? 1 : (num_experts <= 16 ? 2 : (num_experts <= 32 ? 4 : 8));
-    const int smem = (kGateWarps * kGateTok * nt * 8 + kGateTok * num_experts) * static_cast<int>(sizeof(float));
-    // parts of the hidden dimension: while every warp has a step of its own and the CTAs have an SM of their own
-    const int tiles = (ntok + kGateTok - 1) / kGateTok;
-    int parts = 1;
-    while (parts < kGateMaxParts && 2 * parts * kGateWarps * 32 <= hidden && 2 * parts * tiles <= tdist_host::sm_count()) parts *= 2;
+    // A cluster's SMs lie in one GPC: clusters of 2, 4 and 8 CTAs fill 100, 90 and 82 % of the machine (64 experts x 7168, experts shared
+    // by 2 / 4 / 8 CTAs: 240 tokens 11.2 / 8.9 / 8.4 us, 300 tokens 11.3 / 9.0 / 15.6, 592 tokens 11.4 / 17.0 / 23.6). Chains are shared
+    // out where eight CTAs per tile run at once, the experts take one pass (64 tokens x 7168, 256 experts: 52 us, 11.4 by experts),
+    // a chain has two steps or more (4 tokens x 512, 8 experts: 2.5 us, 2.3 on one CTA; x 1024 2.7 and 2.7) and the products
+    // of the steps fit; the experts elsewhere, while each CTA gets some.
+    const int tiles = (ntok + kGateTok - 1) / kGateTok, groups = (num_experts + 7) / 8;
+    const int fit[4] = {100, 100, 90, 82};
+    const auto runs_at_once = [&](int i) { return (100LL * tiles << i) <= static_cast<long long>(fit[i]) * tdist_host::sm_count(); };
+    const auto width = [](int n) { return n <= 1 ? 1 : (n <= 2 ? 2 : (n <= 4 ? 4 : 8)); };
+    static_assert(1 << 3 == kGateMaxParts, "the largest cluster");
+    const bool chains = runs_at_once(3) && groups <= 8 && hidden >= 2 * kGateChains * 32 && gate_chains_smem(hidden, width(groups), num_experts) <= 200 * 1024;
+    int parts = chains ? kGateMaxParts : 1;
+    for (int i = 1; i <= 3 && parts < groups && !chains && runs_at_once(i); ++i) parts *= 2;
+    const int nt = width(chains ? groups : (groups + parts - 1) / parts);
+    const int smem = chains ? gate_chains_smem(hidden, nt, num_experts)
+                            : (kGateWarps * kGateTok * nt * 8 + kGateTok / parts * num_experts) * static_cast<int>(sizeof(float));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(tiles * parts));
     cfg.blockDim = dim3(kGateThreads);
@@ -509,13 +622,21 @@ extern "C" int tdist_moe_gate_topk(const void* x, const void* gate, int ntok, in
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = parts > 1 ? 2 : 1;
-#define TDIST_GATE_CASE(NT)                                                                                                     \
-    {                                                                                                                           \
-        const auto kernel = parts > 1 ? moe_gate_topk_kernel<NT, true> : moe_gate_topk_kernel<NT, false>;                       \
-        if (int rc = ensure_smem(kernel, smem)) return rc;                                                                      \
-        TDIST_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, static_cast<const __nv_bfloat16*>(x),                                    \
-                                         static_cast<const __nv_bfloat16*>(gate), ntok, hidden, num_experts, topk, renormalize, parts, \
-                                         static_cast<int*>(ids), static_cast<float*>(weights), static_cast<float*>(logits)));   \
+    const auto* xp = static_cast<const __nv_bfloat16*>(x);
+    const auto* gp = static_cast<const __nv_bfloat16*>(gate);
+    int* idp = static_cast<int*>(ids);
+    float *wp = static_cast<float*>(weights), *lp = static_cast<float*>(logits);
+#define TDIST_GATE_CASE(NT)                                                                                                              \
+    {                                                                                                                                    \
+        if (chains) {                                                                                                                    \
+            if (int rc = ensure_smem(moe_gate_topk_chains_kernel<NT>, smem)) return rc;                                                  \
+            TDIST_CUDA_OK(cudaLaunchKernelEx(&cfg, moe_gate_topk_chains_kernel<NT>, xp, gp, ntok, hidden, num_experts, topk, renormalize, \
+                                             idp, wp, lp));                                                                              \
+        } else {                                                                                                                         \
+            const auto kernel = parts > 1 ? moe_gate_topk_kernel<NT, true> : moe_gate_topk_kernel<NT, false>;                            \
+            if (int rc = ensure_smem(kernel, smem)) return rc;                                                                           \
+            TDIST_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, xp, gp, ntok, hidden, num_experts, topk, renormalize, parts, idp, wp, lp));   \
+        }                                                                                                                                \
     }
     if (nt == 1) TDIST_GATE_CASE(1)
     else if (nt == 2) TDIST_GATE_CASE(2)

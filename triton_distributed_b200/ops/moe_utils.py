@@ -67,7 +67,8 @@ def topk_softmax(logits: torch.Tensor, topk: int, renormalize: bool = False) -> 
 def gate_topk(x: torch.Tensor, gate: torch.Tensor, topk: int, renormalize: bool = False,
               logits: Optional[torch.Tensor] = None) -> Tuple[torch.Tensor, torch.Tensor]:
     """:func:`topk_softmax` of ``x[T, hidden] @ gate[E, hidden].T`` with fp32 sums; one launch for bf16 operands.
-    ``logits`` (``[T, E]``), if given, receives the product; the launch writes it only as dense fp32."""
+    ``logits`` (``[T, E]``), if given, receives the product; the launch writes it only as dense fp32. What the launch gives a
+    token does not depend on how many others are in the call."""
     global launch_count
     T, hidden = x.shape
     E = gate.shape[0]
