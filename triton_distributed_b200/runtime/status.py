@@ -27,9 +27,11 @@ _TIMEOUT_CACHE = [_CODES, 0]   # setting as the environment keeps it (any other 
 def default_timeout_ns() -> int:
     """Limit of every bounded device wait, from TDIST_WAIT_TIMEOUT_MS (default 4 s); the parsed value is
     cached per distinct setting because this sits on every launch path. The setting is looked up as ``os.environ`` keeps it
-    (its ``get`` encodes the name and decodes the value on every call: 0.5 us of a 10 us call, 0.1 here), and by ``get``
-    where ``os.environ`` is some other mapping."""
-    raw = os.environ._data.get(_TIMEOUT_KEY) if type(os.environ) is _ENVIRON else os.environ.get(_TIMEOUT_NAME)
+    (its ``get`` encodes the name and decodes the value on every call: 0.5 us of a 10 us call, 0.1 here); where ``os.environ``
+    is some other mapping, by ``get`` and parsed on every call."""
+    if type(os.environ) is not _ENVIRON:
+        return int(float(os.environ.get(_TIMEOUT_NAME, "4000")) * 1e6)
+    raw = os.environ._data.get(_TIMEOUT_KEY)
     if raw != _TIMEOUT_CACHE[0]:
         _TIMEOUT_CACHE[1] = int(float(os.environ.get(_TIMEOUT_NAME, "4000")) * 1e6)
         _TIMEOUT_CACHE[0] = raw
