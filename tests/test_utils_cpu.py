@@ -455,6 +455,8 @@ def test_wait_timeout_follows_any_mapping_in_the_place_of_os_environ(monkeypatch
 
 def test_wait_timeout_compares_no_bytes_with_text():
     """Under ``python -bb``, where that is an error, from the process's own settings to another mapping and back."""
+    import subprocess
+    import sys
     code = ("import os; os.environ['TDIST_WAIT_TIMEOUT_MS'] = '250'; own = os.environ; "
             "from triton_distributed_b200.runtime import default_timeout_ns as ns; assert ns() == 250_000_000; "
             "os.environ = {'TDIST_WAIT_TIMEOUT_MS': '125'}; assert ns() == 125_000_000; os.environ = own; assert ns() == 250_000_000")
