@@ -131,6 +131,7 @@ __device__ __forceinline__ uint32_t tile_off(int row, int chunk) {
 // D = 256 -> 3 stages (192 KB, 1 CTA/SM; two would
 // leave one block of a warp in flight).
 __host__ __device__ constexpr int decode_stages(int d) { return d <= 64 ? 4 : 3; }
+__host__ __device__ constexpr int decode_ctas_per_sm(int d) { return d <= 64 ? 3 : (d <= 128 ? 2 : 1); }
 // floats between the heads of a warp's O in shared memory (the four heads a store writes at once lie in different banks)
 __host__ __device__ constexpr int decode_o_pitch(int d) { return d + 4; }
 
@@ -161,7 +162,7 @@ __device__ __forceinline__ int sequence_by_length(const int* kv_lens, int B, int
 }
 
 template <typename T, int D, int NH>
-__global__ void __launch_bounds__(kDecodeThreads, (D <= 64 ? 3 : (D <= 128 ? 2 : 1))) flash_decode_kernel(const DecodeParams p) {
+__global__ void __launch_bounds__(kDecodeThreads, decode_ctas_per_sm(D)) flash_decode_kernel(const DecodeParams p) {
     constexpr int CH = D / 8;                      // 16-byte chunks per row
     constexpr int TILE = kTok * D * 2;             // bytes of one K or V block
     constexpr int NS = decode_stages(D);           // cp.async ring depth per warp
@@ -619,17 +620,21 @@ using tdist_host::fail;
 // partials do not fit the ring, the splits meet in global memory (workspace + arrival counter).
 // Eight is the portable cluster size. Larger ones were measured only while the partials lay behind the ring (133 KB of shared
 // memory per CTA, so that only some 16-CTA clusters were resident at once: batch 1, 8 kv heads, 16384 keys, 16 splits 37.1 us
-// against 22.6 us through global memory); in the ring (100 KB at head_dim 128, two CTAs per SM) they have not been. Up to
-// eight splits the cluster form was 5-10 % faster then (4096 keys: 14.4 / 20.6 us against 15.4 / 22.6 us with 8 / 4 splits).
+// against 22.6 us through global memory); in the ring (96 KB at head_dim 128, two CTAs per SM) they have not been. Up to
+// eight splits the cluster form is 4-8 % faster (batch 1, 4096 keys, 2 / 4 / 8 splits: 30.1 / 17.8 / 11.8 us, through global memory
+// 31.1 / 19.3 / 12.7), except where clusters of eight no longer fit at once (batch 4, 256 CTAs: 23.7 and 18.7 us), which the choice of
+// the splits knows.
 constexpr int kClusterMergeMaxSplits = 8;
 
-// Longest key range per CTA with which a batch of several sequences, all of whose CTAs run at once, overlaps the launch
-// before it. CTAs that take their places as that launch's finish sit where its short sequences were, so that two long
-// ones may share an SM; where the lengths are equal or a second round evens them out this does not matter. Batch 2,
-// lengths ragged up to kv, 18 splits, us per call without / with the overlap: kv 20000 (1111 keys per CTA) 35.4 / 33.8,
-// 40000 (2222) 55.5 / 54.8, 60000 (3333) 75.0 / 75.5, 80000 (4444) 95.7 / 96.5, 110000 (6111) 123.5 / 128.1; 64 query
-// heads, 158353 (8797) 177.5 / 186.6. Batch 1, 200000 keys: 143.5 / 138.0; batch 41, 11127 keys (several rounds): 182.4 /
-// 179.5. The lengths are not known on the host: batch 8 of equal 32768 (8192) would gain too, 173.8 / 171.5.
+// Longest key range per CTA with which a batch of several sequences overlaps the launch before it, up to twice as many CTAs as SMs.
+// CTAs that take their places as that launch's finish sit where its short sequences were, so that two long
+// ones may share an SM; with more CTAs than that the SMs even out. Batch 2,
+// lengths ragged up to kv, 18 splits (through global memory), us per call without / with the overlap: head_dim 128, kv 20000
+// (1111 keys per CTA) 30.6 / 30.1, 40000 (2222) 50.6 / 50.1, 80000 (4444) 89.3 / 89.7; 64 query
+// heads, 158353 (8797) 167.1 / 168.7; head_dim 64, 69120 (3840) 52.6 / 53.2, 138240 (7680) 93.0 / 96.0. Beyond twice the SMs, where
+// three CTAs of head_dim 64 still run at once: 2 x 184320, 384 CTAs of 7680 keys, 114.6 / 113.8; 3 x 138240, 432 CTAs 116.1 / 115.7.
+// The limit is wider than it has to be: with clusters (8 x 32768, 4 splits: 129.6 / 128.5) and with one CTA per SM (head_dim 256, 3 x
+// 46080, 7680 keys per CTA: 160.8 / 159.7) the overlap gains up to 1 % beyond it too.
 constexpr long long kOverlapKeys = 2560;
 
 // Whether the CTAs may take their places while the launch before still runs (programmatic dependent launch).
@@ -684,9 +689,8 @@ static int launch_decode(DecodeParams& p, cudaStream_t stream) {
     p.cluster_merge = cluster ? 1 : 0;
     // Only where some CTAs start after others have ended, and not where CTAs wait for those of another rank: the ranks'
     // lengths differ, and each could wait for a sequence that the other has yet to start.
-    constexpr int per_sm = D <= 64 ? 3 : (D <= 128 ? 2 : 1);
     p.longest_first = p.B > 1 && p.B <= kMaxOrdered && (p.mode != 2 || p.world == 1) &&
-                      static_cast<long long>(p.B) * p.Hkv * p.splits > static_cast<long long>(per_sm) * tdist_host::sm_count();
+                      static_cast<long long>(p.B) * p.Hkv * p.splits > static_cast<long long>(decode_ctas_per_sm(D)) * tdist_host::sm_count();
     TDIST_CUDA_OK(cudaLaunchKernelEx(&cfg, flash_decode_kernel<T, D, NH>, p));
     return 0;
 }

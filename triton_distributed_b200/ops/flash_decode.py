@@ -80,10 +80,11 @@ def ref_lse_merge(parts: torch.Tensor) -> torch.Tensor:
 
 
 def default_splits(B: int, Hkv: int, max_kv: int, device, head_dim: int = 128) -> int:
-    """Enough (batch, kv head, split) CTAs for one wave of the machine (two CTAs fit an SM up to
+    """Enough (batch, kv head, split) CTAs for one wave of the machine (two CTAs per SM up to
     head_dim 128), but at least 256 tokens each: below that the merge of the splits (a round trip through global
-    memory per eight of them) costs more than the shorter KV loop saves (batch 1, 8 kv heads, 4096 keys: 12.4 us with
-    16 splits, 16.5 us with 37, 21.0 us with 64)."""
+    memory per eight of them) costs more than the shorter KV loop saves (batch 1, 8 kv heads, 4096 keys: 10.9 us with
+    16 splits, 14.1 us with 37, 18.6 us with 64). Of head_dim 64 three CTAs fit an SM; two already keep HBM busy (batch 1, 955863
+    keys: 342 us with 37 splits, 356 with 55; batch 2 of 138240 103 and 109, though ragged ones 93 and 86)."""
     per_sm = 2 if head_dim <= 128 else 1
     want = max(1, per_sm * _sm_count(device) // max(1, B * Hkv))
     cap = max(1, (max_kv + 255) // 256)
