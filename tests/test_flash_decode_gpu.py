@@ -349,3 +349,65 @@ def test_a_launch_behind_a_waiting_one_leaves_the_machine_free(cuda_device, monk
     assert free
     torch.testing.assert_close(c.float(), x.float() @ w.float().t(), atol=1e-1, rtol=2e-2)
     assert torch.equal(got, want)
+
+
+def _exact_attn(q, k, v, lens, table, scale):
+    """Output, sum of p |v|, log-sum-exp, in float64."""
+    B, Hq, D = q.shape
+    Hkv, page = k.shape[2], k.shape[1]
+    o, spread = (torch.zeros(B, Hq, D, dtype=torch.float64, device=q.device) for _ in range(2))
+    lse = torch.full((B, Hq), float("-inf"), dtype=torch.float64, device=q.device)
+    for b, n in enumerate(lens.tolist()):
+        if n:
+            pages = table[b, : -(-n // page)].long()
+            kk, vv = (c[pages].reshape(-1, Hkv, D)[:n].double() for c in (k, v))
+            s = torch.einsum("hgd,nhd->hgn", q[b].double().view(Hkv, -1, D), kk) * scale
+            p = torch.softmax(s, -1)
+            o[b], spread[b] = (torch.einsum("hgn,nhd->hgd", p, x).reshape(Hq, D) for x in (vv, vv.abs()))
+            lse[b] = torch.logsumexp(s, -1).reshape(Hq)
+    return o, spread, lse
+
+
+@pytest.mark.parametrize("B,splits,Hq,Hkv,D,most", [
+    (127, 2, 24, 2, 128, 700), (128, 2, 24, 2, 128, 700), (129, 2, 24, 2, 128, 700),   # the largest batch ordered by length, and beyond
+    (128, 1, 8, 4, 64, 600), (50, 2, 8, 2, 256, 300),
+    (24, 10, 8, 2, 128, 2700),                                                         # merged through global memory
+    (128, 12, 8, 2, 64, 700)])                                                         # not ordered: too short for so many rounds
+def test_ragged_batches_of_more_than_one_round(cuda_device, B, splits, Hq, Hkv, D, most):
+    """Sequences of any length, equal and empty ones among them, in a grid of more CTAs than run at once: results, partials with
+    their log-sum-exp, and a captured launch that is replayed with other lengths, with short ones only, and with equal ones. fp16
+    rounds a probability and the result to 2^-11
+    of themselves (small probabilities to 2^-25); scores, exponentials and sums in fp32 add less than 2^-14."""
+    torch.manual_seed(B + splits + D)
+    page = 16
+    k, v, table = _make_cache(B, [most] * B, Hkv, D, page, torch.float16, cuda_device)
+    q = torch.randn(B, Hq, D, device=cuda_device).half()
+    scale = D ** -0.5
+    lens = torch.randint(0, most + 1, (B,), device=cuda_device).to(torch.int32)
+    lens[3], lens[5], lens[6:9], lens[B - 1] = 0, most, most // 2, 1
+
+    def check():
+        o, spread, lse = _exact_attn(q, k, v, lens, table, scale)
+        small = most * 2.0 ** -25 * v.float().abs().max().double()
+        out = FD.gqa_fwd_batch_decode(q, k, v, None, None, lens, table, scale, kv_split=splits)
+        part = FD.gqa_fwd_batch_decode_intra_rank(q, k, v, None, None, lens, table, scale, 0.0, kv_split=splits).double()
+        check_status()
+        assert ((out.double() - o).abs() <= (2.0 ** -11 + 2.0 ** -14) * spread + 2.0 ** -11 * o.abs() + small).all()
+        assert ((part[..., :D] - o).abs() <= (2.0 ** -11 + 2.0 ** -14) * spread + small).all()
+        live = lens > 0
+        assert ((part[live][..., D] - lse[live]).abs() <= 2.0 ** -14).all() and (part[~live][..., D] == float("-inf")).all()
+        return out
+
+    check()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        FD.gqa_fwd_batch_decode(q, k, v, None, None, lens, table, scale, kv_split=splits)
+    torch.cuda.current_stream().wait_stream(side)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        replayed = FD.gqa_fwd_batch_decode(q, k, v, None, None, lens, table, scale, kv_split=splits)
+    for other in (lens[torch.randperm(B, device=cuda_device)], lens[torch.randperm(B, device=cuda_device)], lens // 4, torch.full_like(lens, most)):
+        lens.copy_(other)
+        g.replay()
+        assert torch.equal(replayed, check())

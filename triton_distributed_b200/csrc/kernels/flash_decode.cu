@@ -58,7 +58,7 @@ struct DecodeParams {
     void* out;              // mode 0/2: T [B, Hq, D]; mode 1: float [B, Hq, D + 1]
     char* ll_peer[kMaxRanks];  // SP: this call's parity of every rank: [world][B*Hq*(D+2)/2] packets
     int B, Hq, Hkv, page_size, max_blocks, splits;
-    int longest_first;      // 1: sequences take their places in the order of their lengths
+    int order_from;         // keys of the longest sequence from which on they take their places in the order of their lengths (0: never)
     int page_shift;         // log2(page_size), or -1
     int cluster_merge;      // 1: the splits of a (batch, kv head) are one thread-block cluster and merge through shared memory
     long long stride_block, stride_token, stride_head;  // cache strides in elements
@@ -141,22 +141,30 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
     return r;
 }
 
-// Sequence of the CTAs in place `slot` when the longest come first (ties by number). The grid starts in order of its blocks,
+// Sequence of the CTAs in place `slot`, and its length, when the longest come first (ties by number) and one of them has `least`
+// keys. The grid starts in order of its blocks,
 // so the last ones to start are the shortest (batch 32, 64 query heads, lengths ragged to 8192: 114 us in order of
-// their numbers, 94 us; 51 ragged ones that all start at once: no difference).
+// their numbers, 94 us; 51 ragged ones that all start at once: no difference). A thread per sequence: batches of more than
+// kMaxOrdered keep the order of the numbers.
 constexpr int kMaxOrdered = kDecodeThreads;
-__device__ __forceinline__ int sequence_by_length(const int* kv_lens, int B, int slot) {
-    __shared__ int len_s[kMaxOrdered];
-    __shared__ int pick_s;
+__device__ __forceinline__ int2 sequence_by_length(const int* kv_lens, int B, int slot, int least) {
+    __shared__ __align__(16) int len_s[kMaxOrdered];
+    __shared__ int2 pick_s;
     const int t = static_cast<int>(threadIdx.x);
-    if (t < B) len_s[t] = kv_lens[t];
-    __syncthreads();
-    if (t < B) {
-        const int mine = len_s[t];
-        int rank = 0;
-        for (int j = 0; j < B; ++j) rank += len_s[j] > mine || (len_s[j] == mine && j < t);
-        if (rank == slot) pick_s = t;
+    const int mine = t < B ? kv_lens[t] : -0x7fffffff - 1;   // places without a sequence come last
+    const int first = kv_lens[0];
+    len_s[t] = mine;
+    // nothing to gain where all are short or all alike
+    if (!__syncthreads_or(mine >= least) || !__syncthreads_or(t < B && mine != first)) return make_int2(slot, len_s[slot]);
+    int rank = 0;
+#pragma unroll 8
+    for (int j = 0; j < (B + 3) / 4; ++j) {
+        const int4 v = reinterpret_cast<const int4*>(len_s)[j];
+        const int before = t - 4 * j;   // of equal lengths, those with lower numbers
+        rank += (v.x > mine || (v.x == mine && before > 0)) + (v.y > mine || (v.y == mine && before > 1)) +
+                (v.z > mine || (v.z == mine && before > 2)) + (v.w > mine || (v.w == mine && before > 3));
     }
+    if (t < B && rank == slot) pick_s = make_int2(t, mine);
     __syncthreads();
     return pick_s;
 }
@@ -182,7 +190,14 @@ __global__ void __launch_bounds__(kDecodeThreads, decode_ctas_per_sm(D)) flash_d
     const int split = static_cast<int>(blockIdx.x) % p.splits;
     const int kvh = (static_cast<int>(blockIdx.x) / p.splits) % p.Hkv;
     int b = static_cast<int>(blockIdx.x) / (p.splits * p.Hkv);
-    if (p.longest_first) b = sequence_by_length(p.kv_lens, p.B, b);
+    int kv_len;
+    if (p.order_from > 0) {
+        const int2 pick = sequence_by_length(p.kv_lens, p.B, b, p.order_from);
+        b = pick.x;
+        kv_len = pick.y;
+    } else {
+        kv_len = p.kv_lens[b];
+    }
     const int G = p.Hq / p.Hkv;
     const T* q = static_cast<const T*>(p.q) + (static_cast<size_t>(b) * p.Hq + static_cast<size_t>(kvh) * G) * D;
     const T* kc = static_cast<const T*>(p.k_cache) + static_cast<size_t>(kvh) * p.stride_head;
@@ -190,7 +205,6 @@ __global__ void __launch_bounds__(kDecodeThreads, decode_ctas_per_sm(D)) flash_d
     const int* table = p.block_table + static_cast<size_t>(b) * p.max_blocks;
 
     // ---- this CTA's KV range, in 16-token blocks dealt round-robin to the warps
-    const int kv_len = p.kv_lens[b];
     const int nblk_total = (kv_len + kTok - 1) / kTok;
     const int blk_per_split = (nblk_total + p.splits - 1) / p.splits;
     const int blk0 = split * blk_per_split;
@@ -644,6 +658,23 @@ static bool overlaps_previous(const DecodeParams& p) {
     return p.B == 1 || keys <= kOverlapKeys || ctas > 2LL * tdist_host::sm_count();
 }
 
+// Length of the longest sequence from which on the order by length pays, or 0. Only where some CTAs start after others have ended, and
+// not where CTAs wait for those of another rank: the ranks' lengths differ, and each could wait for a sequence that the other has
+// yet to start. What it gains is the wait for a long sequence that started last; what it costs is a step in front of every CTA, and
+// the short sequences, bound by latencies, no longer run beside long ones that are bound by HBM. So the longest CTA has to
+// be worth more the more rounds of CTAs there are. Ragged batches, 8 kv heads, us per call by number / by length: head_dim 128, 64
+// sequences to 1024 keys (1.7 rounds) 43.6 / 40.0, 64 to 4096 121.5 / 95.2, 100 to 1024 (2.7) 58.6 / 62.3, 100 to 4096 162 / 149,
+// 128 to 64 (3.5) 35.2 / 39.4, 128 to 4096 (6.9, two splits) 196 / 218, 64 to 8192 (3.5, two splits) 202 / 185; head_dim 64, 128 to 64
+// (2.3) 20.6 / 25.0, 100 to 8192 (1.8) 186 / 156; head_dim 256, 24 to 1024 (1.3) 37.5 / 29.2, 40 to 300 (2.2) 26.8 / 28.1.
+constexpr double kOrderValues = 32768;   // keys of a CTA x head_dim
+static int order_from(const DecodeParams& p, int head_dim, int per_sm) {
+    const double rounds = static_cast<double>(p.B) * p.Hkv * p.splits / (per_sm * tdist_host::sm_count());
+    if (p.B < 2 || p.B > kMaxOrdered || (p.mode == 2 && p.world > 1) || rounds <= 1.0) return 0;
+    const double more = 5.0 * (rounds - 1.5);
+    const double keys = kOrderValues * (more > 1.0 ? more : 1.0) / head_dim * p.splits;
+    return keys <= static_cast<double>(p.max_blocks) * p.page_size && keys < 0x7fffffff ? static_cast<int>(keys) : 0;
+}
+
 template <typename T, int D, int NH>
 static int launch_decode(DecodeParams& p, cudaStream_t stream) {
     constexpr int ring = kDecodeWarps * decode_stages(D) * 2 * kTok * D * 2;
@@ -687,10 +718,7 @@ static int launch_decode(DecodeParams& p, cudaStream_t stream) {
         dim.val.clusterDim.z = 1;
     }
     p.cluster_merge = cluster ? 1 : 0;
-    // Only where some CTAs start after others have ended, and not where CTAs wait for those of another rank: the ranks'
-    // lengths differ, and each could wait for a sequence that the other has yet to start.
-    p.longest_first = p.B > 1 && p.B <= kMaxOrdered && (p.mode != 2 || p.world == 1) &&
-                      static_cast<long long>(p.B) * p.Hkv * p.splits > static_cast<long long>(decode_ctas_per_sm(D)) * tdist_host::sm_count();
+    p.order_from = order_from(p, D, decode_ctas_per_sm(D));
     TDIST_CUDA_OK(cudaLaunchKernelEx(&cfg, flash_decode_kernel<T, D, NH>, p));
     return 0;
 }
