@@ -49,7 +49,7 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 // Arrive on the barrier at the same shared-memory offset in CTA `cta` of the cluster, for a thread that hands back what it has
 // READ (TMEM columns whose loads it has waited for): it publishes no writes to the other CTA, and the default semantics (release
 // within this CTA) spare it the wait for its own stores that .release.cluster makes it do (1000 cycles and more: the drain of
-// a GEMM tile ends with it. 4096^3 112.6 -> 110.0 us, m1000 n5504 k4096 47.4 -> 46.0, m8192 n49152 k12288 7237 -> 7182).
+// a GEMM tile ends with it. 4096^3 112.6 -> 110.0 us, m1000 n5504 k4096 47.4 -> 46.0; products of many rounds are within the noise).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar, uint32_t cta) {
     asm volatile(
         "{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, %1;\n\t"

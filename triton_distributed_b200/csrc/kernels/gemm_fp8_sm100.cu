@@ -19,7 +19,8 @@
 // the MMA issuer and the promotion warps: TMEM (512 columns) holds only two 128 x 256 fp32 accumulators,
 // so at most two K blocks of MMA work (~0.5 us) are in flight against a loop of MMA completion latency +
 // TMEM read + barrier hand-over of about 1.3 us. A CTA-pair tiling (cta_group::2, 256 x 256) was built and
-// measured at half this speed, because the same round trip then crosses two SMs; it was removed.
+// removed: at first half this speed, because the arrival that hands an accumulator back to the leader CTA (release at cluster scope)
+// waited for the warp's own stores; with an arrival that does not, 222 us against 228 (m8192 n6144 k4096), 83 against 81 at m2048 n4096 k7168.
 //
 // AG mode is the fp8 twin of gemm_sm100.cu's: pusher CTAs of the same grid stream this rank's rows
 // AND their scales into every peer's workspace, one flag per 128-row block.

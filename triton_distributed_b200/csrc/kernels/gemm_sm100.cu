@@ -1600,7 +1600,7 @@ static GridPlan plan_grid(const TdistGemmArgs* a) {
     const int seg_m_tiles = a->pair_block ? a->num_pairs : (a->m_per_rank + BM * g.ctas_per_tile - 1) / (BM * g.ctas_per_tile);
     int n_tiles = (a->n + BN - 1) / BN;
     if (a->expert_ids != nullptr && g.ctas_per_tile == 1 && a->num_sms <= 0 && (a->a_gather == nullptr || a->gather_dst != nullptr)) {
-        // Grouped GEMM of a decode step: its blocks are a few rows each, so it is bound by the loads of B, and a CTA's rate by
+        // Grouped GEMM on single CTAs. In a decode step its blocks are a few rows each, so it is bound by the loads of B, and a CTA's rate by
         // what an SM takes from L2. While 256-column tiles leave SMs idle, narrower ones that still run as one round bring
         // more of them in (both GEMMs of the experts, 16 tokens, top 2 of 8, 4096 x 2048: 71 -> 67 us; 64 tokens, top 4 of
         // 16, 4096 x 512: 58 -> 51 us).
