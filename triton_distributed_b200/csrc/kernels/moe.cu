@@ -24,7 +24,8 @@ namespace tdist {
 // pair at each sorted position), slot_of[n] (sorted position of each pair). One CTA; a chain of latencies, so few steps: every
 // warp counts a contiguous run of the pairs by itself (position inside the run's group = count so far + equal ids in lower
 // lanes, kept in slot_of meanwhile), prefix sums over the warps and over the experts follow, then every pair's position is
-// known. (Histogram, then 512 pairs at a time with the CTA meeting four times for each: the
+// known. Steps past the end of a run are left out: a match of 32 different values takes longest of all (1024 pairs of 64 experts 7.8 us with
+// them, 4.5 without). (Histogram, then 512 pairs at a time with the CTA meeting four times for each: the
 // whole expert-parallel block of 1194 tokens, top 8 of 16, 280 us, 267 here; 1831 tokens, top 7 of 16, 323 and 314.)
 constexpr int kRouteAhead = 4;   // loads of a lane in flight
 __global__ void __launch_bounds__(1024) moe_route_kernel(const int* ids, int n, int topk, int E, int* splits,
@@ -47,6 +48,7 @@ __global__ void __launch_bounds__(1024) moe_route_kernel(const int* ids, int n, 
         for (int u = 0; u < kRouteAhead; ++u) es[u] = i0 + u * 32 + lane < end ? ids[i0 + u * 32 + lane] : -1;
 #pragma unroll
         for (int u = 0; u < kRouteAhead; ++u) {
+            if (i0 + u * 32 >= end) break;
             const int i = i0 + u * 32 + lane, e = es[u];
             const bool valid = i < end && expert_in_range(e, E);
             if (i < end && !valid) report_bad_expert(w, i, e, E, 1);
