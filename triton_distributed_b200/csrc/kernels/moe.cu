@@ -255,7 +255,7 @@ __global__ void moe_topk_softmax_kernel(const float* logits, int ntok, int E, in
 // That order of the sums is the same in all forms below, which the number of tokens chooses between: a token's logits, and with
 // them the choice between near ties, do not depend on how many others are in the call. The forms, us per call at 16 tokens x 4096,
 // 8 experts / 128 x 7168, 32 / 300 x 7168, 64 / 1200 x 6720, 64:
-//   a CTA per tile, a chain per warp                                        4.4 / 10.2 / 15.5 / 15.3
+//   a CTA per tile, a chain per warp                                        4.0 / 10.2 / 15.5 / 15.3
 //   a cluster of up to eight CTAs per tile, which share the experts           - /  7.6 /  9.0 / 21.6
 //   a cluster of eight CTAs per tile, two chains each                       2.9 /  5.4 / 14.3 / 36
 // (Up to eight parts of the hidden dimension, each a sum of its own, took 2.9 / 5.7 / 9.5 / 15.3: there the order of the sums followed the
@@ -282,7 +282,9 @@ __global__ void __launch_bounds__(kGateThreads, 1) moe_gate_topk_kernel(const __
     const int parts = SPLIT ? split : 1;
     extern __shared__ float gate_sm[];
     constexpr int COLS = NT * 8;
-    constexpr int AHEAD = NT == 1 ? 8 : (NT == 2 ? 4 : (NT == 4 ? 2 : 1));   // steps whose loads are in flight
+    // steps whose loads are in flight: a split tile's CTA has an SM to itself and few steps (more of them cost 4096 tokens x 7168, 8
+    // experts 12.6 us on one CTA per tile, 11.5 so)
+    constexpr int AHEAD = SPLIT ? (NT == 8 ? 1 : (NT == 4 ? 2 : 8 / NT)) : 1, UNROLL = SPLIT || NT == 8 ? 1 : 2;
     float* part = gate_sm;                                   // [warps][16 tokens][COLS]
     float* row_s = gate_sm + kGateWarps * kGateTok * COLS;   // [16 / parts tokens][E]: the tokens this CTA selects for
     const int tid = static_cast<int>(threadIdx.x), warp = tid >> 5, lane = tid & 31;
@@ -304,7 +306,7 @@ __global__ void __launch_bounds__(kGateThreads, 1) moe_gate_topk_kernel(const __
             ge[n] = gate_row(gate, e0 + n * 8 + g, E, hidden, tig);
             acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
         }
-#pragma unroll 1
+#pragma unroll(UNROLL)
         for (int s0 = warp; s0 < steps; s0 += AHEAD * kGateWarps) {
             uint4 a[AHEAD], c[AHEAD], b[AHEAD][NT];
 #pragma unroll
