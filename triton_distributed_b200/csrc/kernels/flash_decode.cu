@@ -214,9 +214,13 @@ __global__ void __launch_bounds__(kDecodeThreads, decode_ctas_per_sm(D)) flash_d
     uint8_t* my_ring = ring + static_cast<size_t>(warp) * NS * 2 * TILE;
     // Page-table lookup of block i of this warp, issued one block ahead of the copies that need it, so that its latency
     // hides behind a block's worth of math instead of stalling the (in-order) warp right before every batch of cp.async.
-    // Pages of a multiple of 16 tokens: a block lies in one page, every lane gets the block's offset. Others: lane r < 16
-    // gets token r's offset, or -1 past the end.
-    const bool whole = (p.page_size & (kTok - 1)) == 0;
+    // Lane r < 16 gets token r's offset, or -1 past the end, and hands it to the lanes that copy the token. With head_dim 64 and
+    // pages of a multiple of 16 tokens a block lies in one page and every lane gets the block's offset (16 heads, 10^6 keys 698 us, by
+    // token 711). Larger heads copy more rows for a block, and an address per row and lane, or only the choice, costs more than the
+    // exchange (head_dim 256, 32 heads on 8: 8 x 32768 keys 348 us, by token 333; 16 x 8192 in pages of one 265 and 198; head_dim
+    // 128: 169.4 and 168.2, 101 and 95).
+    constexpr bool BY_BLOCK = D == 64;
+    const bool whole = BY_BLOCK && (p.page_size & (kTok - 1)) == 0;
     auto lookup = [&](int i) -> long long {
         long long base = -1;
         if (i < my_blocks && (whole || lane < kTok)) {
@@ -241,10 +245,11 @@ __global__ void __launch_bounds__(kDecodeThreads, decode_ctas_per_sm(D)) flash_d
 #pragma unroll
         for (int j = 0; j < kTok / ROWS; ++j) {
             const int row = j * ROWS + lrow;
-            long long off = base + row_off + static_cast<long long>(j * ROWS) * p.stride_token;
+            long long off = base;
+            if (BY_BLOCK) off = base + row_off + static_cast<long long>(j * ROWS) * p.stride_token;
             if (!whole) off = __shfl_sync(0xffffffffu, base, row);
             // rows past the end are zero-filled
-            const int nbytes = row < left ? 16 : 0;
+            const int nbytes = (BY_BLOCK ? row < left : off >= 0) ? 16 : 0;
             if (nbytes == 0) off = 0;
             cp_async16(ks + tile_off<D>(row, lch), kl + off, nbytes);
             cp_async16(ks + TILE + tile_off<D>(row, lch), vl + off, nbytes);
