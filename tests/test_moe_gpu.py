@@ -310,7 +310,8 @@ def test_gate_topk_parts_of_the_hidden_dimension(cuda_device, T, hidden, E, k):
 
 
 @pytest.mark.parametrize("hidden,E,k", [(64, 3, 1), (544, 8, 2), (992, 40, 4), (1024, 16, 4), (2080, 60, 6), (4096, 8, 2), (7168, 64, 8),
-                                        (8192, 64, 8), (7168, 130, 8), (12288, 64, 8), (2048, 520, 6), (512, 1024, 32)])
+                                        (8192, 64, 8), (7168, 130, 8), (12288, 64, 8), (2048, 520, 6), (512, 1024, 32), (2048, 24, 3),
+                                        (4096, 16, 2), (8192, 32, 8), (12288, 32, 4)])
 def test_gate_topk_of_a_token_is_the_same_in_any_batch(cuda_device, hidden, E, k):
     """Every form of the launch, at both sides of the token counts and sizes from which on there is another: bit by bit the
     logits, experts and weights of the largest batch."""

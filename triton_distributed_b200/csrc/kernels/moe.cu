@@ -257,7 +257,7 @@ __global__ void moe_topk_softmax_kernel(const float* logits, int ntok, int E, in
 // 8 experts / 128 x 7168, 32 / 300 x 7168, 64 / 1200 x 6720, 64:
 //   a CTA per tile, a chain per warp                                        4.0 / 10.2 / 15.5 / 15.3
 //   a cluster of up to eight CTAs per tile, which share the experts           - /  7.6 /  9.0 / 21.6
-//   a cluster of eight CTAs per tile, two chains each                       2.9 /  5.4 / 14.3 / 36
+//   a cluster of eight (or four) CTAs per tile, which share the chains      2.9 /  5.4 / 14.3 / 36
 // (Up to eight parts of the hidden dimension, each a sum of its own, took 2.9 / 5.7 / 9.5 / 15.3: there the order of the sums followed the
 // number of parts, and that the number of tokens. Eight such sums whatever the number of CTAs: 29 us for the last of these.)
 constexpr int kGateTok = 16, kGateThreads = 512, kGateWarps = kGateThreads / 32;
@@ -365,31 +365,31 @@ __global__ void __launch_bounds__(kGateThreads, 1) moe_gate_topk_kernel(const __
     if (warp < own && t < ntok) topk_softmax_any(row_s + warp * E, E, topk, renorm, lane, ids + static_cast<size_t>(t) * topk, w + static_cast<size_t>(t) * topk);
 }
 
-// A cluster of eight CTAs per tile, two chains each, for at most 8 NT experts. The products of a chain's steps, which eight warps take
-// in turn, meet in shared memory and are added there in order; the chain's sum goes to the CTA that selects for the token, which
-// adds the 16 chains. Every row is read once per tile.
-constexpr int kGateChains = kGateWarps, kGateOwnChains = kGateChains / kGateMaxParts, kGateStepWarps = kGateWarps / kGateOwnChains;
-constexpr int kGateOwnTok = kGateTok / kGateMaxParts;
+// A cluster of PARTS CTAs per tile, 16 / PARTS chains each, for at most 8 NT experts. The products of a chain's steps, which PARTS
+// warps take in turn, meet in shared memory and are added there in order; the chain's sum goes to the CTA that selects for the
+// token, which adds the 16 chains. Every row is read once per tile.
+constexpr int kGateChains = kGateWarps;
 // floats between the rows of a step's products: those that a warp stores at once spread over the banks
 __host__ __device__ constexpr int gate_pitch(int nt) { return nt * 8 + 8; }
-static int gate_chains_smem(int hidden, int nt, int E) {
+static int gate_chains_smem(int hidden, int nt, int E, int parts) {
     const int most = (hidden / 32 + kGateChains - 1) / kGateChains;   // steps of a chain
-    return (kGateOwnChains * most * kGateTok * gate_pitch(nt) + kGateChains * kGateOwnTok * E) * static_cast<int>(sizeof(float));
+    return (kGateChains / parts * most * kGateTok * gate_pitch(nt) + kGateChains * (kGateTok / parts) * E) * static_cast<int>(sizeof(float));
 }
 
-template <int NT>
+template <int NT, int PARTS>
 __global__ void __launch_bounds__(kGateThreads, 1) moe_gate_topk_chains_kernel(const __nv_bfloat16* x, const __nv_bfloat16* gate, int ntok, int hidden, int E,
                                                                                int topk, int renorm, int* ids, float* w, float* logits) {
     extern __shared__ float gate_sm[];
     constexpr int COLS = NT * 8, PITCH = gate_pitch(NT), STEP = kGateTok * PITCH;
     constexpr int AHEAD = NT == 8 ? 1 : 2;
+    constexpr int OWN_CHAINS = kGateChains / PARTS, OWN_TOK = kGateTok / PARTS;
     const int tid = static_cast<int>(threadIdx.x), warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, tig = lane & 3;
     const int part_id = static_cast<int>(cluster_ctarank());
-    const int t0 = static_cast<int>(blockIdx.x) / kGateMaxParts * kGateTok;
+    const int t0 = static_cast<int>(blockIdx.x) / PARTS * kGateTok;
     const int steps = hidden / 32, most = (steps + kGateChains - 1) / kGateChains;
     float* prod = gate_sm;                                     // [own chains][most][16 tokens][PITCH]
-    float* chain_s = gate_sm + kGateOwnChains * most * STEP;   // [16 chains][own tokens][E]
+    float* chain_s = gate_sm + OWN_CHAINS * most * STEP;   // [16 chains][own tokens][E]
     cluster_arrive();    // its counterpart stands before the first store into another CTA
     pdl_wait_and_release();
     const __nv_bfloat16* xa = gate_row(x, t0 + g, ntok, hidden, tig);
@@ -397,14 +397,14 @@ __global__ void __launch_bounds__(kGateThreads, 1) moe_gate_topk_chains_kernel(c
     const __nv_bfloat16* ge[NT];
 #pragma unroll
     for (int n = 0; n < NT; ++n) ge[n] = gate_row(gate, n * 8 + g, E, hidden, tig);
-    const int mine = warp % kGateOwnChains;                    // this warp's chain, among the CTA's and among all
-    const int chain = part_id * kGateOwnChains + mine;
+    const int mine = warp % OWN_CHAINS;                    // this warp's chain, among the CTA's and among all
+    const int chain = part_id * OWN_CHAINS + mine;
 #pragma unroll 1
-    for (int j0 = warp / kGateOwnChains; chain + j0 * kGateChains < steps; j0 += AHEAD * kGateStepWarps) {
+    for (int j0 = warp / OWN_CHAINS; chain + j0 * kGateChains < steps; j0 += AHEAD * PARTS) {
         uint4 a[AHEAD], c[AHEAD], b[AHEAD][NT];
 #pragma unroll
         for (int u = 0; u < AHEAD; ++u) {
-            const int s = chain + (j0 + u * kGateStepWarps) * kGateChains;
+            const int s = chain + (j0 + u * PARTS) * kGateChains;
             if (s >= steps) break;
             a[u] = ld_v4(xa + s * 32);
             c[u] = ld_v4(xb + s * 32);
@@ -413,7 +413,7 @@ __global__ void __launch_bounds__(kGateThreads, 1) moe_gate_topk_chains_kernel(c
         }
 #pragma unroll
         for (int u = 0; u < AHEAD; ++u) {
-            const int j = j0 + u * kGateStepWarps;
+            const int j = j0 + u * PARTS;
             if (chain + j * kGateChains >= steps) break;
             float* p = prod + (mine * most + j) * STEP + g * PITCH + tig * 2;
 #pragma unroll
@@ -428,28 +428,28 @@ __global__ void __launch_bounds__(kGateThreads, 1) moe_gate_topk_chains_kernel(c
     }
     __syncthreads();
     cluster_wait();   // every CTA of the cluster runs
-    for (int i = tid; i < kGateOwnChains * kGateTok * COLS; i += kGateThreads) {
-        const int k = i / (kGateTok * COLS), t = i / COLS % kGateTok, e = i % COLS, at = part_id * kGateOwnChains + k;
+    for (int i = tid; i < OWN_CHAINS * kGateTok * COLS; i += kGateThreads) {
+        const int k = i / (kGateTok * COLS), t = i / COLS % kGateTok, e = i % COLS, at = part_id * OWN_CHAINS + k;
         if (e >= E) continue;
         float sum = 0.f;
         const float* p = prod + k * most * STEP + t * PITCH + e;
 #pragma unroll 4
         for (int s = at; s < steps; s += kGateChains, p += STEP) sum += *p;
-        st_shared_cluster_f32(mapa_u32(smem_u32(chain_s + (at * kGateOwnTok + t % kGateOwnTok) * E + e), static_cast<uint32_t>(t / kGateOwnTok)), sum);
+        st_shared_cluster_f32(mapa_u32(smem_u32(chain_s + (at * OWN_TOK + t % OWN_TOK) * E + e), static_cast<uint32_t>(t / OWN_TOK)), sum);
     }
     cluster_arrive();
     cluster_wait();
-    for (int i = tid; i < kGateOwnTok * E; i += kGateThreads) {
+    for (int i = tid; i < OWN_TOK * E; i += kGateThreads) {
         float sum = 0.f;
 #pragma unroll
-        for (int k = 0; k < kGateChains; ++k) sum += chain_s[k * kGateOwnTok * E + i];
+        for (int k = 0; k < kGateChains; ++k) sum += chain_s[k * OWN_TOK * E + i];
         chain_s[i] = sum;   // chain 0's own slot: this thread's alone
-        const int t = t0 + part_id * kGateOwnTok + i / E;
+        const int t = t0 + part_id * OWN_TOK + i / E;
         if (logits != nullptr && t < ntok) logits[static_cast<size_t>(t) * E + i % E] = sum;
     }
     __syncthreads();
-    const int t = t0 + part_id * kGateOwnTok + warp;
-    if (warp < kGateOwnTok && t < ntok) topk_softmax_any(chain_s + warp * E, E, topk, renorm, lane, ids + static_cast<size_t>(t) * topk, w + static_cast<size_t>(t) * topk);
+    const int t = t0 + part_id * OWN_TOK + warp;
+    if (warp < OWN_TOK && t < ntok) topk_softmax_any(chain_s + warp * E, E, topk, renorm, lane, ids + static_cast<size_t>(t) * topk, w + static_cast<size_t>(t) * topk);
 }
 
 // ---------------------------------------------------------------------------- row gather / top-k reduce
@@ -599,19 +599,25 @@ extern "C" int tdist_moe_gate_topk(const void* x, const void* gate, int ntok, in
     if (ntok <= 0) return 0;
     // A cluster's SMs lie in one GPC: clusters of 2, 4 and 8 CTAs fill 100, 90 and 82 % of the machine (64 experts x 7168, experts shared
     // by 2 / 4 / 8 CTAs: 240 tokens 11.2 / 8.9 / 8.4 us, 300 tokens 11.3 / 9.0 / 15.6, 592 tokens 11.4 / 17.0 / 23.6). Chains are shared
-    // out where eight CTAs per tile run at once, the experts take one pass (64 tokens x 7168, 256 experts: 52 us, 11.4 by experts),
-    // a chain has two steps or more (4 tokens x 512, 8 experts: 2.5 us, 2.3 on one CTA; x 1024 2.7 and 2.7) and the products
-    // of the steps fit; the experts elsewhere, while each CTA gets some.
+    // out by eight CTAs of a tile where all run at once, the experts take one pass (64 tokens x 7168, 256 experts: 52 us, 11.4 by
+    // experts), a chain has four steps or more (4 tokens x 1024, 64 experts: 4.7 us, 4.1 by experts; 100 x 2048, 32 experts 3.1 and
+    // 3.8) and the products of the steps fit; by four CTAs up to 32 experts, where the experts have few CTAs to go to (cold, 300 tokens x
+    // 4096: 8 experts 4.3 us, 6.3 on one CTA; 32 experts 5.5, 5.7 by experts; 64 experts 8.4 and 7.1). The experts are shared out
+    // elsewhere, while each CTA gets some.
     const int tiles = (ntok + kGateTok - 1) / kGateTok, groups = (num_experts + 7) / 8;
     const int fit[4] = {100, 100, 90, 82};
     const auto runs_at_once = [&](int i) { return (100LL * tiles << i) <= static_cast<long long>(fit[i]) * tdist_host::sm_count(); };
     const auto width = [](int n) { return n <= 1 ? 1 : (n <= 2 ? 2 : (n <= 4 ? 4 : 8)); };
     static_assert(1 << 3 == kGateMaxParts, "the largest cluster");
-    const bool chains = runs_at_once(3) && groups <= 8 && hidden >= 2 * kGateChains * 32 && gate_chains_smem(hidden, width(groups), num_experts) <= 200 * 1024;
-    int parts = chains ? kGateMaxParts : 1;
+    const auto chains_on = [&](int i) {
+        return runs_at_once(i) && groups <= (i == 3 ? 8 : 4) && hidden >= 4 * kGateChains * 32 &&
+               gate_chains_smem(hidden, width(groups), num_experts, 1 << i) <= 200 * 1024;
+    };
+    const bool chains = chains_on(3) || chains_on(2);
+    int parts = chains ? (chains_on(3) ? 8 : 4) : 1;
     for (int i = 1; i <= 3 && parts < groups && !chains && runs_at_once(i); ++i) parts *= 2;
     const int nt = width(chains ? groups : (groups + parts - 1) / parts);
-    const int smem = chains ? gate_chains_smem(hidden, nt, num_experts)
+    const int smem = chains ? gate_chains_smem(hidden, nt, num_experts, parts)
                             : (kGateWarps * kGateTok * nt * 8 + kGateTok / parts * num_experts) * static_cast<int>(sizeof(float));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(tiles * parts));
@@ -633,9 +639,9 @@ extern "C" int tdist_moe_gate_topk(const void* x, const void* gate, int ntok, in
 #define TDIST_GATE_CASE(NT)                                                                                                              \
     {                                                                                                                                    \
         if (chains) {                                                                                                                    \
-            if (int rc = ensure_smem(moe_gate_topk_chains_kernel<NT>, smem)) return rc;                                                  \
-            TDIST_CUDA_OK(cudaLaunchKernelEx(&cfg, moe_gate_topk_chains_kernel<NT>, xp, gp, ntok, hidden, num_experts, topk, renormalize, \
-                                             idp, wp, lp));                                                                              \
+            const auto kernel = parts == 8 ? moe_gate_topk_chains_kernel<NT, 8> : moe_gate_topk_chains_kernel<NT, 4>;                    \
+            if (int rc = ensure_smem(kernel, smem)) return rc;                                                                           \
+            TDIST_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, xp, gp, ntok, hidden, num_experts, topk, renormalize, idp, wp, lp));          \
         } else {                                                                                                                         \
             const auto kernel = parts > 1 ? moe_gate_topk_kernel<NT, true> : moe_gate_topk_kernel<NT, false>;                            \
             if (int rc = ensure_smem(kernel, smem)) return rc;                                                                           \
