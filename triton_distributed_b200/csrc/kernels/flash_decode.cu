@@ -143,7 +143,7 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
 
 // Sequence of the CTAs in place `slot`, and its length, when the longest come first (ties by number) and one of them has `least`
 // keys. The grid starts in order of its blocks,
-// so the last ones to start are the shortest (batch 32, 64 query heads, lengths ragged to 8192: 114 us in order of
+// so the last ones to start are the shortest (batch 32, 64 query heads, lengths ragged to 8192: 111 us in order of
 // their numbers, 94 us; 51 ragged ones that all start at once: no difference). A thread per sequence: batches of more than
 // kMaxOrdered keep the order of the numbers.
 constexpr int kMaxOrdered = kDecodeThreads;
@@ -668,9 +668,9 @@ static bool overlaps_previous(const DecodeParams& p) {
 // yet to start. What it gains is the wait for a long sequence that started last; what it costs is a step in front of every CTA, and
 // the short sequences, bound by latencies, no longer run beside long ones that are bound by HBM. So the longest CTA has to
 // be worth more the more rounds of CTAs there are. Ragged batches, 8 kv heads, us per call by number / by length: head_dim 128, 64
-// sequences to 1024 keys (1.7 rounds) 43.6 / 40.0, 64 to 4096 121.5 / 95.2, 100 to 1024 (2.7) 58.6 / 62.3, 100 to 4096 162 / 149,
-// 128 to 64 (3.5) 35.2 / 39.4, 128 to 4096 (6.9, two splits) 196 / 218, 64 to 8192 (3.5, two splits) 202 / 185; head_dim 64, 128 to 64
-// (2.3) 20.6 / 25.0, 100 to 8192 (1.8) 186 / 156; head_dim 256, 24 to 1024 (1.3) 37.5 / 29.2, 40 to 300 (2.2) 26.8 / 28.1.
+// sequences to 1024 keys (1.7 rounds) 42.1 / 39.2, 64 to 4096 116.3 / 94.4, 100 to 1024 (2.7) 56.4 / 61.9, 100 to 4096 158 / 148,
+// 128 to 64 (3.5) 35.1 / 39.5, 128 to 4096 (6.9, two splits) 191 / 218, 64 to 8192 (3.5, two splits) 195 / 184; head_dim 64, 128 to 64
+// (2.3) 20.7 / 25.1, 100 to 8192 (1.8) 186 / 154; head_dim 256, 24 to 1024 (1.3) 34.7 / 27.2, 40 to 300 (2.2) 25.9 / 27.8.
 constexpr double kOrderValues = 32768;   // keys of a CTA x head_dim
 static int order_from(const DecodeParams& p, int head_dim, int per_sm) {
     const double rounds = static_cast<double>(p.B) * p.Hkv * p.splits / (per_sm * tdist_host::sm_count());
